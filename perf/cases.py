@@ -240,6 +240,128 @@ def run(state):
     return [loss.detach(), dq, dk]
 
 
+# ----------------------------------------------------------------------------------------- exact
+def _rms64(x, w, eps):
+    return x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + eps) * w
+
+
+def _attend64(q, k, v, scale, causal):
+    """q [Hq, S, d], k and v [Hk, S, d] -> [S, Hq * d]; one KV head's group at a time."""
+    groups, S = q.shape[0] // k.shape[0], q.shape[1]
+    out = torch.empty_like(q)
+    mask = torch.ones(S, S, dtype=torch.bool, device=q.device).triu(1) if causal else None
+    for h in range(k.shape[0]):
+        rows = slice(h * groups, (h + 1) * groups)
+        s = torch.matmul(q[rows], k[h].T) * scale
+        if causal:
+            s.masked_fill_(mask, -math.inf)
+        out[rows] = torch.matmul(torch.softmax(s, -1), v[h])
+    return out.transpose(0, 1).reshape(S, -1)
+
+
+def _decoder64(w, cfg, causal, ids):
+    S, d, half = ids.numel(), cfg.head_dim, cfg.head_dim // 2
+    inv = cfg.rope_theta ** (-torch.arange(half, dtype=torch.float64, device="cuda") / half)
+    angle = torch.outer(torch.arange(S, dtype=torch.float64, device="cuda"), inv)
+    cos, sin = angle.cos(), angle.sin()
+
+    def heads(x, n, norm):
+        x = x.view(S, n, d)
+        if norm is not None:
+            x = _rms64(x, norm.double(), cfg.rms_norm_eps)
+        return x.transpose(0, 1)
+
+    def rotate(x):
+        a, b = x[..., :half], x[..., half:]
+        return torch.cat((a * cos - b * sin, b * cos + a * sin), -1)
+
+    x = w["embed_tokens.weight"][ids].double()
+    for i in range(cfg.num_hidden_layers):
+        at = f"layers.{i}."
+
+        def lin(y, name):
+            return y @ w[at + name + ".weight"].double().T
+
+        y = _rms64(x, w[at + "input_layernorm.weight"].double(), cfg.rms_norm_eps)
+        q = heads(lin(y, "self_attn.q_proj"), cfg.num_attention_heads,
+                  w.get(at + "self_attn.q_norm.weight"))
+        k = heads(lin(y, "self_attn.k_proj"), cfg.num_key_value_heads,
+                  w.get(at + "self_attn.k_norm.weight"))
+        v = heads(lin(y, "self_attn.v_proj"), cfg.num_key_value_heads, None)
+        o = _attend64(rotate(q), rotate(k), v, d ** -0.5, causal)
+        x = x + lin(o, "self_attn.o_proj")
+        y = _rms64(x, w[at + "post_attention_layernorm.weight"].double(), cfg.rms_norm_eps)
+        y = torch.nn.functional.silu(lin(y, "mlp.gate_proj")) * lin(y, "mlp.up_proj")
+        x = x + lin(y, "mlp.down_proj")
+    return _rms64(x, w["norm.weight"].double(), cfg.rms_norm_eps)
+
+
+def _bert64(w, cfg, ids):
+    S, n, d = ids.numel(), cfg.num_attention_heads, cfg.hidden_size // cfg.num_attention_heads
+
+    def lin(y, name):
+        return y @ w[name + ".weight"].double().T + w[name + ".bias"].double()
+
+    def norm(y, name):
+        return torch.nn.functional.layer_norm(y, y.shape[-1:], w[name + ".weight"].double(),
+                                              w[name + ".bias"].double(), cfg.layer_norm_eps)
+
+    x = norm((w["embeddings.word_embeddings.weight"][ids].double()
+              + w["embeddings.position_embeddings.weight"][:S].double()
+              + w["embeddings.token_type_embeddings.weight"][0].double()), "embeddings.LayerNorm")
+    for i in range(cfg.num_hidden_layers):
+        at = f"layers.{i}."
+        q, k, v = (lin(x, at + "attention." + p).view(S, n, d).transpose(0, 1)
+                   for p in ("query", "key", "value"))
+        o = _attend64(q, k, v, d ** -0.5, False)
+        x = norm(x + lin(o, at + "attention.dense"), at + "attention.LayerNorm")
+        y = torch.nn.functional.gelu(lin(x, at + "mlp.dense_in"))
+        x = norm(x + lin(y, at + "mlp.dense_out"), at + "mlp.LayerNorm")
+    return x
+
+
+def _encode64(case, seed):
+    if case["model"] == "embeddinggemma":   # four norms a block and two rotary bases: left out
+        return None
+    state = prepare(case, seed)
+    family, cfg = _config(case)
+    w = state["model"].state_dict()
+    out = []
+    for text in state["texts"]:
+        total, acc = 0, 0.0
+        for at in range(0, len(text), 4096 - 128):
+            ids = torch.tensor(text[at:at + 4096], device="cuda")
+            h = _bert64(w, cfg, ids) if family == "bert" else _decoder64(w, cfg, family == "qwen3",
+                                                                         ids)
+            emb = h[-1] if case["pooling"] == "last_token" else h.mean(0)
+            acc, total = acc + emb * ids.numel(), total + ids.numel()
+            if at + 4096 >= len(text):
+                break
+        out.append(torch.nn.functional.normalize(acc / total, dim=-1))
+    return torch.stack(out).cpu().numpy()
+
+
+@torch.no_grad()
+def exact(case, seed):
+    """The outputs of ``run`` in 64 bits. None for training steps: their loss is a single number and
+    the updated weights are the old ones to six digits, so neither says how exact the step was."""
+    if case["kind"] == "encode":
+        return _encode64(case, seed)
+    if case["kind"] == "train":
+        return None
+    state = _prepare_loss(case, seed)
+    q, k = state["q"].double(), state["k"].double()
+    rows = torch.arange(case["q"], device="cuda")
+    target = state["pos_di"] if case["labels"] else rows
+    p = (q @ k.T).div_(TEMPERATURE)      # one positive a row: cross entropy against its column
+    lse = p.logsumexp(1)
+    loss = (lse - p[rows, target]).mean()
+    p.sub_(lse[:, None]).exp_()
+    p[rows, target] -= 1.0
+    p /= TEMPERATURE * case["q"]
+    return [loss, p @ k, p.T @ q]
+
+
 # ------------------------------------------------------------------------------------------ work
 def _linear_params(case):
     family, h, ffn, layers, hq, hk, hd, _ = SIZES[case["model"]]
