@@ -28,4 +28,16 @@ struct AttnPlanView {
   __device__ __forceinline__ int tile(int i) const { return data[2 + 2 * i]; }
 };
 
+// Called by every CTA of a forward kernel when it takes no more work: the last one puts the plan's
+// work counter back to zero for the next layer's launch.
+__device__ __forceinline__ void finish_grid(const int* plan, int capacity) {
+  if (threadIdx.x != 0) return;
+  unsigned* words = reinterpret_cast<unsigned*>(const_cast<int*>(plan)) + 1 + 2 * capacity;
+  __threadfence();
+  if (atomicAdd(&words[2], 1u) + 1u == gridDim.x) {
+    words[0] = 0u;
+    words[2] = 0u;
+  }
+}
+
 }  // namespace lb

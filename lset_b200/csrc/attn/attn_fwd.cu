@@ -1,4 +1,6 @@
 // Varlen (packed) flash attention forward on tcgen05: causal or bidirectional, grouped-query heads.
+// Head dims 64 and 128 run on the two-tile kernel of attn_fwd_pair.cuh; at 256 its accumulators and
+// tiles fit neither tensor nor shared memory, and attn_fwd_kernel below is used:
 //
 // Persistent 128-thread CTAs (two per SM) walk over the (KV head, sequence, query tile) work items;
 // TMEM and the barriers are set up once per CTA and the next item's Q and first K/V block are
@@ -16,6 +18,7 @@
 #include "../common/ptx.cuh"
 #include "../common/tma_desc.h"
 #include "attn_common.cuh"
+#include "attn_fwd_pair.cuh"
 
 namespace lb {
 namespace {
@@ -26,7 +29,7 @@ struct AttnFwdArgs {
   const int* seq_start;  // first token of each sequence
   const int* seq_end;    // one past its last token
   const int* plan;
-  unsigned* work_counter;  // zeroed by the launcher: hands out work items past the first wave
+  unsigned* work_counter;  // hands out work items past the first wave (see finish_grid)
   bf16* O;
   long long ldo;   // elements between consecutive tokens of O
   float* lse;      // [Hq, T]
@@ -34,6 +37,7 @@ struct AttnFwdArgs {
   float scale_log2;  // softmax scale * log2(e)
   int causal;
   int* status;
+  int capacity;
 };
 
 template <int HD>
@@ -62,7 +66,10 @@ __global__ void __launch_bounds__(128)
   AttnPlanView plan{a.plan};
   const int tiles = plan.count();
   const int total = tiles * a.Hk;
-  if (int(blockIdx.x) >= total) return;
+  if (int(blockIdx.x) >= total) {
+    finish_grid(a.plan, a.capacity);
+    return;
+  }
   const int G = a.Hq / a.Hk;
   const int QT = 128 / G;
   auto decode = [&](int w) {
@@ -346,6 +353,7 @@ __global__ void __launch_bounds__(128)
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem_base, C::TMEM_COLS);
+  finish_grid(a.plan, a.capacity);
 }
 
 // One block: prefix over sequences -> (sequence, tile) list. plan[0] = tile count.
@@ -382,10 +390,12 @@ __global__ void attn_plan_kernel(const int* __restrict__ seq_start,
   }
   if (threadIdx.x == 0) {
     plan[0] = s_base < capacity ? s_base : capacity;
-    // second spare word (the first is the forward kernel's work counter): one past the last token
-    // that belongs to a sequence. Tokens behind it (a stream padded to a fixed budget) are
-    // written by no attention kernel; the launchers clear those rows.
+    // spare words: the forward kernel's work counter; one past the last token that belongs to a
+    // sequence (tokens behind it, of a stream padded to a fixed budget, are no work item's: the
+    // forward kernel and the backward's launcher clear those rows); CTAs that have finished.
+    plan[1 + 2 * capacity] = 0;
     plan[1 + 2 * capacity + 1] = seq_end[B - 1];
+    plan[1 + 2 * capacity + 2] = 0;
   }
 }
 
@@ -410,6 +420,19 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+int attn_sms() {
+  static int n = 0;
+  if (n == 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
+      n = 148;
+  }
+  return n;
+}
+
+// Persistent grids: as many CTAs as are resident at once (one per SM), never more than the upper
+// bound of the work items; a CTA beyond the real count finds nothing to do.
 template <int HD>
 int launch_fwd(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV,
                const AttnFwdArgs& a, int max_tiles, cudaStream_t st) {
@@ -422,19 +445,28 @@ int launch_fwd(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap
       return -10;
     configured = true;
   }
-  // persistent: as many CTAs as fit at once (shared memory allows two per SM at head_dim <= 128),
-  // never more than the upper bound of the work items; a CTA beyond the real count exits at once
-  int sms = 148;
-  {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  }
   const long long upper = 1LL * max_tiles * a.Hk;
-  const long long resident = 1LL * sms * (C::SMEM_BYTES <= 113 * 1024 ? 2 : 1);
-  const int grid = static_cast<int>(upper < resident ? upper : resident);
+  const int grid = static_cast<int>(upper < attn_sms() ? upper : attn_sms());
   kern<<<grid, 128, C::SMEM_BYTES, st>>>(tmQ, tmK, tmV, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
+}
+
+template <int HD>
+int launch_pair(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV,
+                const AttnPairArgs& a, int max_tiles, cudaStream_t st) {
+  using C = PairCfg<HD>;
+  auto kern = attn_fwd_pair_kernel<HD>;
+  static bool configured = false;
+  if (!configured) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES) !=
+        cudaSuccess)
+      return -10;
+    configured = true;
+  }
+  const long long upper = 1LL * max_tiles * a.Hk;
+  const int grid = static_cast<int>(upper < attn_sms() ? upper : attn_sms());
+  return launch_pdl(kern, dim3(grid), dim3(kPairThreads), C::SMEM_BYTES, st, pdl_enabled(), 1, tmQ,
+                    tmK, tmV, a);
 }
 
 }  // namespace
@@ -442,8 +474,8 @@ int launch_fwd(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap
 
 using namespace lb;
 
-// plan: int32 [1 + 2 * capacity + 1] (the last word is scratch for the attention kernels);
-// capacity >= ceil(T / tile_tokens) + B always suffices.
+// plan: int32 [1 + 2 * capacity + 3] (the last words are the attention kernels' own, see
+// attn_plan_kernel); capacity >= ceil(T / tile_tokens) + B always suffices.
 // Clears the rows behind the last sequence of a stream (see attn_plan_kernel). plan / capacity as
 // passed to lb_attn_plan; widths in elements, multiples of 8; unused matrices null.
 extern "C" int lb_attn_zero_tail(const int* plan, int capacity, int T, void* p0, long long ld0,
@@ -467,7 +499,12 @@ extern "C" int lb_attn_plan(const int* seq_start, const int* seq_end, int B, int
 // Sequence b owns tokens [seq_start[b], seq_end[b]) of the stream (for a packed batch these are
 // cu_seqlens and cu_seqlens + 1; for a padded batch they skip the padding).
 // q: [T, Hq, hd] with token stride ldq (elements); k, v: [T, Hk, hd] with strides ldk, ldv.
-// plan was built with tile_tokens = 128 / (Hq / Hk). o: [T, Hq, hd] stride ldo; lse: [Hq, T] fp32.
+// plan was built with tile_tokens = lb_attn_fwd_tile_tokens(hd, Hq / Hk). o: [T, Hq, hd] stride ldo;
+// lse: [Hq, T] fp32.
+extern "C" int lb_attn_fwd_tile_tokens(int hd, int group) {
+  return (hd == 256 ? 128 : 256) / group;
+}
+
 extern "C" int lb_attn_fwd(const void* q, long long ldq, const void* k, long long ldk, const void* v,
                            long long ldv, const int* seq_start, const int* seq_end, const int* plan,
                            int max_tiles,
@@ -478,28 +515,30 @@ extern "C" int lb_attn_fwd(const void* q, long long ldq, const void* k, long lon
   const int G = Hq / Hk;
   if (G != 1 && G != 2 && G != 4 && G != 8) return -3;
   if ((ldq | ldk | ldv | ldo) & 7) return -3;
+  if (hd != 128 && hd != 64 && hd != 256) return -3;
   const int QT = 128 / G;
+  const int kv_box = hd == 256 ? kAttnKvBlock : kPairBlock;
   CUtensorMap tmQ, tmK, tmV;
   int rc = make_tmap_2d(&tmQ, q, 2, (uint64_t)Hq * hd, (uint64_t)T, (uint64_t)ldq * 2, 64, QT, true);
   if (rc) return rc;
-  rc = make_tmap_2d(&tmK, k, 2, (uint64_t)Hk * hd, (uint64_t)T, (uint64_t)ldk * 2, 64, kAttnKvBlock,
-                    true);
+  rc = make_tmap_2d(&tmK, k, 2, (uint64_t)Hk * hd, (uint64_t)T, (uint64_t)ldk * 2, 64, kv_box, true);
   if (rc) return rc;
-  rc = make_tmap_2d(&tmV, v, 2, (uint64_t)Hk * hd, (uint64_t)T, (uint64_t)ldv * 2, 64, kAttnKvBlock,
-                    true);
+  rc = make_tmap_2d(&tmV, v, 2, (uint64_t)Hk * hd, (uint64_t)T, (uint64_t)ldv * 2, 64, kv_box, true);
   if (rc) return rc;
-  // the plan buffer carries two spare words behind its 1 + 2 * max_tiles entries: this kernel's
-  // work counter and the end of the stream's last sequence
   unsigned* counter = reinterpret_cast<unsigned*>(const_cast<int*>(plan)) + 1 + 2 * max_tiles;
-  AttnFwdArgs a{seq_start, seq_end, plan, counter, (bf16*)o, ldo, lse, T, Hq, Hk,
-                softmax_scale * kLog2eF, causal, status};
+  const float scale_log2 = softmax_scale * kLog2eF;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (cudaMemsetAsync(counter, 0, sizeof(unsigned), st) != cudaSuccess) return -12;
-  if (hd != 128 && hd != 64 && hd != 256) return -3;
-  rc = lb_attn_zero_tail(plan, max_tiles, T, o, ldo, Hq * hd, nullptr, 0, 0, nullptr, 0, 0, stream);
-  if (rc) return rc;
-  if (hd == 128) return launch_fwd<128>(tmQ, tmK, tmV, a, max_tiles, st);
-  if (hd == 64) return launch_fwd<64>(tmQ, tmK, tmV, a, max_tiles, st);
-  if (hd == 256) return launch_fwd<256>(tmQ, tmK, tmV, a, max_tiles, st);
-  return -3;
+  if (hd == 256) {
+    rc = lb_attn_zero_tail(plan, max_tiles, T, o, ldo, Hq * hd, nullptr, 0, 0, nullptr, 0, 0, stream);
+    if (rc) return rc;
+    AttnFwdArgs a{seq_start, seq_end, plan, counter, (bf16*)o, ldo, lse, T, Hq, Hk,
+                  scale_log2, causal, status, max_tiles};
+    return launch_fwd<256>(tmQ, tmK, tmV, a, max_tiles, st);
+  }
+  // a scale of zero becomes one whose products with finite scores vanish beside the maximum
+  const float mag = scale_log2 < 0.f ? -scale_log2 : scale_log2;
+  AttnPairArgs a{seq_start, seq_end, plan, max_tiles, counter, (bf16*)o, ldo, lse, T, Hq, Hk,
+                 mag > 0.f ? mag : 1e-35f, scale_log2 < 0.f ? 1 : 0, causal, status};
+  return hd == 128 ? launch_pair<128>(tmQ, tmK, tmV, a, max_tiles, st)
+                   : launch_pair<64>(tmQ, tmK, tmV, a, max_tiles, st);
 }

@@ -296,8 +296,8 @@ int block_fwd_tp(const LbBlockDesc* d, const LbStreamCtx* c, const LbBlockIO* io
   if (Tp > T &&  // rows that pad the stream to a multiple of the group size
       cudaMemsetAsync(s.o + (size_t)T * Nq, 0, (size_t)(Tp - T) * Nq * 2, st) != cudaSuccess)
     return -11;
-  LB_TRY(lb_attn_fwd(s.qr, Nq, s.kr, Nk, s.qkv + Nq + Nk, W, c->seq_start, c->seq_end, c->plan_q,
-                     c->cap_q, s.o, Nq, s.lse, T, d->Hq, d->Hk, hd, d->softmax_scale, d->causal,
+  LB_TRY(lb_attn_fwd(s.qr, Nq, s.kr, Nk, s.qkv + Nq + Nk, W, c->seq_start, c->seq_end, c->plan_f,
+                     c->cap_f, s.o, Nq, s.lse, T, d->Hq, d->Hk, hd, d->softmax_scale, d->causal,
                      c->status, c->stream));
   LB_TRY(tp_gemm_rs(r, s.o, Nq, d->o_proj, 0, out, H, Nq, c));
   __nv_bfloat16* x2s = r.next_slot();
@@ -392,9 +392,9 @@ extern "C" size_t lb_block_work_bytes(const LbBlockDesc* d, int T, const LbTpCtx
 extern "C" int lb_block_fwd_launches(const LbBlockDesc* d, const LbStreamCtx* c, int has_residual,
                                      const LbTpCtx* tp) {
   (void)has_residual;
-  if (tp != nullptr)  // two norms, rope, attention (2), glu; 2 gathered GEMMs (own-row copy, barrier,
-    return 6 + 2 * 3 + 2 * 3;  // GEMM) and 2 reduced GEMMs (GEMM, barrier, take-and-clear)
-  int n = 6;  // two norms, rope, attention (tail clear + kernel), glu
+  if (tp != nullptr)  // two norms, rope, attention, glu; 2 gathered GEMMs (own-row copy, barrier,
+    return 5 + 2 * 3 + 2 * 3;  // GEMM) and 2 reduced GEMMs (GEMM, barrier, take-and-clear)
+  int n = d->hd == 256 ? 6 : 5;  // two norms, rope, attention (hd 256: and tail clear), glu
   for (int i = 0; i < 7; ++i) {
     const LbLinear* l = linear_at(d, i);
     if (l != nullptr) n += lin_fwd_launches(*l);
@@ -450,8 +450,8 @@ extern "C" int lb_block_fwd(const LbBlockDesc* d, const LbStreamCtx* c, const Lb
   if (!c->packed) {  // rows of padding are never written by the attention kernel
     if (cudaMemsetAsync(s.o, 0, (size_t)T * Nq * 2, st) != cudaSuccess) return -11;
   }
-  LB_TRY(lb_attn_fwd(s.qr, Nq, s.kr, Nk, s.qkv + Nq + Nk, W, c->seq_start, c->seq_end, c->plan_q,
-                     c->cap_q, s.o, Nq, s.lse, T, d->Hq, d->Hk, hd, d->softmax_scale, d->causal,
+  LB_TRY(lb_attn_fwd(s.qr, Nq, s.kr, Nk, s.qkv + Nq + Nk, W, c->seq_start, c->seq_end, c->plan_f,
+                     c->cap_f, s.o, Nq, s.lse, T, d->Hq, d->Hk, hd, d->softmax_scale, d->causal,
                      c->status, c->stream));
   // attention branch output: staged in `out`, consumed by the second norm before the MLP writes there
   LB_TRY(lin_fwd(d->o_proj, s.o, Nq, out, H, T, s.ts[3], c));

@@ -66,9 +66,11 @@ struct LbStreamCtx {
   int pos_i64;
   const int* seq_start;
   const int* seq_end;
-  const int* plan_q;     // tile list for 128 / (Hq / Hk) tokens per tile
-  int cap_q;
-  const int* plan_kv;    // tile list for 128 tokens per tile (backward)
+  const int* plan_f;     // tile list of the forward (lb_attn_fwd_tile_tokens per tile)
+  int cap_f;
+  const int* plan_q;     // backward: tile list for 128 / (Hq / Hk) tokens per tile (null without
+  int cap_q;             // gradients, as plan_kv)
+  const int* plan_kv;    // tile list for 128 tokens per tile
   int cap_kv;
   int* status;           // device status word for bounded waits
   float* norm_scratch;   // lb_norm_bwd_partial_rows() * H floats

@@ -55,9 +55,9 @@ class AttnPlan:
         if hit is not None:
             return hit
         cap = (self.T + tile_tokens - 1) // tile_tokens + self.B
-        # two spare words behind the entries: the work counter of the persistent forward kernel and
-        # the end of the last sequence (rows behind it are cleared by the attention launchers)
-        plan = torch.empty(1 + 2 * cap + 2, dtype=torch.int32, device=self.seq_start.device)
+        # three spare words behind the entries: the work counter of the persistent forward kernel,
+        # the end of the last sequence (rows behind it are cleared) and the CTAs that have finished
+        plan = torch.empty(1 + 2 * cap + 3, dtype=torch.int32, device=self.seq_start.device)
         rc = nv.load().lb_attn_plan(nv.c_void_p(self.seq_start.data_ptr()),
                                     nv.c_void_p(self.seq_end.data_ptr()), nv.c_int(self.B),
                                     nv.c_int(tile_tokens), nv.c_void_p(plan.data_ptr()),
@@ -97,11 +97,16 @@ def attention_ref(q, k, v, cu_seqlens, causal: bool, scale: float | None = None,
     return out
 
 
+def fwd_tile_tokens(head_dim: int, group: int) -> int:
+    """Tokens per tile of the plan the forward kernel takes (``lb_attn_fwd_tile_tokens``)."""
+    return (128 if head_dim == 256 else 256) // group
+
+
 def _native_fwd(q, k, v, plan: AttnPlan, causal, scale):
     T, Hq, hd = q.shape
     Hk = k.shape[1]
     G = Hq // Hk
-    ptiles, cap = plan.tiles(128 // G)
+    ptiles, cap = plan.tiles(fwd_tile_tokens(hd, G))
     # tokens outside every sequence (padding) are never written by the kernel: keep them zero
     o = (torch.empty if plan.cu_seqlens is not None else torch.zeros)(
         T, Hq, hd, dtype=q.dtype, device=q.device)
@@ -115,7 +120,7 @@ def _native_fwd(q, k, v, plan: AttnPlan, causal, scale):
         nv.c_int(Hq), nv.c_int(Hk), nv.c_int(hd), nv.c_float(scale), nv.c_int(int(causal)),
         nv.c_void_p(nv.status_word(q.device).data_ptr()), nv.c_void_p(nv.stream_ptr()))
     nv.check_rc(rc, "lb_attn_fwd")
-    nv.count_launch(2)
+    nv.count_launch(2 if hd == 256 else 1)
     return o, lse
 
 

@@ -27,6 +27,7 @@ import torch
 
 from . import _ac
 from . import _native as nv
+from .attention import fwd_tile_tokens
 from ._grads import main_grad_of
 from .norm import scratch
 from .runtime_options import enabled, options as _rt
@@ -59,6 +60,7 @@ class LbBlockDesc(ctypes.Structure):
 class LbStreamCtx(ctypes.Structure):
     _fields_ = [("T", ctypes.c_int), ("packed", ctypes.c_int), ("cos", _fp), ("sin", _fp),
                 ("pos", _vp), ("pos_i64", ctypes.c_int), ("seq_start", _ip), ("seq_end", _ip),
+                ("plan_f", _ip), ("cap_f", ctypes.c_int),
                 ("plan_q", _ip), ("cap_q", ctypes.c_int), ("plan_kv", _ip),
                 ("cap_kv", ctypes.c_int), ("status", _ip), ("norm_scratch", _fp),
                 ("rope_scratch", _fp), ("wg_tmp", _fp), ("stream", _vp)]
@@ -360,23 +362,28 @@ def _tp_advance(state) -> None:
 
 # --------------------------------------------------------------------------- stream context
 def _stream_struct(ctx, plan: BlockPlan, device) -> LbStreamCtx:
-    """The per-forward struct, cached on the Python stream context (all blocks share it)."""
+    """The per-forward struct, cached on the Python stream context (all blocks share it). The
+    backward's tile lists are built for a pass that records gradients only."""
     d = plan.desc
-    key = ("_lb", d.hd, d.Hq // d.Hk, plan.rope[1], id(plan.rope[2]))
+    grad = torch.is_grad_enabled()
+    key = ("_lb", grad, d.hd, d.Hq // d.Hk, plan.rope[1], id(plan.rope[2]))
     hit = ctx.tables.get(key)
     if hit is not None:
         return hit
     lib = _library()
     cos, sin = ctx.rope(*plan.rope)
     ap = ctx.plan
-    ptq, capq = ap.tiles(128 // (d.Hq // d.Hk))
-    ptk, capk = ap.tiles(128)
+    G = d.Hq // d.Hk
+    ptf, capf = ap.tiles(fwd_tile_tokens(d.hd, G))
+    ptq, capq = ap.tiles(128 // G) if grad else (None, 0)
+    ptk, capk = ap.tiles(128) if grad else (None, 0)
     s = LbStreamCtx()
     s.T, s.packed = int(ctx.pos.shape[0]), int(ap.cu_seqlens is not None)
     s.cos, s.sin = cos.data_ptr(), sin.data_ptr()
     s.pos, s.pos_i64 = ctx.pos.data_ptr(), int(ctx.pos.dtype == torch.int64)
     s.seq_start, s.seq_end = ap.seq_start.data_ptr(), ap.seq_end.data_ptr()
-    s.plan_q, s.cap_q, s.plan_kv, s.cap_kv = ptq.data_ptr(), capq, ptk.data_ptr(), capk
+    s.plan_f, s.cap_f = ptf.data_ptr(), capf
+    s.plan_q, s.cap_q, s.plan_kv, s.cap_kv = nv.ptr(ptq) or None, capq, nv.ptr(ptk) or None, capk
     s.status = nv.status_word(device).data_ptr()
     s.norm_scratch = scratch("norm_bwd", lib.lb_norm_bwd_partial_rows() * d.H, device).data_ptr()
     s.rope_scratch = scratch("rope_bwd", lib.lb_rope_bwd_partial_rows() * 2 * d.hd,
@@ -384,7 +391,7 @@ def _stream_struct(ctx, plan: BlockPlan, device) -> LbStreamCtx:
     s.wg_tmp = scratch("qk_norm_wgrad", 2 * d.hd, device).data_ptr()
     s.stream = 0
     # keep the tensors the struct points to alive as long as the struct
-    s._keep = (cos, sin, ctx.pos, ap, ptq, ptk)
+    s._keep = (cos, sin, ctx.pos, ap, ptf, ptq, ptk)
     ctx.tables[key] = s
     return s
 

@@ -111,3 +111,26 @@ def test_stream_padded_past_the_last_sequence():
     assert torch.equal(op[:T], o) and not op[T:].any()
     for a, b in ((qp.grad, q.grad), (kp.grad, k.grad), (vp.grad, v.grad)):
         assert torch.equal(a[:T], b) and not a[T:].any()
+
+
+@pytest.mark.parametrize("Hq,Hk,hd", [(2, 2, 128), (4, 2, 128), (8, 2, 64), (8, 1, 128), (3, 3, 64)])
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("scale", [None, -0.2, 0.0])
+def test_forward_tile_edges(Hq, Hk, hd, causal, scale):
+    """Sequences that end on, before and behind the edges of the two-tile kernel: its 32-column
+    chunks, 128-token KV blocks and query tiles of 128 / G tokens, one tile or two; long ones whose
+    running maximum keeps moving; a scale that is not positive.
+
+    Output and LSE are fp32 sums over bf16 probabilities rounded once (2^-9) and bf16 outputs
+    (2^-9): 2^-8 of a value, against the 2-norm of the result."""
+    G = Hq // Hk
+    qt = 128 // G
+    lens = [1, qt - 1, qt, qt + 1, 2 * qt, 2 * qt + 1, 31, 33, 127, 128, 129, 257, 640]
+    q, k, v, cu, plan = _make(lens, Hq, Hk, hd, seed=1)
+    k = (k.float() * torch.linspace(0.2, 4, k.shape[0], device="cuda")[:, None, None]).to(k.dtype)
+    o = varlen_attention(q, k, v, plan, causal, scale)
+    nv.check_status()
+    ref = attention_ref(q.float(), k.float(), v.float(), cu, causal, scale)
+    assert ((o.float() - ref).norm() / ref.norm()).item() < 2 ** -8
+    again = varlen_attention(q, k, v, plan, causal, scale)   # the work counter was put back
+    assert torch.equal(o, again)
