@@ -91,12 +91,6 @@ __device__ __forceinline__ float2 unpair_(unsigned long long v) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
   return f;
 }
-__device__ __forceinline__ unsigned long long fma2_(unsigned long long a, unsigned long long b,
-                                                    unsigned long long c) {
-  unsigned long long d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
 __device__ __forceinline__ unsigned long long add2_(unsigned long long a, unsigned long long b) {
   unsigned long long d;
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
@@ -390,6 +384,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
       if (nblk == 0) continue;
       const int q0 = t.q0 + k * QT;
       const int qpos = q0 + (r & (QT - 1));
+      const bool valid = qpos < t.len;
       const int limit = a.causal ? min(t.len, qpos + 1) : t.len;   // columns this row may see
       const int full_cols = a.causal ? min(t.len, q0 + 1) : t.len; // columns every row may see
       float m_ref = -INFINITY, l_sum = 0.f;
@@ -412,19 +407,25 @@ __global__ void __launch_bounds__(kPairThreads, 1)
           for (int c = 0; c < 128; ++c)
             if (c >= lim) s[c >> 5][c & 31] = __float_as_uint(-INFINITY);
         }
+        // The reference of the exponentials moves by whole halves of 64 columns, and only when the
+        // maximum rose by more than 2^8 somewhere in the warp (lazy rescale); products, differences
+        // and the row sum are rounded one by one, columns in order. These are the roundings of the
+        // one-tile kernel: the two give the same bits unless a second half moves the reference.
         float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-        for (int c = 0; c < 128; c += 2)
-          mx[(c >> 1) & 3] = max3_(mx[(c >> 1) & 3], __uint_as_float(s[c >> 5][c & 31]),
-                                   __uint_as_float(s[c >> 5][(c & 31) + 1]));
-        const float m_new =
-            fmaxf(m_ref, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * scale);
-        // lazy rescale: only when the maximum moved by more than 2^8 somewhere in the warp. The
-        // scores of this block were issued after the previous P·V was complete, so O may be touched.
-        if (__any_sync(0xffffffffu, m_new > m_ref + 8.f)) {
-          const float alpha = m_new == -INFINITY ? 1.f : ex2_(m_ref - m_new);
+        for (int c = 0; c < 128; c += 2) {
+          float& m = mx[(c >> 6) * 2 + ((c >> 1) & 1)];
+          m = max3_(m, __uint_as_float(s[c >> 5][c & 31]), __uint_as_float(s[c >> 5][(c & 31) + 1]));
+        }
+        float m_new = fmaxf(m_ref, fmaxf(mx[0], mx[1]) * scale), m_to = m_ref;
+        if (__any_sync(0xffffffffu, valid && m_new > m_to + 8.f)) m_to = m_new;
+        m_new = fmaxf(m_to, fmaxf(mx[2], mx[3]) * scale);
+        if (__any_sync(0xffffffffu, valid && m_new > m_to + 8.f)) m_to = m_new;
+        // (the scores of this block were issued after the previous P·V was complete: O may be touched)
+        if (__any_sync(0xffffffffu, m_to != m_ref)) {
+          const float alpha = m_to == -INFINITY ? 1.f : ex2_(m_ref - m_to);
           l_sum *= alpha;
-          m_ref = m_new;
+          m_ref = m_to;
           if (j > 0) {
 #pragma unroll 1
             for (int c = 0; c < HD / 32; ++c) {
@@ -438,25 +439,24 @@ __global__ void __launch_bounds__(kPairThreads, 1)
           }
         }
         const float m_use = m_ref == -INFINITY ? 0.f : m_ref;
-        unsigned long long ls[2] = {0ull, 0ull};   // packed pairs: two of everything per instruction
-        const unsigned long long scale2 = pair_(scale, scale), m2 = pair_(-m_use, -m_use);
+        const unsigned long long m2 = pair_(-m_use, -m_use);
 #pragma unroll
         for (int h = 0; h < 4; ++h)
           if (h < nc) {
             uint32_t p[16];
 #pragma unroll
             for (int c = 0; c < 16; ++c) {
-              const float2 x = unpair_(fma2_(pair_(__uint_as_float(s[h][2 * c]),
-                                                   __uint_as_float(s[h][2 * c + 1])),
-                                             scale2, m2));
+              // (the packed product would be contracted with the packed sum)
+              const float2 x = unpair_(add2_(pair_(__fmul_rn(__uint_as_float(s[h][2 * c]), scale),
+                                                   __fmul_rn(__uint_as_float(s[h][2 * c + 1]),
+                                                             scale)), m2));
               const float p0 = ex2_(x.x), p1 = ex2_(x.y);
-              ls[c & 1] = add2_(ls[c & 1], pair_(p0, p1));
+              l_sum += p0;
+              l_sum += p1;
               p[c] = pack_bf16x2(p0, p1);
             }
             tmem_st_32x32b_x16(tS + h * 16, p);
           }
-        const float2 l2 = unpair_(add2_(ls[0], ls[1]));
-        l_sum += l2.x + l2.y;
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
@@ -469,7 +469,6 @@ __global__ void __launch_bounds__(kPairThreads, 1)
       }
       tc_fence_after();
       const float inv = l_sum > 0.f ? 1.f / l_sum : 0.f;
-      const bool valid = qpos < t.len;
       const long long tok = 1LL * t.seq0 + qpos;
       const int head = t.hk * G + (r >> qt_shift);
       // 32 columns at a time through shared memory, so that four lanes store 64 contiguous bytes
