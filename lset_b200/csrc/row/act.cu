@@ -5,6 +5,7 @@
 // and the backward writes d_gate and d_up side by side so a fused projection gets one dgrad GEMM.
 // Counterparts: lset/kernels/swiglu.py:21-74, lset/kernels/geglu.py:22-86, aten GELU in
 // lset/models/encoder/bert/model.py:107.
+#include "../common/pdl.h"
 #include "../common/row.cuh"
 
 namespace lb {
@@ -32,6 +33,8 @@ __global__ void __launch_bounds__(256)
                    bf16* __restrict__ out, long long ld_out, long long T, int I) {
   const int vec_per_row = I / 8;
   const long long total = T * vec_per_row;
+  pdl_wait();
+  pdl_trigger();
   for (long long i = 1LL * blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += 1LL * gridDim.x * blockDim.x) {
     const long long r = i / vec_per_row;
@@ -130,14 +133,9 @@ extern "C" int lb_glu_fwd(int kind, const void* gate, const void* up, long long 
   if (T <= 0 || I <= 0) return 0;
   if ((I & 7) || (ld_in & 7) || (ld_out & 7)) return -3;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  const int grid = flat_grid(T * (I / 8));
-  if (kind == kSwiglu)
-    glu_fwd_kernel<kSwiglu><<<grid, 256, 0, st>>>((const bf16*)gate, (const bf16*)up, ld_in,
-                                                  (bf16*)out, ld_out, T, I);
-  else
-    glu_fwd_kernel<kGeglu><<<grid, 256, 0, st>>>((const bf16*)gate, (const bf16*)up, ld_in,
-                                                 (bf16*)out, ld_out, T, I);
-  return launch_rc();
+  return launch_pdl(kind == kSwiglu ? glu_fwd_kernel<kSwiglu> : glu_fwd_kernel<kGeglu>,
+                    dim3(flat_grid(T * (I / 8))), dim3(256), 0, st, pdl_enabled(), 1,
+                    (const bf16*)gate, (const bf16*)up, ld_in, (bf16*)out, ld_out, T, I);
 }
 
 extern "C" int lb_glu_bwd(int kind, const void* dout, long long ld_dout, const void* gate,

@@ -10,6 +10,7 @@
 //
 // Backward runs on a persistent grid; every CTA writes one fp32 partial row of dW (and dB) to a
 // caller-provided scratch buffer, and a second small kernel sums the partials.
+#include "../common/pdl.h"
 #include "../common/row.cuh"
 
 namespace lb {
@@ -23,48 +24,62 @@ __global__ void __launch_bounds__(kRowThreads)
                    const bf16* __restrict__ w, bf16* __restrict__ y, bf16* __restrict__ res_out,
                    float* __restrict__ rstd_out, int N, int H, float eps, float w_off) {
   __shared__ float sred[8];
-  extern __shared__ float sw[];  // weights (+ offset) as fp32, shared by all rows of the CTA
   constexpr int ROWS = kRowThreads / TPR;
   const int t = threadIdx.x % TPR;
   const int r = threadIdx.x / TPR;
-  for (int i = threadIdx.x; i < H; i += kRowThreads) sw[i] = __bfloat162float(w[i]) + w_off;
-  __syncthreads();
-  for (long long row0 = 1LL * blockIdx.x * ROWS; row0 < N; row0 += 1LL * gridDim.x * ROWS) {
-    const long long row = row0 + r;
-    const bool valid = row < N;
-    float xv[NV][8];
-    float ss = 0.f;
+  const long long row = 1LL * blockIdx.x * ROWS + r;
+  const bool valid = row < N;
+  // Every load of the row is requested before the first is used, the weights (in L1 / L2 after the
+  // first rows) among them; the row stays packed in between, so that more CTAs fit per SM.
+  uint4 xq[NV], rq[NV], wq[NV];
 #pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      const int idx = (v * TPR + t) * 8;
-      if (valid && idx < H) {
-        unpack8(ld16(x + row * H + idx), xv[v]);
-        if (res_in != nullptr) {
-          float rv[8];
-          unpack8(ld16(res_in + row * H + idx), rv);
+  for (int v = 0; v < NV; ++v) {
+    const int idx = (v * TPR + t) * 8;
+    if (valid && idx < H) wq[v] = ld16(w + idx);
+  }
+  pdl_wait();
+  pdl_trigger();
 #pragma unroll
-          for (int i = 0; i < 8; ++i) xv[v][i] = bf16_round(xv[v][i] + rv[i]);
-          st16(res_out + row * H + idx, pack8(xv[v]));
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) ss += xv[v][i] * xv[v][i];
-      }
+  for (int v = 0; v < NV; ++v) {
+    const int idx = (v * TPR + t) * 8;
+    if (valid && idx < H) {
+      xq[v] = ld16(x + row * H + idx);
+      if (res_in != nullptr) rq[v] = ld16(res_in + row * H + idx);
     }
-    ss = row_sum<TPR>(ss, sred);
-    const float rstd = rsqrtf(ss / float(H) + eps);
-    if (valid && t == 0 && rstd_out != nullptr) rstd_out[row] = rstd;
+  }
+  float ss = 0.f;
 #pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      const int idx = (v * TPR + t) * 8;
-      if (valid && idx < H) {
-        float o[8];
-        const float4 w0 = *reinterpret_cast<const float4*>(sw + idx);
-        const float4 w1 = *reinterpret_cast<const float4*>(sw + idx + 4);
-        const float wl[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+  for (int v = 0; v < NV; ++v) {
+    const int idx = (v * TPR + t) * 8;
+    if (valid && idx < H) {
+      float f[8];
+      unpack8(xq[v], f);
+      if (res_in != nullptr) {
+        float rv[8];
+        unpack8(rq[v], rv);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) o[i] = bf16_round(xv[v][i] * rstd) * wl[i];
-        st16(y + row * H + idx, pack8(o));
+        for (int i = 0; i < 8; ++i) f[i] += rv[i];
+        xq[v] = pack8(f);
+        unpack8(xq[v], f);
+        st16(res_out + row * H + idx, xq[v]);
       }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) ss += f[i] * f[i];
+    }
+  }
+  ss = row_sum<TPR>(ss, sred);
+  const float rstd = rsqrtf(ss / float(H) + eps);
+  if (valid && t == 0 && rstd_out != nullptr) rstd_out[row] = rstd;
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    const int idx = (v * TPR + t) * 8;
+    if (valid && idx < H) {
+      float f[8], wl[8];
+      unpack8(xq[v], f);
+      unpack8(wq[v], wl);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) f[i] = bf16_round(f[i] * rstd) * (wl[i] + w_off);
+      st16(y + row * H + idx, pack8(f));
     }
   }
 }
@@ -447,11 +462,10 @@ extern "C" int lb_rms_norm_fwd(const void* x, const void* res_in, const void* w,
   LB_ROW_DISPATCH(H, {
     constexpr int ROWS = kRowThreads / TPR;
     const int grid = (N + ROWS - 1) / ROWS;
-    rms_fwd_kernel<TPR, NV><<<grid, kRowThreads, H * sizeof(float), st>>>(
-        (const bf16*)x, (const bf16*)res_in, (const bf16*)w, (bf16*)y, (bf16*)res_out, rstd, N, H,
-        eps, w_off);
+    return launch_pdl(rms_fwd_kernel<TPR, NV>, dim3(grid), dim3(kRowThreads), 0, st, pdl_enabled(),
+                      1, (const bf16*)x, (const bf16*)res_in, (const bf16*)w, (bf16*)y,
+                      (bf16*)res_out, rstd, N, H, eps, w_off);
   });
-  return launch_rc();
 }
 
 // Fused forward of rmsnorm(a)·w1 → + residual → rmsnorm(·)·w2. Outputs y, res_out (the new

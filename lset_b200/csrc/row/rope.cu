@@ -9,6 +9,7 @@
 // lset/kernels/rope.py:12-75). Inputs may be slices of a fused QKV projection output (row strides
 // are explicit), so no split/copy of the QKV tensor is needed.
 #include "../common/api.h"
+#include "../common/pdl.h"
 #include "../common/row.cuh"
 
 namespace lb {
@@ -35,6 +36,7 @@ struct RopeArgs {
   int T, Hq, Hk;
   float eps, w_off;
   int do_norm;
+  int parts, part_heads;  // lane groups per token, and the heads (of q and k together) each walks over
 };
 
 __device__ __forceinline__ int token_pos(const RopeArgs& a, long long tok) {
@@ -43,7 +45,8 @@ __device__ __forceinline__ int token_pos(const RopeArgs& a, long long tok) {
                    : reinterpret_cast<const int*>(a.pos)[tok];
 }
 
-// A group of HD/8 lanes owns one token at a time and walks over its heads UB at a time: the cos/sin
+// A group of HD/8 lanes owns one token at a time (or, with few tokens, a part of its heads, see
+// rope_parts) and walks over its heads UB at a time: the cos/sin
 // row and the position are fetched once per token, and the 16-byte loads of the next UB heads are
 // already in flight while the current UB heads are normalised, rotated and stored (the kernel is
 // bound by memory latency otherwise).
@@ -55,16 +58,21 @@ __global__ void __launch_bounds__(kRowThreads, 3) qk_rope_fwd_kernel(RopeArgs a)
   __shared__ float swt[2 * HD];  // q then k norm weights (+ offset)
   const int l = threadIdx.x % LPH;
   const int g = threadIdx.x / LPH;
-  const int heads = a.Hq + a.Hk;
   const int e0 = l * 8;
   const int c0 = e0 % (HD / 2);
   const bool first_half = l < LPH / 2;
   for (int i = threadIdx.x; i < 2 * HD; i += kRowThreads)
     swt[i] = a.do_norm ? __bfloat162float(i < HD ? a.qw[i] : a.kw[i - HD]) + a.w_off : 1.f;
   __syncthreads();
-  for (int tok0 = blockIdx.x * TPB; tok0 < a.T; tok0 += gridDim.x * TPB) {
-    const long long tok = tok0 + g;
+  pdl_wait();
+  pdl_trigger();
+  const unsigned total = unsigned(a.T) * a.parts;
+  for (unsigned u0 = blockIdx.x * TPB; u0 < total; u0 += gridDim.x * TPB) {
+    const unsigned tok_u = (u0 + g) / a.parts;
+    const long long tok = tok_u;
     const bool valid = tok < a.T;
+    const int h_first = int(u0 + g - tok_u * a.parts) * a.part_heads;
+    const int heads = min(h_first + a.part_heads, a.Hq + a.Hk);
     const bf16* qrow = a.q_in + tok * a.ldq_in + e0;
     const bf16* krow = a.k_in + tok * a.ldk_in + e0;
     bf16* qdst = a.q_out + tok * a.ldq_out + e0;
@@ -78,7 +86,7 @@ __global__ void __launch_bounds__(kRowThreads, 3) qk_rope_fwd_kernel(RopeArgs a)
       }
     };
     uint4 cur[UB], nxt[UB];
-    load_batch(0, cur);
+    load_batch(h_first, cur);
     float c[8], s[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) c[i] = s[i] = 0.f;
@@ -95,12 +103,13 @@ __global__ void __launch_bounds__(kRowThreads, 3) qk_rope_fwd_kernel(RopeArgs a)
 #pragma unroll
       for (int i = 0; i < 8; ++i) s[i] = -s[i];  // y = x*c - partner*s (first half), + (second)
     }
-    for (int h0 = 0; h0 < heads; h0 += UB) {
-      if (h0 + UB < heads) load_batch(h0 + UB, nxt);
+    for (int b0 = 0; b0 < a.part_heads; b0 += UB) {   // uniform over the CTA
+      const int h0 = h_first + b0;
+      if (b0 + UB < a.part_heads) load_batch(h0 + UB, nxt);
 #pragma unroll
       for (int j = 0; j < UB; ++j) {
         const int h = h0 + j;
-        if (h >= heads) break;  // uniform over the CTA
+        const bool live = valid && h < heads;
         const bool is_q = h < a.Hq;
         float x[8];
         unpack8(cur[j], x);
@@ -111,7 +120,7 @@ __global__ void __launch_bounds__(kRowThreads, 3) qk_rope_fwd_kernel(RopeArgs a)
 #pragma unroll
           for (int o = LPH / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
           const float rstd = rsqrtf(ss / float(HD) + a.eps);
-          if (valid && l == 0) {
+          if (live && l == 0) {
             if (is_q) a.q_rstd[tok * a.Hq + h] = rstd;
             else a.k_rstd[tok * a.Hk + (h - a.Hq)] = rstd;
           }
@@ -128,7 +137,7 @@ __global__ void __launch_bounds__(kRowThreads, 3) qk_rope_fwd_kernel(RopeArgs a)
           const float p = __shfl_xor_sync(0xffffffffu, x[i], LPH / 2);
           y[i] = x[i] * c[i] - p * s[i];
         }
-        if (valid) st16(is_q ? qdst + h * HD : kdst + (h - a.Hq) * HD, pack8(y));
+        if (live) st16(is_q ? qdst + h * HD : kdst + (h - a.Hq) * HD, pack8(y));
       }
 #pragma unroll
       for (int j = 0; j < UB; ++j) cur[j] = nxt[j];
@@ -159,6 +168,7 @@ struct RopeBwdArgs {
   int T, Hq, Hk;
   float w_off;
   int do_norm;
+  int parts, part_heads;
 };
 
 // Same token-per-lane-group walk as the forward kernel, UB heads at a time: the gradient rows, the
@@ -172,7 +182,6 @@ __global__ void __launch_bounds__(kRowThreads, 2) qk_rope_bwd_kernel(RopeBwdArgs
   __shared__ float swt[2 * HD];  // q then k norm weights (+ offset)
   const int l = threadIdx.x % LPH;
   const int g = threadIdx.x / LPH;
-  const int heads = a.Hq + a.Hk;
   const int e0 = l * 8;
   const int c0 = e0 % (HD / 2);
   const bool first_half = l < LPH / 2;
@@ -188,10 +197,16 @@ __global__ void __launch_bounds__(kRowThreads, 2) qk_rope_bwd_kernel(RopeBwdArgs
   pa.pos = a.pos;
   pa.pos_i64 = a.pos_i64;
   pa.pos_mod = a.pos_mod;
+  pdl_wait();
+  pdl_trigger();
 
-  for (int tok0 = blockIdx.x * TPB; tok0 < a.T; tok0 += gridDim.x * TPB) {
-    const long long tok = tok0 + g;
+  const unsigned total = unsigned(a.T) * a.parts;
+  for (unsigned u0 = blockIdx.x * TPB; u0 < total; u0 += gridDim.x * TPB) {
+    const unsigned tok_u = (u0 + g) / a.parts;
+    const long long tok = tok_u;
     const bool valid = tok < a.T;
+    const int h_first = int(u0 + g - tok_u * a.parts) * a.part_heads;
+    const int heads = min(h_first + a.part_heads, a.Hq + a.Hk);
     float c[8], s[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) c[i] = s[i] = 0.f;
@@ -214,7 +229,8 @@ __global__ void __launch_bounds__(kRowThreads, 2) qk_rope_bwd_kernel(RopeBwdArgs
     const bf16* xk = a.k_in + tok * a.ldk_in + e0;
     bf16* oq = a.dq_in + tok * a.lddq_in + e0;
     bf16* ok = a.dk_in + tok * a.lddk_in + e0;
-    for (int h0 = 0; h0 < heads; h0 += UB) {
+    for (int b0 = 0; b0 < a.part_heads; b0 += UB) {
+      const int h0 = h_first + b0;
       uint4 graw[UB], xraw[UB];
       float rs[UB];
 #pragma unroll
@@ -234,7 +250,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) qk_rope_bwd_kernel(RopeBwdArgs
 #pragma unroll
       for (int j = 0; j < UB; ++j) {
         const int h = h0 + j;
-        if (h >= heads) break;  // uniform over the CTA
+        const bool live = valid && h < heads;   // (loads of the others are zero, and add nothing)
         const bool is_q = h < a.Hq;
         float gv[8], gn[8], o[8];
         unpack8(graw[j], gv);
@@ -270,7 +286,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) qk_rope_bwd_kernel(RopeBwdArgs
 #pragma unroll
           for (int i = 0; i < 8; ++i) o[i] = gn[i];
         }
-        if (valid) st16(is_q ? oq + h * HD : ok + (h - a.Hq) * HD, pack8(o));
+        if (live) st16(is_q ? oq + h * HD : ok + (h - a.Hq) * HD, pack8(o));
       }
     }
   }
@@ -291,6 +307,18 @@ __global__ void __launch_bounds__(kRowThreads, 2) qk_rope_bwd_kernel(RopeBwdArgs
 
 using namespace lb;
 
+// Lane groups per token. One walks over all heads, the next loads in flight under the current heads'
+// arithmetic, which is what the kernels are bound by with many tokens (a group for every four heads:
+// 142 against 127 us at 40280 tokens of 16 + 8 heads of 128). With so few tokens that the groups
+// are fewer than the SMs hold, the walk is a chain of latencies, and four heads a group are faster
+// (32 tokens: 21 against 29 us, 1024: 20 against 27; about 10 us of each are the measurement's own).
+static void rope_parts(int T, int heads, int tokens_per_cta, int* parts, int* part_heads) {
+  const int all = (heads + 3) / 4;
+  const bool few = 1LL * T < 3LL * row_num_sms() * tokens_per_cta / 2;
+  *parts = few ? all : 1;
+  *part_heads = few ? 4 : all * 4;
+}
+
 extern "C" int lb_rope_bwd_partial_rows() { return row_num_sms() * 8; }
 
 extern "C" int lb_qk_norm_rope_fwd(const void* q_in, long long ldq_in, const void* k_in,
@@ -305,19 +333,20 @@ extern "C" int lb_qk_norm_rope_fwd(const void* q_in, long long ldq_in, const voi
   if (1LL * T * (Hq + Hk) >= (1LL << 32)) return -3;
   RopeArgs a{(const bf16*)q_in, (const bf16*)k_in, ldq_in, ldk_in, (const bf16*)qw, (const bf16*)kw,
              cos, sin, pos, pos_i64, pos_mod > 0 ? pos_mod : 1, (bf16*)q_out, (bf16*)k_out, ldq_out,
-             ldk_out, q_rstd, k_rstd, T, Hq, Hk, eps, w_off, do_norm};
+             ldk_out, q_rstd, k_rstd, T, Hq, Hk, eps, w_off, do_norm, 1, 0};
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  auto grid_for = [&](int lph) {
-    const long long tpb = kRowThreads / lph;
-    long long g = (T + tpb - 1) / tpb;
+  auto run = [&](auto kern, int lph) {
+    const int tpb = kRowThreads / lph;
+    rope_parts(T, Hq + Hk, tpb, &a.parts, &a.part_heads);
+    const long long g = (1LL * T * a.parts + tpb - 1) / tpb;
     const long long cap = 1LL * row_num_sms() * 6;  // two waves at three CTAs per SM
-    return int(g < cap ? g : cap);
+    return launch_pdl(kern, dim3(unsigned(g < cap ? g : cap)), dim3(kRowThreads), 0, st,
+                      pdl_enabled(), 1, a);
   };
-  if (hd == 128) qk_rope_fwd_kernel<128><<<grid_for(16), kRowThreads, 0, st>>>(a);
-  else if (hd == 64) qk_rope_fwd_kernel<64><<<grid_for(8), kRowThreads, 0, st>>>(a);
-  else if (hd == 256) qk_rope_fwd_kernel<256><<<grid_for(32), kRowThreads, 0, st>>>(a);
-  else return -3;
-  return launch_rc();
+  if (hd == 128) return run(qk_rope_fwd_kernel<128>, 16);
+  if (hd == 64) return run(qk_rope_fwd_kernel<64>, 8);
+  if (hd == 256) return run(qk_rope_fwd_kernel<256>, 32);
+  return -3;
 }
 
 // dw_out: [2, hd] (q weight grad then k weight grad); scratch: lb_rope_bwd_partial_rows()*2*hd floats.
@@ -336,19 +365,22 @@ extern "C" int lb_qk_norm_rope_bwd(const void* dq, long long lddq, const void* d
   RopeBwdArgs a{(const bf16*)dq, (const bf16*)dk, lddq, lddk, (const bf16*)q_in, (const bf16*)k_in,
                 ldq_in, ldk_in, (const bf16*)qw, (const bf16*)kw, cos, sin, pos, pos_i64,
                 pos_mod > 0 ? pos_mod : 1, q_rstd, k_rstd, (bf16*)dq_in, (bf16*)dk_in, lddq_in,
-                lddk_in, scratch, T, Hq, Hk, w_off, do_norm};
+                lddk_in, scratch, T, Hq, Hk, w_off, do_norm, 1, 0};
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  auto grid_for = [&](int lph) {
-    const long long tpb = kRowThreads / lph;
-    long long g = (T + tpb - 1) / tpb;
+  int grid = 1;
+  auto run = [&](auto kern, int lph) {
+    const int tpb = kRowThreads / lph;
+    rope_parts(T, Hq + Hk, tpb, &a.parts, &a.part_heads);
+    const long long g = (1LL * T * a.parts + tpb - 1) / tpb;
     const long long cap = 1LL * row_num_sms() * 4;
-    return int(g < cap ? (g > 0 ? g : 1) : cap);
+    grid = int(g < cap ? g : cap);
+    return launch_pdl(kern, dim3(grid), dim3(kRowThreads), 0, st, pdl_enabled(), 1, a);
   };
-  int grid;
-  if (hd == 128) { grid = grid_for(16); qk_rope_bwd_kernel<128><<<grid, kRowThreads, 0, st>>>(a); }
-  else if (hd == 64) { grid = grid_for(8); qk_rope_bwd_kernel<64><<<grid, kRowThreads, 0, st>>>(a); }
-  else if (hd == 256) { grid = grid_for(32); qk_rope_bwd_kernel<256><<<grid, kRowThreads, 0, st>>>(a); }
-  else return -3;
+  int rc = -3;
+  if (hd == 128) rc = run(qk_rope_bwd_kernel<128>, 16);
+  else if (hd == 64) rc = run(qk_rope_bwd_kernel<64>, 8);
+  else if (hd == 256) rc = run(qk_rope_bwd_kernel<256>, 32);
+  if (rc) return rc;
   if (do_norm && dw_out != nullptr && scratch != nullptr) {
     return lb_colsum(scratch, grid, 2 * hd, dw_out, dw_fp32, dw_accumulate, stream);
   }
