@@ -7,6 +7,8 @@
 #include <stdint.h>
 
 #include "../common/api.h"
+#include "../common/pdl.h"
+#include "../gemm/gemm_small.h"
 
 namespace {
 
@@ -128,6 +130,13 @@ Work carve_work(const LbBlockDesc* d, int T, int R, bool sharded, Arena& a) {
     if (rc_ != 0) return rc_; \
   } while (0)
 
+// Fills in the tile width and split of `g`: whether it is modelled to take less than `alternative`.
+bool small_wins(LbSmallGemm* g, double alternative) {
+  if (!lb_gemm_use_2cta(-1)) return false;
+  const double cost = lb_gemm_small_plan(g, &g->bn, &g->splits);
+  return cost >= 0.0 && cost < alternative;
+}
+
 // y[:, :n_out] (row stride ldy) = x · Wᵀ (+ LoRA). `ts` receives s · x · Aᵀ when the linear has adapters.
 int lin_fwd(const LbLinear& l, const __nv_bfloat16* x, long long ldx, __nv_bfloat16* y,
             long long ldy, int T, __nv_bfloat16* ts, const LbStreamCtx* c) {
@@ -138,6 +147,25 @@ int lin_fwd(const LbLinear& l, const __nv_bfloat16* x, long long ldx, __nv_bfloa
     LB_TRY(scale_bf16(ts, 1LL * T * l.lora_r, l.lora_scale, st));
     return lb_gemm_bf16_ext(x, l.w, ts, l.lora_b, y, T, l.n_out, l.k_in, l.lora_r, ldx, l.ldw,
                             l.lora_r, l.lora_r, ldy, 0, nullptr, c->status, c->stream);
+  }
+  if (c->may_split) {
+    LbSmallGemm g = {};
+    g.A = x;
+    g.B[0] = l.w;
+    g.C[0] = y;
+    g.lda = ldx;
+    g.ldb[0] = l.ldw;
+    g.ldc[0] = ldy;
+    g.M = T;
+    g.N = g.ext[0] = l.n_out;
+    g.K = l.k_in;
+    g.nparts = 1;
+    g.mode = kParallelN;
+    g.b_ready = g.may_split = 1;
+    g.status = c->status;
+    g.stream = c->stream;
+    if (small_wins(&g, lb_gemm_tile_cost(T, l.n_out, l.k_in, lb_gemm_2cta_pairs())))
+      return lb_gemm_small(&g);
   }
   return lb_gemm_bf16(x, l.w, y, T, l.n_out, l.k_in, ldx, l.ldw, ldy, 0, 0, 0, 0, nullptr, 1, 0,
                       c->status, c->stream);
@@ -183,6 +211,162 @@ int lin_wgrad(const LbLinear& l, const __nv_bfloat16* dy, long long lddy, const 
       LB_TRY(lb_gemm_bf16(dy, ts, l.lora_b_grad, l.n_out, l.lora_r, T, lddy, l.lora_r, l.lora_r, 1,
                           1, 1, 1, nullptr, 0, 0, c->status,
                           c->stream));
+  }
+  return 0;
+}
+
+// ---- projections with several linears in one launch -----------------------------------------------
+// A product with few tokens goes to lb_gemm_small, and there all linears of a projection are one
+// launch. `alternative` is the modelled time of the launches it replaces.
+bool plain(const LbProjection& p) {
+  for (int i = 0; i < p.n; ++i)
+    if (p.part[i].lora_r > 0) return false;
+  return true;
+}
+
+thread_local int t_fewer = 0;  // launches saved by the current call
+
+LbSmallGemm small_gemm(const LbProjection& p, int mode, const LbStreamCtx* c) {
+  LbSmallGemm g = {};
+  g.nparts = p.n;
+  g.mode = mode;
+  for (int i = 0; i < p.n; ++i) {
+    g.B[i] = p.part[i].w;
+    g.ldb[i] = p.part[i].ldw;
+    g.ext[i] = p.part[i].n_out;
+  }
+  g.may_split = c->may_split;
+  g.status = c->status;
+  g.stream = c->stream;
+  return g;
+}
+
+// y [T, p.width] = x · [W_0; W_1; ..]ᵀ
+int proj_fwd(const LbProjection& p, const __nv_bfloat16* x, long long ldx, __nv_bfloat16* y, int T,
+             __nv_bfloat16* const* ts, const LbStreamCtx* c) {
+  if (p.n > 1 && plain(p)) {
+    LbSmallGemm g = small_gemm(p, kParallelN, c);
+    double apart = 0.0;
+    __nv_bfloat16* col = y;
+    for (int i = 0; i < p.n; ++i) {
+      g.C[i] = col;
+      g.ldc[i] = p.width;
+      col += p.part[i].n_out;
+      apart += lb_gemm_tile_cost(T, p.part[i].n_out, p.part[i].k_in, lb_gemm_2cta_pairs());
+    }
+    g.A = x;
+    g.lda = ldx;
+    g.M = T;
+    g.N = p.width;
+    g.K = p.part[0].k_in;
+    g.b_ready = 1;
+    if (small_wins(&g, apart)) {
+      t_fewer += p.n - 1;
+      return lb_gemm_small(&g);
+    }
+  }
+  for (int i = 0; i < p.n; ++i) {
+    LB_TRY(lin_fwd(p.part[i], x, ldx, y, p.width, T, ts[i], c));
+    y += p.part[i].n_out;
+  }
+  return 0;
+}
+
+// h [T, I] = act(x · W_gateᵀ) * (x · W_upᵀ), with the two products in gu [T, 2I] (the one-launch form
+// leaves gu unwritten unless it is to be kept).
+int glu_proj_fwd(const LbBlockDesc* d, const __nv_bfloat16* x, __nv_bfloat16* gu, bool keep_gu,
+                 __nv_bfloat16* h, int T, __nv_bfloat16* const* ts, const LbStreamCtx* c) {
+  const LbProjection& p = d->gate_up;
+  const int I = d->I;
+  if (plain(p)) {
+    LbSmallGemm g = small_gemm(p, kParallelN, c);
+    if (p.n == 1) {  // one fused weight: its two halves
+      g.nparts = 2;
+      g.B[1] = static_cast<const __nv_bfloat16*>(p.part[0].w) + I * p.part[0].ldw;
+      g.ldb[1] = p.part[0].ldw;
+    }
+    g.ext[0] = g.ext[1] = I;
+    if (keep_gu) {
+      g.C[0] = gu;
+      g.C[1] = gu + I;
+      g.ldc[0] = g.ldc[1] = 2 * I;
+    }
+    g.glu_h = h;
+    g.ld_h = I;
+    g.glu_kind = d->act_kind;
+    g.A = x;
+    g.lda = d->H;
+    g.M = T;
+    g.N = 2 * I;
+    g.K = d->H;
+    g.b_ready = 1;
+    double apart = 3.0 + 6.0 * T * I / 5e6;  // the activation: a launch, three passes at 5 TB/s
+    for (int i = 0; i < p.n; ++i)
+      apart += lb_gemm_tile_cost(T, p.part[i].n_out, d->H, lb_gemm_2cta_pairs());
+    if (small_wins(&g, apart)) {
+      t_fewer += p.n;
+      return lb_gemm_small(&g);
+    }
+  }
+  LB_TRY(proj_fwd(p, x, d->H, gu, T, ts, c));
+  return lb_glu_fwd(d->act_kind, gu, gu + I, 2 * I, h, I, T, I, c->stream);
+}
+
+// dx [T, k_in] = dy · [W_0; W_1; ..] (the parts' products added up in bf16) and dW_i += dy_iᵀ · x.
+int proj_bwd(const LbProjection& p, const __nv_bfloat16* dy, const __nv_bfloat16* x,
+             __nv_bfloat16* dx, int T, __nv_bfloat16* const* ts, __nv_bfloat16* us,
+             const LbStreamCtx* c) {
+  const int K = p.part[0].k_in;
+  bool dx_done = false, dw_done = false;
+  if (p.n > 1 && plain(p)) {
+    double apart = 0.0, apart_w = 0.0;
+    bool all_w = true;
+    for (int i = 0; i < p.n; ++i) {
+      apart += lb_gemm_tile_cost(T, K, p.part[i].n_out, lb_gemm_2cta_pairs());
+      apart_w += lb_gemm_tile_cost(p.part[i].n_out, K, T, lb_gemm_2cta_pairs());
+      all_w = all_w && p.part[i].wgrad != nullptr;
+    }
+    LbSmallGemm g = small_gemm(p, kParallelK, c);
+    g.A = dy;
+    g.lda = p.width;
+    g.C[0] = dx;
+    g.ldc[0] = K;
+    g.M = T;
+    g.N = K;
+    g.K = p.width;
+    g.b_mn = 1;
+    g.b_ready = 1;
+    if (small_wins(&g, apart)) {
+      LB_TRY(lb_gemm_small(&g));
+      t_fewer += p.n - 1;
+      dx_done = true;
+    }
+    if (all_w) {
+      LbSmallGemm w = small_gemm(p, kParallelM, c);
+      w.A = dy;
+      w.lda = p.width;
+      w.B[0] = x;
+      w.ldb[0] = K;
+      for (int i = 0; i < p.n; ++i) {
+        w.C[i] = p.part[i].wgrad;
+        w.ldc[i] = K;
+      }
+      w.M = p.width;
+      w.N = K;
+      w.K = T;
+      w.a_mn = w.b_mn = w.out_fp32 = 1;
+      if (small_wins(&w, apart_w)) {
+        LB_TRY(lb_gemm_small(&w));
+        t_fewer += p.n - 1;
+        dw_done = true;
+      }
+    }
+  }
+  for (int i = 0, col = 0; i < p.n; ++i) {
+    const LbLinear& l = p.part[i];
+    if (!dx_done) LB_TRY(lin_dgrad(l, dy + col, p.width, dx, T, i > 0, us, c));
+    if (!dw_done) LB_TRY(lin_wgrad(l, dy + col, p.width, x, K, T, ts[i], us, c));
+    col += l.n_out;
   }
   return 0;
 }
@@ -423,7 +607,7 @@ extern "C" int lb_block_bwd_launches(const LbBlockDesc* d, const LbStreamCtx* c,
   return n + (c->packed ? 0 : 3);
 }
 
-extern "C" int lb_block_fwd(const LbBlockDesc* d, const LbStreamCtx* c, const LbBlockIO* io) {
+static int block_fwd(const LbBlockDesc* d, const LbStreamCtx* c, const LbBlockIO* io) {
   const int T = c->T;
   if (T <= 0) return 0;
   if (io->tp != nullptr) return block_fwd_tp(d, c, io);
@@ -437,12 +621,13 @@ extern "C" int lb_block_fwd(const LbBlockDesc* d, const LbStreamCtx* c, const Lb
   const __nv_bfloat16* stream_in = io->residual != nullptr ? s.res1 : branch;
   __nv_bfloat16* out = static_cast<__nv_bfloat16*>(io->out);
 
+  // The first launch of a call is ordered behind everything before it on the stream, weight updates
+  // and events of other streams included; the others may start while the one in front of them runs
+  // and read weights meanwhile.
   LB_TRY(lb_rms_norm_fwd(branch, io->residual, d->ln1_w, s.x1, s.res1, s.rstd1, T, H, d->eps,
                          d->w_off, c->stream));
-  for (int p = 0, col = 0; p < d->qkv.n; ++p) {
-    LB_TRY(lin_fwd(d->qkv.part[p], s.x1, H, s.qkv + col, W, T, s.ts[p], c));
-    col += d->qkv.part[p].n_out;
-  }
+  const lb::PdlScope pdl(true);
+  LB_TRY(proj_fwd(d->qkv, s.x1, H, s.qkv, T, s.ts, c));
   LB_TRY(lb_qk_norm_rope_fwd(s.qkv, W, s.qkv + Nq, W, d->qk_norm ? d->qn_w : nullptr,
                              d->qk_norm ? d->kn_w : nullptr, c->cos, c->sin, c->pos, c->pos_i64, 1,
                              s.qr, Nq, s.kr, Nk, s.q_rstd, s.k_rstd, T, d->Hq, d->Hk, hd, d->eps,
@@ -457,15 +642,12 @@ extern "C" int lb_block_fwd(const LbBlockDesc* d, const LbStreamCtx* c, const Lb
   LB_TRY(lin_fwd(d->o_proj, s.o, Nq, out, H, T, s.ts[3], c));
   LB_TRY(lb_rms_norm_fwd(out, stream_in, d->ln2_w, s.x2, io->res_out, s.rstd2, T, H, d->eps,
                          d->w_off, c->stream));
-  for (int p = 0, col = 0; p < d->gate_up.n; ++p) {
-    LB_TRY(lin_fwd(d->gate_up.part[p], s.x2, H, s.gu + col, 2 * d->I, T, s.ts[4 + p], c));
-    col += d->gate_up.part[p].n_out;
-  }
-  LB_TRY(lb_glu_fwd(d->act_kind, s.gu, s.gu + d->I, 2 * d->I, s.h, d->I, T, d->I, c->stream));
+  // without gradients nothing reads the two products again
+  LB_TRY(glu_proj_fwd(d, s.x2, s.gu, c->plan_q != nullptr, s.h, T, s.ts + 4, c));
   return lin_fwd(d->down, s.h, d->I, out, H, T, s.ts[6], c);
 }
 
-extern "C" int lb_block_bwd(const LbBlockDesc* d, const LbStreamCtx* c, const LbBlockIO* io) {
+static int block_bwd(const LbBlockDesc* d, const LbStreamCtx* c, const LbBlockIO* io) {
   const int T = c->T;
   if (T <= 0) return 0;
   if (io->tp != nullptr) return block_bwd_tp(d, c, io);
@@ -482,15 +664,11 @@ extern "C" int lb_block_bwd(const LbBlockDesc* d, const LbStreamCtx* c, const Lb
 
   // ---- MLP
   LB_TRY(lin_dgrad(d->down, d_out, H, w.dh, T, false, w.us, c));
+  const lb::PdlScope pdl(true);  // from the second launch on, as in the forward
   LB_TRY(lin_wgrad(d->down, d_out, H, s.h, I, T, s.ts[6], w.us, c));
   LB_TRY(lb_glu_bwd(d->act_kind, w.dh, I, s.gu, s.gu + I, 2 * I, w.dgu, w.dgu + I, 2 * I, T, I,
                     c->stream));
-  for (int p = 0, col = 0; p < d->gate_up.n; ++p) {
-    const LbLinear& l = d->gate_up.part[p];
-    LB_TRY(lin_dgrad(l, w.dgu + col, 2 * I, w.dx2, T, p > 0, w.us, c));
-    LB_TRY(lin_wgrad(l, w.dgu + col, 2 * I, s.x2, H, T, s.ts[4 + p], w.us, c));
-    col += l.n_out;
-  }
+  LB_TRY(proj_bwd(d->gate_up, w.dgu, s.x2, w.dx2, T, s.ts + 4, w.us, c));
   // second norm: the gradient of its input is both the attention branch's and the stream's
   LB_TRY(lb_rms_norm_bwd(w.dx2, io->d_res_out, io->res_out, d->ln2_w, s.rstd2, w.dres2,
                          c->norm_scratch, d->ln2_wgrad, 1, 1, T, H, d->w_off, c->stream));
@@ -522,12 +700,21 @@ extern "C" int lb_block_bwd(const LbBlockDesc* d, const LbStreamCtx* c, const Lb
       LB_TRY(lb_colsum(c->wg_tmp + hd, 1, hd, d->kn_wgrad, 1, 1, c->stream));
     }
   }
-  for (int p = 0, col = 0; p < d->qkv.n; ++p) {
-    const LbLinear& l = d->qkv.part[p];
-    LB_TRY(lin_dgrad(l, w.dqkv + col, W, w.dx1, T, p > 0, w.us, c));
-    LB_TRY(lin_wgrad(l, w.dqkv + col, W, s.x1, H, T, s.ts[p], w.us, c));
-    col += l.n_out;
-  }
+  LB_TRY(proj_bwd(d->qkv, w.dqkv, s.x1, w.dx1, T, s.ts, w.us, c));
   return lb_rms_norm_bwd(w.dx1, w.dres2, stream_in, d->ln1_w, s.rstd1, io->dx, c->norm_scratch,
                          d->ln1_wgrad, 1, 1, T, H, d->w_off, c->stream);
+}
+
+extern "C" int lb_block_fwd(const LbBlockDesc* d, const LbStreamCtx* c, LbBlockIO* io) {
+  t_fewer = 0;
+  const int rc = block_fwd(d, c, io);
+  io->fewer_launches = t_fewer;
+  return rc;
+}
+
+extern "C" int lb_block_bwd(const LbBlockDesc* d, const LbStreamCtx* c, LbBlockIO* io) {
+  t_fewer = 0;
+  const int rc = block_bwd(d, c, io);
+  io->fewer_launches = t_fewer;
+  return rc;
 }

@@ -77,6 +77,7 @@ struct LbStreamCtx {
   float* rope_scratch;   // lb_rope_bwd_partial_rows() * 2 * hd floats
   float* wg_tmp;         // 2 * hd floats (QK-norm weight gradient staging)
   void* stream;
+  int may_split;         // inference: contractions may be summed in pieces (LbSmallGemm::may_split)
 };
 
 // Tensor parallelism with a token-sharded residual stream (sequence parallelism): the block's
@@ -119,6 +120,7 @@ struct LbBlockIO {
   void* dx;              // [T, H] gradient of `branch` (and of `residual`: they are equal)
   void* work;            // lb_block_work_bytes() bytes, 256-byte aligned
   const LbTpCtx* tp;     // null: the stream is not token-sharded
+  int fewer_launches;    // out: launches saved against lb_block_*_launches (several linears in one)
 };
 
 // Bytes of the activation arena the forward fills and the backward reads (`tp` may be null; with it
@@ -126,13 +128,14 @@ struct LbBlockIO {
 size_t lb_block_saved_bytes(const LbBlockDesc* d, int T, int has_residual, const LbTpCtx* tp);
 // Bytes of temporary storage the backward needs.
 size_t lb_block_work_bytes(const LbBlockDesc* d, int T, const LbTpCtx* tp);
-// Number of kernel launches the two calls issue (for benchmark reporting).
+// Number of kernel launches the two calls issue when every linear has launches of its own (for
+// benchmark reporting).
 int lb_block_fwd_launches(const LbBlockDesc* d, const LbStreamCtx* c, int has_residual,
                           const LbTpCtx* tp);
 int lb_block_bwd_launches(const LbBlockDesc* d, const LbStreamCtx* c, const LbTpCtx* tp);
 
 // Returns 0, or the negative code of the first launcher that failed.
-int lb_block_fwd(const LbBlockDesc* d, const LbStreamCtx* c, const LbBlockIO* io);
-int lb_block_bwd(const LbBlockDesc* d, const LbStreamCtx* c, const LbBlockIO* io);
+int lb_block_fwd(const LbBlockDesc* d, const LbStreamCtx* c, LbBlockIO* io);
+int lb_block_bwd(const LbBlockDesc* d, const LbStreamCtx* c, LbBlockIO* io);
 
 }  // extern "C"

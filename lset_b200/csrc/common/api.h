@@ -54,6 +54,8 @@ int lb_attn_bwd(const void* dO, long long lddo, const void* q, long long ldq, co
                 int Hk, int hd, float softmax_scale, int causal, int* status, void* stream);
 
 // gemm/gemm_bf16.cu
+int lb_gemm_use_2cta(int v);
+int lb_gemm_2cta_pairs();
 int lb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda,
                  long long ldb, long long ldc, int a_mn, int b_mn, int out_fp32, int accumulate,
                  const void* bias, int splits, int bn, int* status, void* stream);

@@ -24,6 +24,7 @@
 
 #include "../common/ptx.cuh"
 #include "../common/tma_desc.h"
+#include "gemm_small.h"
 
 namespace lb {
 
@@ -978,6 +979,31 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, int M, int N, i
       N >= 256 && c_world <= 8)  // reduce-scatter by slots: rows stored into the owners' areas
     return lb_gemm_bf16_2cta_push(A, B, c_peers, c_world, c_rows_per_peer, M, N, K, lda, ldb, ldc,
                                   a_mn, b_mn, status, stream_);
+  // Few tokens: where cutting the product finer than a tile per pair is modelled to be faster.
+  if (use_2cta() && !scatter && bn == 0 && splits <= 1 && a_mn == out_fp32 &&
+      (out_fp32 ? accumulate != 0 && b_mn != 0 && bias == nullptr : !accumulate)) {
+    LbSmallGemm p = {};
+    p.A = A;
+    p.B[0] = B;
+    p.C[0] = C;
+    p.lda = lda;
+    p.ldb[0] = ldb;
+    p.ldc[0] = ldc;
+    p.M = M;
+    p.N = p.ext[0] = N;
+    p.K = K;
+    p.nparts = 1;
+    p.mode = kParallelN;
+    p.a_mn = a_mn;
+    p.b_mn = b_mn;
+    p.out_fp32 = out_fp32;
+    p.bias[0] = bias;
+    p.status = status;
+    p.stream = stream_;
+    const double cost = lb_gemm_small_plan(&p, &p.bn, &p.splits);
+    if (cost >= 0.0 && cost < lb_gemm_tile_cost(M, N, K, lb_gemm_2cta_pairs()))
+      return lb_gemm_small(&p);
+  }
   if (use_2cta() && bias == nullptr && !scatter && bn == 0 && M >= 256 && N >= 256) {
     int s2 = splits;
     if (s2 == 0) {

@@ -1,0 +1,635 @@
+// bf16 GEMM for products that a 256 x 256 tile per CTA pair leaves most of the chip idle on: few
+// tokens (a query, a small training batch) against weights of any size.
+//
+// Such a product is bound by how fast the weights reach the tensor cores, and one SM takes in
+// about 64 bytes a clock however few rows there are. So the work is cut until every SM has some:
+// 128 x BN tiles (BN 64 or 128), and the contraction of a tile split over a cluster of up to eight
+// CTAs. Each CTA of the cluster leaves its fp32 partial tile in its own shared memory; after a
+// cluster barrier every CTA sums a share of the tile over the cluster through distributed shared
+// memory, in rank order (no atomics: the result does not depend on timing), and stores it. One
+// tile per CTA, about 100 KB of shared memory, so that two CTAs share an SM and one's set-up and
+// epilogue run under the other's main loop.
+//
+//   warp 0      TMA producer          warp 1   tcgen05.mma issuer
+//   warps 2-5   accumulator -> shared memory -> (cluster sum) -> global memory
+//
+// Projections that share an input, an output or a token contraction (q, k, v; gate, up) are one
+// launch: see LbSmallGemm. The gated pair takes gate and up rows of the same features into one
+// tile and writes act(gate) * up from the epilogue.
+//
+// Measurements: see lb_gemm_small_plan.
+#include "gemm_small.h"
+
+#include <cuda_bf16.h>
+
+#include "../common/pdl.h"
+#include "../common/ptx.cuh"
+#include "../common/tma_desc.h"
+
+namespace lb {
+
+namespace {
+
+constexpr int BM = 128;
+constexpr int BK = 64;
+constexpr int kThreads = 192;
+constexpr int kMaxSplits = 8;
+
+struct SmallArgs {
+  int M, N;
+  int kb_total, splits;
+  int nparts, mode;
+  int ext[3];       // extent of each part
+  int first[3];     // first tile (kParallelN / M) or first k-block (kParallelK) of each part
+  int tiles_n;
+  void* C[3];
+  long long ldc[3];
+  const __nv_bfloat16* bias[3];
+  void* glu_h;
+  long long ld_h;
+  int glu_kind;
+  int b_ready;
+  int accs;         // accumulators: one per part of a kParallelK product, else one
+  int tmem_cols;
+  int* status;
+};
+
+template <int BN>
+struct SCfg {
+  static constexpr int A_BYTES = BM * BK * 2;
+  static constexpr int B_BYTES = BN * BK * 2;
+  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+  static constexpr int STAGES = BN == 64 ? 4 : 3;
+  static constexpr int PITCH = BN + 4;  // floats per row of the partial tile: 16-byte row accesses
+                                        // of eight lanes then fall into different banks
+  static constexpr int RING = STAGES * STAGE_BYTES;
+  static constexpr int SMEM_BYTES = RING + 1024 + 256;
+  static_assert(BM * PITCH * 4 <= RING, "the partial tile reuses the operand ring");
+};
+
+__device__ __forceinline__ uint32_t cta_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank) {
+  uint32_t out;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(addr), "r"(rank));
+  return out;
+}
+__device__ __forceinline__ float4 ld_cluster4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(addr)
+               : "memory");
+  return v;
+}
+
+__device__ __forceinline__ float act_of(int kind, float x) {
+  if (kind == 0) return x * (1.f / (1.f + __expf(-x)));
+  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
+  return 0.5f * x * (1.f + tanhf(k0 * (x + k1 * x * x * x)));
+}
+
+__device__ __forceinline__ float bf16_rn(float x) {
+  return __bfloat162float(__float2bfloat16_rn(x));
+}
+
+// Sum over the cluster of four consecutive floats at byte offset `off` of every partial tile.
+__device__ __forceinline__ float4 cluster_sum4(uint32_t base, uint32_t off, int splits) {
+  if (splits == 1) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"(base + off)
+                 : "memory");
+    return v;
+  }
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int s0 = 0; s0 < splits; s0 += 4) {  // all of a group's loads before its additions
+    float4 t[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      t[j] = s0 + j < splits ? ld_cluster4(map_rank(base, s0 + j) + off)
+                             : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      acc.x += t[j].x;
+      acc.y += t[j].y;
+      acc.z += t[j].z;
+      acc.w += t[j].w;
+    }
+  }
+  return acc;
+}
+
+template <int A_MN, int B_MN, int BN, typename OutT, int GLU>
+__global__ void __launch_bounds__(kThreads)
+    gemm_small_kernel(const __grid_constant__ CUtensorMap tmA,
+                      const __grid_constant__ CUtensorMap tmB0,
+                      const __grid_constant__ CUtensorMap tmB1,
+                      const __grid_constant__ CUtensorMap tmB2, SmallArgs g) {
+  using C = SCfg<BN>;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                             ~static_cast<uintptr_t>(1023));
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + C::RING);
+  uint64_t* empty = full + C::STAGES;
+  uint64_t* tfull = empty + C::STAGES;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tfull + 1);
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int S = g.splits;
+  const int rank = S > 1 ? int(cta_rank()) : 0;
+  const int tile = int(blockIdx.x) / S;
+  const int kb0 = rank * g.kb_total / S;
+  const int nkb = (rank + 1) * g.kb_total / S - kb0;   // >= 1: S <= kb_total
+
+  // tile -> part, origin in C, origin of the rows / columns read from A and B
+  const int tm = tile / g.tiles_n, tn = tile - tm * g.tiles_n;
+  int part = 0;
+  if (g.mode != kParallelK) {
+    const int t = g.mode == kParallelN ? tn : tm;
+    while (part + 1 < g.nparts && t >= g.first[part + 1]) ++part;
+  }
+  constexpr int kCols = GLU ? BN / 2 : BN;             // output columns of a tile
+  int m0 = tm * BM, n0 = tn * kCols, am0 = m0, m_ext = g.M, n_ext = g.N;
+  if (g.mode == kParallelN && !GLU) {
+    n0 = (tn - g.first[part]) * BN;
+    n_ext = g.ext[part];
+  } else if (g.mode == kParallelM) {
+    m0 = (tm - g.first[part]) * BM;
+    m_ext = g.ext[part];
+    am0 = m0;
+    for (int p = 0; p < part; ++p) am0 += g.ext[p];
+  }
+  if (GLU) n_ext = g.ext[0];
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < C::STAGES; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    mbar_init(tfull, 1);
+    mbar_fence_init();
+    tma_prefetch_desc(&tmA);
+    tma_prefetch_desc(&tmB0);
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, g.tmem_cols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ TMA producer
+    if (lane == 0) {
+      auto load_a = [&](int i) {
+        uint8_t* sa = smem + (i % C::STAGES) * C::STAGE_BYTES;
+        uint64_t* bar = &full[i % C::STAGES];
+        const int kc = (kb0 + i) * BK;
+        if (A_MN) {
+#pragma unroll
+          for (int c = 0; c < BM / 64; ++c)
+            tma_load_2d(sa + c * (BK * 128), &tmA, bar, am0 + 64 * c, kc);
+        } else {
+          tma_load_2d(sa, &tmA, bar, kc, am0);
+        }
+      };
+      auto load_b = [&](int i) {
+        uint8_t* sb = smem + (i % C::STAGES) * C::STAGE_BYTES + C::A_BYTES;
+        uint64_t* bar = &full[i % C::STAGES];
+        const int kb = kb0 + i;
+        int p = g.mode == kParallelN ? part : 0, kl = kb;
+        if (g.mode == kParallelK) {
+          while (p + 1 < g.nparts && kb >= g.first[p + 1]) ++p;
+          kl = kb - g.first[p];
+        }
+        const CUtensorMap* tb = p == 0 ? &tmB0 : (p == 1 ? &tmB1 : &tmB2);
+        const int kc = kl * BK;
+        if (GLU) {  // gate rows, then up rows of the same features
+          tma_load_2d(sb, &tmB0, bar, kc, n0);
+          tma_load_2d(sb + (BN / 2) * 128, &tmB1, bar, kc, n0);
+        } else if (B_MN) {
+#pragma unroll
+          for (int c = 0; c < BN / 64; ++c)
+            tma_load_2d(sb + c * (BK * 128), tb, bar, n0 + 64 * c, kc);
+        } else {
+          tma_load_2d(sb, tb, bar, kc, n0);
+        }
+      };
+      const int pre = nkb < C::STAGES ? nkb : C::STAGES;
+      for (int i = 0; i < pre; ++i) mbar_expect_tx(&full[i], C::STAGE_BYTES);
+      if (g.b_ready) {
+        for (int i = 0; i < pre; ++i) load_b(i);
+        pdl_wait();
+        for (int i = 0; i < pre; ++i) load_a(i);
+      } else {
+        pdl_wait();
+        for (int i = 0; i < pre; ++i) {
+          load_a(i);
+          load_b(i);
+        }
+      }
+      bool ok = true;
+      for (int i = pre; i < nkb; ++i) {
+        const int s = i % C::STAGES;
+        if (!mbar_wait(&empty[s], ((i / C::STAGES) & 1) ^ 1u)) {
+          report_status(g.status, kStatusTimeoutProducer);
+          ok = false;
+          break;
+        }
+        mbar_expect_tx(&full[s], C::STAGE_BYTES);
+        load_a(i);
+        load_b(i);
+      }
+      if (!ok) {
+        // copies already requested land within microseconds: a bounded grace period before exit
+        const unsigned long long t0 = globaltimer_ns();
+        while (globaltimer_ns() - t0 < 200000ull) {
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer
+    if (lane == 0) {
+      constexpr uint32_t idesc = umma_idesc_bf16(BM, BN, A_MN, B_MN);
+      bool ok = true;
+      int acc = 0;
+      for (int i = 0; i < nkb; ++i) {
+        const int s = i % C::STAGES;
+        bool fresh = i == 0;   // the first k-block of an accumulator overwrites it
+        if (acc + 1 < g.accs && i == g.first[acc + 1]) {
+          ++acc;
+          fresh = true;
+        }
+        if (!mbar_wait(&full[s], (i / C::STAGES) & 1)) {
+          report_status(g.status, kStatusTimeoutMma);
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t sa = smem_u32(smem + s * C::STAGE_BYTES);
+        const uint32_t sb = sa + C::A_BYTES;
+#pragma unroll
+        for (int k = 0; k < BK / 16; ++k) {
+          const uint64_t adesc = A_MN ? umma_smem_desc(sa + k * 2048, BK * 128, 1024)
+                                      : umma_smem_desc(sa + k * 32, 16, 1024);
+          const uint64_t bdesc = B_MN ? umma_smem_desc(sb + k * 2048, BK * 128, 1024)
+                                      : umma_smem_desc(sb + k * 32, 16, 1024);
+          umma_bf16(tmem_base + acc * BN, adesc, bdesc, idesc, (!fresh || k > 0) ? 1u : 0u);
+        }
+        umma_commit(&empty[s]);
+      }
+      if (ok) umma_commit(tfull);
+    }
+    __syncwarp();
+  } else {
+    // ------------------------------------------------------------------ accumulator -> shared memory
+    pdl_wait();  // also the only wait of a thread that writes global memory
+    pdl_trigger();
+    const int q = warp & 3;
+    const bool ok = mbar_wait(tfull, 0);
+    if (!ok && lane == 0) report_status(g.status, kStatusTimeoutEpilogue);
+    tc_fence_after();
+    if (__all_sync(0xffffffffu, ok) && m0 + q * 32 < m_ext) {
+      float* prow = reinterpret_cast<float*>(smem) + (q * 32 + lane) * C::PITCH;
+#pragma unroll
+      for (int c = 0; c < BN / 32; ++c) {
+        uint32_t r[32];
+        tmem_ld_32x32b_x32(tmem_base + (uint32_t(q * 32) << 16) + c * 32, r);
+        tmem_ld_wait();
+        if constexpr (B_MN && !A_MN) {
+          // the parts' products added up in bf16, one after the other: the roundings of launches
+          // that each add to the result in memory
+          for (int p = 1; p < g.accs; ++p) {
+            uint32_t t[32];
+            tmem_ld_32x32b_x32(tmem_base + (uint32_t(q * 32) << 16) + p * BN + c * 32, t);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              const float sum = bf16_rn(__uint_as_float(r[j])) + bf16_rn(__uint_as_float(t[j]));
+              r[j] = __float_as_uint(bf16_rn(sum));
+            }
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          *reinterpret_cast<float4*>(prow + c * 32 + 4 * j) =
+              make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
+                          __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
+      }
+    }
+    tc_fence_before();
+  }
+  if (S > 1)
+    cluster_sync_();
+  else
+    __syncthreads();
+
+  // ---------------------------------------------------------------------- sum and store
+  // (all 192 threads; after a failed wait the values are meaningless and the status word says so)
+  const int rows = min(BM, m_ext - m0);
+  const uint32_t base = smem_u32(smem);
+  if (sizeof(OutT) == 2) {
+    constexpr int VPR = kCols / 8;
+    const int total = rows * VPR;
+    const int per = (total + S - 1) / S;
+    const int hi = min(total, (rank + 1) * per);
+    for (int v = rank * per + int(threadIdx.x); v < hi; v += kThreads) {
+      const int row = v / VPR, c = (v % VPR) * 8;
+      if (n0 + c >= n_ext) continue;
+      const uint32_t off = uint32_t(row * C::PITCH + c) * 4u;
+      float4 a0 = cluster_sum4(base, off, S), a1 = cluster_sum4(base, off + 16u, S);
+      if (!GLU && g.bias[part] != nullptr) {
+        const uint4 bq = *reinterpret_cast<const uint4*>(g.bias[part] + n0 + c);
+        const float2 b0 = unpack_bf16x2(bq.x), b1 = unpack_bf16x2(bq.y);
+        const float2 b2 = unpack_bf16x2(bq.z), b3 = unpack_bf16x2(bq.w);
+        a0 = make_float4(a0.x + b0.x, a0.y + b0.y, a0.z + b1.x, a0.w + b1.y);
+        a1 = make_float4(a1.x + b2.x, a1.y + b2.y, a1.z + b3.x, a1.w + b3.y);
+      }
+      uint4 pk;
+      pk.x = pack_bf16x2(a0.x, a0.y);
+      pk.y = pack_bf16x2(a0.z, a0.w);
+      pk.z = pack_bf16x2(a1.x, a1.y);
+      pk.w = pack_bf16x2(a1.z, a1.w);
+      const long long grow = m0 + row;
+      if constexpr (GLU) {
+        const float4 u0 = cluster_sum4(base, off + BN / 2 * 4u, S);
+        const float4 u1 = cluster_sum4(base, off + BN / 2 * 4u + 16u, S);
+        uint4 pu;
+        pu.x = pack_bf16x2(u0.x, u0.y);
+        pu.y = pack_bf16x2(u0.z, u0.w);
+        pu.z = pack_bf16x2(u1.x, u1.y);
+        pu.w = pack_bf16x2(u1.z, u1.w);
+        if (g.C[0] != nullptr) {
+          *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(g.C[0]) + grow * g.ldc[0] +
+                                    n0 + c) = pk;
+          *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(g.C[1]) + grow * g.ldc[1] +
+                                    n0 + c) = pu;
+        }
+        const uint32_t gw[4] = {pk.x, pk.y, pk.z, pk.w}, uw[4] = {pu.x, pu.y, pu.z, pu.w};
+        uint32_t hw[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 gv = unpack_bf16x2(gw[j]), uv = unpack_bf16x2(uw[j]);
+          hw[j] = pack_bf16x2(act_of(g.glu_kind, gv.x) * uv.x, act_of(g.glu_kind, gv.y) * uv.y);
+        }
+        *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(g.glu_h) + grow * g.ld_h + n0 +
+                                  c) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+      } else {
+        *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(g.C[part]) +
+                                  grow * g.ldc[part] + n0 + c) = pk;
+      }
+    }
+  } else {
+    constexpr int VPR = kCols / 4;
+    const int total = rows * VPR;
+    const int per = (total + S - 1) / S;
+    const int hi = min(total, (rank + 1) * per);
+    for (int v = rank * per + int(threadIdx.x); v < hi; v += kThreads) {
+      const int row = v / VPR, c = (v % VPR) * 4;
+      if (n0 + c >= n_ext) continue;
+      const float4 a = cluster_sum4(base, uint32_t(row * C::PITCH + c) * 4u, S);
+      asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(
+                       reinterpret_cast<float*>(g.C[part]) + (m0 + row) * g.ldc[part] + n0 + c),
+                   "f"(a.x), "f"(a.y), "f"(a.z), "f"(a.w)
+                   : "memory");
+    }
+  }
+  // nobody gives its shared memory back while a peer may still read it
+  if (S > 1)
+    cluster_sync_();
+  else
+    __syncthreads();
+  if (warp == 1) tmem_dealloc(tmem_base, g.tmem_cols);
+}
+
+int small_sms() {
+  static int n = 0;
+  if (n == 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
+      n = 148;
+  }
+  return n;
+}
+
+inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
+
+int kblocks(const LbSmallGemm* p) {
+  if (p->mode != kParallelK) return ceil_div(p->K, BK);
+  int n = 0;
+  for (int i = 0; i < p->nparts; ++i) n += ceil_div(p->ext[i], BK);
+  return n;
+}
+
+int tiles_along(const LbSmallGemm* p, int mode, int whole, int tile) {
+  if (p->mode != mode) return ceil_div(whole, tile);
+  int n = 0;
+  for (int i = 0; i < p->nparts; ++i) n += ceil_div(p->ext[i], tile);
+  return n;
+}
+
+int accumulators(const LbSmallGemm* p) { return p->mode == kParallelK ? p->nparts : 1; }
+
+int count_tiles(const LbSmallGemm* p, int bn, int* tiles_n) {
+  const int tm = tiles_along(p, kParallelM, p->M, BM);
+  const int tn = p->glu_h != nullptr ? ceil_div(p->ext[0], bn / 2)
+                                     : tiles_along(p, kParallelN, p->N, bn);
+  *tiles_n = tn;
+  return tm * tn;
+}
+
+bool shape_ok(const LbSmallGemm* p) {
+  if (p->M <= 0 || p->N <= 0 || p->K <= 0 || p->nparts < 1 || p->nparts > 3) return false;
+  if (p->lda & 7) return false;
+  for (int i = 0; i < p->nparts; ++i) {
+    if (p->ext[i] <= 0 || (p->ext[i] & 7)) return false;
+    if (p->mode != kParallelM && (p->ldb[i] & 7)) return false;
+    if (p->mode == kParallelK && (p->ext[i] % BK) != 0) return false;  // a k-block has one weight
+  }
+  if (p->mode == kParallelM && (p->ldb[0] & 7)) return false;
+  if (p->mode != kParallelN && (p->N & 7)) return false;
+  for (int i = 0; i < (p->mode == kParallelK ? 1 : p->nparts); ++i)
+    if (p->C[i] != nullptr && (p->ldc[i] & (p->out_fp32 ? 3 : 7))) return false;
+  if (p->glu_h != nullptr &&
+      (p->mode != kParallelN || p->nparts != 2 || p->ext[0] != p->ext[1] || p->a_mn || p->b_mn ||
+       p->out_fp32 || (p->ld_h & 7)))
+    return false;
+  if (p->a_mn && !p->b_mn) return false;        // not a product of a linear layer
+  if (p->out_fp32 != (p->a_mn ? 1 : 0)) return false;
+  for (int i = 0; i < p->nparts; ++i)
+    if (p->bias[i] != nullptr &&
+        (p->mode != kParallelN || p->glu_h != nullptr || p->out_fp32 ||
+         (reinterpret_cast<uintptr_t>(p->bias[i]) & 15u) != 0))
+      return false;
+  return true;
+}
+
+template <int A_MN, int B_MN, int BN, typename OutT, int GLU>
+int launch_small(const CUtensorMap& tA, const CUtensorMap* tB, const SmallArgs& g, int grid,
+                 cudaStream_t st) {
+  auto kern = gemm_small_kernel<A_MN, B_MN, BN, OutT, GLU>;
+  static bool configured = false;
+  if (!configured) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             SCfg<BN>::SMEM_BYTES) != cudaSuccess)
+      return -10;
+    configured = true;
+  }
+  return launch_pdl(kern, dim3(grid), dim3(kThreads), SCfg<BN>::SMEM_BYTES, st, pdl_enabled(),
+                    g.splits, tA, tB[0], tB[1], tB[2], g);
+}
+
+template <int BN>
+int dispatch(const LbSmallGemm* p, const CUtensorMap& tA, const CUtensorMap* tB, const SmallArgs& g,
+             int grid, cudaStream_t st) {
+  if (p->glu_h != nullptr) return launch_small<0, 0, BN, __nv_bfloat16, 1>(tA, tB, g, grid, st);
+  if (p->a_mn) return launch_small<1, 1, BN, float, 0>(tA, tB, g, grid, st);
+  if (p->b_mn) return launch_small<0, 1, BN, __nv_bfloat16, 0>(tA, tB, g, grid, st);
+  return launch_small<0, 0, BN, __nv_bfloat16, 0>(tA, tB, g, grid, st);
+}
+
+}  // namespace
+}  // namespace lb
+
+using namespace lb;
+
+// Microseconds, fitted to measurements of 13 products of transformer blocks (H 768 and 1024) at 32
+// to 2048 tokens with both tile widths and all splits; the choice it leads to is within 10 % of the
+// best of the eight for all but a few of them. W waves of two CTAs per SM pay for launch, set-up,
+// pipeline fill and the store of the tile, a split for the cluster's barriers; a k-block costs what
+// the SM needs to take it in, but no less than its share of the latency of the loads in flight.
+//   tokens x N x K                     tile kernels      this kernel (us, L2 flushed)
+//   32 x (2048, 1024, 1024) x 1024     37.8 (3 launches) 12.7
+//   32 x 1024 x 3072                   26.2              12.7
+//   660 x (768, 768, 768) x 768        39.8 (3 launches) 12.7
+//   1024 x (3072, 3072) x 1024         31.7 (2 launches) 26.3
+//   1024 x 1024 x (2048, 1024, 1024)   48.0 (3 launches) 23.3
+//   (3072, 3072) x 1024 x 1024 (grad)  35.2 (2 launches) 28.9
+// (about 5 us of each are the measurement's own).
+extern "C" double lb_gemm_small_plan(const LbSmallGemm* p, int* bn_out, int* splits_out) {
+  if (!shape_ok(p)) return -1.0;
+  const int sms = small_sms();
+  const int kb = kblocks(p);
+  const int a_rows = p->M < BM && !p->a_mn ? p->M : BM;
+  // Split only where the caller takes sums in another order (in a training step a different
+  // rounding of one layer shows in the loss after the next update): an unsplit product has the bits
+  // that the tile kernels give. Nothing is lost for the weight gradients, which are never faster split.
+  const int max_splits = p->a_mn || !p->may_split || accumulators(p) > 1 ? 1 : kMaxSplits;
+  double best = 1e30;
+  for (int bn = 64; bn <= 128; bn += 64) {
+    if (accumulators(p) > 2 && bn > 64) break;   // two CTAs per SM have 256 columns each
+    int tn;
+    const int tiles = count_tiles(p, bn, &tn);
+    const double stages = bn == 64 ? SCfg<64>::STAGES : SCfg<128>::STAGES;
+    for (int s = 1; s <= max_splits && s <= kb; s *= 2) {
+      const int ctas = tiles * s;
+      const double waves = ceil_div(ctas, 2 * sms);
+      const double per_sm = ctas < sms ? 1.0 : (s == 1 ? ceil_div(ctas, sms) : double(ctas) / sms);
+      const double store = (p->out_fp32 ? 1.8 : 2.6) * a_rows * bn / 8192.0;
+      const double split = (s > 1 ? 2.3 : 0.0) + (s > 2 ? 0.7 : 0.0) + (s > 4 ? 1.8 : 0.0);
+      const double block = per_sm * (a_rows + bn) * 2.0, latency = 1400.0 / stages;
+      const double cost = 2.0 + waves * (1.1 + split + store) +
+                          ceil_div(kb, s) * (block > latency ? block : latency) / 1900.0;
+      if (cost < best) {
+        best = cost;
+        *bn_out = bn;
+        *splits_out = s;
+      }
+    }
+  }
+  return best;
+}
+
+// The same for one product of lb_gemm_bf16_2cta: measured 14.5 us (of them 5 the measurement's) and
+// a 256 x 256 tile per pair and wave at 0.27 us a 64-deep k-block.
+extern "C" double lb_gemm_tile_cost(int M, int N, int K, int pairs) {
+  const double tiles = double(ceil_div(M, 256)) * ceil_div(N, 256);
+  const double waves = tiles < pairs ? 1.0 : double(ceil_div(int(tiles), pairs));
+  const int kb = ceil_div(K, BK);
+  return 10.0 + waves * kb * 0.27;
+}
+
+extern "C" int lb_gemm_small(const LbSmallGemm* p) {
+  if (p->M <= 0 || p->N <= 0) return 0;
+  if (!shape_ok(p)) return -3;
+  int bn = p->bn, splits = p->splits;
+  if (bn != 64 && bn != 128) bn = 0;
+  if (bn == 0 || splits <= 0) {
+    int b2 = 64, s2 = 1;
+    lb_gemm_small_plan(p, &b2, &s2);
+    if (bn == 0) bn = b2;
+    if (splits <= 0) splits = s2;
+  }
+  if (splits != 1 && splits != 2 && splits != 4 && splits != 8) return -3;
+  const int kb = kblocks(p);
+  while (splits > kb) splits /= 2;
+  const int accs = accumulators(p);
+  if (accs > 1) splits = 1;
+
+  CUtensorMap tA, tB[3];
+  int rc;
+  int a_inner = p->a_mn ? p->M : p->K;
+  rc = p->a_mn ? make_tmap_2d(&tA, p->A, 2, (uint64_t)a_inner, (uint64_t)p->K,
+                              (uint64_t)p->lda * 2, 64, BK, true)
+               : make_tmap_2d(&tA, p->A, 2, (uint64_t)a_inner, (uint64_t)p->M,
+                              (uint64_t)p->lda * 2, BK, BM, true);
+  if (rc) return rc;
+  const int nb = p->mode == kParallelM ? 1 : p->nparts;
+  for (int i = 0; i < nb; ++i) {
+    const int n = p->mode == kParallelN ? p->ext[i] : p->N;
+    const int k = p->mode == kParallelK ? p->ext[i] : p->K;
+    rc = p->b_mn ? make_tmap_2d(&tB[i], p->B[i], 2, (uint64_t)n, (uint64_t)k,
+                                (uint64_t)p->ldb[i] * 2, 64, BK, true)
+                 : make_tmap_2d(&tB[i], p->B[i], 2, (uint64_t)k, (uint64_t)n,
+                                (uint64_t)p->ldb[i] * 2, BK, p->glu_h != nullptr ? bn / 2 : bn,
+                                true);
+    if (rc) return rc;
+  }
+  for (int i = nb; i < 3; ++i) tB[i] = tB[0];
+
+  SmallArgs g{};
+  g.M = p->M;
+  g.N = p->N;
+  g.kb_total = kb;
+  g.splits = splits;
+  g.nparts = p->nparts;
+  g.mode = p->mode;
+  const int unit = p->mode == kParallelN ? bn : (p->mode == kParallelK ? BK : BM);
+  int at = 0;
+  for (int i = 0; i < 3; ++i) {
+    g.first[i] = at;
+    if (i < p->nparts) {
+      g.ext[i] = p->ext[i];
+      g.C[i] = p->C[i];
+      g.bias[i] = static_cast<const __nv_bfloat16*>(p->bias[i]);
+      g.ldc[i] = p->ldc[i];
+      at += ceil_div(p->ext[i], unit);
+    }
+  }
+  const int tiles = count_tiles(p, bn, &g.tiles_n);
+  g.glu_h = p->glu_h;
+  g.ld_h = p->ld_h;
+  g.glu_kind = p->glu_kind;
+  g.b_ready = p->b_ready && pdl_enabled();
+  g.accs = accs;
+  g.tmem_cols = bn;
+  while (g.tmem_cols < accs * bn) g.tmem_cols *= 2;
+  g.status = p->status;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(p->stream);
+  const int grid = tiles * splits;
+  return bn == 64 ? dispatch<64>(p, tA, tB, g, grid, st) : dispatch<128>(p, tA, tB, g, grid, st);
+}

@@ -63,7 +63,8 @@ class LbStreamCtx(ctypes.Structure):
                 ("plan_f", _ip), ("cap_f", ctypes.c_int),
                 ("plan_q", _ip), ("cap_q", ctypes.c_int), ("plan_kv", _ip),
                 ("cap_kv", ctypes.c_int), ("status", _ip), ("norm_scratch", _fp),
-                ("rope_scratch", _fp), ("wg_tmp", _fp), ("stream", _vp)]
+                ("rope_scratch", _fp), ("wg_tmp", _fp), ("stream", _vp),
+                ("may_split", ctypes.c_int)]
 
 
 class LbTpCtx(ctypes.Structure):
@@ -78,7 +79,7 @@ class LbTpCtx(ctypes.Structure):
 class LbBlockIO(ctypes.Structure):
     _fields_ = [("branch", _vp), ("residual", _vp), ("out", _vp), ("res_out", _vp),
                 ("saved", _vp), ("d_out", _vp), ("d_res_out", _vp), ("dx", _vp), ("work", _vp),
-                ("tp", _vp)]
+                ("tp", _vp), ("fewer_launches", ctypes.c_int)]
 
 
 _lib = None
@@ -361,12 +362,15 @@ def _tp_advance(state) -> None:
 
 
 # --------------------------------------------------------------------------- stream context
-def _stream_struct(ctx, plan: BlockPlan, device) -> LbStreamCtx:
+def _stream_struct(ctx, plan: BlockPlan, device, training: bool) -> LbStreamCtx:
     """The per-forward struct, cached on the Python stream context (all blocks share it). The
     backward's tile lists are built for a pass that records gradients only."""
     d = plan.desc
     grad = torch.is_grad_enabled()
-    key = ("_lb", grad, d.hd, d.Hq // d.Hk, plan.rope[1], id(plan.rope[2]))
+    # a model in training mode keeps one order of summation, with and without gradients: what an
+    # activation checkpoint recomputes has the bits of the first pass
+    may_split = not grad and not training
+    key = ("_lb", grad, may_split, d.hd, d.Hq // d.Hk, plan.rope[1], id(plan.rope[2]))
     hit = ctx.tables.get(key)
     if hit is not None:
         return hit
@@ -390,6 +394,7 @@ def _stream_struct(ctx, plan: BlockPlan, device) -> LbStreamCtx:
                              device).data_ptr()
     s.wg_tmp = scratch("qk_norm_wgrad", 2 * d.hd, device).data_ptr()
     s.stream = 0
+    s.may_split = int(may_split)
     # keep the tensors the struct points to alive as long as the struct
     s._keep = (cos, sin, ctx.pos, ap, ptf, ptq, ptk)
     ctx.tables[key] = s
@@ -431,7 +436,7 @@ class _BlockFn(torch.autograd.Function):
             n = lib.lb_block_fwd_launches(ctypes.addressof(d), ctypes.addressof(sctx), int(has_res),
                                           tp_ptr)
             plan._launches[("f", sctx.packed)] = n
-        nv.count_launch(n)
+        nv.count_launch(n - io.fewer_launches)
         ctx.save_for_backward(branch, residual, saved, res_out)
         ctx.plan, ctx.sctx, ctx.stream_ctx = plan, sctx, stream_ctx
         return out, res_out
@@ -486,7 +491,7 @@ class _BlockFn(torch.autograd.Function):
         if n is None:
             n = lib.lb_block_bwd_launches(ctypes.addressof(d), ctypes.addressof(sctx), tp_ptr)
             plan._launches[key] = n
-        nv.count_launch(n)
+        nv.count_launch(n - io.fewer_launches)
         pgrads = tuple(None if t is None else t.to(p.dtype) for t, p in zip(temps, plan.params))
         return (dx, dx if residual is not None else None, None, None, None) + pgrads
 
@@ -494,5 +499,5 @@ class _BlockFn(torch.autograd.Function):
 def run(block, branch, residual, ctx):
     """``(mlp_out, residual_out)`` of one decoder block, as ``DecoderBlock.forward`` returns them."""
     plan = plan_of(block)
-    sctx = _stream_struct(ctx, plan, branch.device)
+    sctx = _stream_struct(ctx, plan, branch.device, block.training)
     return _BlockFn.apply(branch, residual, plan, sctx, ctx, *plan.params)

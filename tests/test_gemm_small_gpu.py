@@ -1,0 +1,161 @@
+"""The GEMM for few tokens (``lb_gemm_small``): one to three weights side by side, along the output
+columns, the contraction or the output rows, split over clusters or not, against fp64 products."""
+import ctypes
+
+import pytest
+import torch
+
+from lset_b200.ops import _native as nv
+
+pytestmark = pytest.mark.gpu
+_vp, _ll, _ci = ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int
+N_PARTS, K_PARTS, M_PARTS = 0, 1, 2
+
+
+class SmallGemm(ctypes.Structure):      # LbSmallGemm of csrc/gemm/gemm_small.h
+    _fields_ = [("A", _vp), ("B", _vp * 3), ("C", _vp * 3), ("lda", _ll), ("ldb", _ll * 3),
+                ("ldc", _ll * 3), ("M", _ci), ("N", _ci), ("K", _ci), ("ext", _ci * 3),
+                ("nparts", _ci), ("mode", _ci), ("a_mn", _ci), ("b_mn", _ci), ("out_fp32", _ci),
+                ("bias", _vp * 3), ("glu_h", _vp), ("ld_h", _ll), ("glu_kind", _ci),
+                ("b_ready", _ci), ("may_split", _ci), ("bn", _ci), ("splits", _ci), ("status", _vp), ("stream", _vp)]
+
+
+def _call(a, bs, cs, M, N, K, ext, mode, a_mn=0, b_mn=0, fp32=0, bias=(), h=None, bn=0, splits=0):
+    g = SmallGemm()
+    g.A, g.lda = a.data_ptr(), a.stride(0)
+    for i, b in enumerate(bs):
+        g.B[i], g.ldb[i] = b.data_ptr(), b.stride(0)
+    for i, c in enumerate(cs):
+        g.C[i], g.ldc[i] = c.data_ptr(), c.stride(0)
+    for i, e in enumerate(ext):
+        g.ext[i] = e
+    for i, b in enumerate(bias):
+        g.bias[i] = b.data_ptr()
+    g.M, g.N, g.K, g.nparts, g.mode = M, N, K, len(ext), mode
+    g.a_mn, g.b_mn, g.out_fp32, g.bn, g.splits = a_mn, b_mn, fp32, bn, splits
+    if h is not None:
+        g.glu_h, g.ld_h = h.data_ptr(), h.stride(0)
+    g.status, g.stream = nv.status_word(a.device).data_ptr(), nv.stream_ptr()
+    return nv.load().lb_gemm_small(ctypes.byref(g))
+
+
+def _rand(*shape):
+    return torch.randn(*shape, device="cuda").to(torch.bfloat16)
+
+
+def _rel(x, ref):
+    return ((x.double() - ref).norm() / ref.norm()).item()
+
+
+def _columns(c, ext):
+    at, out = 0, []
+    for e in ext:
+        out.append(c[:, at:at + e])
+        at += e
+    return out
+
+
+FORMS = [(bn, s) for bn in (64, 128) for s in (1, 2, 8)] + [(0, 0)]
+ROUND = 2 ** -8   # one rounding to bf16 (2^-9 at most, less in the 2-norm)
+
+
+@pytest.mark.parametrize("T", [1, 33, 128, 257])
+@pytest.mark.parametrize("ext,K", [([72], 64), ([128, 64, 136], 200), ([768, 768, 768], 2048)])
+def test_parts_along_the_columns(T, ext, K):
+    torch.manual_seed(T)
+    a, bs, bias = _rand(T, K), [_rand(e, K) for e in ext], [_rand(e) for e in ext]
+    ref = a.double() @ torch.cat(bs).double().t()
+    for bn, s in FORMS:
+        c = torch.full((T, sum(ext)), float("nan"), device="cuda", dtype=torch.bfloat16)
+        assert _call(a, bs, _columns(c, ext), T, sum(ext), K, ext, N_PARTS, bn=bn, splits=s) == 0
+        assert _rel(c, ref) < ROUND, (bn, s)
+        assert _call(a, bs, _columns(c, ext), T, sum(ext), K, ext, N_PARTS, bias=bias, bn=bn,
+                     splits=s) == 0
+        assert _rel(c, ref + torch.cat(bias).double()) < ROUND, (bn, s)
+    nv.check_status()
+
+
+@pytest.mark.parametrize("T", [1, 128, 257])
+@pytest.mark.parametrize("ext,N", [([64], 72), ([128, 64, 192], 200), ([3072, 3072], 1024)])
+def test_parts_along_the_contraction(T, ext, N):
+    torch.manual_seed(T)
+    a, bs = _rand(T, sum(ext)), [_rand(e, N) for e in ext]
+    ref = a.double() @ torch.cat(bs).double()
+    for bn, s in FORMS:
+        c = torch.full((T, N), float("nan"), device="cuda", dtype=torch.bfloat16)
+        assert _call(a, bs, [c], T, N, sum(ext), ext, K_PARTS, b_mn=1, bn=bn, splits=s) == 0
+        # every product and every sum is rounded once
+        assert _rel(c, ref) < (2 * len(ext) - 1) * ROUND, (bn, s)
+        apart = [torch.empty(T, N, device="cuda", dtype=torch.bfloat16) for _ in ext]
+        for x, b, e, out in zip(_columns(a, ext), bs, ext, apart):
+            assert _call(x, [b], [out], T, N, e, [N], N_PARTS, b_mn=1, bn=bn, splits=1) == 0
+        for x in apart[1:]:
+            apart[0] += x
+        assert torch.equal(c, apart[0]), (bn, s)
+    nv.check_status()
+
+
+@pytest.mark.parametrize("T", [1, 64, 300])
+@pytest.mark.parametrize("ext,N", [([72], 64), ([128, 64, 136], 200)])
+def test_parts_along_the_rows_add_to_fp32(T, ext, N):
+    torch.manual_seed(T)
+    a, b = _rand(T, sum(ext)), _rand(T, N)
+    ref = a.double().t() @ b.double() + 3
+    for bn, s in FORMS:
+        cs = [torch.full((e, N), 3.0, device="cuda") for e in ext]
+        assert _call(a, [b], cs, sum(ext), N, T, ext, M_PARTS, a_mn=1, b_mn=1, fp32=1, bn=bn,
+                     splits=s) == 0
+        # fp32 sums of at most 300 products, one more addition
+        assert _rel(torch.cat(cs), ref) < 300 ** 0.5 * 2 ** -23, (bn, s)
+    nv.check_status()
+
+
+@pytest.mark.parametrize("T,I", [(1, 40), (130, 1152), (32, 3072)])
+@pytest.mark.parametrize("keep", [True, False])
+def test_gated_pair(T, I, keep):
+    K = 1024
+    torch.manual_seed(I)
+    a, w = _rand(T, K), [_rand(I, K) * 0.05, _rand(I, K) * 0.05]
+    gate, up = (a.double() @ x.double().t() for x in w)
+    want = torch.nn.functional.silu(gate) * up
+    for bn, s in FORMS:
+        gu = torch.full((T, 2 * I), float("nan"), device="cuda", dtype=torch.bfloat16)
+        h = torch.full((T, I), float("nan"), device="cuda", dtype=torch.bfloat16)
+        assert _call(a, w, [gu[:, :I], gu[:, I:]] if keep else [], T, 2 * I, K, [I, I], N_PARTS,
+                     h=h, bn=bn, splits=s) == 0
+        # both factors are rounded (2^-9 each, the gate's amplified by at most 1.1 through SiLU),
+        # then their product
+        assert _rel(h, want) < 2 * ROUND, (bn, s)
+        if keep:
+            assert _rel(gu, torch.cat([gate, up], 1)) < ROUND
+        else:
+            assert torch.isnan(gu).all()
+    nv.check_status()
+
+
+def test_shapes_it_does_not_take():
+    a, b, c = _rand(8, 64), _rand(16, 64), _rand(8, 16)
+    assert _call(a, [b], [c], 8, 12, 64, [12], N_PARTS) == -3          # columns not a multiple of 8
+    assert _call(a, [_rand(40, 16), _rand(24, 16)], [c], 8, 16, 64, [40, 24], K_PARTS,
+                 b_mn=1) == -3                                          # a k-block over two weights
+    assert _call(a, [b], [c.float()], 8, 16, 64, [16], N_PARTS, fp32=1) == -3
+
+
+@pytest.mark.parametrize("T,N,K", [(40, 1024, 2048), (304, 768, 3072), (1000, 2048, 1024)])
+@pytest.mark.parametrize("a_mn,b_mn", [(0, 0), (0, 1), (1, 1)])
+def test_unsplit_it_has_the_bits_of_the_tile_kernels(T, N, K, a_mn, b_mn):
+    from lset_b200.ops.gemm import matmul_abt
+
+    torch.manual_seed(T)
+    a = _rand(K, T) if a_mn else _rand(T, K)
+    b = _rand(K, N) if b_mn else _rand(N, K)
+    dtype = torch.float32 if a_mn else torch.bfloat16
+    before = nv.load().lb_gemm_use_2cta(-1)
+    out = {}
+    for on in (0, 1):
+        nv.load().lb_gemm_use_2cta(on)
+        out[on] = torch.zeros(T, N, device="cuda", dtype=dtype)
+        matmul_abt(a, b, a_mn=bool(a_mn), b_mn=bool(b_mn), out=out[on], accumulate=bool(a_mn))
+    nv.load().lb_gemm_use_2cta(before)
+    nv.check_status()
+    assert torch.equal(out[0], out[1])
