@@ -167,9 +167,9 @@ class _VarlenAttn(torch.autograd.Function):
     def backward(ctx, do):
         q, k, v, o, lse = ctx.saved_tensors
         do = do if do.is_contiguous() else do.contiguous()
-        dq = torch.empty(q.shape, dtype=q.dtype, device=q.device)
-        dk = torch.empty(k.shape, dtype=k.dtype, device=k.device)
-        dv = torch.empty(v.shape, dtype=v.dtype, device=v.device)
+        # rows of padding are written by no kernel
+        empty = torch.empty if ctx.plan.cu_seqlens is not None else torch.zeros
+        dq, dk, dv = (empty(t.shape, dtype=t.dtype, device=t.device) for t in (q, k, v))
         _native_bwd(do, q, k, v, o, lse, ctx.plan, ctx.causal, ctx.scale, dq, dk, dv)
         return dq, dk, dv, None, None, None
 

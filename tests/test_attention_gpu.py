@@ -134,3 +134,24 @@ def test_forward_tile_edges(Hq, Hk, hd, causal, scale):
     assert ((o.float() - ref).norm() / ref.norm()).item() < 2 ** -8
     again = varlen_attention(q, k, v, plan, causal, scale)   # the work counter was put back
     assert torch.equal(o, again)
+
+
+def test_padded_plan_clears_the_gradient_rows_of_padding():
+    """Rows of a padded batch that belong to no sequence get zero gradients, not what the buffers
+    held before: the projections sum over all rows."""
+    B, S, H, hd = 3, 96, 2, 64
+    mask = torch.zeros(B, S, dtype=torch.long, device="cuda")
+    for i, n in enumerate((40, 7, 96)):
+        mask[i, :n] = 1
+    plan = AttnPlan.from_mask(mask)
+    q, k, v = (torch.randn(B * S, H, hd, device="cuda").to(torch.bfloat16).requires_grad_()
+               for _ in range(3))
+    o = varlen_attention(q, k, v, plan, False)
+    junk = [torch.full((B * S, H, hd), float("nan"), device="cuda", dtype=torch.bfloat16)
+            for _ in range(8)]
+    del junk
+    o.backward(torch.randn_like(o))
+    nv.check_status()
+    pad = mask.reshape(-1) == 0
+    for t in (q, k, v):
+        assert not t.grad[pad].any() and t.grad[~pad].abs().max() > 0
