@@ -47,7 +47,6 @@ struct SmallArgs {
   const __nv_bfloat16* bias[3];
   void* glu_h;
   long long ld_h;
-  int glu_kind;
   int b_ready;
   int accs;         // accumulators: one per part of a kParallelK product, else one
   int tmem_cols;
@@ -90,10 +89,16 @@ __device__ __forceinline__ float4 ld_cluster4(uint32_t addr) {
   return v;
 }
 
-__device__ __forceinline__ float act_of(int kind, float x) {
-  if (kind == 0) return x * (1.f / (1.f + __expf(-x)));
-  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-  return 0.5f * x * (1.f + tanhf(k0 * (x + k1 * x * x * x)));
+// The values of the stand-alone activation kernel (row/act.cu): the same bits. GLU: 1 = SiLU, 2 =
+// tanh-GELU.
+template <int GLU>
+__device__ __forceinline__ float act_of(float x) {
+  if constexpr (GLU == 1) {
+    return x * __frcp_rn(1.f + __expf(-x));
+  } else {
+    const float k0 = 0.7978845608028654f, k1 = 0.044715f;
+    return 0.5f * x * (1.f + tanhf(k0 * (x + k1 * x * x * x)));
+  }
 }
 
 __device__ __forceinline__ float bf16_rn(float x) {
@@ -383,7 +388,7 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const float2 gv = unpack_bf16x2(gw[j]), uv = unpack_bf16x2(uw[j]);
-          hw[j] = pack_bf16x2(act_of(g.glu_kind, gv.x) * uv.x, act_of(g.glu_kind, gv.y) * uv.y);
+          hw[j] = pack_bf16x2(act_of<GLU>(gv.x) * uv.x, act_of<GLU>(gv.y) * uv.y);
         }
         *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(g.glu_h) + grow * g.ld_h + n0 +
                                   c) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
@@ -496,7 +501,9 @@ int launch_small(const CUtensorMap& tA, const CUtensorMap* tB, const SmallArgs& 
 template <int BN>
 int dispatch(const LbSmallGemm* p, const CUtensorMap& tA, const CUtensorMap* tB, const SmallArgs& g,
              int grid, cudaStream_t st) {
-  if (p->glu_h != nullptr) return launch_small<0, 0, BN, __nv_bfloat16, 1>(tA, tB, g, grid, st);
+  if (p->glu_h != nullptr)
+    return p->glu_kind == 0 ? launch_small<0, 0, BN, __nv_bfloat16, 1>(tA, tB, g, grid, st)
+                            : launch_small<0, 0, BN, __nv_bfloat16, 2>(tA, tB, g, grid, st);
   if (p->a_mn) return launch_small<1, 1, BN, float, 0>(tA, tB, g, grid, st);
   if (p->b_mn) return launch_small<0, 1, BN, __nv_bfloat16, 0>(tA, tB, g, grid, st);
   return launch_small<0, 0, BN, __nv_bfloat16, 0>(tA, tB, g, grid, st);
@@ -623,7 +630,6 @@ extern "C" int lb_gemm_small(const LbSmallGemm* p) {
   const int tiles = count_tiles(p, bn, &g.tiles_n);
   g.glu_h = p->glu_h;
   g.ld_h = p->ld_h;
-  g.glu_kind = p->glu_kind;
   g.b_ready = p->b_ready && pdl_enabled();
   g.accs = accs;
   g.tmem_cols = bn;

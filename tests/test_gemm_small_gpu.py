@@ -159,3 +159,28 @@ def test_unsplit_it_has_the_bits_of_the_tile_kernels(T, N, K, a_mn, b_mn):
     nv.load().lb_gemm_use_2cta(before)
     nv.check_status()
     assert torch.equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("T,I,K", [(256, 256, 64), (257, 264, 200), (700, 1160, 1024)])
+@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("keep", [True, False])
+def test_gated_pair_on_cta_pairs(T, I, K, kind, keep):
+    """``lb_gemm_glu_2cta`` has the bits of the two products and the activation kernel."""
+    from lset_b200.ops.gemm import matmul_abt
+
+    torch.manual_seed(T)
+    lib, a, w = nv.load(), _rand(T, K), _rand(2 * I, K) * 0.1
+    gu = matmul_abt(a, w)
+    want = torch.empty(T, I, device="cuda", dtype=torch.bfloat16)
+    stream = _vp(nv.stream_ptr())
+    assert lib.lb_glu_fwd(_ci(kind), _vp(gu.data_ptr()), _vp(gu.data_ptr() + 2 * I), _ll(2 * I),
+                          _vp(want.data_ptr()), _ll(I), _ll(T), _ci(I), stream) == 0
+    got, h = torch.full_like(gu, float("nan")), torch.full_like(want, float("nan"))
+    ptr = got.data_ptr() if keep else 0
+    assert lib.lb_gemm_glu_2cta(
+        _vp(a.data_ptr()), _vp(w.data_ptr()), _vp(w.data_ptr() + 2 * I * K), _vp(ptr),
+        _vp(ptr + 2 * I if keep else 0), _vp(h.data_ptr()), _ci(T), _ci(I), _ci(K), _ll(K), _ll(K),
+        _ll(2 * I), _ll(I), _ci(kind), _vp(nv.status_word(a.device).data_ptr()), stream) == 0
+    nv.check_status()
+    assert torch.equal(h, want)
+    assert torch.equal(got, gu) if keep else torch.isnan(got).all()
