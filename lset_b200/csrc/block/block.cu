@@ -730,3 +730,183 @@ extern "C" int lb_block_bwd(const LbBlockDesc* d, const LbStreamCtx* c, LbBlockI
   io->fewer_launches = t_fewer;
   return rc;
 }
+
+// ---- encoder block ---------------------------------------------------------------------------
+namespace {
+
+struct EncSaved {
+  __nv_bfloat16 *qkv, *o, *nr1, *y1, *u, *g, *nr2, *tmp;
+  float *lse, *mean1, *rstd1, *mean2, *rstd2;
+};
+
+EncSaved carve_enc_saved(const LbEncoderDesc* d, int T, Arena& a) {
+  EncSaved s{};
+  const size_t t = (size_t)T;
+  s.qkv = a.bf(t * d->qkv.width);
+  s.o = a.bf(t * d->H);
+  s.lse = a.f32(t * d->heads);
+  s.nr1 = a.bf(t * d->H);
+  s.y1 = a.bf(t * d->H);
+  s.mean1 = a.f32(t);
+  s.rstd1 = a.f32(t);
+  s.u = a.bf(t * d->I);
+  s.g = a.bf(t * d->I);
+  s.nr2 = a.bf(t * d->H);
+  s.mean2 = a.f32(t);
+  s.rstd2 = a.f32(t);
+  s.tmp = a.bf(t * d->H);
+  return s;
+}
+
+struct EncWork {
+  __nv_bfloat16 *dnr2, *dg, *du, *dy1, *dnr1, *dO, *dqkv;
+  float* delta;
+};
+
+EncWork carve_enc_work(const LbEncoderDesc* d, int T, Arena& a) {
+  EncWork w{};
+  const size_t t = (size_t)T;
+  w.dnr2 = a.bf(t * d->H);
+  w.dy1 = a.bf(t * d->H);
+  w.dnr1 = a.bf(t * d->H);
+  const size_t mark = a.off;  // the MLP half is finished before the attention half starts
+  w.dg = a.bf(t * d->I);
+  w.du = a.bf(t * d->I);
+  const size_t end = a.off;
+  a.off = mark;
+  w.dO = a.bf(t * d->H);
+  w.dqkv = a.bf(t * d->qkv.width);
+  w.delta = a.f32(t * d->heads);
+  if (a.off < end) a.off = end;
+  return w;
+}
+
+// Gradient of LN's input; weight and bias gradients straight into the accumulators where these lie
+// one behind the other.
+int enc_norm_bwd(const __nv_bfloat16* dy, const __nv_bfloat16* nr, const void* w, const float* mean,
+                 const float* rstd, __nv_bfloat16* dx, float* wgrad, float* bgrad, int T, int H,
+                 const LbStreamCtx* c, int* n) {
+  const bool want = wgrad != nullptr || bgrad != nullptr;
+  const bool direct = wgrad != nullptr && bgrad == wgrad + H;
+  float* dst = !want ? nullptr : (direct ? wgrad : c->wg_tmp);
+  LB_TRY(lb_layer_norm_bwd(dy, nullptr, nr, w, mean, rstd, dx, c->norm_scratch, dst, 1,
+                           direct ? 1 : 0, T, H, c->stream));
+  *n += want ? 2 : 1;
+  if (want && !direct) {
+    if (wgrad != nullptr) LB_TRY(lb_colsum(c->wg_tmp, 1, H, wgrad, 1, 1, c->stream));
+    if (bgrad != nullptr) LB_TRY(lb_colsum(c->wg_tmp + H, 1, H, bgrad, 1, 1, c->stream));
+    *n += (wgrad != nullptr) + (bgrad != nullptr);
+  }
+  return 0;
+}
+
+int enc_linear_bwd(const LbLinear& l, float* bgrad, const __nv_bfloat16* dy, const __nv_bfloat16* x,
+                   __nv_bfloat16* dx, int T, const LbStreamCtx* c, int* n) {
+  LB_TRY(lin_dgrad(l, dy, l.n_out, dx, T, false, nullptr, c));
+  LB_TRY(lin_wgrad(l, dy, l.n_out, x, l.k_in, T, nullptr, nullptr, c));
+  *n += 1 + (l.wgrad != nullptr);
+  if (bgrad != nullptr) {
+    LB_TRY(lb_bias_grad(dy, l.n_out, T, l.n_out, 0, 0, bgrad, nullptr, nullptr, c->stream));
+    ++*n;
+  }
+  return 0;
+}
+
+bool enc_ok(const LbEncoderDesc* d) {
+  return (d->qkv.n == 1 || d->qkv.n == 3) && d->qkv.width == 3 * d->H && d->heads * d->hd == d->H;
+}
+
+}  // namespace
+
+extern "C" size_t lb_encoder_saved_bytes(const LbEncoderDesc* d, int T) {
+  Arena a(nullptr);
+  carve_enc_saved(d, T, a);
+  return a.off;
+}
+
+extern "C" size_t lb_encoder_work_bytes(const LbEncoderDesc* d, int T) {
+  Arena a(nullptr);
+  carve_enc_work(d, T, a);
+  return a.off;
+}
+
+extern "C" int lb_encoder_fwd(const LbEncoderDesc* d, const LbStreamCtx* c, LbBlockIO* io) {
+  const int T = c->T, H = d->H, I = d->I, W = d->qkv.width;
+  io->launches = 0;
+  if (T <= 0) return 0;
+  if (!enc_ok(d)) return -3;
+  t_fewer = 0;
+  Arena arena(io->saved);
+  const EncSaved s = carve_enc_saved(d, T, arena);
+  const __nv_bfloat16* x = static_cast<const __nv_bfloat16*>(io->branch);
+  __nv_bfloat16* no_ts[3] = {nullptr, nullptr, nullptr};
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(c->stream);
+  if (!c->packed) {  // rows of padding are never written by the attention kernel
+    if (cudaMemsetAsync(s.o, 0, (size_t)T * H * 2, st) != cudaSuccess) return -11;
+    ++io->launches;
+  }
+  // ordered behind everything before it on the stream; the others as in block_fwd
+  LB_TRY(proj_fwd(d->qkv, x, H, s.qkv, T, no_ts, c, d->bias));
+  const lb::PdlScope pdl(true);
+  LB_TRY(lb_attn_fwd(s.qkv, W, s.qkv + H, W, s.qkv + 2 * H, W, c->seq_start, c->seq_end, c->plan_f,
+                     c->cap_f, s.o, H, s.lse, T, d->heads, d->heads, d->hd, d->softmax_scale, 0,
+                     c->status, c->stream));
+  LB_TRY(lin_fwd(d->o_proj, s.o, H, s.tmp, H, T, nullptr, c, d->bias[3]));
+  LB_TRY(lb_layer_norm_fwd(s.tmp, x, d->ln1_w, d->ln1_b, s.y1, s.nr1, s.mean1, s.rstd1, T, H, d->eps,
+                           c->stream));
+  LB_TRY(lin_fwd(d->in, s.y1, H, s.u, I, T, nullptr, c, d->bias[4]));
+  LB_TRY(lb_gelu_fwd(s.u, s.g, 1LL * T * I, c->stream));
+  LB_TRY(lin_fwd(d->out, s.g, I, s.tmp, H, T, nullptr, c, d->bias[5]));
+  LB_TRY(lb_layer_norm_fwd(s.tmp, s.y1, d->ln2_w, d->ln2_b, io->out, s.nr2, s.mean2, s.rstd2, T, H,
+                           d->eps, c->stream));
+  io->launches += 7 + d->qkv.n - t_fewer;
+  return 0;
+}
+
+extern "C" int lb_encoder_bwd(const LbEncoderDesc* d, const LbStreamCtx* c, LbBlockIO* io) {
+  const int T = c->T, H = d->H, W = d->qkv.width;
+  io->launches = 0;
+  if (T <= 0) return 0;
+  if (!enc_ok(d)) return -3;
+  t_fewer = 0;
+  int n = 0;
+  Arena sa(io->saved), wa(io->work);
+  const EncSaved s = carve_enc_saved(d, T, sa);
+  const EncWork w = carve_enc_work(d, T, wa);
+  const __nv_bfloat16* x = static_cast<const __nv_bfloat16*>(io->branch);
+  const __nv_bfloat16* dy = static_cast<const __nv_bfloat16*>(io->d_out);
+  __nv_bfloat16* dx = static_cast<__nv_bfloat16*>(io->dx);
+  __nv_bfloat16* no_ts[3] = {nullptr, nullptr, nullptr};
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(c->stream);
+  LB_TRY(enc_norm_bwd(dy, s.nr2, d->ln2_w, s.mean2, s.rstd2, w.dnr2, d->ln2_wgrad, d->ln2_bgrad, T, H,
+                      c, &n));
+  const lb::PdlScope pdl(true);
+  LB_TRY(enc_linear_bwd(d->out, d->bias_grad[5], w.dnr2, s.g, w.dg, T, c, &n));
+  LB_TRY(lb_gelu_bwd(w.dg, s.u, w.du, 1LL * T * d->I, c->stream));
+  LB_TRY(enc_linear_bwd(d->in, d->bias_grad[4], w.du, s.y1, w.dy1, T, c, &n));
+  LB_TRY(lb_add_bf16(w.dy1, w.dnr2, 1LL * T * H, c->stream));
+  LB_TRY(enc_norm_bwd(w.dy1, s.nr1, d->ln1_w, s.mean1, s.rstd1, w.dnr1, d->ln1_wgrad, d->ln1_bgrad, T,
+                      H, c, &n));
+  LB_TRY(enc_linear_bwd(d->o_proj, d->bias_grad[3], w.dnr1, s.o, w.dO, T, c, &n));
+  if (!c->packed) {
+    if (cudaMemsetAsync(w.dqkv, 0, (size_t)T * W * 2, st) != cudaSuccess) return -11;
+    ++n;
+  }
+  LB_TRY(lb_attn_bwd(w.dO, H, s.qkv, W, s.qkv + H, W, s.qkv + 2 * H, W, s.o, H, s.lse, w.delta,
+                     c->seq_start, c->seq_end, c->plan_q, c->cap_q, c->plan_kv, c->cap_kv, w.dqkv, W,
+                     w.dqkv + H, W, w.dqkv + 2 * H, W, T, d->heads, d->heads, d->hd,
+                     d->softmax_scale, 0, c->status, c->stream));
+  LB_TRY(proj_bwd(d->qkv, w.dqkv, x, dx, T, no_ts, nullptr, c));
+  float* const* bg = d->bias_grad;
+  if (bg[0] != nullptr || bg[1] != nullptr || bg[2] != nullptr) {
+    const int parts = d->qkv.n;
+    LB_TRY(lb_bias_grad(w.dqkv, W, T, d->qkv.part[0].n_out, parts == 3 ? H : 0, parts == 3 ? H : 0,
+                        bg[0], bg[1], bg[2], c->stream));
+    ++n;
+  }
+  LB_TRY(lb_add_bf16(dx, w.dnr1, 1LL * T * H, c->stream));
+  n += 3 + 4 + d->qkv.n;  // gelu, two additions; attention; input gradients of the projections
+  for (int i = 0; i < d->qkv.n; ++i) n += d->qkv.part[i].wgrad != nullptr;
+  io->launches = n - t_fewer;
+  return 0;
+}

@@ -121,7 +121,28 @@ struct LbBlockIO {
   void* work;            // lb_block_work_bytes() bytes, 256-byte aligned
   const LbTpCtx* tp;     // null: the stream is not token-sharded
   int fewer_launches;    // out: launches saved against lb_block_*_launches (several linears in one)
+  int launches;          // out: launches of an encoder block's call
 };
+
+// A post-LayerNorm encoder block (BERT): projections with biases, bidirectional attention, two
+// residual LayerNorms, GELU (erf) between the MLP's linears. The same calls as the decoder block's:
+//   nr1 = x + o_proj(attention(qkv(x)));  y1 = LN1(nr1);  nr2 = y1 + out(gelu(in(y1)));  y = LN2(nr2)
+struct LbEncoderDesc {
+  int H, heads, hd, I;
+  float eps, softmax_scale;
+  const void *ln1_w, *ln1_b, *ln2_w, *ln2_b;
+  float *ln1_wgrad, *ln1_bgrad, *ln2_wgrad, *ln2_bgrad;  // fp32 accumulators, or null (frozen)
+  LbProjection qkv;
+  LbLinear o_proj, in, out;
+  const void* bias[6];    // q, k, v (or the fused one first), o_proj, in, out
+  float* bias_grad[6];
+};
+// io: branch = x, out = y; d_out, dx and the arenas as for the decoder block. The stream context's
+// norm_scratch has room for 2 * H columns here, wg_tmp for 2 * H floats.
+size_t lb_encoder_saved_bytes(const LbEncoderDesc* d, int T);
+size_t lb_encoder_work_bytes(const LbEncoderDesc* d, int T);
+int lb_encoder_fwd(const LbEncoderDesc* d, const LbStreamCtx* c, LbBlockIO* io);
+int lb_encoder_bwd(const LbEncoderDesc* d, const LbStreamCtx* c, LbBlockIO* io);
 
 // Bytes of the activation arena the forward fills and the backward reads (`tp` may be null; with it
 // T is ignored and the sizes follow world * rows gathered tokens and `rows` local ones).

@@ -15,6 +15,12 @@ int lb_rms_norm_bwd(const void* dy, const void* dres, const void* xin, const voi
                     const float* rstd, void* dx, float* scratch, void* dw_out, int dw_fp32,
                     int dw_accumulate, int N, int H, float w_off, void* stream);
 
+int lb_layer_norm_fwd(const void* x, const void* res_in, const void* w, const void* b, void* y,
+                      void* res_out, float* mean, float* rstd, int N, int H, float eps, void* stream);
+int lb_layer_norm_bwd(const void* dy, const void* dres, const void* xin, const void* w,
+                      const float* mean, const float* rstd, void* dx, float* scratch, void* dwb_out,
+                      int dw_fp32, int dw_accumulate, int N, int H, void* stream);
+
 // row/rope.cu
 int lb_rope_bwd_partial_rows();
 int lb_qk_norm_rope_fwd(const void* q_in, long long ldq_in, const void* k_in, long long ldk_in,
@@ -38,6 +44,12 @@ int lb_glu_bwd(int kind, const void* dout, long long ld_dout, const void* gate, 
                long long ld_in, void* dgate, void* dup, long long ld_d, long long T, int I,
                void* stream);
 
+int lb_gelu_fwd(const void* x, void* y, long long n, void* stream);
+int lb_gelu_bwd(const void* dy, const void* x, void* dx, long long n, void* stream);
+int lb_add_bf16(void* x, const void* y, long long n, void* stream);
+int lb_bias_grad(const void* dy, long long ld, int T, int n0, int n1, int n2, float* g0, float* g1,
+                 float* g2, void* stream);
+
 // attn/
 int lb_attn_zero_tail(const int* plan, int capacity, int T, void* p0, long long ld0, int w0,
                       void* p1, long long ld1, int w1, void* p2, long long ld2, int w2,
@@ -54,6 +66,9 @@ int lb_attn_bwd(const void* dO, long long lddo, const void* q, long long ldq, co
                 int Hk, int hd, float softmax_scale, int causal, int* status, void* stream);
 
 // gemm/gemm_bf16.cu
+int lb_gemm_glu_2cta(const void* A, const void* Wg, const void* Wu, void* gate, void* up, void* h,
+                     int M, int I, int K, long long lda, long long ldw, long long ld_gu,
+                     long long ld_h, int kind, int* status, void* stream);
 int lb_gemm_use_2cta(int v);
 int lb_gemm_2cta_pairs();
 int lb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda,

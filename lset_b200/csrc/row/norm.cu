@@ -276,6 +276,8 @@ __global__ void __launch_bounds__(kRowThreads)
       }
     }
   }
+  pdl_wait();
+  pdl_trigger();
   for (long long row0 = 1LL * blockIdx.x * ROWS; row0 < N; row0 += 1LL * gridDim.x * ROWS) {
     const long long row = row0 + r;
     const bool valid = row < N;
@@ -520,11 +522,10 @@ extern "C" int lb_layer_norm_fwd(const void* x, const void* res_in, const void* 
   LB_ROW_DISPATCH(H, {
     constexpr int ROWS = kRowThreads / TPR;
     const int grid = (N + ROWS - 1) / ROWS;
-    ln_fwd_kernel<TPR, NV><<<grid, kRowThreads, 0, st>>>(
-        (const bf16*)x, (const bf16*)res_in, (const bf16*)w, (const bf16*)b, (bf16*)y,
-        (bf16*)res_out, mean, rstd, N, H, eps);
+    return launch_pdl(ln_fwd_kernel<TPR, NV>, dim3(grid), dim3(kRowThreads), 0, st, pdl_enabled(),
+                      1, (const bf16*)x, (const bf16*)res_in, (const bf16*)w, (const bf16*)b,
+                      (bf16*)y, (bf16*)res_out, mean, rstd, N, H, eps);
   });
-  return launch_rc();
 }
 
 // dwb_out: [2, H] (dW then dB), fp32 or bf16; scratch: lb_norm_bwd_partial_rows() * 2H floats.

@@ -15,6 +15,7 @@ import torch.nn as nn
 from ..ops import activation as act_ops
 from ..ops import attention as attn_ops
 from ..ops import embedding as emb_ops
+from ..ops import encoder_block as block_ops
 from ..ops import norm as norm_ops
 from .configs import BertConfig
 from .layers import Linear, StreamCtx, make_stream_ctx
@@ -93,6 +94,8 @@ class BertBlock(nn.Module):
         self.mlp = BertMLP(config)
 
     def forward(self, x, ctx: StreamCtx):
+        if block_ops.usable(self, x):
+            return block_ops.run(self, x, ctx)   # the whole block in one native call
         return self.mlp(self.attention(x, ctx))
 
 

@@ -79,7 +79,7 @@ class LbTpCtx(ctypes.Structure):
 class LbBlockIO(ctypes.Structure):
     _fields_ = [("branch", _vp), ("residual", _vp), ("out", _vp), ("res_out", _vp),
                 ("saved", _vp), ("d_out", _vp), ("d_res_out", _vp), ("dx", _vp), ("work", _vp),
-                ("tp", _vp), ("fewer_launches", ctypes.c_int)]
+                ("tp", _vp), ("fewer_launches", ctypes.c_int), ("launches", ctypes.c_int)]
 
 
 _lib = None

@@ -1,0 +1,241 @@
+"""Whole post-LayerNorm encoder block (BERT / XLM-R) forward and backward in two native calls.
+
+Op by op a block is eight launches forward and about thirty backward, each with an autograd node and
+a foreign call of its own: at the batch sizes such encoders are used with, the host needs several
+times longer to issue them than the GPU to run them. ``run`` hands the sequence to
+``lb_encoder_fwd`` / ``lb_encoder_bwd`` (``csrc/block/block.cu``), as ``ops/block.py`` does for the
+decoder block; autograd sees one node. Forward values have the bits of the op-by-op path; bias
+gradients are added to their fp32 accumulators without a rounding to bf16 in between.
+
+Taken for blocks of plain bf16 ``Linear`` layers with biases (fused or separate query / key / value)
+on the GPU; everything else (tensor parallelism, 8-bit layers, adapters, selective activation
+checkpointing, wrapped or hooked submodules) keeps the op-by-op path.
+
+Replaces the Python block of the reference (lset/models/encoder/bert/model.py:53-142).
+"""
+from __future__ import annotations
+
+import ctypes
+import math
+
+import torch
+
+from . import _ac
+from . import _native as nv
+from ._grads import main_grad_of
+from .attention import fwd_tile_tokens
+from .block import (LbBlockIO, LbLinear, LbProjection, LbStreamCtx, _arena_size, _fp, _vp,
+                    _work_arena)
+from .norm import scratch
+from .runtime_options import enabled, options as _rt
+
+
+class LbEncoderDesc(ctypes.Structure):
+    _fields_ = [("H", ctypes.c_int), ("heads", ctypes.c_int), ("hd", ctypes.c_int),
+                ("I", ctypes.c_int), ("eps", ctypes.c_float), ("softmax_scale", ctypes.c_float),
+                ("ln1_w", _vp), ("ln1_b", _vp), ("ln2_w", _vp), ("ln2_b", _vp),
+                ("ln1_wgrad", _fp), ("ln1_bgrad", _fp), ("ln2_wgrad", _fp), ("ln2_bgrad", _fp),
+                ("qkv", LbProjection), ("o_proj", LbLinear), ("in_", LbLinear), ("out", LbLinear),
+                ("bias", _vp * 6), ("bias_grad", _fp * 6)]
+
+
+_lib = None
+calls = 0     # blocks taken by the runner (for tests)
+
+
+def _library():
+    global _lib
+    if _lib is None:
+        lib = nv.load()
+        for fn in (lib.lb_encoder_saved_bytes, lib.lb_encoder_work_bytes):
+            fn.restype, fn.argtypes = ctypes.c_size_t, [_vp, ctypes.c_int]
+        for fn in (lib.lb_encoder_fwd, lib.lb_encoder_bwd):
+            fn.argtypes = [_vp, _vp, _vp]
+        _lib = lib
+    return _lib
+
+
+def _modules(block):
+    att, mlp = block.attention, block.mlp
+    qkv = [att.qkv_proj] if att.fused_qkv else [att.query, att.key, att.value]
+    return qkv, att.dense, mlp.dense_in, mlp.dense_out, att.LayerNorm, mlp.LayerNorm
+
+
+def _plain(m) -> bool:
+    from ..models.layers import Linear
+
+    return (type(m) is Linear and m.bias is not None and "forward" not in m.__dict__
+            and not hasattr(m, "_tp_kind") and not m._forward_hooks and not m._forward_pre_hooks
+            and not m._backward_hooks and not m._backward_pre_hooks
+            and m.weight.dtype == torch.bfloat16 and m.bias.dtype == torch.bfloat16
+            and m.weight.is_cuda and m.weight.is_contiguous() and m.bias.is_contiguous()
+            and m.weight.shape[0] % 8 == 0 and m.weight.shape[1] % 8 == 0)
+
+
+class EncoderPlan:
+    """The tensors that feed the descriptor; pointers are read again on every call."""
+
+    def __init__(self, block):
+        self.ok = False
+        self.signature = self._signature(block)
+        qkv, o, fin, fout, ln1, ln2 = _modules(block)
+        att = block.attention
+        H, hd = o.weight.shape[0], att.head_dim
+        if hd not in (64, 128) or att.num_heads * hd != H or H % 8:
+            return
+        if not all(_plain(m) for m in qkv + [o, fin, fout]):
+            return
+        if any(m.weight.shape != (3 * H // len(qkv), H) for m in qkv):
+            return
+        if (o.weight.shape != (H, H) or fin.weight.shape[1] != H
+                or fout.weight.shape != (H, fin.weight.shape[0])):
+            return
+        for ln in (ln1, ln2):
+            if (type(ln) is not torch.nn.LayerNorm or ln.weight is None or ln.bias is None
+                    or ln.weight.dtype != torch.bfloat16 or ln.bias.dtype != torch.bfloat16
+                    or not ln.weight.is_cuda or ln.eps != ln1.eps):
+                return
+        d = LbEncoderDesc()
+        d.H, d.heads, d.hd, d.I = H, att.num_heads, hd, fin.weight.shape[0]
+        d.eps, d.softmax_scale = float(ln1.eps), 1.0 / math.sqrt(hd)
+        d.qkv.n, d.qkv.width = len(qkv), 3 * H
+        self.desc = d
+        self.linears = [(m, d.qkv.part[i], i) for i, m in enumerate(qkv)]
+        self.linears += [(o, d.o_proj, 3), (fin, d.in_, 4), (fout, d.out, 5)]
+        self.norms = [(ln1, "ln1"), (ln2, "ln2")]
+        self.params = [p for ln, _ in self.norms for p in (ln.weight, ln.bias)]
+        self.params += [p for m, _, _ in self.linears for p in (m.weight, m.bias)]
+        self.ok = True
+
+    @staticmethod
+    def _signature(block):
+        """Changes when a submodule is wrapped, replaced, hooked, moved or cast."""
+        qkv, *rest = _modules(block)
+        return tuple((id(m), id(m.weight), id(m.bias), "forward" in m.__dict__, m.weight.dtype,
+                      m.weight.device, len(m._forward_hooks), len(m._forward_pre_hooks),
+                      len(m._backward_hooks)) for m in qkv + rest) + tuple(
+            len(h) for m in (block.attention, block.mlp)
+            for h in (m._forward_hooks, m._forward_pre_hooks, m._backward_hooks))
+
+    def fill(self, grads: dict) -> LbEncoderDesc:
+        d = self.desc
+        for ln, name in self.norms:
+            setattr(d, name + "_w", ln.weight.data_ptr())
+            setattr(d, name + "_b", ln.bias.data_ptr())
+            setattr(d, name + "_wgrad", grads.get(id(ln.weight)))
+            setattr(d, name + "_bgrad", grads.get(id(ln.bias)))
+        for m, dst, i in self.linears:
+            w = m.weight
+            dst.w, dst.wgrad, dst.ldw = w.data_ptr(), grads.get(id(w)), w.stride(0)
+            dst.n_out, dst.k_in = w.shape
+            d.bias[i], d.bias_grad[i] = m.bias.data_ptr(), grads.get(id(m.bias))
+        return d
+
+
+def plan_of(block):
+    plan = block.__dict__.get("_lb_plan")
+    if plan is None or plan.signature != plan._signature(block):
+        plan = EncoderPlan(block)
+        block.__dict__["_lb_plan"] = plan
+    return plan if plan.ok else None
+
+
+def usable(block, x) -> bool:
+    if not (x.is_cuda and x.dtype == torch.bfloat16 and x.dim() == 2 and x.shape[0] > 0):
+        return False
+    if _ac._active is not None or not enabled("block_runner") or _rt.attention_backend == "sdpa":
+        return False
+    if not enabled("fused_layernorm") or any(
+            m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks
+            for m in (block.attention, block.mlp)):
+        return False
+    return plan_of(block) is not None
+
+
+def _stream_struct(ctx, plan: EncoderPlan, device, training: bool) -> LbStreamCtx:
+    d = plan.desc
+    grad = torch.is_grad_enabled()
+    may_split = not grad and not training
+    key = ("_lb_enc", grad, may_split, d.hd, d.H)
+    hit = ctx.tables.get(key)
+    if hit is not None:
+        return hit
+    ap = ctx.plan
+    ptf, capf = ap.tiles(fwd_tile_tokens(d.hd, 1))
+    ptq, capq = ap.tiles(128) if grad else (None, 0)
+    s = LbStreamCtx()
+    s.T, s.packed = int(ctx.pos.shape[0]), int(ap.cu_seqlens is not None)
+    s.seq_start, s.seq_end = ap.seq_start.data_ptr(), ap.seq_end.data_ptr()
+    s.plan_f, s.cap_f = ptf.data_ptr(), capf
+    s.plan_q = s.plan_kv = nv.ptr(ptq) or None      # one query head per KV head: the same tiles
+    s.cap_q = s.cap_kv = capq
+    s.status = nv.status_word(device).data_ptr()
+    s.norm_scratch = scratch("norm_bwd", _library().lb_norm_bwd_partial_rows() * 2 * d.H,
+                             device).data_ptr()
+    s.wg_tmp = scratch("ln_wgrad", 2 * d.H, device).data_ptr()
+    s.may_split = int(may_split)
+    s._keep = (ctx.pos, ap, ptf, ptq)
+    ctx.tables[key] = s
+    return s
+
+
+class _EncoderBlockFn(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, plan, sctx, stream_ctx, *params):
+        global calls
+        lib = _library()
+        d = plan.fill({})
+        x = x if x.is_contiguous() else x.contiguous()
+        T, H = x.shape
+        nbytes = lib.lb_encoder_saved_bytes(ctypes.addressof(d), T)
+        saved = torch.empty(_arena_size(nbytes), dtype=torch.uint8, device=x.device)
+        out = torch.empty_like(x)
+        io = LbBlockIO()
+        io.branch, io.out, io.saved = x.data_ptr(), out.data_ptr(), saved.data_ptr()
+        sctx.stream = nv.stream_ptr()
+        rc = lib.lb_encoder_fwd(ctypes.addressof(d), ctypes.addressof(sctx), ctypes.addressof(io))
+        if rc != 0:
+            nv.check_rc(rc, "lb_encoder_fwd")
+        nv.count_launch(io.launches)
+        calls += 1
+        ctx.save_for_backward(x, saved)
+        ctx.plan, ctx.sctx, ctx.stream_ctx = plan, sctx, stream_ctx
+        return out
+
+    @staticmethod
+    def backward(ctx, d_out):
+        lib = _library()
+        x, saved = ctx.saved_tensors
+        plan, sctx = ctx.plan, ctx.sctx
+        T, H = x.shape
+        d_out = d_out.to(x.dtype).contiguous()
+        # weight gradients go straight into the sharding runtime's fp32 accumulators; a parameter
+        # without one gets a temporary that is returned to autograd
+        grads, temps = {}, []
+        for p in plan.params:
+            mg = main_grad_of(p) if p.requires_grad else None
+            temp = None
+            if p.requires_grad and mg is None:
+                mg = temp = torch.zeros(p.shape, dtype=torch.float32, device=x.device)
+            temps.append(temp)
+            if mg is not None:
+                grads[id(p)] = mg.data_ptr()
+        d = plan.fill(grads)
+        work = _work_arena(lib.lb_encoder_work_bytes(ctypes.addressof(d), T), x.device)
+        dx = torch.empty_like(x)
+        io = LbBlockIO()
+        io.branch, io.saved, io.work = x.data_ptr(), saved.data_ptr(), work.data_ptr()
+        io.d_out, io.dx = d_out.data_ptr(), dx.data_ptr()
+        sctx.stream = nv.stream_ptr()
+        rc = lib.lb_encoder_bwd(ctypes.addressof(d), ctypes.addressof(sctx), ctypes.addressof(io))
+        if rc != 0:
+            nv.check_rc(rc, "lb_encoder_bwd")
+        nv.count_launch(io.launches)
+        pgrads = tuple(None if t is None else t.to(p.dtype) for t, p in zip(temps, plan.params))
+        return (dx, None, None, None) + pgrads
+
+
+def run(block, x, ctx):
+    plan = plan_of(block)
+    sctx = _stream_struct(ctx, plan, x.device, block.training)
+    return _EncoderBlockFn.apply(x, plan, sctx, ctx, *plan.params)
