@@ -70,33 +70,29 @@ def panel_cols(M: int, N: int) -> int:
 
 
 def streamed_loss_backward(launch_pgrad, q, k, need_dq: bool, need_dk: bool):
-    """``launch_pgrad(c0, c1, W)`` fills ``W [Mp, c1 - c0]`` (bf16, rows past M zero) for the
-    passage columns ``[c0, c1)``. Returns ``(dq, dk)`` in the inputs' dtype."""
+    """``launch_pgrad(c0, c1, W)`` fills ``W [M, c1 - c0]`` (bf16) for the passage columns
+    ``[c0, c1)``. Returns ``(dq, dk)`` in the inputs' dtype."""
     M, D = q.shape
     N = k.shape[0]
-    Mp = (M + 7) // 8 * 8
     step = panel_cols(M, N)
     single = step >= N
-    qp = q if Mp == M else torch.cat([q, q.new_zeros(Mp - M, D)])
     dq = dk = dq32 = None
     if need_dk:
         dk = torch.empty(N, D, dtype=k.dtype, device=k.device)
-    W = torch.empty(Mp, step, dtype=torch.bfloat16, device=q.device)
-    if Mp != M:
-        W[M:].zero_()
+    W = torch.empty(M, step, dtype=torch.bfloat16, device=q.device)
     for c0 in range(0, N, step):
         c1 = min(N, c0 + step)
         Wp = W if c1 - c0 == step else W[:, :c1 - c0]
         launch_pgrad(c0, c1, Wp)
         if need_dq:
             if single:
-                dq = matmul_abt(Wp[:M], k, b_mn=True)                       # [M, D] = W · K
+                dq = matmul_abt(Wp, k, b_mn=True)                       # [M, D] = W · K
             elif dq32 is None:
-                dq32 = matmul_abt(Wp[:M], k[c0:c1], b_mn=True, out_dtype=torch.float32)
+                dq32 = matmul_abt(Wp, k[c0:c1], b_mn=True, out_dtype=torch.float32)
             else:
-                matmul_abt(Wp[:M], k[c0:c1], b_mn=True, out=dq32, accumulate=True)
+                matmul_abt(Wp, k[c0:c1], b_mn=True, out=dq32, accumulate=True)
         if need_dk:
-            matmul_abt(Wp, qp, a_mn=True, b_mn=True, out=dk[c0:c1])         # [n, D] = Wᵀ · Q
+            matmul_abt(Wp, q, a_mn=True, b_mn=True, out=dk[c0:c1])          # [n, D] = Wᵀ · Q
     if need_dq and dq is None:
         dq = dq32.to(q.dtype)
     return dq, dk
@@ -242,6 +238,26 @@ def _pad_rows8(k):
     return k if extra == 0 else torch.cat([k, k.new_zeros(extra, k.shape[1])], dim=0)
 
 
+_LABEL_KINDS = {torch.float32: 0, torch.int64: 1, torch.int32: 2, torch.int8: 3, torch.bool: 3}
+
+
+def _label_prep(labels, kind: int, Kp: int):
+    """``(int8 labels [Q, Kp], row_scale [Q], row_w [Q])`` of a 0/1/-1 label matrix in one launch."""
+    Q, K = labels.shape
+    dev = labels.device
+    lab8 = torch.empty(Q, Kp, dtype=torch.int8, device=dev)
+    stats = torch.empty(2, Q, dtype=torch.float32, device=dev)
+    counters = torch.zeros(2, dtype=torch.int32, device=dev)
+    rc = nv.load().lb_label_prep(
+        nv.c_void_p(labels.data_ptr()), nv.c_int(kind), nv.c_ll(labels.stride(0)), nv.c_int(Q),
+        nv.c_int(K), nv.c_int(Kp), nv.c_void_p(lab8.data_ptr()), nv.c_void_p(stats.data_ptr()),
+        nv.c_void_p(stats.data_ptr() + 4 * Q), nv.c_void_p(counters.data_ptr()),
+        nv.c_void_p(nv.stream_ptr()))
+    nv.check_rc(rc, "lb_label_prep")
+    nv.count_launch()
+    return lab8, stats[0], stats[1]
+
+
 def fused_label_loss(q, k, labels, temperature: float, scores=None):
     """Label-matrix contrastive loss on the streaming kernels. ``labels [Q, K]``: 1 positive,
     0 negative, negative values ignored. Without ``scores``: multi-positive NCE
@@ -251,6 +267,12 @@ def fused_label_loss(q, k, labels, temperature: float, scores=None):
     Q, K = labels.shape
     dev = q.device
     Kp = (K + 31) // 32 * 32
+    kind = _LABEL_KINDS.get(labels.dtype)
+    if (scores is None and kind is not None and labels.device == dev and Q > 0 and K > 0
+            and (K == 1 or labels.stride(1) == 1)):
+        lab8, row_scale, row_w = _label_prep(labels, kind, Kp)
+        return _FusedLabelLoss.apply(q.contiguous(), _pad_rows8(k).contiguous(), lab8, None,
+                                     row_scale, row_w, 1.0 / float(temperature))
     lab8 = torch.full((Q, Kp), -1, dtype=torch.int8, device=dev)
     lab8[:, :K].copy_(labels)           # converts in the copy: no fp32 [Q, K] temporary
     labels = lab8[:, :K]

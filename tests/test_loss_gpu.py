@@ -248,3 +248,25 @@ def test_fused_label_loss_reads_missing_teacher_scores_as_zero_targets():
     assert ref.item() > 0 and abs(loss.item() - ref.item()) < 2e-2 * max(1.0, abs(ref.item()))
     for a, b in ((q.grad, qr.grad), (k.grad, kr.grad)):
         assert (a.float() - b).abs().max().item() < 3e-2 * (b.abs().max().item() + 1e-6)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.int64, torch.int32, torch.int8, torch.bool])
+@pytest.mark.parametrize("Q,K", [(1, 1), (7, 33), (1009, 4036), (3000, 64)])
+def test_label_prep_is_the_elementwise_computation(dtype, Q, K):
+    from lset_b200.ops.loss import _LABEL_KINDS, _label_prep
+
+    g = torch.Generator(device="cuda").manual_seed(Q)
+    wide = torch.randint(-1, 2, (Q, K + 3), generator=g, device="cuda")
+    wide[::3] = -1                       # rows without a valid column
+    wide[1::3] = wide[1::3].clamp(max=0)  # rows without a positive
+    labels = (wide > 0 if dtype == torch.bool else wide.to(dtype))[:, :K]   # strided rows
+    Kp = (K + 31) // 32 * 32
+    for _ in range(2):
+        lab8, row_scale, row_w = _label_prep(labels, _LABEL_KINDS[dtype], Kp)
+        want = torch.full((Q, Kp), -1, dtype=torch.int8, device="cuda")
+        want[:, :K] = labels
+        n_pos = want.clamp(min=0).sum(1)
+        keep = ((n_pos > 0) & (want.amax(1) >= 0)).float()
+        assert torch.equal(lab8, want)
+        assert torch.equal(row_scale, 1.0 / n_pos.clamp(min=1).float())
+        assert torch.equal(row_w, keep / keep.sum().clamp(min=1.0))
