@@ -236,14 +236,23 @@ class BlockPlan:
 
     @staticmethod
     def _signature(block):
-        """Changes when a projection is wrapped, replaced, moved or cast after the plan was made."""
-        att, mlp = block.self_attn, block.mlp
-        mods = (([att.qkv_proj] if att.fused_qkv else [att.q_proj, att.k_proj, att.v_proj])
-                + [att.o_proj]
-                + ([mlp.gate_up_proj] if mlp.fused_gate_up else [mlp.gate_proj, mlp.up_proj])
-                + [mlp.down_proj])
-        return tuple((id(m), "forward" in m.__dict__, id(getattr(m, "_sp_state", None)),
-                      m.weight.dtype, m.weight.device, m.training) for m in mods)
+        """Changes when a projection is wrapped, replaced, moved or cast after the plan was made.
+        (Modules and parameters are looked up in their dicts: attribute access on a module costs
+        more than the rest of this, which runs for every block of every pass.)"""
+        att, mlp = block._modules["self_attn"], block._modules["mlp"]
+        am, mm = att._modules, mlp._modules
+        mods = ((am["qkv_proj"],) if att.fused_qkv else (am["q_proj"], am["k_proj"], am["v_proj"]))
+        mods += (am["o_proj"],)
+        mods += ((mm["gate_up_proj"],) if mlp.fused_gate_up else (mm["gate_proj"], mm["up_proj"]))
+        sig = []
+        for m in mods + (mm["down_proj"],):
+            d = m.__dict__
+            w = d["_parameters"].get("weight")
+            if w is None:
+                w = m.weight
+            sig.append((id(m), "forward" in d, id(d.get("_sp_state")), w.dtype, w.device,
+                        d["training"]))
+        return sig
 
     def still_valid(self, block) -> bool:
         return self.signature == self._signature(block)
@@ -280,6 +289,14 @@ class BlockPlan:
         self._fill_linear(d.o_proj, self.o, grads)
         self._fill_linear(d.down, self.down, grads)
         return d
+
+
+def node_inputs(params):
+    """The parameters an autograd node lists: those of a pass that records no derivatives are left
+    out (each costs the call a look at its wrapper)."""
+    if torch.is_grad_enabled() or torch.autograd.forward_ad._current_level >= 0:
+        return params
+    return ()
 
 
 def plan_of(block):
@@ -497,7 +514,8 @@ class _BlockFn(torch.autograd.Function):
 
 
 def run(block, branch, residual, ctx):
-    """``(mlp_out, residual_out)`` of one decoder block, as ``DecoderBlock.forward`` returns them."""
-    plan = plan_of(block)
+    """``(mlp_out, residual_out)`` of one decoder block, as ``DecoderBlock.forward`` returns them, for
+    a block that ``usable`` has just accepted."""
+    plan = block.__dict__["_lb_plan"]
     sctx = _stream_struct(ctx, plan, branch.device, block.training)
-    return _BlockFn.apply(branch, residual, plan, sctx, ctx, *plan.params)
+    return _BlockFn.apply(branch, residual, plan, sctx, ctx, *node_inputs(plan.params))

@@ -25,7 +25,7 @@ from . import _native as nv
 from ._grads import main_grad_of
 from .attention import fwd_tile_tokens
 from .block import (LbBlockIO, LbLinear, LbProjection, LbStreamCtx, _arena_size, _fp, _vp,
-                    _work_arena)
+                    _work_arena, node_inputs)
 from .norm import scratch
 from .runtime_options import enabled, options as _rt
 
@@ -78,6 +78,8 @@ class EncoderPlan:
     def __init__(self, block):
         self.ok = False
         self.signature = self._signature(block)
+        if self.signature is None:
+            return
         qkv, o, fin, fout, ln1, ln2 = _modules(block)
         att = block.attention
         H, hd = o.weight.shape[0], att.head_dim
@@ -109,13 +111,23 @@ class EncoderPlan:
 
     @staticmethod
     def _signature(block):
-        """Changes when a submodule is wrapped, replaced, hooked, moved or cast."""
-        qkv, *rest = _modules(block)
-        return tuple((id(m), id(m.weight), id(m.bias), "forward" in m.__dict__, m.weight.dtype,
-                      m.weight.device, len(m._forward_hooks), len(m._forward_pre_hooks),
-                      len(m._backward_hooks)) for m in qkv + rest) + tuple(
-            len(h) for m in (block.attention, block.mlp)
-            for h in (m._forward_hooks, m._forward_pre_hooks, m._backward_hooks))
+        """Changes when a submodule is wrapped, replaced, hooked, moved or cast (looked up in the
+        modules' dicts, see ``BlockPlan._signature``)."""
+        att, mlp = block._modules["attention"], block._modules["mlp"]
+        am, mm = att._modules, mlp._modules
+        mods = (am["qkv_proj"],) if att.fused_qkv else (am["query"], am["key"], am["value"])
+        mods += (am["dense"], mm["dense_in"], mm["dense_out"], am["LayerNorm"], mm["LayerNorm"])
+        sig = []
+        for m in mods:
+            d = m.__dict__
+            p = d["_parameters"]
+            w = p.get("weight")
+            if w is None:
+                return None
+            sig.append((id(m), id(w), id(p.get("bias")), "forward" in d, w.dtype, w.device,
+                        len(d["_forward_hooks"]), len(d["_forward_pre_hooks"]),
+                        len(d["_backward_hooks"])))
+        return sig
 
     def fill(self, grads: dict) -> LbEncoderDesc:
         d = self.desc
@@ -134,7 +146,7 @@ class EncoderPlan:
 
 def plan_of(block):
     plan = block.__dict__.get("_lb_plan")
-    if plan is None or plan.signature != plan._signature(block):
+    if plan is None or plan.signature is None or plan.signature != plan._signature(block):
         plan = EncoderPlan(block)
         block.__dict__["_lb_plan"] = plan
     return plan if plan.ok else None
@@ -236,6 +248,6 @@ class _EncoderBlockFn(torch.autograd.Function):
 
 
 def run(block, x, ctx):
-    plan = plan_of(block)
+    plan = block.__dict__["_lb_plan"]     # ``usable`` has just accepted it
     sctx = _stream_struct(ctx, plan, x.device, block.training)
-    return _EncoderBlockFn.apply(x, plan, sctx, ctx, *plan.params)
+    return _EncoderBlockFn.apply(x, plan, sctx, ctx, *node_inputs(plan.params))

@@ -3,23 +3,24 @@
 lset/train/data/packed_collator.py:27-67)."""
 from __future__ import annotations
 
+import itertools
 from typing import List, Sequence
 
+import numpy as np
 import torch
 
 
 def pack_sequences(sequences: Sequence[Sequence[int]]) -> dict:
     """``{input_ids [T] int64, cu_seqlens [N+1] int32, max_seqlen int, position_ids [T] int64}``;
     positions restart at 0 for every sequence."""
-    lens = [len(s) for s in sequences]
-    flat = [t for s in sequences for t in s]
-    cu = torch.zeros(len(lens) + 1, dtype=torch.int32)
-    if lens:
-        cu[1:] = torch.tensor(lens, dtype=torch.int64).cumsum(0).to(torch.int32)
-    pos = torch.cat([torch.arange(n, dtype=torch.int64) for n in lens]) if lens else \
-        torch.zeros(0, dtype=torch.int64)
-    return {"input_ids": torch.tensor(flat, dtype=torch.int64), "cu_seqlens": cu,
-            "max_seqlen": max(lens) if lens else 0, "position_ids": pos}
+    lens = np.fromiter(map(len, sequences), dtype=np.int64, count=len(sequences))
+    total = int(lens.sum())
+    ids = np.fromiter(itertools.chain.from_iterable(sequences), dtype=np.int64, count=total)
+    cu = np.zeros(len(lens) + 1, dtype=np.int32)
+    np.cumsum(lens, out=cu[1:])
+    pos = np.arange(total, dtype=np.int64) - np.repeat(cu[:-1].astype(np.int64), lens)
+    return {"input_ids": torch.from_numpy(ids), "cu_seqlens": torch.from_numpy(cu),
+            "max_seqlen": int(lens.max()) if len(lens) else 0, "position_ids": torch.from_numpy(pos)}
 
 
 def pack_fixed_budget(sequences: Sequence[Sequence[int]], token_budget: int, pad_token_id: int = 0) -> dict:
