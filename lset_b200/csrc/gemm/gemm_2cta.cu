@@ -25,6 +25,9 @@
 // waiting.
 //
 // Operand layouts, split-K and the output forms are those of lb_gemm_bf16 (see gemm_bf16.cu).
+// 8-bit float operands (F8 kernels, K-major) use the same bytes: a row of a tile is 128 bytes, now 128
+// elements, an instruction contracts 32 bytes of it, and the dequantisation factors are applied to
+// the accumulator in the epilogue.
 #include <cuda_bf16.h>
 #include <stdlib.h>
 
@@ -83,6 +86,10 @@ struct Args2 {
   void* up_out;
   void* glu_h;
   long long ld_h;
+  // 8-bit operands (F8 kernels): element (r, c) is multiplied by f8_sa[r * f8_sa_stride] *
+  // f8_sb[c * f8_sb_stride]; formats 0 = e4m3, 1 = e5m2
+  const float *f8_sa, *f8_sb;
+  int f8_sa_stride, f8_sb_stride, f8_a_e5m2, f8_b_e5m2;
   int* status;
 };
 
@@ -147,6 +154,18 @@ __device__ __forceinline__ void umma2_bf16(uint32_t tmem_d, uint64_t adesc, uint
       : "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+__device__ __forceinline__ void umma2_f8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
+                                         uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n"
+      "}\n"
+      :
+      : "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
 // Arrive on the barrier at this shared-memory offset in both CTAs of the pair once the tcgen05
 // operations issued so far have completed: one commit per CTA, the peer's barrier through its
 // address in the cluster's shared-memory window.
@@ -193,11 +212,14 @@ constexpr int kPullWarps = 2;
 //   40280 x (3072, 3072) x 1024    487 -> 445 -> 389
 //   20000 x (9728, 9728) x 2560   1565 -> 1567 -> 1451
 //   20000 x (8192, 8192) x 2048   1186 -> 1021 -> 930
-template <int A_MN, int B_MN, typename OutT, int GATHER = 0, int GLU = 0>
+template <int A_MN, int B_MN, typename OutT, int GATHER = 0, int GLU = 0, int F8 = 0>
 __global__ void __launch_bounds__(kThreads + (GATHER ? 32 * kPullWarps : 0), 1)
     gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                      const __grid_constant__ CUtensorMap tmA2,
                      const __grid_constant__ CUtensorMap tmB2, Args2 g) {
+  static_assert(!F8 || (!A_MN && !B_MN && !GATHER && !GLU), "8-bit operands: plain products only");
+  constexpr int BKE = F8 ? 2 * BK : BK;      // elements per stage
+  constexpr int BKTE = F8 ? 2 * BKT : BKT;   // elements per row of a TMA box
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -245,7 +267,7 @@ __global__ void __launch_bounds__(kThreads + (GATHER ? 32 * kPullWarps : 0), 1)
   const int tiles_m = GATHER ? g.world * tiles_per_peer : (g.M + 2 * BMc - 1) / (2 * BMc);
   constexpr int kTileN = GLU ? BNh : BNp;   // output columns (features) of a tile
   const int tiles_n = (g.N + kTileN - 1) / kTileN;
-  const int kb_first = (g.K + BK - 1) / BK;                    // k-blocks of the first operand pair
+  const int kb_first = (g.K + BKE - 1) / BKE;                  // k-blocks of the first operand pair
   const int kb_total = kb_first + (g.K2 + BK - 1) / BK;
   const int total = tiles_m * tiles_n * g.splits;
   const int pair = blockIdx.x >> 1;
@@ -327,7 +349,7 @@ __global__ void __launch_bounds__(kThreads + (GATHER ? 32 * kPullWarps : 0), 1)
           const bool second = kb >= kb_first;   // past the first pair: rows beyond K2 read as zero
           const CUtensorMap* ta = second ? &tmA2 : &tmA;
           const CUtensorMap* tb = (GLU ? !leader : second) ? &tmB2 : &tmB;
-          const int kc = (second ? kb - kb_first : kb) * BK;
+          const int kc = (second ? kb - kb_first : kb) * BKE;
           if (A_MN) {
 #pragma unroll
             for (int c = 0; c < BMc / 64; ++c)
@@ -335,7 +357,7 @@ __global__ void __launch_bounds__(kThreads + (GATHER ? 32 * kPullWarps : 0), 1)
           } else {
 #pragma unroll
             for (int h = 0; h < BK / BKT; ++h)
-              tma_load_2d_pair(sa + h * (BMc * 128), ta, bar, kc + BKT * h, m0);
+              tma_load_2d_pair(sa + h * (BMc * 128), ta, bar, kc + BKTE * h, m0);
           }
           if (B_MN) {
 #pragma unroll
@@ -344,7 +366,7 @@ __global__ void __launch_bounds__(kThreads + (GATHER ? 32 * kPullWarps : 0), 1)
           } else {
 #pragma unroll
             for (int h = 0; h < BK / BKT; ++h)
-              tma_load_2d_pair(sb + h * (BNh * 128), tb, bar, kc + BKT * h, nb);
+              tma_load_2d_pair(sb + h * (BNh * 128), tb, bar, kc + BKTE * h, nb);
           }
           if (++stage == kStages) {
             stage = 0;
@@ -364,7 +386,8 @@ __global__ void __launch_bounds__(kThreads + (GATHER ? 32 * kPullWarps : 0), 1)
   } else if (warp == 1) {
     if (lane == 0 && leader) {
       // ---------------------------------------------------------------- MMA issuer (leader)
-      const uint32_t idesc = umma_idesc_bf16(2 * BMc, BNp, A_MN, B_MN);
+      const uint32_t idesc = F8 ? umma_idesc_f8(2 * BMc, BNp, g.f8_a_e5m2, g.f8_b_e5m2)
+                                : umma_idesc_bf16(2 * BMc, BNp, A_MN, B_MN);
       int stage = 0;
       uint32_t phase = 0;
       int it = 0;
@@ -398,7 +421,10 @@ __global__ void __launch_bounds__(kThreads + (GATHER ? 32 * kPullWarps : 0), 1)
             const uint64_t bdesc =
                 B_MN ? umma_smem_desc(sb + k * 2048, BK * 128, 1024)
                      : umma_smem_desc(sb + (k / 4) * (BNh * 128) + (k % 4) * 32, 16, 1024);
-            umma2_bf16(d_tmem, adesc, bdesc, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+            if constexpr (F8)
+              umma2_f8(d_tmem, adesc, bdesc, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+            else
+              umma2_bf16(d_tmem, adesc, bdesc, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
           }
           umma2_commit_both(&empty[stage], 1u);
           if (++stage == kStages) {
@@ -527,12 +553,27 @@ __global__ void __launch_bounds__(kThreads + (GATHER ? 32 * kPullWarps : 0), 1)
           }
         }
       } else {
+      [[maybe_unused]] float f8_row = 1.f;
+      if constexpr (F8) {
+        f8_row = row < m_limit ? g.f8_sa[static_cast<long long>(row) * g.f8_sa_stride] : 0.f;
+        if (g.f8_sb_stride == 0) f8_row *= g.f8_sb[0];   // one factor for all of B
+      }
 #pragma unroll 1
       for (int c = half * kChunks; c < (half + 1) * kChunks; ++c) {
         uint32_t r[32];
         tmem_ld_32x32b_x32(tmem_base + (uint32_t(q * 32) << 16) + acc * BNp + c * 32, r);
         tmem_ld_wait();
         const int col0 = n0 + c * 32;
+        if constexpr (F8) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * f8_row);
+          if (g.f8_sb_stride != 0) {
+            const float sb = col0 + lane < g.N ? g.f8_sb[col0 + lane] : 0.f;
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              r[j] = __float_as_uint(__uint_as_float(r[j]) * __shfl_sync(0xffffffffu, sb, j));
+          }
+        }
         if constexpr (sizeof(OutT) == 2) {
           uint8_t* sblk = reinterpret_cast<uint8_t*>(epi_stage + (warp - 2) * EPI_WORDS);
           uint8_t* srow = sblk + lane * 80;
@@ -622,10 +663,10 @@ __global__ void __launch_bounds__(kThreads + (GATHER ? 32 * kPullWarps : 0), 1)
 // SMs / 2; a persistent grid larger than it would run in two waves.
 int g_max_pairs = 0;
 
-template <int A_MN, int B_MN, typename OutT, int GATHER = 0, int GLU = 0>
+template <int A_MN, int B_MN, typename OutT, int GATHER = 0, int GLU = 0, int F8 = 0>
 int launch2(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmA2,
             const CUtensorMap& tmB2, const Args2& g, long long total, cudaStream_t stream) {
-  auto kern = gemm_2cta_kernel<A_MN, B_MN, OutT, GATHER, GLU>;
+  auto kern = gemm_2cta_kernel<A_MN, B_MN, OutT, GATHER, GLU, F8>;
   static bool configured = false;
   if (!configured) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) !=
@@ -876,4 +917,45 @@ extern "C" int lb_gemm_glu_2cta(const void* A, const void* Wg, const void* Wu, v
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   return kind == 0 ? launch2<0, 0, __nv_bfloat16, 0, 1>(tmA, tmG, tmA, tmU, g, total, stream)
                    : launch2<0, 0, __nv_bfloat16, 0, 2>(tmA, tmG, tmA, tmU, g, total, stream);
+}
+
+// lb_gemm_fp8 (gemm_bf16.cu) without bias on CTA pairs; splits given explicitly (>= 1).
+extern "C" int lb_gemm_fp8_2cta(const void* A, const void* B, void* C, int M, int N, int K,
+                                long long lda, long long ldb, long long ldc, int a_e5m2, int b_e5m2,
+                                const float* sa, int sa_stride, const float* sb, int sb_stride,
+                                int out_fp32, int accumulate, int splits, int* status,
+                                void* stream_) {
+  using namespace lb;
+  CUtensorMap tmA, tmB;
+  int rc = make_tmap_2d(&tmA, A, 1, (uint64_t)K, (uint64_t)M, (uint64_t)lda, 2 * BKT, BMc, true);
+  if (rc) return rc;
+  rc = make_tmap_2d(&tmB, B, 1, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, 2 * BKT, BNh, true);
+  if (rc) return rc;
+  const int kb_total = (K + 2 * BK - 1) / (2 * BK);
+  if (splits < 1) splits = 1;
+  if (splits > kb_total) splits = kb_total;
+  const int kb_per = (kb_total + splits - 1) / splits;
+  splits = (kb_total + kb_per - 1) / kb_per;
+  const int tiles_m = (M + 2 * BMc - 1) / (2 * BMc), tiles_n = (N + BNp - 1) / BNp;
+  Args2 g{};
+  g.M = M;
+  g.N = N;
+  g.K = K;
+  g.C = C;
+  g.ldc = ldc;
+  g.accumulate = accumulate || splits > 1;
+  g.splits = splits;
+  g.kb_per_split = kb_per;
+  g.raster_m_fast = tiles_n > tiles_m ? 1 : 0;
+  g.f8_sa = sa;
+  g.f8_sb = sb;
+  g.f8_sa_stride = sa_stride ? 1 : 0;
+  g.f8_sb_stride = sb_stride ? 1 : 0;
+  g.f8_a_e5m2 = a_e5m2 ? 1 : 0;
+  g.f8_b_e5m2 = b_e5m2 ? 1 : 0;
+  g.status = status;
+  const long long total = 1LL * tiles_m * tiles_n * splits;
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
+  return out_fp32 ? launch2<0, 0, float, 0, 0, 1>(tmA, tmB, tmA, tmB, g, total, stream)
+                  : launch2<0, 0, __nv_bfloat16, 0, 0, 1>(tmA, tmB, tmA, tmB, g, total, stream);
 }

@@ -158,3 +158,25 @@ def test_engine_trains_with_fp8_linears(recipe):
     eng.optimizer_step()
     losses = [float(eng.train_step(batch)) for _ in range(8)]
     assert losses[-1] < losses[0], losses
+
+
+@pytest.mark.parametrize("M,N,K", [(256, 256, 16), (257, 264, 272), (700, 520, 1040)])
+@pytest.mark.parametrize("per_row", [True, False])
+@pytest.mark.parametrize("fp32", [True, False])
+def test_cta_pair_kernel_has_the_bits_of_the_one_cta_kernel(M, N, K, per_row, fp32):
+    from lset_b200.ops import fp8 as f8
+
+    torch.manual_seed(M)
+    mode = f8.PER_ROW if per_row else f8.PER_TENSOR
+    a, _ = f8.quantize_fp8(torch.randn(M, K, device="cuda").to(torch.bfloat16), mode)
+    b, _ = f8.quantize_fp8(torch.randn(N, K, device="cuda").to(torch.bfloat16), mode, e5m2=True)
+    lib, out = nv.load(), []
+    before = lib.lb_gemm_use_2cta(-1)
+    for on in (0, 1):
+        lib.lb_gemm_use_2cta(on)
+        out.append(f8.matmul_fp8(a, b, out_dtype=torch.float32 if fp32 else torch.bfloat16))
+        if fp32:
+            f8.matmul_fp8(a, b, out=out[-1], accumulate=True)
+    lib.lb_gemm_use_2cta(before)
+    nv.check_status()
+    assert torch.equal(*out)
