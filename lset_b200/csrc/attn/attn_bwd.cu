@@ -5,10 +5,11 @@
 //             blocks of 64:
 //               S = Q·Kᵀ, dP = dO·Vᵀ (TMEM) -> dS = P∘(dP − delta)·scale (bf16, written over the V
 //               block in smem) -> dQ += dS·K
-//   dK/dV     one 256-thread CTA per (sequence, 128-row KV tile, KV head), walking (query block,
+//   dK/dV     one CTA per (sequence, 128-row KV tile, KV head), walking (query block,
 //             head) pairs through a 3-deep TMA ring, with Sᵀ/dPᵀ double-buffered in TMEM so the
 //             score products of step i+1 run while step i is in the softmax-gradient math:
 //               Sᵀ = K·Qᵀ, dPᵀ = V·dOᵀ (TMEM) -> Pᵀ, dSᵀ (bf16, smem) -> dV += Pᵀ·dO, dK += dSᵀ·Q
+//             Sixteen warps do the math, one requests the loads, one issues the products.
 // Thread t owns accumulator row t % 128 and a half (dQ kernel, 256 threads) or a quarter (dK/dV
 // kernel, 512 threads) of the 64 columns of a score block.
 // The Q / dO / K / V tiles are loaded once by TMA and serve both as K-major operands (contraction
@@ -396,8 +397,9 @@ struct DkvCfg {
   static constexpr int QB_BYTES = 64 * HD * 2;   // one query block of Q or dO
   static constexpr int QBUFS = 3;                // TMA ring depth for (Q, dO) blocks
   static constexpr int PT_BYTES = 128 * 64 * 2;
-  static constexpr int SMEM_BYTES =
-      2 * KV_BYTES + 2 * QBUFS * QB_BYTES + 2 * PT_BYTES + 1024 /*stats*/ + 1024 /*align*/ + 128;
+  static constexpr int STAT_BYTES = QBUFS * 128 * 4;   // lse and delta of a block's 64 queries
+  static constexpr int SMEM_BYTES = 2 * KV_BYTES + 2 * QBUFS * QB_BYTES + 2 * PT_BYTES + STAT_BYTES +
+                                    1024 /*align*/ + 256;
   // TMEM: two (Sᵀ, dPᵀ) buffers of 64 + 64 columns, then the dV and dK accumulators.
   static constexpr int DV_COL = 256;
   static constexpr int DK_COL = 256 + HD;
@@ -405,13 +407,18 @@ struct DkvCfg {
   static_assert(256 + 2 * HD <= 512, "head_dim too large for the dK/dV accumulators");
 };
 
-// 512 threads: thread t owns accumulator row t % 128 and a quarter (t / 128) of the 64 columns of
-// a score block. With 256 threads (two warps per scheduler) the softmax-gradient math of a step
-// was bound by instruction latency, not by the tensor pipe.
-constexpr int kDkvThreads = 512;
+// Math thread t (of 512) owns accumulator row t % 128 and a quarter (t / 128) of the 64 columns of a
+// score block. With 256 (two warps per scheduler) the softmax-gradient math of a step was bound by
+// instruction latency, not by the tensor pipe. Loads and products have warps of their own: when
+// thread 0 issued them between its own loads and stores, all others waited 3800 of the 5600 clocks
+// of a step for its warp. What is left per step is the tensor work (four products of 128 x 64 x HD) and
+// the chain scores -> math -> shared memory -> accumulation, overlapped over two steps.
+// Measured with dQ and delta (us): BWD_FIG
+constexpr int kDkvMath = 512;
+constexpr int kDkvThreads = kDkvMath + 64;
 
 template <int HD>
-__global__ void __launch_bounds__(kDkvThreads)
+__global__ void __launch_bounds__(kDkvThreads, 1)
     attn_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmdO,
                     const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                     AttnBwdArgs a) {
@@ -427,7 +434,7 @@ __global__ void __launch_bounds__(kDkvThreads)
   const int kv0 = kt * 128;
   const int nqb = (len + 63) / 64;
   const int qb_start = a.causal ? (kv0 / 64) : 0;
-  const int n_inner = (nqb - qb_start) * G;
+  const int n_inner = (nqb - qb_start) * G;   // >= 1: the tile's own rows are queries too
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -438,50 +445,40 @@ __global__ void __launch_bounds__(kDkvThreads)
   uint8_t* sdO = sQ + C::QBUFS * C::QB_BYTES;   // [QBUFS]
   uint8_t* sPT = sdO + C::QBUFS * C::QB_BYTES;
   uint8_t* sdST = sPT + C::PT_BYTES;
-  float* sStat = reinterpret_cast<float*>(sdST + C::PT_BYTES);  // [2 bufs][2][64]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sStat + 256);
+  float* sStat = reinterpret_cast<float*>(sdST + C::PT_BYTES);  // [QBUFS][2][64]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sStat + C::STAT_BYTES / 4);
   uint64_t* bar_kv = bars;
-  uint64_t* bar_q = bars + 1;    // [QBUFS]
-  uint64_t* bar_s = bars + 4;    // [2]
-  uint64_t* bar_acc = bars + 6;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 7);
+  uint64_t* bar_q = bars + 1;     // [QBUFS] Q and dO of a step have landed
+  uint64_t* bar_st = bars + 4;    // [QBUFS] its lse and delta are in place
+  uint64_t* bar_e = bars + 7;     // [QBUFS] its accumulation products are complete: slot free
+  uint64_t* bar_s = bars + 10;    // [2] scores of a step are in tensor memory
+  uint64_t* bar_p = bars + 12;    // Pᵀ and dSᵀ of a step are in shared memory
+  uint64_t* bar_acc = bars + 13;  // ... and have been read by its accumulation products
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
-  const int quarter = warp >> 2;  // which 16 of the 64 score columns this thread handles
-  constexpr uint32_t idesc_s = umma_idesc_bf16(128, 64, 0, 0);
-  constexpr uint32_t idesc_acc = umma_idesc_bf16(128, HD, 0, 1);
+  const int lane = tid & 31;
 
-  auto load_q = [&](int i) {
-    const int buf = i % C::QBUFS;
-    const int qb = qb_start + i / G;
-    const int head = hk * G + i % G;
-    mbar_expect_tx(&bar_q[buf], 2 * C::QB_BYTES);
-#pragma unroll
-    for (int p = 0; p < C::PANELS; ++p) {
-      tma_load_2d(sQ + buf * C::QB_BYTES + p * (64 * 128), &tmQ, &bar_q[buf], head * HD + p * 64,
-                  seq0 + qb * 64);
-      tma_load_2d(sdO + buf * C::QB_BYTES + p * (64 * 128), &tmdO, &bar_q[buf], head * HD + p * 64,
-                  seq0 + qb * 64);
-    }
-  };
-  // Barriers, then the K / V tile and the first two (Q, dO) blocks are requested before the TMEM
-  // allocation and the CTA barrier, so the load latency runs under that set-up.
-  if (tid == 0) {
+  if (tid == kDkvMath) {
     mbar_init(bar_kv, 1);
-    for (int i = 0; i < C::QBUFS; ++i) mbar_init(&bar_q[i], 1);
+    for (int i = 0; i < C::QBUFS; ++i) {
+      mbar_init(&bar_q[i], 1);
+      mbar_init(&bar_st[i], 32);
+      mbar_init(&bar_e[i], 1);
+    }
     mbar_init(&bar_s[0], 1);
     mbar_init(&bar_s[1], 1);
+    mbar_init(bar_p, kDkvMath / 32);
     mbar_init(bar_acc, 1);
     mbar_fence_init();
+    // the K / V tile is requested before the TMEM allocation and the CTA barrier
     mbar_expect_tx(bar_kv, 2 * C::KV_BYTES);
 #pragma unroll
     for (int p = 0; p < C::PANELS; ++p) {
       tma_load_2d(sK + p * (128 * 128), &tmK, bar_kv, hk * HD + p * 64, seq0 + kv0);
       tma_load_2d(sV + p * (128 * 128), &tmV, bar_kv, hk * HD + p * 64, seq0 + kv0);
     }
-    if (n_inner > 0) load_q(0);
-    if (n_inner > 1) load_q(1);
   }
   if (warp == 0) {
     tmem_alloc(tmem_slot, C::TMEM_COLS);
@@ -491,141 +488,160 @@ __global__ void __launch_bounds__(kDkvThreads)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem_row = tmem_base + (uint32_t((warp & 3) * 32) << 16);
 
-  // Sᵀ = K·Qᵀ and dPᵀ = V·dOᵀ of inner step i into TMEM buffer i & 1 (issued by thread 0).
-  auto issue_scores = [&](int i) -> bool {
-    const int buf = i % C::QBUFS;
-    if (!mbar_wait(&bar_q[buf], (i / C::QBUFS) & 1)) {
-      report_status(a.status, kStatusTimeoutProducer);
-      return false;
-    }
-    tc_fence_after();
-    const uint32_t ka = smem_u32(sK), va = smem_u32(sV);
-    const uint32_t qa = smem_u32(sQ + buf * C::QB_BYTES);
-    const uint32_t da = smem_u32(sdO + buf * C::QB_BYTES);
-    const uint32_t dcol = tmem_base + (i & 1) * 128;
-#pragma unroll
-    for (int ks = 0; ks < HD / 16; ++ks) {
-      const uint32_t aoff = (ks / 4) * (128 * 128) + (ks % 4) * 32;
-      const uint32_t boff = (ks / 4) * (64 * 128) + (ks % 4) * 32;
-      umma_bf16(dcol, umma_smem_desc(ka + aoff, 16, 1024), umma_smem_desc(qa + boff, 16, 1024),
-                idesc_s, ks > 0 ? 1u : 0u);
-    }
-#pragma unroll
-    for (int ks = 0; ks < HD / 16; ++ks) {
-      const uint32_t aoff = (ks / 4) * (128 * 128) + (ks % 4) * 32;
-      const uint32_t boff = (ks / 4) * (64 * 128) + (ks % 4) * 32;
-      umma_bf16(dcol + 64, umma_smem_desc(va + aoff, 16, 1024), umma_smem_desc(da + boff, 16, 1024),
-                idesc_s, ks > 0 ? 1u : 0u);
-    }
-    umma_commit(&bar_s[i & 1]);
-    return true;
-  };
-
-  const int r = tid & 127;
-  const int kvpos = kv0 + r;
-  const bool row_valid = kvpos < len;
-  bool failed = false;
-  // lse / delta of a block's 64 queries (read by every row), staged one step ahead
-  auto stage_stats = [&](int i) {
-    if (tid < 64) {
-      const int qp = (qb_start + i / G) * 64 + tid;
+  if (warp == kDkvMath / 32) {
+    // -------------------------------------------------------------------- loads
+    bool ok = true;
+    for (int i = 0; i < n_inner; ++i) {
+      const int buf = i % C::QBUFS;
+      ok = __all_sync(0xffffffffu, mbar_wait(&bar_e[buf], ((i / C::QBUFS) & 1) ^ 1u));
+      if (!ok) break;
+      const int qb = qb_start + i / G;
       const int head = hk * G + i % G;
-      const bool v = qp < len;
-      sStat[(i & 1) * 128 + tid] = v ? a.lse[1LL * head * a.T + seq0 + qp] * kLog2eF : 0.f;
-      sStat[(i & 1) * 128 + 64 + tid] = v ? a.delta[1LL * head * a.T + seq0 + qp] : 0.f;
-    }
-  };
-  if (n_inner > 0) stage_stats(0);
-  {
-    const bool ok = mbar_wait(bar_kv, 0);
-    if (__syncthreads_or(!ok)) {
-      report_status(a.status, kStatusTimeoutProducer);
-      failed = true;
-    }
-  }
-  if (!failed && tid == 0 && n_inner > 0) issue_scores(0);
-
-  // One CTA-wide barrier per step (before the accumulation products are issued). Every thread
-  // waits on the mbarriers itself; whether a wait ran out anywhere is agreed on at that barrier.
-  for (int i = 0; i < n_inner && !failed; ++i) {
-    const int sb = i & 1;
-    const int qbuf = i % C::QBUFS;
-    const int qb = qb_start + i / G;
-    bool ok = mbar_wait(&bar_s[sb], (i >> 1) & 1);
-    tc_fence_after();
-    // The score products of the next step go to the tensor pipe now: their TMEM buffer was last
-    // read by step i - 1 (complete in every thread before that step's barrier), and they then run
-    // under this step's softmax-gradient math instead of behind this step's accumulation products.
-    if (tid == 0 && ok && i + 1 < n_inner) ok = issue_scores(i + 1);
-    if (i + 1 < n_inner) stage_stats(i + 1);
-    float pt[16], dst[16];
-    ld_row16(tmem_row + sb * 128 + quarter * 16, pt);
-    ld_row16(tmem_row + sb * 128 + 64 + quarter * 16, dst);
-    {
-      const float* lse2 = sStat + sb * 128 + quarter * 16;
-      const float* dl = lse2 + 64;
-      const int qbase = qb * 64 + quarter * 16;
+      if (lane == 0) {
+        mbar_expect_tx(&bar_q[buf], 2 * C::QB_BYTES);
 #pragma unroll
-      for (int c = 0; c < 16; ++c) {
-        const int qp = qbase + c;
-        const bool valid = row_valid && qp < len && (!a.causal || kvpos <= qp);
-        const float p = valid ? exp2f(pt[c] * a.scale_log2 - lse2[c]) : 0.f;
-        pt[c] = p;
-        dst[c] = p * (dst[c] - dl[c]) * a.scale;
+        for (int p = 0; p < C::PANELS; ++p) {
+          tma_load_2d(sQ + buf * C::QB_BYTES + p * (64 * 128), &tmQ, &bar_q[buf],
+                      head * HD + p * 64, seq0 + qb * 64);
+          tma_load_2d(sdO + buf * C::QB_BYTES + p * (64 * 128), &tmdO, &bar_q[buf],
+                      head * HD + p * 64, seq0 + qb * 64);
+        }
+      }
+      float* st = sStat + buf * 128;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int c = lane + 32 * h;
+        const int qp = qb * 64 + c;
+        const long long at = 1LL * head * a.T + seq0 + qp;
+        st[c] = qp < len ? a.lse[at] * kLog2eF : 0.f;
+        st[64 + c] = qp < len ? a.delta[at] : 0.f;
+      }
+      mbar_arrive(&bar_st[buf]);
+    }
+    if (!ok) {
+      if (lane == 0) report_status(a.status, kStatusTimeoutProducer);
+      const unsigned long long t0 = globaltimer_ns();   // copies in flight land meanwhile
+      while (globaltimer_ns() - t0 < 200000ull) {
       }
     }
-    if (i > 0) {
-      // previous dV/dK products done: the Pᵀ/dSᵀ tiles and ring slot (i-1) % 3 are free
-      ok = mbar_wait(bar_acc, (i - 1) & 1) && ok;
-      tc_fence_after();
-    }
-    if (tid == 0 && ok && i + 2 < n_inner) load_q(i + 2);
-    st_quarter_row_bf16_swz(sPT, r, quarter, pt);
-    st_quarter_row_bf16_swz(sdST, r, quarter, dst);
-    fence_proxy_async_smem();
-    tc_fence_before();
-    if (__syncthreads_or(!ok)) {
-      report_status(a.status, kStatusTimeoutMma);
-      failed = true;
-      break;
-    }
-    if (tid == 0) {
-      tc_fence_after();
-      const uint32_t pa = smem_u32(sPT), sa = smem_u32(sdST);
-      const uint32_t qa = smem_u32(sQ + qbuf * C::QB_BYTES);
-      const uint32_t da = smem_u32(sdO + qbuf * C::QB_BYTES);
+    __syncwarp();
+  } else if (warp == kDkvMath / 32 + 1) {
+    // -------------------------------------------------------------------- products
+    if (lane == 0) {
+      constexpr uint32_t idesc_s = umma_idesc_bf16(128, 64, 0, 0);
+      constexpr uint32_t idesc_acc = umma_idesc_bf16(128, HD, 0, 1);
+      const uint64_t kd = umma_smem_desc(smem_u32(sK), 16, 1024);
+      const uint64_t vd = umma_smem_desc(smem_u32(sV), 16, 1024);
+      const uint64_t pd = umma_smem_desc(smem_u32(sPT), 16, 1024);
+      const uint64_t sd = umma_smem_desc(smem_u32(sdST), 16, 1024);
+      // Step i issues the scores of block i (Sᵀ = K·Qᵀ, dPᵀ = V·dOᵀ, into TMEM buffer i & 1, which
+      // step i - 2's math has read) and the accumulation products of block i - 1.
+      bool ok = mbar_wait(bar_kv, 0);
+      for (int i = 0; i <= n_inner && ok; ++i) {
+        if (i < n_inner) {
+          const int buf = i % C::QBUFS;
+          ok = mbar_wait(&bar_q[buf], (i / C::QBUFS) & 1);
+          if (!ok) break;
+          tc_fence_after();
+          const uint64_t qd = umma_smem_desc(smem_u32(sQ + buf * C::QB_BYTES), 16, 1024);
+          const uint64_t dd = umma_smem_desc(smem_u32(sdO + buf * C::QB_BYTES), 16, 1024);
+          const uint32_t dcol = tmem_base + (i & 1) * 128;
 #pragma unroll
-      for (int ks = 0; ks < 4; ++ks)
-        umma_bf16(tmem_base + C::DV_COL, umma_smem_desc(pa + ks * 32, 16, 1024),
-                  umma_smem_desc(da + ks * 2048, 64 * 128, 1024), idesc_acc,
-                  (i > 0 || ks > 0) ? 1u : 0u);
+          for (int ks = 0; ks < HD / 16; ++ks) {
+            const int aoff = ((ks / 4) * (128 * 128) + (ks % 4) * 32) >> 4;
+            const int boff = ((ks / 4) * (64 * 128) + (ks % 4) * 32) >> 4;
+            umma_bf16(dcol, kd + aoff, qd + boff, idesc_s, ks > 0 ? 1u : 0u);
+          }
 #pragma unroll
-      for (int ks = 0; ks < 4; ++ks)
-        umma_bf16(tmem_base + C::DK_COL, umma_smem_desc(sa + ks * 32, 16, 1024),
-                  umma_smem_desc(qa + ks * 2048, 64 * 128, 1024), idesc_acc,
-                  (i > 0 || ks > 0) ? 1u : 0u);
-      umma_commit(bar_acc);
+          for (int ks = 0; ks < HD / 16; ++ks) {
+            const int aoff = ((ks / 4) * (128 * 128) + (ks % 4) * 32) >> 4;
+            const int boff = ((ks / 4) * (64 * 128) + (ks % 4) * 32) >> 4;
+            umma_bf16(dcol + 64, vd + aoff, dd + boff, idesc_s, ks > 0 ? 1u : 0u);
+          }
+          umma_commit(&bar_s[i & 1]);
+        }
+        if (i > 0) {
+          const int j = i - 1, buf = j % C::QBUFS;
+          ok = mbar_wait(bar_p, j & 1);
+          if (!ok) break;
+          tc_fence_after();
+          const uint64_t qd = umma_smem_desc(smem_u32(sQ + buf * C::QB_BYTES), 64 * 128, 1024);
+          const uint64_t dd = umma_smem_desc(smem_u32(sdO + buf * C::QB_BYTES), 64 * 128, 1024);
+#pragma unroll
+          for (int ks = 0; ks < 4; ++ks)
+            umma_bf16(tmem_base + C::DV_COL, pd + ks * 2, dd + ks * (2048 >> 4), idesc_acc,
+                      (j > 0 || ks > 0) ? 1u : 0u);
+#pragma unroll
+          for (int ks = 0; ks < 4; ++ks)
+            umma_bf16(tmem_base + C::DK_COL, sd + ks * 2, qd + ks * (2048 >> 4), idesc_acc,
+                      (j > 0 || ks > 0) ? 1u : 0u);
+          umma_commit(bar_acc);
+          umma_commit(&bar_e[buf]);
+        }
+      }
+      if (!ok) report_status(a.status, kStatusTimeoutMma);
     }
-  }
-  if (!failed && n_inner > 0) {
-    const bool ok = mbar_wait(bar_acc, (n_inner - 1) & 1);
-    if (__syncthreads_or(!ok)) {
-      report_status(a.status, kStatusTimeoutMma);
-      failed = true;
+    __syncwarp();
+  } else {
+    // -------------------------------------------------------------------- softmax gradient
+    const int quarter = warp >> 2;  // which 16 of the 64 score columns this thread handles
+    const uint32_t tmem_row = tmem_base + (uint32_t((warp & 3) * 32) << 16);
+    const int r = tid & 127;
+    const int kvpos = kv0 + r;
+    const bool row_valid = kvpos < len;
+    bool ok = true;
+    for (int i = 0; i < n_inner; ++i) {
+      const int sb = i & 1, buf = i % C::QBUFS;
+      ok = mbar_wait(&bar_st[buf], (i / C::QBUFS) & 1) && mbar_wait(&bar_s[sb], (i >> 1) & 1);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc_fence_after();
+      uint32_t t0[16], t1[16];
+      tmem_ld_32x32b_x16(tmem_row + sb * 128 + quarter * 16, t0);
+      tmem_ld_32x32b_x16(tmem_row + sb * 128 + 64 + quarter * 16, t1);
+      tmem_ld_wait();
+      float pt[16], dst[16];
+      {
+        const float* lse2 = sStat + buf * 128 + quarter * 16;
+        const float* dl = lse2 + 64;
+        const int qbase = (qb_start + i / G) * 64 + quarter * 16;
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
+          const int qp = qbase + c;
+          const bool valid = row_valid && qp < len && (!a.causal || kvpos <= qp);
+          const float p = valid ? exp2f(__uint_as_float(t0[c]) * a.scale_log2 - lse2[c]) : 0.f;
+          pt[c] = p;
+          dst[c] = p * (__uint_as_float(t1[c]) - dl[c]) * a.scale;
+        }
+      }
+      if (i > 0) {
+        // the previous step's products have read the Pᵀ / dSᵀ tiles
+        ok = __all_sync(0xffffffffu, mbar_wait(bar_acc, (i - 1) & 1));
+        if (!ok) break;
+      }
+      st_quarter_row_bf16_swz(sPT, r, quarter, pt);
+      st_quarter_row_bf16_swz(sdST, r, quarter, dst);
+      fence_proxy_async_smem();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_p);
     }
-  }
-  if (!failed && n_inner > 0) {
-    tc_fence_after();
-    const long long tok = 1LL * seq0 + kvpos;
-    store_acc_cols16<HD / 4>(tmem_row + C::DV_COL + quarter * (HD / 4),
-                             a.dV + tok * a.lddv + hk * HD + quarter * (HD / 4), row_valid);
-    store_acc_cols16<HD / 4>(tmem_row + C::DK_COL + quarter * (HD / 4),
-                             a.dK + tok * a.lddk + hk * HD + quarter * (HD / 4), row_valid);
+    if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_acc, (n_inner - 1) & 1));
+    if (ok) {
+      tc_fence_after();
+      const long long tok = 1LL * seq0 + kvpos;
+      store_acc_cols16<HD / 4>(tmem_row + C::DV_COL + quarter * (HD / 4),
+                               a.dV + tok * a.lddv + hk * HD + quarter * (HD / 4), row_valid);
+      store_acc_cols16<HD / 4>(tmem_row + C::DK_COL + quarter * (HD / 4),
+                               a.dK + tok * a.lddk + hk * HD + quarter * (HD / 4), row_valid);
+    } else if (lane == 0) {
+      report_status(a.status, kStatusTimeoutEpilogue);
+    }
   }
   tc_fence_before();
   __syncthreads();
+  tc_fence_after();
   if (warp == 0) tmem_dealloc(tmem_base, C::TMEM_COLS);
 }
 
