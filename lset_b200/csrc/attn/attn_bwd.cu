@@ -5,11 +5,12 @@
 //             blocks of 64:
 //               S = Q·Kᵀ, dP = dO·Vᵀ (TMEM) -> dS = P∘(dP − delta)·scale (bf16, written over the V
 //               block in smem) -> dQ += dS·K
-//   dK/dV     one CTA per (sequence, 128-row KV tile, KV head), walking (query block,
+//   dK/dV     work item = (sequence, 128-row KV tile, KV head), walking (query block,
 //             head) pairs through a 3-deep TMA ring, with Sᵀ/dPᵀ double-buffered in TMEM so the
 //             score products of step i+1 run while step i is in the softmax-gradient math:
 //               Sᵀ = K·Qᵀ, dPᵀ = V·dOᵀ (TMEM) -> Pᵀ, dSᵀ (bf16, smem) -> dV += Pᵀ·dO, dK += dSᵀ·Q
-//             Sixteen warps do the math, one requests the loads, one issues the products.
+//             Sixteen warps do the math, one requests the loads, one issues the products; the grid
+//             is persistent, and an item's loads run under the end of the one before it.
 // Thread t owns accumulator row t % 128 and a half (dQ kernel, 256 threads) or a quarter (dK/dV
 // kernel, 512 threads) of the 64 columns of a score block.
 // The Q / dO / K / V tiles are loaded once by TMA and serve both as K-major operands (contraction
@@ -75,6 +76,8 @@ struct AttnBwdArgs {
   float scale_log2;  // scale * log2(e)
   int causal;
   int* status;
+  int capacity;      // of the plan
+  unsigned* counter; // its work counter (persistent kernel; see finish_grid)
 };
 
 __device__ __forceinline__ void ld_row32(uint32_t taddr, float (&s)[32]) {
@@ -413,9 +416,24 @@ struct DkvCfg {
 // thread 0 issued them between its own loads and stores, all others waited 3800 of the 5600 clocks
 // of a step for its warp. What is left per step is the tensor work (four products of 128 x 64 x HD) and
 // the chain scores -> math -> shared memory -> accumulation, overlapped over two steps.
-// Measured with dQ and delta (us): BWD_FIG
+// Measured (whole backward, us; products issued by thread 0 -> warps of their own -> persistent grid):
+//   64 sequences of 16..64 and 64 of 128..512 tokens, 16/8 heads of 128   588 -> 484 -> 458
+//   8 x 2048 tokens, 16/8 heads                                          1341 -> 972 -> 936
+//   32 of 256..1024 tokens, 32/8 heads                                   1438 -> 1062 -> 1049
 constexpr int kDkvMath = 512;
 constexpr int kDkvThreads = kDkvMath + 64;
+
+// A work item of the persistent grid: one 128-row KV tile (hk < 0: no more items), its first query
+// block and its steps (query blocks x heads of the group).
+struct DkvItem {
+  int hk, seq0, len, kv0;
+};
+__device__ __forceinline__ int dkv_first(const DkvItem& t, int causal) {
+  return causal ? t.kv0 / 64 : 0;
+}
+__device__ __forceinline__ int dkv_steps(const DkvItem& t, int causal, int G) {
+  return ((t.len + 63) / 64 - dkv_first(t, causal)) * G;   // >= 1: the tile's rows are queries too
+}
 
 template <int HD>
 __global__ void __launch_bounds__(kDkvThreads, 1)
@@ -423,19 +441,7 @@ __global__ void __launch_bounds__(kDkvThreads, 1)
                     const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                     AttnBwdArgs a) {
   using C = DkvCfg<HD>;
-  AttnPlanView plan{a.plan};
-  if (int(blockIdx.x) >= plan.count()) return;
-  const int b = plan.seq(blockIdx.x);
-  const int kt = plan.tile(blockIdx.x);
-  const int hk = blockIdx.y;
   const int G = a.Hq / a.Hk;
-  const int seq0 = a.seq_start[b];
-  const int len = a.seq_end[b] - seq0;
-  const int kv0 = kt * 128;
-  const int nqb = (len + 63) / 64;
-  const int qb_start = a.causal ? (kv0 / 64) : 0;
-  const int n_inner = (nqb - qb_start) * G;   // >= 1: the tile's own rows are queries too
-
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -454,7 +460,11 @@ __global__ void __launch_bounds__(kDkvThreads, 1)
   uint64_t* bar_s = bars + 10;    // [2] scores of a step are in tensor memory
   uint64_t* bar_p = bars + 12;    // Pᵀ and dSᵀ of a step are in shared memory
   uint64_t* bar_acc = bars + 13;  // ... and have been read by its accumulation products
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
+  uint64_t* bar_kve = bars + 14;  // the item's last scores are complete: K and V may be replaced
+  uint64_t* work_full = bars + 15;   // [2]
+  uint64_t* work_empty = bars + 17;  // [2]
+  DkvItem* s_work = reinterpret_cast<DkvItem*>(bars + 20);  // [2]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_work + 2);
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
@@ -471,14 +481,12 @@ __global__ void __launch_bounds__(kDkvThreads, 1)
     mbar_init(&bar_s[1], 1);
     mbar_init(bar_p, kDkvMath / 32);
     mbar_init(bar_acc, 1);
-    mbar_fence_init();
-    // the K / V tile is requested before the TMEM allocation and the CTA barrier
-    mbar_expect_tx(bar_kv, 2 * C::KV_BYTES);
-#pragma unroll
-    for (int p = 0; p < C::PANELS; ++p) {
-      tma_load_2d(sK + p * (128 * 128), &tmK, bar_kv, hk * HD + p * 64, seq0 + kv0);
-      tma_load_2d(sV + p * (128 * 128), &tmV, bar_kv, hk * HD + p * 64, seq0 + kv0);
+    mbar_init(bar_kve, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&work_full[i], 1);
+      mbar_init(&work_empty[i], kDkvMath / 32 + 1);   // the math warps and the products' issuer
     }
+    mbar_fence_init();
   }
   if (warp == 0) {
     tmem_alloc(tmem_slot, C::TMEM_COLS);
@@ -490,35 +498,74 @@ __global__ void __launch_bounds__(kDkvThreads, 1)
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == kDkvMath / 32) {
-    // -------------------------------------------------------------------- loads
+    // -------------------------------------------------------------------- work items, loads
+    AttnPlanView plan{a.plan};
+    const int total = plan.count() * a.Hk;
+    int w = int(blockIdx.x), n = 0;   // n: steps so far, over all items
     bool ok = true;
-    for (int i = 0; i < n_inner; ++i) {
-      const int buf = i % C::QBUFS;
-      ok = __all_sync(0xffffffffu, mbar_wait(&bar_e[buf], ((i / C::QBUFS) & 1) ^ 1u));
-      if (!ok) break;
-      const int qb = qb_start + i / G;
-      const int head = hk * G + i % G;
-      if (lane == 0) {
-        mbar_expect_tx(&bar_q[buf], 2 * C::QB_BYTES);
+    for (int it = 0; ok; ++it) {
+      DkvItem t{-1, 0, 0, 0};
+      if (w < total) {                // heads vary fastest; the first KV tiles have the most queries
+        const int i = w / a.Hk;
+        const int b = plan.seq(i);
+        t.hk = w - i * a.Hk;
+        t.seq0 = a.seq_start[b];
+        t.len = a.seq_end[b] - t.seq0;
+        t.kv0 = plan.tile(i) * 128;
+      }
+      const int slot = it & 1;
+      ok = mbar_wait(&work_empty[slot], ((it >> 1) & 1) ^ 1u);
+      if (ok && lane == 0) {
+        s_work[slot] = t;
+        mbar_arrive(&work_full[slot]);
+      }
+      if (!ok || t.hk < 0) break;
+      // K and V of the item as soon as the last one's scores are complete: under its last math,
+      // its accumulation products and its store
+      ok = mbar_wait(bar_kve, (it & 1) ^ 1u);
+      if (ok && lane == 0) {
+        mbar_expect_tx(bar_kv, 2 * C::KV_BYTES);
 #pragma unroll
         for (int p = 0; p < C::PANELS; ++p) {
-          tma_load_2d(sQ + buf * C::QB_BYTES + p * (64 * 128), &tmQ, &bar_q[buf],
-                      head * HD + p * 64, seq0 + qb * 64);
-          tma_load_2d(sdO + buf * C::QB_BYTES + p * (64 * 128), &tmdO, &bar_q[buf],
-                      head * HD + p * 64, seq0 + qb * 64);
+          tma_load_2d(sK + p * (128 * 128), &tmK, bar_kv, t.hk * HD + p * 64, t.seq0 + t.kv0);
+          tma_load_2d(sV + p * (128 * 128), &tmV, bar_kv, t.hk * HD + p * 64, t.seq0 + t.kv0);
         }
       }
-      float* st = sStat + buf * 128;
+      const int qb_start = dkv_first(t, a.causal), steps = dkv_steps(t, a.causal, G);
+      for (int i = 0; i < steps && ok; ++i, ++n) {
+        const int buf = n % C::QBUFS;
+        ok = mbar_wait(&bar_e[buf], ((n / C::QBUFS) & 1) ^ 1u);
+        if (!ok) break;
+        const int qb = qb_start + i / G;
+        const int head = t.hk * G + i % G;
+        if (lane == 0) {
+          mbar_expect_tx(&bar_q[buf], 2 * C::QB_BYTES);
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int c = lane + 32 * h;
-        const int qp = qb * 64 + c;
-        const long long at = 1LL * head * a.T + seq0 + qp;
-        st[c] = qp < len ? a.lse[at] * kLog2eF : 0.f;
-        st[64 + c] = qp < len ? a.delta[at] : 0.f;
+          for (int p = 0; p < C::PANELS; ++p) {
+            tma_load_2d(sQ + buf * C::QB_BYTES + p * (64 * 128), &tmQ, &bar_q[buf],
+                        head * HD + p * 64, t.seq0 + qb * 64);
+            tma_load_2d(sdO + buf * C::QB_BYTES + p * (64 * 128), &tmdO, &bar_q[buf],
+                        head * HD + p * 64, t.seq0 + qb * 64);
+          }
+        }
+        float* st = sStat + buf * 128;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int c = lane + 32 * h;
+          const int qp = qb * 64 + c;
+          const long long at = 1LL * head * a.T + t.seq0 + qp;
+          st[c] = qp < t.len ? a.lse[at] * kLog2eF : 0.f;
+          st[64 + c] = qp < t.len ? a.delta[at] : 0.f;
+        }
+        mbar_arrive(&bar_st[buf]);
       }
-      mbar_arrive(&bar_st[buf]);
+      // the next item is drawn when this one's last loads are out, three steps before its end: drawn
+      // earlier it would wait here while other SMs run out of work
+      unsigned drawn = 0;
+      if (lane == 0) drawn = atomicAdd(a.counter, 1u);
+      w = int(__shfl_sync(0xffffffffu, drawn, 0)) + int(gridDim.x);
     }
+    ok = __all_sync(0xffffffffu, ok);
     if (!ok) {
       if (lane == 0) report_status(a.status, kStatusTimeoutProducer);
       const unsigned long long t0 = globaltimer_ns();   // copies in flight land meanwhile
@@ -537,48 +584,62 @@ __global__ void __launch_bounds__(kDkvThreads, 1)
       const uint64_t sd = umma_smem_desc(smem_u32(sdST), 16, 1024);
       // Step i issues the scores of block i (Sᵀ = K·Qᵀ, dPᵀ = V·dOᵀ, into TMEM buffer i & 1, which
       // step i - 2's math has read) and the accumulation products of block i - 1.
-      bool ok = mbar_wait(bar_kv, 0);
-      for (int i = 0; i <= n_inner && ok; ++i) {
-        if (i < n_inner) {
-          const int buf = i % C::QBUFS;
-          ok = mbar_wait(&bar_q[buf], (i / C::QBUFS) & 1);
-          if (!ok) break;
-          tc_fence_after();
-          const uint64_t qd = umma_smem_desc(smem_u32(sQ + buf * C::QB_BYTES), 16, 1024);
-          const uint64_t dd = umma_smem_desc(smem_u32(sdO + buf * C::QB_BYTES), 16, 1024);
-          const uint32_t dcol = tmem_base + (i & 1) * 128;
+      int n = 0;   // steps so far, over all items
+      bool ok = true;
+      for (int it = 0; ok; ++it) {
+        const int slot = it & 1;
+        ok = mbar_wait(&work_full[slot], (it >> 1) & 1);
+        if (!ok) break;
+        const DkvItem t = s_work[slot];
+        mbar_arrive(&work_empty[slot]);
+        if (t.hk < 0) break;
+        const int steps = dkv_steps(t, a.causal, G);
+        ok = mbar_wait(bar_kv, it & 1);
+#pragma unroll 1
+        for (int i = 0; i <= steps && ok; ++i) {
+          if (i < steps) {
+            const int buf = (n + i) % C::QBUFS;
+            ok = mbar_wait(&bar_q[buf], ((n + i) / C::QBUFS) & 1);
+            if (!ok) break;
+            tc_fence_after();
+            const uint64_t qd = umma_smem_desc(smem_u32(sQ + buf * C::QB_BYTES), 16, 1024);
+            const uint64_t dd = umma_smem_desc(smem_u32(sdO + buf * C::QB_BYTES), 16, 1024);
+            const uint32_t dcol = tmem_base + ((n + i) & 1) * 128;
 #pragma unroll
-          for (int ks = 0; ks < HD / 16; ++ks) {
-            const int aoff = ((ks / 4) * (128 * 128) + (ks % 4) * 32) >> 4;
-            const int boff = ((ks / 4) * (64 * 128) + (ks % 4) * 32) >> 4;
-            umma_bf16(dcol, kd + aoff, qd + boff, idesc_s, ks > 0 ? 1u : 0u);
+            for (int ks = 0; ks < HD / 16; ++ks) {
+              const int aoff = ((ks / 4) * (128 * 128) + (ks % 4) * 32) >> 4;
+              const int boff = ((ks / 4) * (64 * 128) + (ks % 4) * 32) >> 4;
+              umma_bf16(dcol, kd + aoff, qd + boff, idesc_s, ks > 0 ? 1u : 0u);
+            }
+#pragma unroll
+            for (int ks = 0; ks < HD / 16; ++ks) {
+              const int aoff = ((ks / 4) * (128 * 128) + (ks % 4) * 32) >> 4;
+              const int boff = ((ks / 4) * (64 * 128) + (ks % 4) * 32) >> 4;
+              umma_bf16(dcol + 64, vd + aoff, dd + boff, idesc_s, ks > 0 ? 1u : 0u);
+            }
+            umma_commit(&bar_s[(n + i) & 1]);
+            if (i + 1 == steps) umma_commit(bar_kve);
           }
+          if (i > 0) {
+            const int j = i - 1, buf = (n + j) % C::QBUFS;
+            ok = mbar_wait(bar_p, (n + j) & 1);
+            if (!ok) break;
+            tc_fence_after();
+            const uint64_t qd = umma_smem_desc(smem_u32(sQ + buf * C::QB_BYTES), 64 * 128, 1024);
+            const uint64_t dd = umma_smem_desc(smem_u32(sdO + buf * C::QB_BYTES), 64 * 128, 1024);
 #pragma unroll
-          for (int ks = 0; ks < HD / 16; ++ks) {
-            const int aoff = ((ks / 4) * (128 * 128) + (ks % 4) * 32) >> 4;
-            const int boff = ((ks / 4) * (64 * 128) + (ks % 4) * 32) >> 4;
-            umma_bf16(dcol + 64, vd + aoff, dd + boff, idesc_s, ks > 0 ? 1u : 0u);
+            for (int ks = 0; ks < 4; ++ks)
+              umma_bf16(tmem_base + C::DV_COL, pd + ks * 2, dd + ks * (2048 >> 4), idesc_acc,
+                        (j > 0 || ks > 0) ? 1u : 0u);
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks)
+              umma_bf16(tmem_base + C::DK_COL, sd + ks * 2, qd + ks * (2048 >> 4), idesc_acc,
+                        (j > 0 || ks > 0) ? 1u : 0u);
+            umma_commit(bar_acc);
+            umma_commit(&bar_e[buf]);
           }
-          umma_commit(&bar_s[i & 1]);
         }
-        if (i > 0) {
-          const int j = i - 1, buf = j % C::QBUFS;
-          ok = mbar_wait(bar_p, j & 1);
-          if (!ok) break;
-          tc_fence_after();
-          const uint64_t qd = umma_smem_desc(smem_u32(sQ + buf * C::QB_BYTES), 64 * 128, 1024);
-          const uint64_t dd = umma_smem_desc(smem_u32(sdO + buf * C::QB_BYTES), 64 * 128, 1024);
-#pragma unroll
-          for (int ks = 0; ks < 4; ++ks)
-            umma_bf16(tmem_base + C::DV_COL, pd + ks * 2, dd + ks * (2048 >> 4), idesc_acc,
-                      (j > 0 || ks > 0) ? 1u : 0u);
-#pragma unroll
-          for (int ks = 0; ks < 4; ++ks)
-            umma_bf16(tmem_base + C::DK_COL, sd + ks * 2, qd + ks * (2048 >> 4), idesc_acc,
-                      (j > 0 || ks > 0) ? 1u : 0u);
-          umma_commit(bar_acc);
-          umma_commit(&bar_e[buf]);
-        }
+        n += steps;
       }
       if (!ok) report_status(a.status, kStatusTimeoutMma);
     }
@@ -588,61 +649,78 @@ __global__ void __launch_bounds__(kDkvThreads, 1)
     const int quarter = warp >> 2;  // which 16 of the 64 score columns this thread handles
     const uint32_t tmem_row = tmem_base + (uint32_t((warp & 3) * 32) << 16);
     const int r = tid & 127;
-    const int kvpos = kv0 + r;
-    const bool row_valid = kvpos < len;
-    bool ok = true;
-    for (int i = 0; i < n_inner; ++i) {
-      const int sb = i & 1, buf = i % C::QBUFS;
-      ok = mbar_wait(&bar_st[buf], (i / C::QBUFS) & 1) && mbar_wait(&bar_s[sb], (i >> 1) & 1);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
-      tc_fence_after();
-      uint32_t t0[16], t1[16];
-      tmem_ld_32x32b_x16(tmem_row + sb * 128 + quarter * 16, t0);
-      tmem_ld_32x32b_x16(tmem_row + sb * 128 + 64 + quarter * 16, t1);
-      tmem_ld_wait();
-      float pt[16], dst[16];
-      {
-        const float* lse2 = sStat + buf * 128 + quarter * 16;
-        const float* dl = lse2 + 64;
-        const int qbase = (qb_start + i / G) * 64 + quarter * 16;
-#pragma unroll
-        for (int c = 0; c < 16; ++c) {
-          const int qp = qbase + c;
-          const bool valid = row_valid && qp < len && (!a.causal || kvpos <= qp);
-          const float p = valid ? exp2f(__uint_as_float(t0[c]) * a.scale_log2 - lse2[c]) : 0.f;
-          pt[c] = p;
-          dst[c] = p * (__uint_as_float(t1[c]) - dl[c]) * a.scale;
-        }
+    int n = 0;   // steps so far, over all items
+    for (int it = 0;; ++it) {
+      const int slot = it & 1;
+      bool ok = __all_sync(0xffffffffu, mbar_wait(&work_full[slot], (it >> 1) & 1));
+      if (!ok) {
+        if (lane == 0) report_status(a.status, kStatusTimeoutEpilogue);
+        break;
       }
-      if (i > 0) {
-        // the previous step's products have read the Pᵀ / dSᵀ tiles
-        ok = __all_sync(0xffffffffu, mbar_wait(bar_acc, (i - 1) & 1));
-        if (!ok) break;
-      }
-      st_quarter_row_bf16_swz(sPT, r, quarter, pt);
-      st_quarter_row_bf16_swz(sdST, r, quarter, dst);
-      fence_proxy_async_smem();
-      tc_fence_before();
+      const DkvItem t = s_work[slot];
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar_p);
-    }
-    if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_acc, (n_inner - 1) & 1));
-    if (ok) {
-      tc_fence_after();
-      const long long tok = 1LL * seq0 + kvpos;
-      store_acc_cols16<HD / 4>(tmem_row + C::DV_COL + quarter * (HD / 4),
-                               a.dV + tok * a.lddv + hk * HD + quarter * (HD / 4), row_valid);
-      store_acc_cols16<HD / 4>(tmem_row + C::DK_COL + quarter * (HD / 4),
-                               a.dK + tok * a.lddk + hk * HD + quarter * (HD / 4), row_valid);
-    } else if (lane == 0) {
-      report_status(a.status, kStatusTimeoutEpilogue);
+      if (lane == 0) mbar_arrive(&work_empty[slot]);
+      if (t.hk < 0) break;
+      const int qb_start = dkv_first(t, a.causal), steps = dkv_steps(t, a.causal, G);
+      const int kvpos = t.kv0 + r, len = t.len;
+      const bool row_valid = kvpos < len;
+      for (int i = 0; i < steps; ++i, ++n) {
+        const int sb = n & 1, buf = n % C::QBUFS;
+        ok = mbar_wait(&bar_st[buf], (n / C::QBUFS) & 1) && mbar_wait(&bar_s[sb], (n >> 1) & 1);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after();
+        uint32_t t0[16], t1[16];
+        tmem_ld_32x32b_x16(tmem_row + sb * 128 + quarter * 16, t0);
+        tmem_ld_32x32b_x16(tmem_row + sb * 128 + 64 + quarter * 16, t1);
+        tmem_ld_wait();
+        float pt[16], dst[16];
+        {
+          const float* lse2 = sStat + buf * 128 + quarter * 16;
+          const float* dl = lse2 + 64;
+          const int qbase = (qb_start + i / G) * 64 + quarter * 16;
+#pragma unroll
+          for (int c = 0; c < 16; ++c) {
+            const int qp = qbase + c;
+            const bool valid = row_valid && qp < len && (!a.causal || kvpos <= qp);
+            const float p = valid ? exp2f(__uint_as_float(t0[c]) * a.scale_log2 - lse2[c]) : 0.f;
+            pt[c] = p;
+            dst[c] = p * (__uint_as_float(t1[c]) - dl[c]) * a.scale;
+          }
+        }
+        if (n > 0) {
+          // the previous step's products have read the Pᵀ / dSᵀ tiles
+          ok = __all_sync(0xffffffffu, mbar_wait(bar_acc, (n - 1) & 1));
+          if (!ok) break;
+        }
+        st_quarter_row_bf16_swz(sPT, r, quarter, pt);
+        st_quarter_row_bf16_swz(sdST, r, quarter, dst);
+        fence_proxy_async_smem();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_p);
+      }
+      if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar_acc, (n - 1) & 1));
+      if (ok) {
+        tc_fence_after();
+        const long long tok = 1LL * t.seq0 + kvpos;
+        store_acc_cols16<HD / 4>(tmem_row + C::DV_COL + quarter * (HD / 4),
+                                 a.dV + tok * a.lddv + t.hk * HD + quarter * (HD / 4), row_valid);
+        store_acc_cols16<HD / 4>(tmem_row + C::DK_COL + quarter * (HD / 4),
+                                 a.dK + tok * a.lddk + t.hk * HD + quarter * (HD / 4), row_valid);
+        // (the next item's first products into these accumulators wait for bar_p, behind the reads)
+        tc_fence_before();
+      } else {
+        if (lane == 0) report_status(a.status, kStatusTimeoutEpilogue);
+        break;
+      }
     }
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   if (warp == 0) tmem_dealloc(tmem_base, C::TMEM_COLS);
+  finish_grid(a.plan, a.capacity);
 }
 
 template <int HD>
@@ -696,7 +774,11 @@ int launch_bwd(const void* dO, long long lddo, const void* q, long long ldq, con
       configured = true;
     }
     a.plan = plan_kv;
-    kern<<<dim3(cap_kv, a.Hk), kDkvThreads, C::SMEM_BYTES, st>>>(tmQ, tmdO, tmK, tmV, a);
+    a.capacity = cap_kv;
+    a.counter = reinterpret_cast<unsigned*>(const_cast<int*>(plan_kv)) + 1 + 2 * cap_kv;
+    const long long upper = 1LL * cap_kv * a.Hk;
+    const int grid = int(upper < row_num_sms() ? upper : row_num_sms());
+    kern<<<grid, kDkvThreads, C::SMEM_BYTES, st>>>(tmQ, tmdO, tmK, tmV, a);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
@@ -721,7 +803,7 @@ extern "C" int lb_attn_bwd(const void* dO, long long lddo, const void* q, long l
   if (G != 1 && G != 2 && G != 4 && G != 8) return -3;
   if ((lddo | ldq | ldk | ldv | ldo | lddq | lddk | lddv) & 7) return -3;
   AttnBwdArgs a{seq_start, seq_end, nullptr, lse, delta, (bf16*)dq, lddq, (bf16*)dk, lddk, (bf16*)dv, lddv,
-                T, Hq, Hk, softmax_scale, softmax_scale * kLog2eF, causal, status};
+                T, Hq, Hk, softmax_scale, softmax_scale * kLog2eF, causal, status, 0, nullptr};
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (hd != 128 && hd != 64) return -3;
   // gradient rows of tokens behind the last sequence are written by no kernel below

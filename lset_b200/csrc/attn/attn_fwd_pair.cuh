@@ -244,7 +244,6 @@ __global__ void __launch_bounds__(kPairThreads, 1)
         s_work[slot] = t;
         mbar_arrive(&work_full[slot]);
         if (t.hk < 0) break;
-        const unsigned drawn = atomicAdd(a.counter, 1u);   // answered while the loads are requested
         if (!pair_wait(q_empty, (it & 1) ^ 1u)) {
           report_status(a.status, kStatusTimeoutProducer);
           break;
@@ -275,7 +274,9 @@ __global__ void __launch_bounds__(kPairThreads, 1)
           ++n;
         }
         if (!ok) report_status(a.status, kStatusTimeoutProducer);
-        w = int(drawn) + int(gridDim.x);
+        // the next item is drawn when this one's last loads are out: drawn earlier it would wait
+        // here while other SMs run out of work
+        w = int(atomicAdd(a.counter, 1u)) + int(gridDim.x);
       }
       if (!ok) {
         const unsigned long long t0 = globaltimer_ns();   // copies in flight land meanwhile
