@@ -166,7 +166,7 @@ int lin_fwd(const LbLinear& l, const __nv_bfloat16* x, long long ldx, __nv_bfloa
     g.bias[0] = bias;
     g.status = c->status;
     g.stream = c->stream;
-    if (small_wins(&g, lb_gemm_tile_cost(T, l.n_out, l.k_in, lb_gemm_2cta_pairs())))
+    if (small_wins(&g, lb_gemm_tile_cost(T, l.n_out, l.k_in, 0)))
       return lb_gemm_small(&g);
   }
   return lb_gemm_bf16(x, l.w, y, T, l.n_out, l.k_in, ldx, l.ldw, ldy, 0, 0, 0, 0, bias, 1, 0,
@@ -255,7 +255,7 @@ int proj_fwd(const LbProjection& p, const __nv_bfloat16* x, long long ldx, __nv_
       g.bias[i] = bias != nullptr ? bias[i] : nullptr;
       g.ldc[i] = p.width;
       col += p.part[i].n_out;
-      apart += lb_gemm_tile_cost(T, p.part[i].n_out, p.part[i].k_in, lb_gemm_2cta_pairs());
+      apart += lb_gemm_tile_cost(T, p.part[i].n_out, p.part[i].k_in, 0);
     }
     g.A = x;
     g.lda = ldx;
@@ -305,7 +305,7 @@ int glu_proj_fwd(const LbBlockDesc* d, const __nv_bfloat16* x, __nv_bfloat16* gu
     g.b_ready = 1;
     double apart = 3.0 + 6.0 * T * I / 5e6;  // the activation: a launch, three passes at 5 TB/s
     for (int i = 0; i < p.n; ++i)
-      apart += lb_gemm_tile_cost(T, p.part[i].n_out, d->H, lb_gemm_2cta_pairs());
+      apart += lb_gemm_tile_cost(T, p.part[i].n_out, d->H, 0);
     if (small_wins(&g, apart)) {
       t_fewer += p.n;
       return lb_gemm_small(&g);
@@ -334,8 +334,8 @@ int proj_bwd(const LbProjection& p, const __nv_bfloat16* dy, const __nv_bfloat16
     double apart = 0.0, apart_w = 0.0;
     bool all_w = true;
     for (int i = 0; i < p.n; ++i) {
-      apart += lb_gemm_tile_cost(T, K, p.part[i].n_out, lb_gemm_2cta_pairs());
-      apart_w += lb_gemm_tile_cost(p.part[i].n_out, K, T, lb_gemm_2cta_pairs());
+      apart += lb_gemm_tile_cost(T, K, p.part[i].n_out, 0);
+      apart_w += lb_gemm_tile_cost(p.part[i].n_out, K, T, 1);
       all_w = all_w && p.part[i].wgrad != nullptr;
     }
     LbSmallGemm g = small_gemm(p, kParallelK, c);

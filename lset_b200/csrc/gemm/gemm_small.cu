@@ -561,15 +561,6 @@ extern "C" double lb_gemm_small_plan(const LbSmallGemm* p, int* bn_out, int* spl
   return best;
 }
 
-// The same for one product of lb_gemm_bf16_2cta: measured 14.5 us (of them 5 the measurement's) and
-// a 256 x 256 tile per pair and wave at 0.27 us a 64-deep k-block.
-extern "C" double lb_gemm_tile_cost(int M, int N, int K, int pairs) {
-  const double tiles = double(ceil_div(M, 256)) * ceil_div(N, 256);
-  const double waves = tiles < pairs ? 1.0 : double(ceil_div(int(tiles), pairs));
-  const int kb = ceil_div(K, BK);
-  return 10.0 + waves * kb * 0.27;
-}
-
 extern "C" int lb_gemm_small(const LbSmallGemm* p) {
   if (p->M <= 0 || p->N <= 0) return 0;
   if (!shape_ok(p)) return -3;

@@ -35,9 +35,10 @@ struct LbSmallGemm {
 };
 
 // Modelled time of the product on this kernel and the tile width and split it would take (a negative
-// value: not taken), and of one product on the CTA-pair kernel.
+// value: not taken), and of one product on the CTA-pair kernel (fp32: a weight gradient, whose
+// contraction that kernel splits).
 double lb_gemm_small_plan(const LbSmallGemm* p, int* bn, int* splits);
-double lb_gemm_tile_cost(int M, int N, int K, int pairs);
+double lb_gemm_tile_cost(int M, int N, int K, int fp32);
 int lb_gemm_small(const LbSmallGemm* p);
 
 }  // extern "C"
