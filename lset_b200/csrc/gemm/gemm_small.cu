@@ -48,8 +48,7 @@ struct SmallArgs {
   void* glu_h;
   long long ld_h;
   int b_ready;
-  int accs;         // accumulators: one per part of a kParallelK product, else one
-  int tmem_cols;
+  int by_part;      // kParallelK of several parts: CTA r of a cluster contracts part r
   int* status;
 };
 
@@ -105,8 +104,11 @@ __device__ __forceinline__ float bf16_rn(float x) {
   return __bfloat162float(__float2bfloat16_rn(x));
 }
 
-// Sum over the cluster of four consecutive floats at byte offset `off` of every partial tile.
-__device__ __forceinline__ float4 cluster_sum4(uint32_t base, uint32_t off, int splits) {
+// Sum over the cluster of four consecutive floats at byte offset `off` of every partial tile. Products
+// of several parts (by_part) are added up in bf16, one after the other: the roundings of launches
+// that each add to the result in memory.
+__device__ __forceinline__ float4 cluster_sum4(uint32_t base, uint32_t off, int splits,
+                                               int by_part = 0) {
   if (splits == 1) {
     float4 v;
     asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
@@ -122,6 +124,18 @@ __device__ __forceinline__ float4 cluster_sum4(uint32_t base, uint32_t off, int 
     for (int j = 0; j < 4; ++j)
       t[j] = s0 + j < splits ? ld_cluster4(map_rank(base, s0 + j) + off)
                              : make_float4(0.f, 0.f, 0.f, 0.f);
+    if (by_part) {  // (at most three parts: one group)
+      acc = t[0];
+#pragma unroll
+      for (int j = 1; j < 3; ++j)
+        if (j < splits) {
+          acc.x = bf16_rn(bf16_rn(acc.x) + bf16_rn(t[j].x));
+          acc.y = bf16_rn(bf16_rn(acc.y) + bf16_rn(t[j].y));
+          acc.z = bf16_rn(bf16_rn(acc.z) + bf16_rn(t[j].z));
+          acc.w = bf16_rn(bf16_rn(acc.w) + bf16_rn(t[j].w));
+        }
+      return acc;
+    }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       acc.x += t[j].x;
@@ -153,8 +167,11 @@ __global__ void __launch_bounds__(kThreads)
   const int S = g.splits;
   const int rank = S > 1 ? int(cta_rank()) : 0;
   const int tile = int(blockIdx.x) / S;
-  const int kb0 = rank * g.kb_total / S;
-  const int nkb = (rank + 1) * g.kb_total / S - kb0;   // >= 1: S <= kb_total
+  // contraction of this CTA: a share of the whole (>= 1 block: S <= kb_total), or one part
+  const int kb0 = g.by_part ? g.first[rank] : rank * g.kb_total / S;
+  const int kb1 = g.by_part ? (rank + 1 < S ? g.first[rank + 1] : g.kb_total)
+                            : (rank + 1) * g.kb_total / S;
+  const int nkb = kb1 - kb0;
 
   // tile -> part, origin in C, origin of the rows / columns read from A and B
   const int tm = tile / g.tiles_n, tn = tile - tm * g.tiles_n;
@@ -187,7 +204,7 @@ __global__ void __launch_bounds__(kThreads)
     tma_prefetch_desc(&tmB0);
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, g.tmem_cols);
+    tmem_alloc(tmem_slot, BN);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -270,14 +287,8 @@ __global__ void __launch_bounds__(kThreads)
     if (lane == 0) {
       constexpr uint32_t idesc = umma_idesc_bf16(BM, BN, A_MN, B_MN);
       bool ok = true;
-      int acc = 0;
       for (int i = 0; i < nkb; ++i) {
         const int s = i % C::STAGES;
-        bool fresh = i == 0;   // the first k-block of an accumulator overwrites it
-        if (acc + 1 < g.accs && i == g.first[acc + 1]) {
-          ++acc;
-          fresh = true;
-        }
         if (!mbar_wait(&full[s], (i / C::STAGES) & 1)) {
           report_status(g.status, kStatusTimeoutMma);
           ok = false;
@@ -292,7 +303,7 @@ __global__ void __launch_bounds__(kThreads)
                                       : umma_smem_desc(sa + k * 32, 16, 1024);
           const uint64_t bdesc = B_MN ? umma_smem_desc(sb + k * 2048, BK * 128, 1024)
                                       : umma_smem_desc(sb + k * 32, 16, 1024);
-          umma_bf16(tmem_base + acc * BN, adesc, bdesc, idesc, (!fresh || k > 0) ? 1u : 0u);
+          umma_bf16(tmem_base, adesc, bdesc, idesc, (i > 0 || k > 0) ? 1u : 0u);
         }
         umma_commit(&empty[s]);
       }
@@ -314,20 +325,6 @@ __global__ void __launch_bounds__(kThreads)
         uint32_t r[32];
         tmem_ld_32x32b_x32(tmem_base + (uint32_t(q * 32) << 16) + c * 32, r);
         tmem_ld_wait();
-        if constexpr (B_MN && !A_MN) {
-          // the parts' products added up in bf16, one after the other: the roundings of launches
-          // that each add to the result in memory
-          for (int p = 1; p < g.accs; ++p) {
-            uint32_t t[32];
-            tmem_ld_32x32b_x32(tmem_base + (uint32_t(q * 32) << 16) + p * BN + c * 32, t);
-            tmem_ld_wait();
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              const float sum = bf16_rn(__uint_as_float(r[j])) + bf16_rn(__uint_as_float(t[j]));
-              r[j] = __float_as_uint(bf16_rn(sum));
-            }
-          }
-        }
 #pragma unroll
         for (int j = 0; j < 8; ++j)
           *reinterpret_cast<float4*>(prow + c * 32 + 4 * j) =
@@ -355,7 +352,8 @@ __global__ void __launch_bounds__(kThreads)
       const int row = v / VPR, c = (v % VPR) * 8;
       if (n0 + c >= n_ext) continue;
       const uint32_t off = uint32_t(row * C::PITCH + c) * 4u;
-      float4 a0 = cluster_sum4(base, off, S), a1 = cluster_sum4(base, off + 16u, S);
+      float4 a0 = cluster_sum4(base, off, S, g.by_part);
+      float4 a1 = cluster_sum4(base, off + 16u, S, g.by_part);
       if (!GLU && g.bias[part] != nullptr) {
         const uint4 bq = *reinterpret_cast<const uint4*>(g.bias[part] + n0 + c);
         const float2 b0 = unpack_bf16x2(bq.x), b1 = unpack_bf16x2(bq.y);
@@ -417,7 +415,7 @@ __global__ void __launch_bounds__(kThreads)
     cluster_sync_();
   else
     __syncthreads();
-  if (warp == 1) tmem_dealloc(tmem_base, g.tmem_cols);
+  if (warp == 1) tmem_dealloc(tmem_base, BN);
 }
 
 int small_sms() {
@@ -447,7 +445,7 @@ int tiles_along(const LbSmallGemm* p, int mode, int whole, int tile) {
   return n;
 }
 
-int accumulators(const LbSmallGemm* p) { return p->mode == kParallelK ? p->nparts : 1; }
+bool by_part(const LbSmallGemm* p) { return p->mode == kParallelK && p->nparts > 1; }
 
 int count_tiles(const LbSmallGemm* p, int bn, int* tiles_n) {
   const int tm = tiles_along(p, kParallelM, p->M, BM);
@@ -524,7 +522,7 @@ using namespace lb;
 //   32 x 1024 x 3072                   26.2              12.7
 //   660 x (768, 768, 768) x 768        39.8 (3 launches) 12.7
 //   1024 x (3072, 3072) x 1024         31.7 (2 launches) 26.3
-//   1024 x 1024 x (2048, 1024, 1024)   48.0 (3 launches) 23.3
+//   1024 x 1024 x (2048, 1024, 1024)   48.0 (3 launches) 30.2
 //   (3072, 3072) x 1024 x 1024 (grad)  35.2 (2 launches) 28.9
 // (about 5 us of each are the measurement's own).
 extern "C" double lb_gemm_small_plan(const LbSmallGemm* p, int* bn_out, int* splits_out) {
@@ -534,15 +532,20 @@ extern "C" double lb_gemm_small_plan(const LbSmallGemm* p, int* bn_out, int* spl
   const int a_rows = p->M < BM && !p->a_mn ? p->M : BM;
   // Split only where the caller takes sums in another order (in a training step a different
   // rounding of one layer shows in the loss after the next update): an unsplit product has the bits
-  // that the tile kernels give. Nothing is lost for the weight gradients, which are never faster split.
-  const int max_splits = p->a_mn || !p->may_split || accumulators(p) > 1 ? 1 : kMaxSplits;
+  // that the tile kernels give. Nothing is lost for the weight gradients, which are never faster
+  // split. A product of several parts always has a CTA per part.
+  const bool parts = by_part(p);
+  const int max_splits = p->a_mn || !p->may_split || parts ? 1 : kMaxSplits;
+  int kb_part = 0;
+  for (int i = 0; parts && i < p->nparts; ++i)
+    kb_part = ceil_div(p->ext[i], BK) > kb_part ? ceil_div(p->ext[i], BK) : kb_part;
   double best = 1e30;
   for (int bn = 64; bn <= 128; bn += 64) {
-    if (accumulators(p) > 2 && bn > 64) break;   // two CTAs per SM have 256 columns each
     int tn;
     const int tiles = count_tiles(p, bn, &tn);
     const double stages = bn == 64 ? SCfg<64>::STAGES : SCfg<128>::STAGES;
-    for (int s = 1; s <= max_splits && s <= kb; s *= 2) {
+    for (int s1 = 1; s1 <= max_splits && s1 <= kb; s1 *= 2) {
+      const int s = parts ? p->nparts : s1;
       const int ctas = tiles * s;
       const double waves = ceil_div(ctas, 2 * sms);
       const double per_sm = ctas < sms ? 1.0 : (s == 1 ? ceil_div(ctas, sms) : double(ctas) / sms);
@@ -550,7 +553,8 @@ extern "C" double lb_gemm_small_plan(const LbSmallGemm* p, int* bn_out, int* spl
       const double split = (s > 1 ? 2.3 : 0.0) + (s > 2 ? 0.7 : 0.0) + (s > 4 ? 1.8 : 0.0);
       const double block = per_sm * (a_rows + bn) * 2.0, latency = 1400.0 / stages;
       const double cost = 2.0 + waves * (1.1 + split + store) +
-                          ceil_div(kb, s) * (block > latency ? block : latency) / 1900.0;
+                          (parts ? kb_part : ceil_div(kb, s)) *
+                              (block > latency ? block : latency) / 1900.0;
       if (cost < best) {
         best = cost;
         *bn_out = bn;
@@ -572,11 +576,13 @@ extern "C" int lb_gemm_small(const LbSmallGemm* p) {
     if (bn == 0) bn = b2;
     if (splits <= 0) splits = s2;
   }
-  if (splits != 1 && splits != 2 && splits != 4 && splits != 8) return -3;
   const int kb = kblocks(p);
-  while (splits > kb) splits /= 2;
-  const int accs = accumulators(p);
-  if (accs > 1) splits = 1;
+  if (by_part(p)) {
+    splits = p->nparts;
+  } else {
+    if (splits != 1 && splits != 2 && splits != 4 && splits != 8) return -3;
+    while (splits > kb) splits /= 2;
+  }
 
   CUtensorMap tA, tB[3];
   int rc;
@@ -622,9 +628,7 @@ extern "C" int lb_gemm_small(const LbSmallGemm* p) {
   g.glu_h = p->glu_h;
   g.ld_h = p->ld_h;
   g.b_ready = p->b_ready && pdl_enabled();
-  g.accs = accs;
-  g.tmem_cols = bn;
-  while (g.tmem_cols < accs * bn) g.tmem_cols *= 2;
+  g.by_part = by_part(p);
   g.status = p->status;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(p->stream);
   const int grid = tiles * splits;
