@@ -100,42 +100,65 @@ __global__ void __launch_bounds__(kRowThreads)
   }
 }
 
-// One CTA per segment. Threads are (column-vector, token-subset) pairs; subsets are combined in
-// shared memory. weighted = 1 weights token j (1-based inside its segment) by j / sum(j).
-__global__ void __launch_bounds__(kRowThreads)
+// Means over a segment's tokens: what bounds this is the latency of a long segment's loads (its sums are
+// serial in each token subset, and their order is kept). One CTA per segment with a lane per eight
+// columns and one load in flight took 611 us for 17 segments of 4096 x 1024 and 1208 for a longest one
+// of 8192; with 64 columns a CTA, a lane per two and 32 loads in flight 135 and 244 (24 of 30 x 768:
+// 12.5 -> 8.2). Loads behind a condition of their own were not batched: 238 and 447. A warp is a token
+// subset, and the subsets are combined in shared memory. weighted = 1 weights token j (1-based inside
+// its segment) by j / sum(j).
+constexpr int kSegCols = 64, kSegMaxSubsets = 32;
+
+__global__ void __launch_bounds__(32 * kSegMaxSubsets)
     segment_mean_fwd_kernel(const bf16* __restrict__ x, const int* __restrict__ cu,
                             bf16* __restrict__ out, int H, int weighted) {
-  extern __shared__ float sacc[];  // [S, H]
+  __shared__ float sacc[kSegMaxSubsets][kSegCols];
   const int seg = blockIdx.x;
   const int t0 = cu[seg], t1 = cu[seg + 1];
   const int len = t1 - t0;
-  const int CV = min(H / 8, kRowThreads);
-  const int S = kRowThreads / CV;
-  const int cvi = threadIdx.x % CV;
-  const int sub = threadIdx.x / CV;
-  const bool active = sub < S;
+  const int S = blockDim.x / 32;       // a warp's tokens: t0 + sub, t0 + sub + S, ..
+  const int sub = threadIdx.x / 32;
+  const int lc = (threadIdx.x & 31) * 2;
+  const int c = blockIdx.y * kSegCols + lc;
   const float wden = weighted ? 0.5f * float(len) * float(len + 1) : float(len);
-  for (int c = cvi * 8; c < H; c += CV * 8) {
-    float acc[8];
+  float acc[2] = {0.f, 0.f};
+  if (c < H) {
+    constexpr int kDepth = 32;         // tokens in flight per thread
+    const bf16* src = x + 1LL * (t0 + sub) * H + c;
+    const long long step = 1LL * S * H;
+    for (int tok = sub; tok < len; tok += kDepth * S) {
+      __nv_bfloat162 q[kDepth];
+      const bool whole = tok + (kDepth - 1) * S < len;
+      if (whole) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i] = 0.f;
-    if (active) {
-      for (int tok = t0 + sub; tok < t1; tok += S) {
-        float v[8];
-        unpack8(ld16(x + 1LL * tok * H + c), v);
-        const float wt = weighted ? float(tok - t0 + 1) : 1.f;
+        for (int k = 0; k < kDepth; ++k, src += step)
+          q[k] = *reinterpret_cast<const __nv_bfloat162*>(src);
+      } else {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) acc[i] += wt * v[i];
+        for (int k = 0; k < kDepth; ++k, src += step) {
+          q[k] = __nv_bfloat162{};
+          if (tok + k * S < len) q[k] = *reinterpret_cast<const __nv_bfloat162*>(src);
+        }
       }
 #pragma unroll
-      for (int i = 0; i < 8; ++i) sacc[sub * H + c + i] = acc[i];
+      for (int k = 0; k < kDepth; ++k)
+        if (whole || tok + k * S < len) {
+          const float2 v = __bfloat1622float2(q[k]);
+          const float wt = weighted ? float(tok + k * S + 1) : 1.f;
+          acc[0] += wt * v.x;
+          acc[1] += wt * v.y;
+        }
     }
   }
+  sacc[sub][lc] = acc[0];
+  sacc[sub][lc + 1] = acc[1];
   __syncthreads();
-  for (int c = threadIdx.x; c < H; c += kRowThreads) {
+  for (int i = threadIdx.x; i < kSegCols; i += blockDim.x) {
+    const int col = blockIdx.y * kSegCols + i;
+    if (col >= H) continue;
     float s = 0.f;
-    for (int k = 0; k < S; ++k) s += sacc[k * H + c];
-    out[1LL * seg * H + c] = __float2bfloat16_rn(len > 0 ? s / wden : 0.f);
+    for (int k = 0; k < S; ++k) s += sacc[k][i];
+    out[1LL * seg * H + col] = __float2bfloat16_rn(len > 0 ? s / wden : 0.f);
   }
 }
 
@@ -201,12 +224,13 @@ extern "C" int lb_l2norm_bwd(const void* gy, long long ldgy, const void* y, long
 extern "C" int lb_segment_mean_fwd(const void* x, const int* cu_seqlens, void* out, int M, int H,
                                    int weighted, void* stream) {
   if (M <= 0) return 0;
-  if (H & 7) return -3;
+  if ((H & 7) || H > 12288) return -3;
+  // token subsets as many as lanes of eight columns leave of a CTA of kRowThreads, at most 32
   const int CV = (H / 8) < kRowThreads ? (H / 8) : kRowThreads;
-  const int S = kRowThreads / CV;
-  const size_t smem = size_t(S) * H * sizeof(float);
-  if (smem > 48 * 1024) return -3;
-  segment_mean_fwd_kernel<<<M, kRowThreads, smem, reinterpret_cast<cudaStream_t>(stream)>>>(
+  int S = kRowThreads / CV;
+  if (S > kSegMaxSubsets) S = kSegMaxSubsets;
+  segment_mean_fwd_kernel<<<dim3(M, (H + kSegCols - 1) / kSegCols), 32 * S, 0,
+                            reinterpret_cast<cudaStream_t>(stream)>>>(
       (const bf16*)x, cu_seqlens, (bf16*)out, H, weighted);
   return launch_rc();
 }

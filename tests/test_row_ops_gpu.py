@@ -249,3 +249,28 @@ def test_poll_status_raises_one_call_late_without_blocking():
     assert word.item() == 0
     nv.poll_status()
     nv.poll_status()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("H", [8, 64, 136, 768, 1024, 2560])
+def test_segment_mean_chunk_edges(H, weighted):
+    """Segments around the 32 tokens a thread has in flight (per token subset), and empty ones."""
+    from lset_b200.ops.pooling import segment_mean
+
+    subsets = max(1, min(32, 256 // (H // 8)))
+    whole = 32 * subsets
+    lens = [1, 0, subsets, whole - 1, whole, whole + 1, 2 * whole - subsets, 2 * whole + 3]
+    cu = torch.tensor([0] + lens).cumsum(0).int().cuda()
+    x = torch.randn(sum(lens), H, generator=torch.Generator().manual_seed(H)).bfloat16().cuda()
+    got = segment_mean(x, cu, weighted).double()
+    for m, n in enumerate(lens):
+        seg = x[int(cu[m]):int(cu[m + 1])].double()
+        w = torch.arange(1, n + 1, device="cuda").double() if weighted else torch.ones(n).double().cuda()
+        if n == 0:
+            assert torch.equal(got[m], torch.zeros_like(got[m]))
+            continue
+        want = (w[:, None] * seg).sum(0) / w.sum()
+        # one rounding to bf16, and fp32 sums of n terms in any order
+        tol = want.abs() * 2.0 ** -8 + n * 2.0 ** -23 * (w[:, None] * seg.abs()).sum(0) / w.sum()
+        assert ((got[m] - want).abs() <= tol + 1e-30).all(), (m, n)
