@@ -55,8 +55,9 @@ class AttnPlan:
         if hit is not None:
             return hit
         cap = (self.T + tile_tokens - 1) // tile_tokens + self.B
-        # three spare words behind the entries: the work counter of the persistent forward kernel,
-        # the end of the last sequence (rows behind it are cleared) and the CTAs that have finished
+        # three spare words behind the entries: the work counter of the persistent kernels (forward,
+        # dK/dV), the end of the last sequence (rows behind it are cleared) and the CTAs that have
+        # finished: launches with one plan follow each other on a stream
         plan = torch.empty(1 + 2 * cap + 3, dtype=torch.int32, device=self.seq_start.device)
         rc = nv.load().lb_attn_plan(nv.c_void_p(self.seq_start.data_ptr()),
                                     nv.c_void_p(self.seq_end.data_ptr()), nv.c_int(self.B),

@@ -21,7 +21,7 @@ class RuntimeOptions:
     fused_rmsnorm: bool = True
     fused_qk_norm_rope: bool = True
     fused_double_rmsnorm: bool = True
-    block_runner: bool = True       # whole decoder blocks issued by the native block runner
+    block_runner: bool = True       # whole decoder / encoder blocks issued by the native block runner
     tp_block_runner: bool = True    # ... also tensor-parallel blocks on a token-sharded stream
     fused_glu_gemm: bool = False    # gated-MLP activation in the epilogue of the gate/up GEMM (measured slower: off)
     attention_backend: str = "auto"  # auto | native | sdpa
