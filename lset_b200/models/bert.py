@@ -94,7 +94,7 @@ class BertBlock(nn.Module):
         self.mlp = BertMLP(config)
 
     def forward(self, x, ctx: StreamCtx):
-        if block_ops.usable(self, x):
+        if block_ops.usable(self, x, ctx):
             return block_ops.run(self, x, ctx)   # the whole block in one native call
         return self.mlp(self.attention(x, ctx))
 

@@ -68,7 +68,8 @@ def _plain(m) -> bool:
             and not hasattr(m, "_tp_kind") and not m._forward_hooks and not m._forward_pre_hooks
             and not m._backward_hooks and not m._backward_pre_hooks
             and m.weight.dtype == torch.bfloat16 and m.bias.dtype == torch.bfloat16
-            and m.weight.is_cuda and m.weight.is_contiguous() and m.bias.is_contiguous()
+            and m.weight.is_cuda and m.bias.is_cuda
+            and m.weight.is_contiguous() and m.bias.is_contiguous()
             and m.weight.shape[0] % 8 == 0 and m.weight.shape[1] % 8 == 0)
 
 
@@ -89,13 +90,19 @@ class EncoderPlan:
             return
         if any(m.weight.shape != (3 * H // len(qkv), H) for m in qkv):
             return
+        if any(m.bias.shape != m.weight.shape[:1] for m in qkv + [o, fin, fout]):
+            return
         if (o.weight.shape != (H, H) or fin.weight.shape[1] != H
                 or fout.weight.shape != (H, fin.weight.shape[0])):
             return
         for ln in (ln1, ln2):
             if (type(ln) is not torch.nn.LayerNorm or ln.weight is None or ln.bias is None
                     or ln.weight.dtype != torch.bfloat16 or ln.bias.dtype != torch.bfloat16
-                    or not ln.weight.is_cuda or ln.eps != ln1.eps):
+                    or not ln.weight.is_cuda or ln.eps != ln1.eps
+                    or ln.weight.shape != (H,) or ln.bias.shape != (H,)
+                    or not ln.weight.is_contiguous() or not ln.bias.is_contiguous()
+                    or ln._forward_hooks or ln._forward_pre_hooks or ln._backward_hooks
+                    or ln._backward_pre_hooks or "forward" in ln.__dict__):
                 return
         d = LbEncoderDesc()
         d.H, d.heads, d.hd, d.I = H, att.num_heads, hd, fin.weight.shape[0]
@@ -111,8 +118,8 @@ class EncoderPlan:
 
     @staticmethod
     def _signature(block):
-        """Changes when a submodule is wrapped, replaced, hooked, moved or cast (looked up in the
-        modules' dicts, see ``BlockPlan._signature``)."""
+        """Changes when a submodule is wrapped, replaced, hooked, moved, cast or given other
+        data (looked up in the modules' dicts, see ``BlockPlan._signature``)."""
         att, mlp = block._modules["attention"], block._modules["mlp"]
         am, mm = att._modules, mlp._modules
         mods = (am["qkv_proj"],) if att.fused_qkv else (am["query"], am["key"], am["value"])
@@ -121,12 +128,14 @@ class EncoderPlan:
         for m in mods:
             d = m.__dict__
             p = d["_parameters"]
-            w = p.get("weight")
-            if w is None:
+            w, b = p.get("weight"), p.get("bias")
+            if w is None or b is None:
                 return None
-            sig.append((id(m), id(w), id(p.get("bias")), "forward" in d, w.dtype, w.device,
+            # (``.data`` of a parameter can be exchanged under the same object)
+            sig.append((id(m), id(w), id(b), "forward" in d, w.dtype, w.device, w.shape,
+                        w.is_contiguous(), b.dtype, b.device, b.shape, b.is_contiguous(), d.get("eps"),
                         len(d["_forward_hooks"]), len(d["_forward_pre_hooks"]),
-                        len(d["_backward_hooks"])))
+                        len(d["_backward_hooks"]), len(d["_backward_pre_hooks"])))
         return sig
 
     def fill(self, grads: dict) -> LbEncoderDesc:
@@ -152,7 +161,7 @@ def plan_of(block):
     return plan if plan.ok else None
 
 
-def usable(block, x) -> bool:
+def usable(block, x, ctx) -> bool:
     if not (x.is_cuda and x.dtype == torch.bfloat16 and x.dim() == 2 and x.shape[0] > 0):
         return False
     if _ac._active is not None or not enabled("block_runner") or _rt.attention_backend == "sdpa":
@@ -161,7 +170,8 @@ def usable(block, x) -> bool:
             m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks
             for m in (block.attention, block.mlp)):
         return False
-    return plan_of(block) is not None
+    plan = plan_of(block)
+    return plan is not None and x.shape[1] == plan.desc.H and ctx.pos.shape[0] == x.shape[0]
 
 
 def _stream_struct(ctx, plan: EncoderPlan, device, training: bool) -> LbStreamCtx:

@@ -106,6 +106,26 @@ def test_hooked_or_replaced_submodules_keep_the_op_path():
     assert enc_ops.calls == before and seen
 
 
+def test_data_exchanged_under_the_same_parameter():
+    """Other storage, another eps: what the runner has looked at once is looked at again."""
+    model, inputs = _model(128, 2, 256, False), _inputs([20, 9], False)
+    _run(model, inputs, True)
+    before = enc_ops.calls
+    layers = model.layers
+    w = layers[0].mlp.dense_in.weight
+    w.data = w.data.t().contiguous().t()               # same values, column by column in memory
+    got = _run(model, inputs, True)
+    assert enc_ops.calls == before + len(layers) - 1   # that block goes op by op
+    assert torch.allclose(got.float(), _run(model, inputs, False).float(), atol=6e-2)
+    w.data = w.data.contiguous()
+    for layer in layers:
+        layer.attention.LayerNorm.eps = layer.mlp.LayerNorm.eps = 0.5
+    before = enc_ops.calls
+    got = _run(model, inputs, True)
+    assert enc_ops.calls == before + len(layers)
+    assert torch.allclose(got.float(), _run(model, inputs, False).float(), atol=6e-2)
+
+
 @pytest.mark.parametrize("T,parts", [(1, (64, 0, 0)), (700, (768, 768, 768)), (5000, (72, 0, 0))])
 def test_bias_grad(T, parts):
     import ctypes
