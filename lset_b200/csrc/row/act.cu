@@ -102,6 +102,8 @@ __global__ void __launch_bounds__(256)
 __global__ void __launch_bounds__(256)
     gelu_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, bf16* __restrict__ dx,
                     long long n8) {
+  pdl_wait();
+  pdl_trigger();
   for (long long i = 1LL * blockIdx.x * blockDim.x + threadIdx.x; i < n8;
        i += 1LL * gridDim.x * blockDim.x) {
     float v[8], g[8];
