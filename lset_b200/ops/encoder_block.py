@@ -26,7 +26,6 @@ from ._grads import main_grad_of
 from .attention import fwd_tile_tokens
 from .block import (LbBlockIO, LbLinear, LbProjection, LbStreamCtx, _arena_size, _fp, _vp,
                     _work_arena, node_inputs)
-from .norm import scratch
 from .runtime_options import enabled, options as _rt
 
 
@@ -192,11 +191,15 @@ def _stream_struct(ctx, plan: EncoderPlan, device, training: bool) -> LbStreamCt
     s.plan_q = s.plan_kv = nv.ptr(ptq) or None      # one query head per KV head: the same tiles
     s.cap_q = s.cap_kv = capq
     s.status = nv.status_word(device).data_ptr()
-    s.norm_scratch = scratch("norm_bwd", _library().lb_norm_bwd_partial_rows() * 2 * d.H,
-                             device).data_ptr()
-    s.wg_tmp = scratch("ln_wgrad", 2 * d.H, device).data_ptr()
+    # partial sums of the backward's norms: the struct's own, as its backward comes later than other
+    # callers' passes, which would grow or write a shared buffer
+    sums = None
+    if grad:
+        partial = _library().lb_norm_bwd_partial_rows() * 2 * d.H
+        sums = torch.empty(partial + 2 * d.H, dtype=torch.float32, device=device)
+        s.norm_scratch, s.wg_tmp = sums.data_ptr(), sums.data_ptr() + 4 * partial
     s.may_split = int(may_split)
-    s._keep = (ctx.pos, ap, ptf, ptq)
+    s._keep = (ctx.pos, ap, ptf, ptq, sums)
     ctx.tables[key] = s
     return s
 

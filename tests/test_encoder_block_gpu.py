@@ -118,6 +118,32 @@ def test_gradients_below_frozen_parameters(T, trained):
             assert (got[n] - want).norm().item() < 2e-2 * size, n
 
 
+def test_passes_of_models_of_different_width_interleaved(monkeypatch):
+    """The wider model's pass, between the narrower one's two, asks for larger buffers."""
+    from lset_b200.ops import norm
+
+    models = [_model(128, 2, 256, False), _model(768, 12, 3072, False)]
+    inputs = _inputs([20, 70, 9], False)
+    want = []
+    for m in models:
+        _run(m, inputs, True)
+        want.append({n: p.grad for n, p in m.named_parameters()})
+        for p in m.parameters():
+            p.grad = None
+    monkeypatch.setattr(norm, "_scratch", {})
+    outs = [m(**inputs)["hidden_states"] for m in models]
+    held = [torch.full((1 << k,), 3.0, device="cuda") for k in range(8, 22) for _ in range(4)]
+    for m, out in zip(models, outs):
+        torch.manual_seed(9)
+        (out.float() * torch.randn(out.shape, device="cuda")).sum().backward()
+    nv.check_status()
+    assert all((t == 3.0).all() for t in held)      # nobody else's memory was written
+    for m, grads in zip(models, want):
+        for n, p in m.named_parameters():
+            size = grads[n.replace("key.bias", "value.bias")].float().norm().item()
+            assert (p.grad.float() - grads[n].float()).norm().item() < 2e-2 * size, n
+
+
 def test_hooked_or_replaced_submodules_keep_the_op_path():
     model, inputs = _model(128, 2, 256, False), _inputs([20, 9], False)
     seen = []
