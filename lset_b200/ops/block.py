@@ -29,7 +29,6 @@ from . import _ac
 from . import _native as nv
 from .attention import fwd_tile_tokens
 from ._grads import main_grad_of
-from .norm import scratch
 from .runtime_options import enabled, options as _rt
 
 _vp, _fp, _ip = ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p
@@ -406,14 +405,19 @@ def _stream_struct(ctx, plan: BlockPlan, device, training: bool) -> LbStreamCtx:
     s.plan_f, s.cap_f = ptf.data_ptr(), capf
     s.plan_q, s.cap_q, s.plan_kv, s.cap_kv = nv.ptr(ptq) or None, capq, nv.ptr(ptk) or None, capk
     s.status = nv.status_word(device).data_ptr()
-    s.norm_scratch = scratch("norm_bwd", lib.lb_norm_bwd_partial_rows() * d.H, device).data_ptr()
-    s.rope_scratch = scratch("rope_bwd", lib.lb_rope_bwd_partial_rows() * 2 * d.hd,
-                             device).data_ptr()
-    s.wg_tmp = scratch("qk_norm_wgrad", 2 * d.hd, device).data_ptr()
+    # partial sums of the backward's norms: the struct's own, as its backward comes later than other
+    # callers' passes, which would grow or write a shared buffer
+    sums = None
+    if grad:
+        norm, rope = lib.lb_norm_bwd_partial_rows() * d.H, lib.lb_rope_bwd_partial_rows() * 2 * d.hd
+        sums = torch.empty(norm + rope + 2 * d.hd, dtype=torch.float32, device=device)
+        s.norm_scratch = sums.data_ptr()
+        s.rope_scratch = sums.data_ptr() + 4 * norm
+        s.wg_tmp = sums.data_ptr() + 4 * (norm + rope)
     s.stream = 0
     s.may_split = int(may_split)
     # keep the tensors the struct points to alive as long as the struct
-    s._keep = (cos, sin, ctx.pos, ap, ptf, ptq, ptk)
+    s._keep = (cos, sin, ctx.pos, ap, ptf, ptq, ptk, sums)
     ctx.tables[key] = s
     return s
 

@@ -31,12 +31,14 @@ def _stream_struct(ops, monkeypatch, training=True):
     return ops._stream_struct(ctx, plan, torch.device("cpu"), training)
 
 
-@pytest.mark.parametrize("ops", [enc_ops])
+@pytest.mark.parametrize("ops", [enc_ops, dec_ops])
 def test_stream_struct_owns_the_buffers_of_the_backward(ops, monkeypatch):
     """The backward comes later than other callers' passes: a buffer that one of them may replace
     or write is not what the struct can point to."""
     structs = [_stream_struct(ops, monkeypatch) for _ in range(2)]
-    for name, n in (("norm_scratch", 8 * 2 * 16), ("wg_tmp", 2 * 16)):
+    sizes = ([("norm_scratch", 8 * 2 * 16), ("wg_tmp", 2 * 16)] if ops is enc_ops else
+             [("norm_scratch", 8 * 16), ("rope_scratch", 8 * 2 * 64), ("wg_tmp", 2 * 64)])
+    for name, n in sizes:
         at = [ctypes.cast(getattr(s, name), ctypes.c_void_p).value for s in structs]
         for a, s in zip(at, structs):
             assert any(torch.is_tensor(t) and t.data_ptr() <= a
