@@ -9,7 +9,7 @@ gradients are added to their fp32 accumulators without a rounding to bf16 in bet
 
 Taken for blocks of plain bf16 ``Linear`` layers with biases (fused or separate query / key / value)
 on the GPU; everything else (tensor parallelism, 8-bit layers, adapters, selective activation
-checkpointing, wrapped or hooked submodules) keeps the op-by-op path.
+checkpointing, wrapped, hooked or subclassed submodules) keeps the op-by-op path.
 
 Replaces the Python block of the reference (lset/models/encoder/bert/model.py:53-142).
 """
@@ -19,6 +19,7 @@ import ctypes
 import math
 
 import torch
+from torch.nn.modules.module import _has_any_global_hook
 
 from . import _ac
 from . import _native as nv
@@ -131,7 +132,7 @@ class EncoderPlan:
             if w is None or b is None:
                 return None
             # (``.data`` of a parameter can be exchanged under the same object)
-            sig.append((id(m), id(w), id(b), "forward" in d, w.dtype, w.device, w.shape,
+            sig.append((id(m), type(m), id(w), id(b), "forward" in d, w.dtype, w.device, w.shape,
                         w.is_contiguous(), b.dtype, b.device, b.shape, b.is_contiguous(), d.get("eps"),
                         len(d["_forward_hooks"]), len(d["_forward_pre_hooks"]),
                         len(d["_backward_hooks"]), len(d["_backward_pre_hooks"])))
@@ -160,14 +161,34 @@ def plan_of(block):
     return plan if plan.ok else None
 
 
+_types = None
+
+
+def _own_forwards(block) -> bool:
+    """Whether calling the block's two halves would run the forwards that the runner stands for."""
+    global _types
+    if _types is None:
+        from ..models.bert import BertAttention, BertMLP
+
+        _types = (BertAttention, BertMLP)
+    mods = block._modules
+    att, mlp = mods["attention"], mods["mlp"]
+    if type(att) is not _types[0] or type(mlp) is not _types[1] or _has_any_global_hook():
+        return False
+    for m in (att, mlp):
+        d = m.__dict__
+        if ("forward" in d or d["_forward_hooks"] or d["_forward_pre_hooks"]
+                or d["_backward_hooks"] or d["_backward_pre_hooks"]):
+            return False
+    return True
+
+
 def usable(block, x, ctx) -> bool:
     if not (x.is_cuda and x.dtype == torch.bfloat16 and x.dim() == 2 and x.shape[0] > 0):
         return False
     if _ac._active is not None or not enabled("block_runner") or _rt.attention_backend == "sdpa":
         return False
-    if not enabled("fused_layernorm") or any(
-            m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks
-            for m in (block.attention, block.mlp)):
+    if not enabled("fused_layernorm") or not _own_forwards(block):
         return False
     plan = plan_of(block)
     return plan is not None and x.shape[1] == plan.desc.H and ctx.pos.shape[0] == x.shape[0]

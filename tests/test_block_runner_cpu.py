@@ -46,3 +46,73 @@ def test_stream_struct_owns_the_buffers_of_the_backward(ops, monkeypatch):
         assert abs(at[0] - at[1]) >= 4 * n, name
     with torch.no_grad():
         assert not _stream_struct(ops, monkeypatch).norm_scratch
+
+
+class _Accepted(RuntimeError):
+    pass
+
+
+@pytest.fixture
+def decide(monkeypatch):
+    """``usable`` on the CPU: everything but the device is real."""
+    def plan_of(block):
+        raise _Accepted
+
+    def call(ops, block, ctx):
+        monkeypatch.setattr(ops, "plan_of", plan_of)
+        x = SimpleNamespace(is_cuda=True, dtype=torch.bfloat16, shape=(5, 128), dim=lambda: 2)
+        try:
+            assert ops.usable(block, x, ctx) is False
+            return False
+        except _Accepted:      # everything that is looked at before the plan is accepted
+            return True
+    return call
+
+
+def _bert_block():
+    from lset_b200.models.bert import BertBlock
+    from lset_b200.models.configs import BertConfig
+
+    return BertBlock(BertConfig(vocab_size=8, hidden_size=128, intermediate_size=256,
+                                num_hidden_layers=1, num_attention_heads=2))
+
+
+def _subclass(m):
+    m.__class__ = type("Own", (type(m),), {"forward": lambda self, x, *a: x})
+
+
+def _patched(m):
+    m.forward = lambda x, *a: x
+
+
+def _hooked(m):
+    m.register_forward_hook(lambda *a: None)
+
+
+@pytest.mark.parametrize("half", ["attention", "mlp"])
+@pytest.mark.parametrize("change", [_subclass, _patched, _hooked])
+def test_encoder_blocks_with_a_forward_of_their_own_are_not_taken(decide, half, change):
+    block = _bert_block()
+    assert decide(enc_ops, block, None)
+    change(getattr(block, half))
+    assert not decide(enc_ops, block, None)
+
+
+def test_encoder_block_with_another_mlp_or_under_a_global_hook_is_not_taken(decide):
+    block = _bert_block()
+    handle = torch.nn.modules.module.register_module_forward_hook(lambda *a: None)
+    try:
+        assert not decide(enc_ops, block, None)
+    finally:
+        handle.remove()
+    assert decide(enc_ops, block, None)
+    block.mlp = torch.nn.Linear(128, 128)      # no dense_in
+    assert not decide(enc_ops, block, None)
+
+
+def test_encoder_signature_sees_a_linear_that_became_another_class():
+    block = _bert_block()
+    before = enc_ops.EncoderPlan._signature(block)
+    assert enc_ops.EncoderPlan._signature(block) == before
+    _subclass(block.mlp.dense_in)              # as the 8-bit conversion does
+    assert enc_ops.EncoderPlan._signature(block) != before
