@@ -249,7 +249,7 @@ class BlockPlan:
             w = d["_parameters"].get("weight")
             if w is None:
                 w = m.weight
-            sig.append((id(m), "forward" in d, id(d.get("_sp_state")), w.dtype, w.device,
+            sig.append((id(m), type(m), "forward" in d, id(d.get("_sp_state")), w.dtype, w.device,
                         d["training"]))
         return sig
 
@@ -306,6 +306,22 @@ def plan_of(block):
     return plan if plan.ok else None
 
 
+_types = None
+
+
+def _own_forwards(block) -> bool:
+    """Whether calling the block's two halves would run the forwards that the runner stands for."""
+    global _types
+    if _types is None:
+        from ..models.layers import Attention, GatedMLP
+
+        _types = (Attention, GatedMLP)
+    mods = block._modules
+    att, mlp = mods["self_attn"], mods["mlp"]
+    return (type(att) is _types[0] and type(mlp) is _types[1]
+            and "forward" not in att.__dict__ and "forward" not in mlp.__dict__)
+
+
 def usable(block, branch, ctx) -> bool:
     """True when this call can go through the block runner."""
     if not (branch.is_cuda and branch.dtype == torch.bfloat16 and branch.dim() == 2):
@@ -315,6 +331,8 @@ def usable(block, branch, ctx) -> bool:
     for name in ("fused_rmsnorm", "fused_residual_rmsnorm", "fused_qk_norm_rope"):
         if not enabled(name):
             return False
+    if not _own_forwards(block):
+        return False
     plan = plan_of(block)
     if plan is None:
         return False

@@ -89,6 +89,24 @@ def _hooked(m):
     m.register_forward_hook(lambda *a: None)
 
 
+def _decoder_block():
+    from lset_b200.models import Qwen3Config
+    from lset_b200.models.decoder import Qwen3Decoder
+
+    return Qwen3Decoder(Qwen3Config(vocab_size=8, hidden_size=128, intermediate_size=256,
+                                    num_hidden_layers=1, num_attention_heads=2,
+                                    num_key_value_heads=1, head_dim=64)).layers[0]
+
+
+@pytest.mark.parametrize("half", ["self_attn", "mlp"])
+@pytest.mark.parametrize("change", [_subclass, _patched])
+def test_decoder_blocks_with_a_forward_of_their_own_are_not_taken(decide, half, change):
+    block = _decoder_block()
+    assert decide(dec_ops, block, None)
+    change(getattr(block, half))
+    assert not decide(dec_ops, block, None)
+
+
 @pytest.mark.parametrize("half", ["attention", "mlp"])
 @pytest.mark.parametrize("change", [_subclass, _patched, _hooked])
 def test_encoder_blocks_with_a_forward_of_their_own_are_not_taken(decide, half, change):
@@ -110,9 +128,11 @@ def test_encoder_block_with_another_mlp_or_under_a_global_hook_is_not_taken(deci
     assert not decide(enc_ops, block, None)
 
 
-def test_encoder_signature_sees_a_linear_that_became_another_class():
-    block = _bert_block()
-    before = enc_ops.EncoderPlan._signature(block)
-    assert enc_ops.EncoderPlan._signature(block) == before
-    _subclass(block.mlp.dense_in)              # as the 8-bit conversion does
-    assert enc_ops.EncoderPlan._signature(block) != before
+@pytest.mark.parametrize("make,plan,name", [(_bert_block, enc_ops.EncoderPlan, "dense_in"),
+                                            (_decoder_block, dec_ops.BlockPlan, "down_proj")])
+def test_signature_sees_a_linear_that_became_another_class(make, plan, name):
+    block = make()
+    before = plan._signature(block)
+    assert plan._signature(block) == before
+    _subclass(getattr(block.mlp, name))        # as the 8-bit conversion does
+    assert plan._signature(block) != before
