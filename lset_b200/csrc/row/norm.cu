@@ -18,7 +18,15 @@ namespace {
 
 using bf16 = __nv_bfloat16;
 
-template <int TPR, int NV>
+// Eight weights of a slice that does not start at a 16-byte boundary.
+__device__ __forceinline__ uint4 ld8_unaligned(const bf16* p) {
+  float f[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) f[i] = __bfloat162float(p[i]);
+  return pack8(f);
+}
+
+template <int TPR, int NV, bool W_ALIGNED>
 __global__ void __launch_bounds__(kRowThreads)
     rms_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ res_in,
                    const bf16* __restrict__ w, bf16* __restrict__ y, bf16* __restrict__ res_out,
@@ -35,7 +43,7 @@ __global__ void __launch_bounds__(kRowThreads)
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
     const int idx = (v * TPR + t) * 8;
-    if (valid && idx < H) wq[v] = ld16(w + idx);
+    if (valid && idx < H) wq[v] = W_ALIGNED ? ld16(w + idx) : ld8_unaligned(w + idx);
   }
   pdl_wait();
   pdl_trigger();
@@ -464,9 +472,11 @@ extern "C" int lb_rms_norm_fwd(const void* x, const void* res_in, const void* w,
   LB_ROW_DISPATCH(H, {
     constexpr int ROWS = kRowThreads / TPR;
     const int grid = (N + ROWS - 1) / ROWS;
-    return launch_pdl(rms_fwd_kernel<TPR, NV>, dim3(grid), dim3(kRowThreads), 0, st, pdl_enabled(),
-                      1, (const bf16*)x, (const bf16*)res_in, (const bf16*)w, (bf16*)y,
-                      (bf16*)res_out, rstd, N, H, eps, w_off);
+    const bool aligned = (reinterpret_cast<uintptr_t>(w) & 15u) == 0;
+    return launch_pdl(aligned ? rms_fwd_kernel<TPR, NV, true> : rms_fwd_kernel<TPR, NV, false>,
+                      dim3(grid), dim3(kRowThreads), 0, st, pdl_enabled(), 1, (const bf16*)x,
+                      (const bf16*)res_in, (const bf16*)w, (bf16*)y, (bf16*)res_out, rstd, N, H, eps,
+                      w_off);
   });
 }
 

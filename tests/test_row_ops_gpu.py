@@ -274,3 +274,20 @@ def test_segment_mean_chunk_edges(H, weighted):
         # one rounding to bf16, and fp32 sums of n terms in any order
         tol = want.abs() * 2.0 ** -8 + n * 2.0 ** -23 * (w[:, None] * seg.abs()).sum(0) / w.sum()
         assert ((got[m] - want).abs() <= tol + 1e-30).all(), (m, n)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("offset", [1, 4])
+@pytest.mark.parametrize("H", [64, 136, 1024, 2560])
+def test_rms_norm_takes_a_weight_that_starts_anywhere(H, offset):
+    """A slice of a flat buffer that does not start at a 16-byte boundary; the same bits."""
+    from lset_b200.ops.norm import residual_rms_norm, rms_norm
+
+    g = torch.Generator().manual_seed(H)
+    x, r = (torch.randn(37, H, generator=g).bfloat16().cuda() for _ in range(2))
+    flat = torch.randn(H + offset, generator=g).bfloat16().cuda()
+    w = flat[offset:]
+    assert w.data_ptr() % 16 != 0
+    assert torch.equal(rms_norm(x, w), rms_norm(x, w.clone()))
+    for a, b in zip(residual_rms_norm(r, x, w), residual_rms_norm(r, x, w.clone())):
+        assert torch.equal(a, b)
