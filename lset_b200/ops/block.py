@@ -273,9 +273,10 @@ class BlockPlan:
             dst.lora_r, dst.lora_scale = 0, 0.0
 
     def fill(self, grads: dict) -> LbBlockDesc:
-        """Refresh every pointer. ``grads`` maps ``id(param)`` to the address of its fp32 gradient
-        accumulator (absent = no weight gradient wanted)."""
-        d = self.desc
+        """A descriptor of its own for the call (another thread may be in a pass of the same block),
+        with the tensors' present addresses. ``grads`` maps ``id(param)`` to the address of its fp32
+        gradient accumulator (absent = no weight gradient wanted)."""
+        d = LbBlockDesc.from_buffer_copy(self.desc)
         d.ln1_w, d.ln1_wgrad = self.ln1.weight.data_ptr(), grads.get(id(self.ln1.weight))
         d.ln2_w, d.ln2_wgrad = self.ln2.weight.data_ptr(), grads.get(id(self.ln2.weight))
         if self.qn is not None:

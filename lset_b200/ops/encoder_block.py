@@ -74,7 +74,7 @@ def _plain(m) -> bool:
 
 
 class EncoderPlan:
-    """The tensors that feed the descriptor; pointers are read again on every call."""
+    """The tensors that feed the descriptor (``desc``: its sizes); addresses are read on every call."""
 
     def __init__(self, block):
         self.ok = False
@@ -109,11 +109,10 @@ class EncoderPlan:
         d.eps, d.softmax_scale = float(ln1.eps), 1.0 / math.sqrt(hd)
         d.qkv.n, d.qkv.width = len(qkv), 3 * H
         self.desc = d
-        self.linears = [(m, d.qkv.part[i], i) for i, m in enumerate(qkv)]
-        self.linears += [(o, d.o_proj, 3), (fin, d.in_, 4), (fout, d.out, 5)]
+        self.linears = [*enumerate(qkv), (3, o), (4, fin), (5, fout)]
         self.norms = [(ln1, "ln1"), (ln2, "ln2")]
         self.params = [p for ln, _ in self.norms for p in (ln.weight, ln.bias)]
-        self.params += [p for m, _, _ in self.linears for p in (m.weight, m.bias)]
+        self.params += [p for _, m in self.linears for p in (m.weight, m.bias)]
         self.ok = True
 
     @staticmethod
@@ -139,14 +138,18 @@ class EncoderPlan:
         return sig
 
     def fill(self, grads: dict) -> LbEncoderDesc:
-        d = self.desc
+        """A descriptor of its own for the call (another thread may be in a pass of the same block),
+        with the tensors' present addresses; ``grads`` as in ``BlockPlan.fill``."""
+        d = LbEncoderDesc.from_buffer_copy(self.desc)
+        part = d.qkv.part
+        slots = (part[0], part[1], part[2], d.o_proj, d.in_, d.out)
         for ln, name in self.norms:
             setattr(d, name + "_w", ln.weight.data_ptr())
             setattr(d, name + "_b", ln.bias.data_ptr())
             setattr(d, name + "_wgrad", grads.get(id(ln.weight)))
             setattr(d, name + "_bgrad", grads.get(id(ln.bias)))
-        for m, dst, i in self.linears:
-            w = m.weight
+        for i, m in self.linears:
+            dst, w = slots[i], m.weight
             dst.w, dst.wgrad, dst.ldw = w.data_ptr(), grads.get(id(w)), w.stride(0)
             dst.n_out, dst.k_in = w.shape
             d.bias[i], d.bias_grad[i] = m.bias.data_ptr(), grads.get(id(m.bias))

@@ -136,3 +136,35 @@ def test_signature_sees_a_linear_that_became_another_class(make, plan, name):
     assert plan._signature(block) == before
     _subclass(getattr(block.mlp, name))        # as the 8-bit conversion does
     assert plan._signature(block) != before
+
+
+def _encoder_plan():
+    block, plan = _bert_block(), enc_ops.EncoderPlan.__new__(enc_ops.EncoderPlan)
+    qkv, o, fin, fout, ln1, ln2 = enc_ops._modules(block)
+    plan.desc = enc_ops.LbEncoderDesc()
+    plan.linears = list(enumerate(qkv + [o, fin, fout]))
+    plan.norms = [(ln1, "ln1"), (ln2, "ln2")]
+    return plan, fout.weight, lambda d: d.out
+
+
+def _decoder_plan():
+    block, plan = _decoder_block(), dec_ops.BlockPlan.__new__(dec_ops.BlockPlan)
+    plan.desc = dec_ops.LbBlockDesc()
+    plan.ln1, plan.ln2, plan.qn, plan.kn = block.input_layernorm, block.input_layernorm, None, None
+    parts = [(m.weight, None, None, 0.0) for m in (block.self_attn.q_proj, block.self_attn.o_proj,
+                                                   block.mlp.up_proj, block.mlp.down_proj)]
+    plan.qkv, plan.o, plan.gate_up, plan.down = parts[:1], parts[1], parts[2:3], parts[3]
+    return plan, block.mlp.down_proj.weight, lambda d: d.down
+
+
+@pytest.mark.parametrize("make", [_encoder_plan, _decoder_plan])
+def test_every_call_has_a_descriptor_of_its_own(make):
+    """A forward in one thread does not clear the gradient addresses that another thread's backward
+    has just filled in."""
+    plan, w, linear = make()
+    backward = plan.fill({id(w): 4096})
+    forward = plan.fill({})
+    assert linear(backward).wgrad and not linear(forward).wgrad
+    assert ctypes.cast(linear(backward).wgrad, ctypes.c_void_p).value == 4096
+    assert linear(backward).w == linear(forward).w == w.data_ptr()
+    assert not linear(plan.desc).w
