@@ -103,9 +103,6 @@ def _library():
     return _lib
 
 
-_arenas = {}
-
-
 def _arena_size(nbytes: int) -> int:
     """``nbytes`` rounded up to the next size of a geometric series (eight sizes per octave, at
     most 12.5 % more). Packed batches differ in token count from step to step; with exact sizes
@@ -120,13 +117,9 @@ def _arena_size(nbytes: int) -> int:
 
 
 def _work_arena(nbytes: int, device) -> torch.Tensor:
-    """Temporary storage of the block backward: one buffer per device, grown on demand. Blocks run
-    their backward one after the other on the same stream, so they share it."""
-    t = _arenas.get(device)
-    if t is None or t.numel() < nbytes:
-        t = torch.empty(_arena_size(nbytes), dtype=torch.uint8, device=device)
-        _arenas[device] = t
-    return t
+    """Temporary storage of one block's backward. Each call has its own: passes of other streams run
+    at the same time, and the allocator hands blocks of one stream's passes the same memory."""
+    return torch.empty(_arena_size(nbytes), dtype=torch.uint8, device=device)
 
 
 # --------------------------------------------------------------------------- eligibility

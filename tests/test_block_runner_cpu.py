@@ -168,3 +168,9 @@ def test_every_call_has_a_descriptor_of_its_own(make):
     assert ctypes.cast(linear(backward).wgrad, ctypes.c_void_p).value == 4096
     assert linear(backward).w == linear(forward).w == w.data_ptr()
     assert not linear(plan.desc).w
+
+
+def test_backward_passes_that_overlap_do_not_share_their_temporary_storage():
+    a, b = (dec_ops._work_arena(3 << 20, torch.device("cpu")) for _ in range(2))
+    assert a.numel() >= 3 << 20
+    assert a.data_ptr() + a.numel() <= b.data_ptr() or b.data_ptr() + b.numel() <= a.data_ptr()
