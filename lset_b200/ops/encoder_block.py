@@ -113,6 +113,7 @@ class EncoderPlan:
         self.norms = [(ln1, "ln1"), (ln2, "ln2")]
         self.params = [p for ln, _ in self.norms for p in (ln.weight, ln.bias)]
         self.params += [p for _, m in self.linears for p in (m.weight, m.bias)]
+        self.weights = [ln.weight for ln, _ in self.norms] + [m.weight for _, m in self.linears]
         self.ok = True
 
     @staticmethod
@@ -247,14 +248,15 @@ class _EncoderBlockFn(torch.autograd.Function):
             nv.check_rc(rc, "lb_encoder_fwd")
         nv.count_launch(io.launches)
         calls += 1
-        ctx.save_for_backward(x, saved)
+        # the weights, for autograd to see that the backward reads what the forward read
+        ctx.save_for_backward(x, saved, *plan.weights)
         ctx.plan, ctx.sctx, ctx.stream_ctx = plan, sctx, stream_ctx
         return out
 
     @staticmethod
     def backward(ctx, d_out):
         lib = _library()
-        x, saved = ctx.saved_tensors
+        x, saved = ctx.saved_tensors[:2]
         plan, sctx = ctx.plan, ctx.sctx
         T, H = x.shape
         d_out = d_out.to(x.dtype).contiguous()

@@ -174,6 +174,22 @@ def test_data_exchanged_under_the_same_parameter():
     assert torch.allclose(got.float(), _run(model, inputs, False).float(), atol=6e-2)
 
 
+@pytest.mark.parametrize("name", ["attention.query", "mlp.dense_out", "attention.LayerNorm"])
+def test_weights_changed_in_place_before_the_backward_are_refused(name):
+    """The backward reads the weights of the forward: autograd refuses others, as op by op."""
+    model, inputs = _model(128, 2, 256, False), _inputs([20, 9], False)
+    for on in (True, False):
+        configure(block_runner=on)
+        try:
+            out = model(**inputs)["hidden_states"]
+            with torch.no_grad():
+                model.layers[1].get_submodule(name).weight.mul_(2)
+            with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+                out.float().sum().backward()
+        finally:
+            configure(block_runner=True)
+
+
 @pytest.mark.parametrize("T,parts", [(1, (64, 0, 0)), (700, (768, 768, 768)), (5000, (72, 0, 0))])
 def test_bias_grad(T, parts):
     import ctypes
