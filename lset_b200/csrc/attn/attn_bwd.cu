@@ -499,6 +499,9 @@ __global__ void __launch_bounds__(kDkvThreads, 1)
 
   if (warp == kDkvMath / 32) {
     // -------------------------------------------------------------------- work items, loads
+    // (the lanes agree on the waits before they go on to the next item: where one ran out in some
+    // of them only, those would leave the loop whose shuffles the others take part in. A vote per
+    // step took 0.5-1.5 % of the backward; within an item they meet behind the loop.)
     AttnPlanView plan{a.plan};
     const int total = plan.count() * a.Hk;
     int w = int(blockIdx.x), n = 0;   // n: steps so far, over all items
@@ -514,7 +517,7 @@ __global__ void __launch_bounds__(kDkvThreads, 1)
         t.kv0 = plan.tile(i) * 128;
       }
       const int slot = it & 1;
-      ok = mbar_wait(&work_empty[slot], ((it >> 1) & 1) ^ 1u);
+      ok = __all_sync(0xffffffffu, mbar_wait(&work_empty[slot], ((it >> 1) & 1) ^ 1u));
       if (ok && lane == 0) {
         s_work[slot] = t;
         mbar_arrive(&work_full[slot]);
@@ -522,7 +525,7 @@ __global__ void __launch_bounds__(kDkvThreads, 1)
       if (!ok || t.hk < 0) break;
       // K and V of the item as soon as the last one's scores are complete: under its last math,
       // its accumulation products and its store
-      ok = mbar_wait(bar_kve, (it & 1) ^ 1u);
+      ok = __all_sync(0xffffffffu, mbar_wait(bar_kve, (it & 1) ^ 1u));
       if (ok && lane == 0) {
         mbar_expect_tx(bar_kv, 2 * C::KV_BYTES);
 #pragma unroll
@@ -563,9 +566,9 @@ __global__ void __launch_bounds__(kDkvThreads, 1)
       // earlier it would wait here while other SMs run out of work
       unsigned drawn = 0;
       if (lane == 0) drawn = atomicAdd(a.counter, 1u);
+      ok = __all_sync(0xffffffffu, ok);
       w = int(__shfl_sync(0xffffffffu, drawn, 0)) + int(gridDim.x);
     }
-    ok = __all_sync(0xffffffffu, ok);
     if (!ok) {
       if (lane == 0) report_status(a.status, kStatusTimeoutProducer);
       const unsigned long long t0 = globaltimer_ns();   // copies in flight land meanwhile

@@ -38,3 +38,17 @@ def test_kernels_launched_as_programmatic_dependents_wait():
         body = _kernel_body(name)
         assert "pdl_wait();" in body, name
         assert 0 <= body.find("pdl_wait();") < body.find("pdl_trigger();"), name
+
+
+def test_lanes_of_the_load_warp_of_dkv_agree_on_their_waits():
+    """Every wait is bounded, and may run out in some lanes only: all 32 take part in the shuffles
+    behind it, so they have to leave the loops together."""
+    body = _kernel_body("attn_dkv_kernel")
+    loads = body[body.index("if (warp == kDkvMath / 32) {"):
+                 body.index("if (warp == kDkvMath / 32 + 1) {")]
+    per_item, per_step = loads.split("i < steps && ok;")
+    waits = re.findall(r"(.*)mbar_wait\(", per_item)
+    assert len(waits) == 2 and all(w.endswith("__all_sync(0xffffffffu, ") for w in waits)
+    # lanes that left the inner loop meet the others behind it
+    behind = per_step[per_step.index("unsigned drawn"):]
+    assert behind.index("ok = __all_sync(0xffffffffu, ok);") < behind.index("__shfl_sync")
