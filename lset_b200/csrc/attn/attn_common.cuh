@@ -28,7 +28,18 @@ struct AttnPlanView {
   __device__ __forceinline__ int tile(int i) const { return data[2 + 2 * i]; }
 };
 
-// Called by every CTA of a forward kernel when it takes no more work: the last one puts the plan's
+// Rows of the stream behind the last sequence belong to no work item: every CTA clears a share of O's
+// (`vec` = 16-byte pieces of a row).
+__device__ __forceinline__ void clear_tail(const int* plan, int capacity, __nv_bfloat16* O,
+                                           long long ldo, int T, int vec) {
+  const int end = plan[1 + 2 * capacity + 1];
+  if (end < 0) return;
+  for (int row = end + int(blockIdx.x); row < T; row += gridDim.x)
+    for (int v = threadIdx.x; v < vec; v += blockDim.x)
+      *reinterpret_cast<uint4*>(O + 1LL * row * ldo + v * 8) = make_uint4(0u, 0u, 0u, 0u);
+}
+
+// Called by every CTA of a persistent kernel when it takes no more work: the last one puts the plan's
 // work counter back to zero for the next layer's launch.
 __device__ __forceinline__ void finish_grid(const int* plan, int capacity) {
   if (threadIdx.x != 0) return;

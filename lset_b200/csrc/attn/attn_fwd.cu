@@ -1,8 +1,9 @@
 // Varlen (packed) flash attention forward on tcgen05: causal or bidirectional, grouped-query heads.
-// Head dims 64 and 128 run on the two-tile kernel of attn_fwd_pair.cuh; at 256 its accumulators and
-// tiles fit neither tensor nor shared memory, and attn_fwd_kernel below is used:
+// Head dims 64 and 128 run on the two-tile kernel of attn_fwd_pair.cuh, except where the sequences are
+// short (AttnPlan in ops/attention.py has the rule); these, and head dim 256, for which that kernel's
+// accumulators and tiles fit neither tensor nor shared memory, run on attn_fwd_kernel below:
 //
-// Persistent 128-thread CTAs (two per SM) walk over the (KV head, sequence, query tile) work items;
+// Persistent 128-thread CTAs (two per SM, at head dim 256 one) walk over the (KV head, sequence, query tile) work items;
 // TMEM and the barriers are set up once per CTA and the next item's Q and first K/V block are
 // requested during the last block of the current one. Per KV block of 64:
 //   S = Q·Kᵀ          tcgen05.mma, A = Q tile (128 x hd), B = K block (64 x hd), S in TMEM
@@ -63,10 +64,13 @@ __global__ void __launch_bounds__(128)
     attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, AttnFwdArgs a) {
   using C = FwdCfg<HD>;
+  pdl_wait();
+  pdl_trigger();
   AttnPlanView plan{a.plan};
   const int tiles = plan.count();
   const int total = tiles * a.Hk;
   if (int(blockIdx.x) >= total) {
+    clear_tail(a.plan, a.capacity, a.O, a.ldo, a.T, a.Hq * HD / 8);
     finish_grid(a.plan, a.capacity);
     return;
   }
@@ -353,6 +357,7 @@ __global__ void __launch_bounds__(128)
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem_base, C::TMEM_COLS);
+  clear_tail(a.plan, a.capacity, a.O, a.ldo, a.T, a.Hq * HD / 8);
   finish_grid(a.plan, a.capacity);
 }
 
@@ -431,8 +436,9 @@ int attn_sms() {
   return n;
 }
 
-// Persistent grids: as many CTAs as are resident at once (one per SM), never more than the upper
-// bound of the work items; a CTA beyond the real count finds nothing to do.
+// Persistent grids: as many CTAs as are resident at once (one per SM, two of the one-tile kernel where
+// its shared memory allows), never more than the upper bound of the work items; a CTA beyond the real
+// count finds nothing to do.
 template <int HD>
 int launch_fwd(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV,
                const AttnFwdArgs& a, int max_tiles, cudaStream_t st) {
@@ -446,9 +452,10 @@ int launch_fwd(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap
     configured = true;
   }
   const long long upper = 1LL * max_tiles * a.Hk;
-  const int grid = static_cast<int>(upper < attn_sms() ? upper : attn_sms());
-  kern<<<grid, 128, C::SMEM_BYTES, st>>>(tmQ, tmK, tmV, a);
-  return cudaGetLastError() == cudaSuccess ? 0 : -11;
+  const long long resident = attn_sms() * (C::SMEM_BYTES <= 113 * 1024 ? 2LL : 1LL);
+  const int grid = static_cast<int>(upper < resident ? upper : resident);
+  return launch_pdl(kern, dim3(grid), dim3(128), C::SMEM_BYTES, st, pdl_enabled(), 1, tmQ, tmK, tmV,
+                    a);
 }
 
 template <int HD>
@@ -499,15 +506,11 @@ extern "C" int lb_attn_plan(const int* seq_start, const int* seq_end, int B, int
 // Sequence b owns tokens [seq_start[b], seq_end[b]) of the stream (for a packed batch these are
 // cu_seqlens and cu_seqlens + 1; for a padded batch they skip the padding).
 // q: [T, Hq, hd] with token stride ldq (elements); k, v: [T, Hk, hd] with strides ldk, ldv.
-// plan was built with tile_tokens = lb_attn_fwd_tile_tokens(hd, Hq / Hk). o: [T, Hq, hd] stride ldo;
-// lse: [Hq, T] fp32.
-extern "C" int lb_attn_fwd_tile_tokens(int hd, int group) {
-  return (hd == 256 ? 128 : 256) / group;
-}
-
+// plan was built with tile_tokens = 256 / (Hq / Hk) for the two-tile kernel, 128 / (Hq / Hk) for the
+// one-tile kernel (the only one for hd 256). o: [T, Hq, hd] stride ldo; lse: [Hq, T] fp32.
 extern "C" int lb_attn_fwd(const void* q, long long ldq, const void* k, long long ldk, const void* v,
                            long long ldv, const int* seq_start, const int* seq_end, const int* plan,
-                           int max_tiles,
+                           int max_tiles, int tile_tokens,
                            void* o, long long ldo, float* lse, int T, int Hq, int Hk, int hd,
                            float softmax_scale, int causal, int* status, void* stream) {
   if (T <= 0 || max_tiles <= 0) return 0;
@@ -517,7 +520,9 @@ extern "C" int lb_attn_fwd(const void* q, long long ldq, const void* k, long lon
   if ((ldq | ldk | ldv | ldo) & 7) return -3;
   if (hd != 128 && hd != 64 && hd != 256) return -3;
   const int QT = 128 / G;
-  const int kv_box = hd == 256 ? kAttnKvBlock : kPairBlock;
+  const bool one_tile = tile_tokens == QT;
+  if (!one_tile && (tile_tokens != 2 * QT || hd == 256)) return -3;
+  const int kv_box = one_tile ? kAttnKvBlock : kPairBlock;
   CUtensorMap tmQ, tmK, tmV;
   int rc = make_tmap_2d(&tmQ, q, 2, (uint64_t)Hq * hd, (uint64_t)T, (uint64_t)ldq * 2, 64, QT, true);
   if (rc) return rc;
@@ -528,12 +533,12 @@ extern "C" int lb_attn_fwd(const void* q, long long ldq, const void* k, long lon
   unsigned* counter = reinterpret_cast<unsigned*>(const_cast<int*>(plan)) + 1 + 2 * max_tiles;
   const float scale_log2 = softmax_scale * kLog2eF;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (hd == 256) {
-    rc = lb_attn_zero_tail(plan, max_tiles, T, o, ldo, Hq * hd, nullptr, 0, 0, nullptr, 0, 0, stream);
-    if (rc) return rc;
+  if (one_tile) {
     AttnFwdArgs a{seq_start, seq_end, plan, counter, (bf16*)o, ldo, lse, T, Hq, Hk,
                   scale_log2, causal, status, max_tiles};
-    return launch_fwd<256>(tmQ, tmK, tmV, a, max_tiles, st);
+    if (hd == 256) return launch_fwd<256>(tmQ, tmK, tmV, a, max_tiles, st);
+    return hd == 128 ? launch_fwd<128>(tmQ, tmK, tmV, a, max_tiles, st)
+                     : launch_fwd<64>(tmQ, tmK, tmV, a, max_tiles, st);
   }
   // a scale of zero becomes one whose products with finite scores vanish beside the maximum
   const float mag = scale_log2 < 0.f ? -scale_log2 : scale_log2;

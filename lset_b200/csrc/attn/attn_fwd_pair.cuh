@@ -522,14 +522,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
   __syncthreads();
   tc_fence_after();
   if (warp == 9) tmem_dealloc(tmem_base, C::TMEM_COLS);
-  // rows of the stream behind the last sequence belong to no work item
-  const int end = a.plan[1 + 2 * a.capacity + 1];
-  if (end >= 0) {
-    const int vec = a.Hq * HD / 8;
-    for (int row = end + int(blockIdx.x); row < a.T; row += gridDim.x)
-      for (int v = threadIdx.x; v < vec; v += kPairThreads)
-        *reinterpret_cast<uint4*>(a.O + 1LL * row * a.ldo + v * 8) = make_uint4(0u, 0u, 0u, 0u);
-  }
+  clear_tail(a.plan, a.capacity, a.O, a.ldo, a.T, a.Hq * HD / 8);
   finish_grid(a.plan, a.capacity);   // thread 0 belongs to warp 0; the item counter is final: the
                                      // barrier above came after the last item was drawn
 }

@@ -493,8 +493,8 @@ int block_fwd_tp(const LbBlockDesc* d, const LbStreamCtx* c, const LbBlockIO* io
       cudaMemsetAsync(s.o + (size_t)T * Nq, 0, (size_t)(Tp - T) * Nq * 2, st) != cudaSuccess)
     return -11;
   LB_TRY(lb_attn_fwd(s.qr, Nq, s.kr, Nk, s.qkv + Nq + Nk, W, c->seq_start, c->seq_end, c->plan_f,
-                     c->cap_f, s.o, Nq, s.lse, T, d->Hq, d->Hk, hd, d->softmax_scale, d->causal,
-                     c->status, c->stream));
+                     c->cap_f, c->tile_f, s.o, Nq, s.lse, T, d->Hq, d->Hk, hd, d->softmax_scale,
+                     d->causal, c->status, c->stream));
   LB_TRY(tp_gemm_rs(r, s.o, Nq, d->o_proj, 0, out, H, Nq, c));
   __nv_bfloat16* x2s = r.next_slot();
   LB_TRY(lb_rms_norm_fwd(out, stream_in, d->ln2_w, x2s, io->res_out, s.rstd2, R, H, d->eps,
@@ -590,7 +590,7 @@ extern "C" int lb_block_fwd_launches(const LbBlockDesc* d, const LbStreamCtx* c,
   (void)has_residual;
   if (tp != nullptr)  // two norms, rope, attention, glu; 2 gathered GEMMs (own-row copy, barrier,
     return 5 + 2 * 3 + 2 * 3;  // GEMM) and 2 reduced GEMMs (GEMM, barrier, take-and-clear)
-  int n = d->hd == 256 ? 6 : 5;  // two norms, rope, attention (hd 256: and tail clear), glu
+  int n = 5;  // two norms, rope, attention, glu
   for (int i = 0; i < 7; ++i) {
     const LbLinear* l = linear_at(d, i);
     if (l != nullptr) n += lin_fwd_launches(*l);
@@ -648,8 +648,8 @@ static int block_fwd(const LbBlockDesc* d, const LbStreamCtx* c, const LbBlockIO
     if (cudaMemsetAsync(s.o, 0, (size_t)T * Nq * 2, st) != cudaSuccess) return -11;
   }
   LB_TRY(lb_attn_fwd(s.qr, Nq, s.kr, Nk, s.qkv + Nq + Nk, W, c->seq_start, c->seq_end, c->plan_f,
-                     c->cap_f, s.o, Nq, s.lse, T, d->Hq, d->Hk, hd, d->softmax_scale, d->causal,
-                     c->status, c->stream));
+                     c->cap_f, c->tile_f, s.o, Nq, s.lse, T, d->Hq, d->Hk, hd, d->softmax_scale,
+                     d->causal, c->status, c->stream));
   // attention branch output: staged in `out`, consumed by the second norm before the MLP writes there
   LB_TRY(lin_fwd(d->o_proj, s.o, Nq, out, H, T, s.ts[3], c));
   LB_TRY(lb_rms_norm_fwd(out, stream_in, d->ln2_w, s.x2, io->res_out, s.rstd2, T, H, d->eps,
@@ -849,8 +849,8 @@ extern "C" int lb_encoder_fwd(const LbEncoderDesc* d, const LbStreamCtx* c, LbBl
   LB_TRY(proj_fwd(d->qkv, x, H, s.qkv, T, no_ts, c, d->bias));
   const lb::PdlScope pdl(true);
   LB_TRY(lb_attn_fwd(s.qkv, W, s.qkv + H, W, s.qkv + 2 * H, W, c->seq_start, c->seq_end, c->plan_f,
-                     c->cap_f, s.o, H, s.lse, T, d->heads, d->heads, d->hd, d->softmax_scale, 0,
-                     c->status, c->stream));
+                     c->cap_f, c->tile_f, s.o, H, s.lse, T, d->heads, d->heads, d->hd,
+                     d->softmax_scale, 0, c->status, c->stream));
   LB_TRY(lin_fwd(d->o_proj, s.o, H, s.tmp, H, T, nullptr, c, d->bias[3]));
   LB_TRY(lb_layer_norm_fwd(s.tmp, x, d->ln1_w, d->ln1_b, s.y1, s.nr1, s.mean1, s.rstd1, T, H, d->eps,
                            c->stream));

@@ -66,8 +66,8 @@ struct LbStreamCtx {
   int pos_i64;
   const int* seq_start;
   const int* seq_end;
-  const int* plan_f;     // tile list of the forward (lb_attn_fwd_tile_tokens per tile)
-  int cap_f;
+  const int* plan_f;     // tile list of the forward, tile_f tokens per tile
+  int cap_f, tile_f;
   const int* plan_q;     // backward: tile list for 128 / (Hq / Hk) tokens per tile (null without
   int cap_q;             // gradients, as plan_kv)
   const int* plan_kv;    // tile list for 128 tokens per tile

@@ -56,8 +56,8 @@ int lb_attn_zero_tail(const int* plan, int capacity, int T, void* p0, long long 
                       void* stream);
 int lb_attn_fwd(const void* q, long long ldq, const void* k, long long ldk, const void* v,
                 long long ldv, const int* seq_start, const int* seq_end, const int* plan,
-                int max_tiles, void* o, long long ldo, float* lse, int T, int Hq, int Hk, int hd,
-                float softmax_scale, int causal, int* status, void* stream);
+                int max_tiles, int tile_tokens, void* o, long long ldo, float* lse, int T, int Hq, int Hk,
+                int hd, float softmax_scale, int causal, int* status, void* stream);
 int lb_attn_bwd(const void* dO, long long lddo, const void* q, long long ldq, const void* k,
                 long long ldk, const void* v, long long ldv, const void* o, long long ldo,
                 const float* lse, float* delta, const int* seq_start, const int* seq_end,

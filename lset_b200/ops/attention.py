@@ -68,6 +68,28 @@ class AttnPlan:
         self._plans[tile_tokens] = (plan, cap)
         return plan, cap
 
+    def fwd_tiles(self, heads: int, kv_heads: int, head_dim: int):
+        """(plan tensor, capacity, tokens per tile) of the forward: a tile of 128 rows (the query heads
+        of a KV head stacked) for the one-tile kernel, of 256 for the two-tile kernel."""
+        rows = 256 // (heads // kv_heads)
+        if head_dim == 256 or self._one_tile(heads, kv_heads, head_dim):
+            rows //= 2
+        return (*self.tiles(rows), rows)
+
+    def _one_tile(self, heads: int, kv_heads: int, head_dim: int) -> bool:
+        """Whether all sequences, or most of them, fit in one tile, and there are more of them than SMs:
+        the second tile of a CTA would be idle, and of the one-tile kernel two CTAs share an SM. (At
+        head dim 64 a tile of more than 64 tokens has two KV blocks there, and the two-tile kernel is as
+        fast.) Two-tile / one-tile (us, 2000 sequences of 24 tokens):
+        16/16 heads of 128 666 / 487, 12/12 of 64 429 / 328, 16/8 of 128 368 / 286; 4000 (sequence, KV
+        head) pairs of 0.9 tiles: 16/8 of 128 143 / 102, of 1.3 tiles 172 / 197; 12/12 of 64 at 64
+        tokens 98 / 74, at 90 105 / 107; 16/16 of 128 at 128 tokens 154 / 136, at 90 ragged up to 150
+        156 / 149, at 115 ragged up to 190 183 / 190."""
+        tile = 128 // (heads // kv_heads)
+        if self.B * kv_heads <= 148 or (head_dim == 64 and self.T > 64 * self.B):
+            return False
+        return self.max_seqlen <= tile or self.T <= self.B * min(0.9 * tile, 96)
+
 
 def attention_ref(q, k, v, cu_seqlens, causal: bool, scale: float | None = None, seq_end=None):
     """Eager oracle: per-sequence softmax attention in fp32. q: [T,Hq,hd]; k, v: [T,Hk,hd].
@@ -98,16 +120,10 @@ def attention_ref(q, k, v, cu_seqlens, causal: bool, scale: float | None = None,
     return out
 
 
-def fwd_tile_tokens(head_dim: int, group: int) -> int:
-    """Tokens per tile of the plan the forward kernel takes (``lb_attn_fwd_tile_tokens``)."""
-    return (128 if head_dim == 256 else 256) // group
-
-
 def _native_fwd(q, k, v, plan: AttnPlan, causal, scale):
     T, Hq, hd = q.shape
     Hk = k.shape[1]
-    G = Hq // Hk
-    ptiles, cap = plan.tiles(fwd_tile_tokens(hd, G))
+    ptiles, cap, tile = plan.fwd_tiles(Hq, Hk, hd)
     # tokens outside every sequence (padding) are never written by the kernel: keep them zero
     o = (torch.empty if plan.cu_seqlens is not None else torch.zeros)(
         T, Hq, hd, dtype=q.dtype, device=q.device)
@@ -116,12 +132,12 @@ def _native_fwd(q, k, v, plan: AttnPlan, causal, scale):
         nv.c_void_p(q.data_ptr()), nv.c_ll(q.stride(0)), nv.c_void_p(k.data_ptr()),
         nv.c_ll(k.stride(0)), nv.c_void_p(v.data_ptr()), nv.c_ll(v.stride(0)),
         nv.c_void_p(plan.seq_start.data_ptr()), nv.c_void_p(plan.seq_end.data_ptr()),
-        nv.c_void_p(ptiles.data_ptr()), nv.c_int(cap),
+        nv.c_void_p(ptiles.data_ptr()), nv.c_int(cap), nv.c_int(tile),
         nv.c_void_p(o.data_ptr()), nv.c_ll(Hq * hd), nv.c_void_p(lse.data_ptr()), nv.c_int(T),
         nv.c_int(Hq), nv.c_int(Hk), nv.c_int(hd), nv.c_float(scale), nv.c_int(int(causal)),
         nv.c_void_p(nv.status_word(q.device).data_ptr()), nv.c_void_p(nv.stream_ptr()))
     nv.check_rc(rc, "lb_attn_fwd")
-    nv.count_launch(2 if hd == 256 else 1)
+    nv.count_launch()
     return o, lse
 
 

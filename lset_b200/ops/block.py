@@ -27,7 +27,6 @@ import torch
 
 from . import _ac
 from . import _native as nv
-from .attention import fwd_tile_tokens
 from ._grads import main_grad_of
 from .runtime_options import enabled, options as _rt
 
@@ -59,7 +58,7 @@ class LbBlockDesc(ctypes.Structure):
 class LbStreamCtx(ctypes.Structure):
     _fields_ = [("T", ctypes.c_int), ("packed", ctypes.c_int), ("cos", _fp), ("sin", _fp),
                 ("pos", _vp), ("pos_i64", ctypes.c_int), ("seq_start", _ip), ("seq_end", _ip),
-                ("plan_f", _ip), ("cap_f", ctypes.c_int),
+                ("plan_f", _ip), ("cap_f", ctypes.c_int), ("tile_f", ctypes.c_int),
                 ("plan_q", _ip), ("cap_q", ctypes.c_int), ("plan_kv", _ip),
                 ("cap_kv", ctypes.c_int), ("status", _ip), ("norm_scratch", _fp),
                 ("rope_scratch", _fp), ("wg_tmp", _fp), ("stream", _vp),
@@ -406,7 +405,7 @@ def _stream_struct(ctx, plan: BlockPlan, device, training: bool) -> LbStreamCtx:
     cos, sin = ctx.rope(*plan.rope)
     ap = ctx.plan
     G = d.Hq // d.Hk
-    ptf, capf = ap.tiles(fwd_tile_tokens(d.hd, G))
+    ptf, capf, tile = ap.fwd_tiles(d.Hq, d.Hk, d.hd)
     ptq, capq = ap.tiles(128 // G) if grad else (None, 0)
     ptk, capk = ap.tiles(128) if grad else (None, 0)
     s = LbStreamCtx()
@@ -414,7 +413,7 @@ def _stream_struct(ctx, plan: BlockPlan, device, training: bool) -> LbStreamCtx:
     s.cos, s.sin = cos.data_ptr(), sin.data_ptr()
     s.pos, s.pos_i64 = ctx.pos.data_ptr(), int(ctx.pos.dtype == torch.int64)
     s.seq_start, s.seq_end = ap.seq_start.data_ptr(), ap.seq_end.data_ptr()
-    s.plan_f, s.cap_f = ptf.data_ptr(), capf
+    s.plan_f, s.cap_f, s.tile_f = ptf.data_ptr(), capf, tile
     s.plan_q, s.cap_q, s.plan_kv, s.cap_kv = nv.ptr(ptq) or None, capq, nv.ptr(ptk) or None, capk
     s.status = nv.status_word(device).data_ptr()
     # partial sums of the backward's norms: the struct's own, as its backward comes later than other

@@ -24,7 +24,6 @@ from torch.nn.modules.module import _has_any_global_hook
 from . import _ac
 from . import _native as nv
 from ._grads import main_grad_of
-from .attention import fwd_tile_tokens
 from .block import (LbBlockIO, LbLinear, LbProjection, LbStreamCtx, _arena_size, _fp, _vp,
                     _work_arena, node_inputs)
 from .runtime_options import enabled, options as _rt
@@ -207,12 +206,12 @@ def _stream_struct(ctx, plan: EncoderPlan, device, training: bool) -> LbStreamCt
     if hit is not None:
         return hit
     ap = ctx.plan
-    ptf, capf = ap.tiles(fwd_tile_tokens(d.hd, 1))
+    ptf, capf, tile = ap.fwd_tiles(d.heads, d.heads, d.hd)
     ptq, capq = ap.tiles(128) if grad else (None, 0)
     s = LbStreamCtx()
     s.T, s.packed = int(ctx.pos.shape[0]), int(ap.cu_seqlens is not None)
     s.seq_start, s.seq_end = ap.seq_start.data_ptr(), ap.seq_end.data_ptr()
-    s.plan_f, s.cap_f = ptf.data_ptr(), capf
+    s.plan_f, s.cap_f, s.tile_f = ptf.data_ptr(), capf, tile
     s.plan_q = s.plan_kv = nv.ptr(ptq) or None      # one query head per KV head: the same tiles
     s.cap_q = s.cap_kv = capq
     s.status = nv.status_word(device).data_ptr()

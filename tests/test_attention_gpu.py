@@ -155,3 +155,29 @@ def test_padded_plan_clears_the_gradient_rows_of_padding():
     pad = mask.reshape(-1) == 0
     for t in (q, k, v):
         assert not t.grad[pad].any() and t.grad[~pad].abs().max() > 0
+
+
+@pytest.mark.parametrize("Hq,Hk,hd", [(2, 2, 128), (4, 2, 128), (8, 2, 64), (8, 1, 128), (3, 3, 64)])
+@pytest.mark.parametrize("causal", [True, False])
+def test_forward_of_the_one_tile_kernel(Hq, Hk, hd, causal, monkeypatch):
+    """The kernel that short sequences take, on the sequences and with the bound of
+    ``test_forward_tile_edges``, and on a stream with rows behind the last sequence."""
+    test_forward_tile_edges(Hq, Hk, hd, causal, -0.2)
+    monkeypatch.setattr(AttnPlan, "_one_tile", lambda *a: True)
+    test_forward_tile_edges(Hq, Hk, hd, causal, None)
+    test_forward_tile_edges(Hq, Hk, hd, causal, -0.2)
+    test_stream_padded_past_the_last_sequence()
+
+
+def test_short_sequences_take_the_one_tile_kernel():
+    def tile(n, length, Hq, Hk, hd, longest=0):
+        cu = torch.arange(n + 1, dtype=torch.int32, device="cuda") * length
+        return AttnPlan(cu, longest or length, n * length).fwd_tiles(Hq, Hk, hd)[2]
+
+    assert tile(256, 30, 12, 12, 64) == 128 and tile(256, 64, 12, 12, 64) == 128
+    assert tile(256, 65, 12, 12, 64) == 256
+    assert tile(256, 64, 16, 8, 128) == 64 and tile(256, 65, 16, 8, 128) == 128
+    assert tile(256, 57, 16, 8, 128, 90) == 64 and tile(256, 58, 16, 8, 128, 90) == 128
+    assert tile(256, 128, 16, 16, 128) == 128
+    assert tile(1, 30, 16, 8, 128) == 128          # fewer sequences than SMs
+    assert tile(256, 300, 4, 4, 256) == 128
