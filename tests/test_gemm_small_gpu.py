@@ -75,6 +75,25 @@ def test_parts_along_the_columns(T, ext, K):
     nv.check_status()
 
 
+@pytest.mark.parametrize("T,N", [(1, 8), (7, 16), (100, 56), (127, 120), (300, 16)])
+def test_operands_with_fewer_rows_than_a_tile(T, N):
+    """Loaded as they are: what lies below them in shared memory is read by no one. Not finite here,
+    from the product before."""
+    K = 1024
+    bad = torch.full((256, K), float("nan"), device="cuda", dtype=torch.bfloat16)
+    junk = torch.empty(256, 128, device="cuda", dtype=torch.bfloat16)
+    a, b = _rand(T, K), _rand(N, K)
+    ref = a.double() @ b.double().t()
+    for bn, s in FORMS:
+        for _ in range(2):      # 2 x 148 CTAs and more: every SM's shared memory
+            assert _call(bad, [bad.repeat(80, 1)], [junk.new_empty(256, 20480)], 256, 20480, K, [20480],
+                         N_PARTS, bn=64, splits=1) == 0
+        c = torch.full((T, N), float("nan"), device="cuda", dtype=torch.bfloat16)
+        assert _call(a, [b], [c], T, N, K, [N], N_PARTS, bn=bn, splits=s) == 0
+        assert _rel(c, ref) < ROUND, (bn, s)
+    nv.check_status()
+
+
 @pytest.mark.parametrize("T", [1, 128, 257])
 @pytest.mark.parametrize("ext,N", [([64], 72), ([128, 64, 192], 200), ([3072, 3072], 1024)])
 def test_parts_along_the_contraction(T, ext, N):
