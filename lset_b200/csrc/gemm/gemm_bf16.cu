@@ -958,14 +958,30 @@ extern "C" int lb_gemm_use_2cta(int v) {
   return use_2cta();
 }
 
-// Measured 14.5 us a launch (of them 5 the measurement's) and, per wave of 256 x 256 tiles, 0.27 us for
-// 64 of contraction depth; a split weight gradient adds its reductions.
+// Columns of a tile of the one-CTA kernel: 256 unless 128 fill the SMs' last wave better.
+static int one_cta_bn(int M, int N) {
+  const int sms = lb::num_sms(), tiles_m = (M + lb::BM - 1) / lb::BM;
+  auto eff = [&](int b) {
+    const long long t = 1LL * tiles_m * ((N + b - 1) / b);
+    const long long waves = (t + sms - 1) / sms;
+    return double(t) * b / double(waves * sms);  // useful columns per SM-slot
+  };
+  return (N > 128 && eff(256) >= eff(128)) ? 256 : 128;
+}
+
+// Fitted with lb_gemm_small_plan, against which it is compared: a launch, and per wave of tiles and 64 of
+// contraction depth 0.33 us on CTA pairs, on the one-CTA kernel (for products smaller than a pair's
+// tile) 0.37 with 256 columns a tile and 0.27 with 128; a split weight gradient adds its reductions.
 extern "C" double lb_gemm_tile_cost(int M, int N, int K, int fp32) {
-  const long long tiles = 1LL * ((M + 255) / 256) * ((N + 255) / 256);
-  const int kb = (K + lb::BK - 1) / lb::BK, pairs = lb_gemm_2cta_pairs();
-  const int s = fp32 ? lb::auto_splits(tiles, kb, pairs) : 1;
-  const long long waves = (tiles * s + pairs - 1) / pairs;
-  return 10.0 + double(waves) * ((kb + s - 1) / s) * 0.27 + (s > 1 ? 4.0 : 0.0);
+  const bool pair = M >= 256 && N >= 256;
+  const int bm = pair ? 256 : lb::BM, bn = pair ? 256 : one_cta_bn(M, N);
+  const int slots = pair ? lb_gemm_2cta_pairs() : lb::num_sms();
+  const long long tiles = 1LL * ((M + bm - 1) / bm) * ((N + bn - 1) / bn);
+  const int kb = (K + lb::BK - 1) / lb::BK;
+  const int s = fp32 ? lb::auto_splits(tiles, kb, slots) : 1;
+  const long long waves = (tiles * s + slots - 1) / slots;
+  const double block = pair ? 0.33 : (bn == 256 ? 0.37 : 0.27);
+  return 11.0 + double(waves) * ((kb + s - 1) / s) * block + (s > 1 ? 4.0 : 0.0);
 }
 
 static int gemm_bf16_impl(const void* A, const void* B, void* C, int M, int N, int K,
@@ -1029,14 +1045,7 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, int M, int N, i
     return lb_gemm_bf16_2cta(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_fp32, accumulate, s2,
                              status, stream_);
   }
-  if (bn != 128 && bn != 256) {
-    auto eff = [&](int b) {
-      const long long t = 1LL * tiles_m * ((N + b - 1) / b);
-      const long long waves = (t + sms - 1) / sms;
-      return double(t) * b / double(waves * sms);  // useful columns per SM-slot
-    };
-    bn = (N > 128 && eff(256) >= eff(128)) ? 256 : 128;
-  }
+  if (bn != 128 && bn != 256) bn = one_cta_bn(M, N);
   const int tiles_n = (N + bn - 1) / bn;
   const int kb_total = (K + BK - 1) / BK;
   if (splits == 0)

@@ -513,11 +513,11 @@ int dispatch(const LbSmallGemm* p, const CUtensorMap& tA, const CUtensorMap* tB,
 
 using namespace lb;
 
-// Microseconds, fitted to measurements of 13 products of transformer blocks (H 768 and 1024) at 32
-// to 2048 tokens with both tile widths and all splits; the choice it leads to is within 10 % of the
-// best of the eight for all but a few of them. W waves of two CTAs per SM pay for launch, set-up,
-// pipeline fill and the store of the tile, a split for the cluster's barriers; a k-block costs what
-// the SM needs to take it in, but no less than its share of the latency of the loads in flight.
+// Microseconds, fitted to measurements of 40 products of transformer blocks (widths 768 to 4096, their
+// FFNs up to 12288, rank-16 adapters) at 1 to 20000 tokens with both tile widths and all splits: no
+// choice between this kernel and the tile kernels that it leads to is more than 3 % behind the other. W waves of two CTAs per SM pay for launch, set-up, pipeline fill and
+// the store of the tile, a split for the cluster's barriers; a k-block costs what the SM needs to
+// take it in, but no less than its share of the latency of the loads in flight in every wave.
 //   tokens x N x K                     tile kernels      this kernel (us, L2 flushed)
 //   32 x (2048, 1024, 1024) x 1024     37.8 (3 launches) 12.7
 //   32 x 1024 x 3072                   26.2              12.7
@@ -552,7 +552,7 @@ extern "C" double lb_gemm_small_plan(const LbSmallGemm* p, int* bn_out, int* spl
       const double per_sm = ctas < sms ? 1.0 : (s == 1 ? ceil_div(ctas, sms) : double(ctas) / sms);
       const double store = (p->out_fp32 ? 1.8 : 2.6) * a_rows * bn / 8192.0;
       const double split = (s > 1 ? 2.3 : 0.0) + (s > 2 ? 0.7 : 0.0) + (s > 4 ? 1.8 : 0.0);
-      const double block = per_sm * (a_rows + bn) * 2.0, latency = 1400.0 / stages;
+      const double block = per_sm * (a_rows + bn) * 2.0, latency = waves * 2600.0 / stages;
       const double cost = 2.0 + waves * (1.1 + split + store) +
                           (parts ? kb_part : ceil_div(kb, s)) *
                               (block > latency ? block : latency) / 1900.0;
