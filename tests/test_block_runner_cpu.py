@@ -19,6 +19,9 @@ class Plan:
     def tiles(self, tokens):
         return torch.zeros(8, dtype=torch.int32), 2
 
+    def fwd_tiles(self, heads, kv_heads, head_dim):
+        return (*self.tiles(128), 128)
+
 
 def _stream_struct(ops, monkeypatch, training=True):
     monkeypatch.setattr(ops, "_library", lambda: LIB)
@@ -27,7 +30,7 @@ def _stream_struct(ops, monkeypatch, training=True):
     table = torch.zeros(4, 4)
     ctx = SimpleNamespace(plan=Plan(), pos=torch.zeros(5, dtype=torch.int64), tables={},
                           rope=lambda *a: (table, table))
-    plan = SimpleNamespace(desc=SimpleNamespace(H=16, hd=64, Hq=2, Hk=1), rope=(64, 1e4, None))
+    plan = SimpleNamespace(desc=SimpleNamespace(H=16, hd=64, heads=2, Hq=2, Hk=1), rope=(64, 1e4, None))
     return ops._stream_struct(ctx, plan, torch.device("cpu"), training)
 
 
