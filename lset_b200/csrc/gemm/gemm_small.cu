@@ -71,7 +71,9 @@ __device__ __forceinline__ uint32_t cta_rank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
+// (the aligned forms want the whole warp: threads that left a loop early meet the others first)
 __device__ __forceinline__ void cluster_sync_() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -313,7 +315,7 @@ __global__ void __launch_bounds__(kThreads)
     __syncwarp();
   } else {
     // ------------------------------------------------------------------ accumulator -> shared memory
-    pdl_wait();  // also the only wait of a thread that writes global memory
+    pdl_wait();
     pdl_trigger();
     const int q = warp & 3;
     const bool ok = mbar_wait(tfull, 0);
@@ -335,6 +337,7 @@ __global__ void __launch_bounds__(kThreads)
     }
     tc_fence_before();
   }
+  pdl_wait();   // for itself in every thread: all of them store below
   if (S > 1)
     cluster_sync_();
   else

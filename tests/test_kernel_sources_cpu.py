@@ -52,3 +52,14 @@ def test_lanes_of_the_load_warp_of_dkv_agree_on_their_waits():
     # lanes that left the inner loop meet the others behind it
     behind = per_step[per_step.index("unsigned drawn"):]
     assert behind.index("ok = __all_sync(0xffffffffu, ok);") < behind.index("__shfl_sync")
+
+
+def test_every_thread_of_the_small_gemm_waits_before_it_stores():
+    """The loading and the issuing warp store results too, and a cluster barrier of the aligned form
+    wants whole warps, which the loops in front of it do not leave together."""
+    body = _kernel_body("gemm_small_kernel")
+    joined = body[:body.index("sum and store")].rsplit("\n  }\n", 1)[1]    # behind the warps' roles
+    assert "pdl_wait();" in joined
+    text = next(t for t in TEXTS.values() if "void cluster_sync_()" in t)
+    barrier = text[text.index("void cluster_sync_()"):]
+    assert barrier.index("__syncwarp();") < barrier.index("barrier.cluster.arrive")
