@@ -9,6 +9,10 @@ out-of-memory batches are retried in halves; large results stream into a memmap.
 The batching is different on purpose: chunks are *packed* into streams of at most
 ``token_budget`` tokens (no padding at all) and run through the model's packed path, instead of
 padded ``(B+1)·max_len ≤ budget`` rectangles.
+
+The encoder's passes are declared to be inference (``ops.block.inference_pass``): products of few tokens
+are then summed in pieces whose number follows the token count. An embedding's last bits (differences
+of the size of the bf16 roundings) therefore depend on the texts it is encoded with.
 """
 from __future__ import annotations
 
@@ -20,6 +24,7 @@ from typing import Callable, List, Optional, Sequence
 import numpy as np
 import torch
 
+from ..ops.block import inference_pass
 from ..ops.pooling import packed_pool
 from ..train.data.packing import pack_sequences
 
@@ -105,7 +110,7 @@ def encode_chunked(model, tokenize_fn, pool_fn, texts: Sequence[str], *, device,
         packed = pack_sequences([chunks[i] for i in idx])
         ids = packed["input_ids"].to(device)
         cu = packed["cu_seqlens"].to(device)
-        with torch.no_grad():
+        with torch.no_grad(), inference_pass():
             hid = model(ids, position_ids=packed["position_ids"].to(device), cu_seqlens=cu,
                         max_seqlen=packed["max_seqlen"])["hidden_states"]
             return packed_pool(hid, cu, pooling, False).float()

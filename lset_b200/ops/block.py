@@ -20,8 +20,10 @@ Replaces the Python block of the reference (lset/models/decoder/qwen3/block.py:2
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import math
+import threading
 
 import torch
 
@@ -388,16 +390,39 @@ def _tp_advance(state) -> None:
     tok.epoch += 4
 
 
+# --------------------------------------------------------------------------- order of summation
+_thread = threading.local()
+
+
+@contextlib.contextmanager
+def inference_pass():
+    """The forwards of this thread within it are for their results alone: no later pass with gradients
+    has to reproduce their bits. Their products may then be summed in pieces, which is faster with few
+    tokens, and how many pieces depends on the number of tokens."""
+    before = getattr(_thread, "inference", False)
+    _thread.inference = True
+    try:
+        yield
+    finally:
+        _thread.inference = before
+
+
+def may_split(training: bool) -> bool:
+    """Whether products may be summed in pieces: in passes declared to be inference (torch's inference
+    mode declares it too) of a model in evaluation mode. Other passes without gradients keep the order
+    of those with gradients: a checkpoint or a cached-gradient step recomputes what they computed."""
+    return (not training and not torch.is_grad_enabled()
+            and (getattr(_thread, "inference", False) or torch.is_inference_mode_enabled()))
+
+
 # --------------------------------------------------------------------------- stream context
 def _stream_struct(ctx, plan: BlockPlan, device, training: bool) -> LbStreamCtx:
     """The per-forward struct, cached on the Python stream context (all blocks share it). The
     backward's tile lists are built for a pass that records gradients only."""
     d = plan.desc
     grad = torch.is_grad_enabled()
-    # a model in training mode keeps one order of summation, with and without gradients: what an
-    # activation checkpoint recomputes has the bits of the first pass
-    may_split = not grad and not training
-    key = ("_lb", grad, may_split, d.hd, d.Hq // d.Hk, plan.rope[1], id(plan.rope[2]))
+    split = may_split(training)
+    key = ("_lb", grad, split, d.hd, d.Hq // d.Hk, plan.rope[1], id(plan.rope[2]))
     hit = ctx.tables.get(key)
     if hit is not None:
         return hit
@@ -426,7 +451,7 @@ def _stream_struct(ctx, plan: BlockPlan, device, training: bool) -> LbStreamCtx:
         s.rope_scratch = sums.data_ptr() + 4 * norm
         s.wg_tmp = sums.data_ptr() + 4 * (norm + rope)
     s.stream = 0
-    s.may_split = int(may_split)
+    s.may_split = int(split)
     # keep the tensors the struct points to alive as long as the struct
     s._keep = (cos, sin, ctx.pos, ap, ptf, ptq, ptk, sums)
     ctx.tables[key] = s

@@ -25,7 +25,7 @@ from . import _ac
 from . import _native as nv
 from ._grads import main_grad_of
 from .block import (LbBlockIO, LbLinear, LbProjection, LbStreamCtx, _arena_size, _fp, _vp,
-                    _work_arena, node_inputs)
+                    _work_arena, may_split, node_inputs)
 from .runtime_options import enabled, options as _rt
 
 
@@ -200,8 +200,8 @@ def usable(block, x, ctx) -> bool:
 def _stream_struct(ctx, plan: EncoderPlan, device, training: bool) -> LbStreamCtx:
     d = plan.desc
     grad = torch.is_grad_enabled()
-    may_split = not grad and not training
-    key = ("_lb_enc", grad, may_split, d.hd, d.H)
+    split = may_split(training)
+    key = ("_lb_enc", grad, split, d.hd, d.H)
     hit = ctx.tables.get(key)
     if hit is not None:
         return hit
@@ -222,7 +222,7 @@ def _stream_struct(ctx, plan: EncoderPlan, device, training: bool) -> LbStreamCt
         partial = _library().lb_norm_bwd_partial_rows() * 2 * d.H
         sums = torch.empty(partial + 2 * d.H, dtype=torch.float32, device=device)
         s.norm_scratch, s.wg_tmp = sums.data_ptr(), sums.data_ptr() + 4 * partial
-    s.may_split = int(may_split)
+    s.may_split = int(split)
     s._keep = (ctx.pos, ap, ptf, ptq, sums)
     ctx.tables[key] = s
     return s

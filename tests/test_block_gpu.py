@@ -156,3 +156,14 @@ def test_full_activation_checkpointing_recomputes_through_the_runner():
     for n, p in model.named_parameters():
         a, b = grads[n].float(), p.grad.float()
         assert torch.allclose(a, b, rtol=2e-2, atol=2e-2 * a.abs().max().item() + 1e-6), n
+
+
+@pytest.mark.parametrize("kind", ["qwen3", "llama"])
+def test_eval_passes_with_and_without_gradients_have_the_same_bits(kind):
+    """A cached-gradient step encodes without gradients first and again with them."""
+    model = _build(kind, False).eval()
+    inputs = _packed_inputs(lens=(9, 20, 3))
+    with torch.no_grad():
+        first = model(**inputs)["hidden_states"]
+    assert torch.equal(first, model(**inputs)["hidden_states"])
+    nv.check_status()

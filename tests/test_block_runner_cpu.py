@@ -51,6 +51,27 @@ def test_stream_struct_owns_the_buffers_of_the_backward(ops, monkeypatch):
         assert not _stream_struct(ops, monkeypatch).norm_scratch
 
 
+@pytest.mark.parametrize("ops", [enc_ops, dec_ops])
+def test_only_passes_declared_to_be_inference_are_summed_in_pieces(ops, monkeypatch):
+    """What a checkpoint or a cached-gradient step computes without gradients is recomputed with them,
+    in evaluation mode too: the same order of summation."""
+    def splits(training):
+        return bool(_stream_struct(ops, monkeypatch, training).may_split)
+
+    with torch.no_grad():
+        assert not splits(False) and not splits(True)
+        with dec_ops.inference_pass():
+            assert splits(False) and not splits(True)
+            with dec_ops.inference_pass():
+                pass
+            assert splits(False)
+        assert not splits(False)
+    with torch.inference_mode():
+        assert splits(False) and not splits(True)
+    with dec_ops.inference_pass():
+        assert not splits(False)          # gradients are recorded
+
+
 class _Accepted(RuntimeError):
     pass
 

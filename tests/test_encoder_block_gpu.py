@@ -118,6 +118,14 @@ def test_gradients_below_frozen_parameters(T, trained):
             assert (got[n] - want).norm().item() < 2e-2 * size, n
 
 
+def test_eval_passes_with_and_without_gradients_have_the_same_bits():
+    model, inputs = _model(768, 12, 3072, False).eval(), _inputs([9, 20, 3], False)
+    with torch.no_grad():
+        first = model(**inputs)["hidden_states"]
+    assert torch.equal(first, model(**inputs)["hidden_states"])
+    nv.check_status()
+
+
 def test_passes_of_models_of_different_width_interleaved(monkeypatch):
     """The wider model's pass, between the narrower one's two, asks for larger buffers."""
     from lset_b200.ops import norm
