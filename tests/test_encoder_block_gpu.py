@@ -213,3 +213,20 @@ def test_bias_grad(T, parts):
     ref = dy.double().sum(0) + 2
     # fp32 sums of T terms
     assert (torch.cat(outs).double() - ref).abs().max().item() < T * 2 ** -23 * 8
+
+
+@pytest.mark.parametrize("T", [4096, 4097, 8191, 20000])
+def test_bias_grad_sums_in_a_fixed_order(T):
+    """Pass after pass the same bits, from one chunk of rows to a cluster of eight."""
+    import ctypes
+
+    N = 776
+    dy = torch.randn(T, N, device="cuda").to(torch.bfloat16)
+    vp, outs = ctypes.c_void_p, []
+    for _ in range(20):
+        out = torch.zeros(N, device="cuda")
+        assert nv.load().lb_bias_grad(vp(dy.data_ptr()), ctypes.c_longlong(N), T, N, 0, 0,
+                                      vp(out.data_ptr()), vp(0), vp(0), vp(nv.stream_ptr())) == 0
+        outs.append(out)
+    assert all(torch.equal(o, outs[0]) for o in outs)
+    assert (outs[0].double() - dy.double().sum(0)).abs().max().item() < T * 2 ** -23 * 8
