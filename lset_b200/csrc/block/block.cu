@@ -303,18 +303,25 @@ int glu_proj_fwd(const LbBlockDesc* d, const __nv_bfloat16* x, __nv_bfloat16* gu
     g.N = 2 * I;
     g.K = d->H;
     g.b_ready = 1;
-    double apart = 3.0 + 6.0 * T * I / 5e6;  // the activation: a launch, three passes at 5 TB/s
-    for (int i = 0; i < p.n; ++i)
-      apart += lb_gemm_tile_cost(T, p.part[i].n_out, d->H, 0);
-    if (small_wins(&g, apart)) {
+    // On the CTA-pair kernel the activation costs the epilogue (3 us of the model) and saves a launch and
+    // its passes over memory. With one fused weight and the products kept that is even up to some
+    // thousand tokens (2048: 46.8 against 45.3 us, 4100: 71 against 68, 22627: 257 against 266).
+    const bool pair = T >= 256 && I >= 256 && g.ldb[0] == g.ldb[1] && lb_gemm_use_2cta(-1) &&
+                      (p.n == 2 || !keep_gu || T >= 8192);
+    double other = 3.0;
+    if (pair) {
+      other += lb_gemm_tile_cost(T, 2 * I, d->H, 0);
+    } else {
+      other += 6.0 * T * I / 5e6;   // the activation: a launch, three passes at 5 TB/s
+      for (int i = 0; i < p.n; ++i) other += lb_gemm_tile_cost(T, p.part[i].n_out, d->H, 0);
+    }
+    // (measured, small / pair: 520 x 3072 x 1024 25 / 29 us, 800 x 9728 x 2560 175 / 121, 1500 x 1152 x 768
+    // 21 / 25, 6000 x 1152 x 768 48 / 39)
+    if (small_wins(&g, other)) {
       t_fewer += p.n;
       return lb_gemm_small(&g);
     }
-    // On the CTA-pair kernel the activation costs the epilogue and saves a launch and its passes over
-    // memory. With one fused weight and the products kept that is even up to some thousand tokens
-    // (2048: 46.8 against 45.3 us, 4100: 71 against 68, 22627: 257 against 266).
-    if (T >= 256 && I >= 256 && g.ldb[0] == g.ldb[1] && lb_gemm_use_2cta(-1) &&
-        (p.n == 2 || !keep_gu || T >= 8192)) {
+    if (pair) {
       t_fewer += p.n;
       return lb_gemm_glu_2cta(x, g.B[0], g.B[1], g.C[0], g.C[1], h, T, I, d->H, d->H, g.ldb[0], 2 * I,
                               I, d->act_kind, c->status, c->stream);
