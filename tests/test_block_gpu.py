@@ -167,3 +167,43 @@ def test_eval_passes_with_and_without_gradients_have_the_same_bits(kind):
         first = model(**inputs)["hidden_states"]
     assert torch.equal(first, model(**inputs)["hidden_states"])
     nv.check_status()
+
+
+@pytest.mark.parametrize("kind", ["qwen3", "llama"])
+@pytest.mark.parametrize("trained", ["embed_tokens", "norm", "q_proj", "o_proj", "down_proj", "gate_proj"])
+def test_gradients_with_most_of_the_block_frozen(kind, trained):
+    """The launches of a backward follow each other differently with every set of frozen parameters;
+    the later ones may start while those in front of them run."""
+    model = _build(kind, False)
+    for n, p in model.named_parameters():
+        p.requires_grad_(trained in n)
+    inputs, grads = _packed_inputs(lens=(37, 130, 5)), []
+    for use in (True, True, True, False):
+        _run(model, inputs, use)
+        grads.append({n: p.grad.float() for n, p in model.named_parameters() if p.requires_grad})
+    assert grads[0]
+    for n, want in grads[-1].items():
+        for got in grads[:-1]:       # atomics order the sums of weight gradients
+            assert (got[n] - want).norm().item() <= 2e-2 * want.norm().item(), n
+
+
+def test_models_of_different_width_with_interleaved_passes():
+    """Each pass has sums and storage of its own."""
+    models, inputs = [_build("qwen3", False), _build("llama", True)], _packed_inputs()
+    wide = LlamaBidirectionalModel(LlamaConfig(vocab_size=1024, hidden_size=1024, intermediate_size=2048,
+                                               num_hidden_layers=1, num_attention_heads=16,
+                                               num_key_value_heads=8, head_dim=64))
+    models.append(wide.cuda().to(torch.bfloat16))
+    want = []
+    for m in models:
+        _run(m, inputs, True)
+        want.append({n: p.grad.float() for n, p in m.named_parameters()})
+        for p in m.parameters():
+            p.grad = None
+    outs = [m(**inputs)["hidden_states"] for m in models]
+    for m, out in zip(models, outs):
+        (out.float() * torch.linspace(-1, 1, out.shape[-1], device=out.device)).sum().backward()
+    nv.check_status()
+    for m, grads in zip(models, want):
+        for n, p in m.named_parameters():
+            assert (p.grad.float() - grads[n]).norm().item() <= 2e-2 * grads[n].norm().item(), n

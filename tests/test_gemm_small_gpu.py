@@ -176,8 +176,13 @@ def test_unsplit_it_has_the_bits_of_the_tile_kernels(T, N, K, a_mn, b_mn):
         out[on] = torch.zeros(T, N, device="cuda", dtype=dtype)
         matmul_abt(a, b, a_mn=bool(a_mn), b_mn=bool(b_mn), out=out[on], accumulate=bool(a_mn))
     nv.load().lb_gemm_use_2cta(before)
-    nv.check_status()
     assert torch.equal(out[0], out[1])
+    for bn in (64, 128):         # the kernel itself: what the dispatch above takes is the model's choice
+        c = torch.zeros_like(out[0])
+        assert _call(a, [b], [c], T, N, K, [N], N_PARTS, a_mn=a_mn, b_mn=b_mn, fp32=a_mn, bn=bn,
+                     splits=1) == 0
+        assert torch.equal(c, out[0]), bn
+    nv.check_status()
 
 
 @pytest.mark.parametrize("T,I,K", [(256, 256, 64), (257, 264, 200), (700, 1160, 1024)])
