@@ -156,7 +156,19 @@ def _linear_parts(m):
     return None
 
 
-class BlockPlan:
+def _no_plan():
+    return None
+
+
+class Plan:
+    """Kept in its block's ``__dict__``. A copy or a pickle of the model is without it (the descriptor
+    holds addresses) and makes its own."""
+
+    def __reduce__(self):
+        return _no_plan, ()
+
+
+class BlockPlan(Plan):
     """What the runner needs to know about one ``DecoderBlock``: which tensors feed which field of
     the descriptor. Pointers are re-read on every call (parameters may be re-homed into flat
     buffers after the plan was made)."""

@@ -24,7 +24,7 @@ from torch.nn.modules.module import _has_any_global_hook
 from . import _ac
 from . import _native as nv
 from ._grads import main_grad_of
-from .block import (LbBlockIO, LbLinear, LbProjection, LbStreamCtx, _arena_size, _fp, _vp,
+from .block import (LbBlockIO, LbLinear, LbProjection, LbStreamCtx, Plan, _arena_size, _fp, _vp,
                     _work_arena, may_split, node_inputs)
 from .runtime_options import enabled, options as _rt
 
@@ -72,7 +72,7 @@ def _plain(m) -> bool:
             and m.weight.shape[0] % 8 == 0 and m.weight.shape[1] % 8 == 0)
 
 
-class EncoderPlan:
+class EncoderPlan(Plan):
     """The tensors that feed the descriptor (``desc``: its sizes); addresses are read on every call."""
 
     def __init__(self, block):

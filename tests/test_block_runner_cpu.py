@@ -1,5 +1,7 @@
 """Host side of the block runners: what their structs point to, and which blocks they take."""
+import copy
 import ctypes
+import pickle
 from types import SimpleNamespace
 
 import pytest
@@ -198,3 +200,14 @@ def test_backward_passes_that_overlap_do_not_share_their_temporary_storage():
     a, b = (dec_ops._work_arena(3 << 20, torch.device("cpu")) for _ in range(2))
     assert a.numel() >= 3 << 20
     assert a.data_ptr() + a.numel() <= b.data_ptr() or b.data_ptr() + b.numel() <= a.data_ptr()
+
+
+@pytest.mark.parametrize("make,plan", [(_bert_block, _encoder_plan), (_decoder_block, _decoder_plan)])
+@pytest.mark.parametrize("copied", [copy.deepcopy, lambda m: pickle.loads(pickle.dumps(m))])
+def test_a_block_that_has_run_can_be_copied_and_pickled(make, plan, copied):
+    block = make()
+    block.__dict__["_lb_plan"] = plan()[0]      # as after a pass on the GPU
+    other = copied(block)
+    assert other.__dict__["_lb_plan"] is None
+    for a, b in zip(block.parameters(), other.parameters()):
+        assert torch.equal(a, b)

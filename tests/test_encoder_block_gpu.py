@@ -118,6 +118,16 @@ def test_gradients_below_frozen_parameters(T, trained):
             assert (got[n] - want).norm().item() < 2e-2 * size, n
 
 
+def test_copy_of_a_model_that_has_run():
+    import copy
+
+    model, inputs = _model(128, 2, 256, False), _inputs([20, 9], False)
+    want = _run(model, inputs, True)
+    before = enc_ops.calls
+    assert torch.equal(_run(copy.deepcopy(model), inputs, True), want)
+    assert enc_ops.calls == before + len(model.layers)
+
+
 def test_eval_passes_with_and_without_gradients_have_the_same_bits():
     model, inputs = _model(768, 12, 3072, False).eval(), _inputs([9, 20, 3], False)
     with torch.no_grad():
