@@ -269,25 +269,26 @@ class BlockPlan(Plan):
         dst.w = w.data_ptr()
         dst.ldw = w.stride(0)
         dst.n_out, dst.k_in = w.shape
-        dst.wgrad = grads.get(id(w))
+        if grads:            # (of a pass without gradients the accumulators stay null)
+            dst.wgrad = grads.get(id(w))
         if a is not None:
             dst.lora_a, dst.lora_b = a.data_ptr(), b.data_ptr()
             dst.lora_a_grad, dst.lora_b_grad = grads.get(id(a)), grads.get(id(b))
             dst.lora_r, dst.lora_scale = a.shape[0], scale
-        else:
-            dst.lora_a = dst.lora_b = dst.lora_a_grad = dst.lora_b_grad = None
-            dst.lora_r, dst.lora_scale = 0, 0.0
 
     def fill(self, grads: dict) -> LbBlockDesc:
         """A descriptor of its own for the call (another thread may be in a pass of the same block),
         with the tensors' present addresses. ``grads`` maps ``id(param)`` to the address of its fp32
         gradient accumulator (absent = no weight gradient wanted)."""
         d = LbBlockDesc.from_buffer_copy(self.desc)
-        d.ln1_w, d.ln1_wgrad = self.ln1.weight.data_ptr(), grads.get(id(self.ln1.weight))
-        d.ln2_w, d.ln2_wgrad = self.ln2.weight.data_ptr(), grads.get(id(self.ln2.weight))
+        ln1, ln2 = self.ln1.weight, self.ln2.weight
+        d.ln1_w, d.ln2_w = ln1.data_ptr(), ln2.data_ptr()
         if self.qn is not None:
-            d.qn_w, d.qn_wgrad = self.qn.data_ptr(), grads.get(id(self.qn))
-            d.kn_w, d.kn_wgrad = self.kn.data_ptr(), grads.get(id(self.kn))
+            d.qn_w, d.kn_w = self.qn.data_ptr(), self.kn.data_ptr()
+        if grads:
+            d.ln1_wgrad, d.ln2_wgrad = grads.get(id(ln1)), grads.get(id(ln2))
+            if self.qn is not None:
+                d.qn_wgrad, d.kn_wgrad = grads.get(id(self.qn)), grads.get(id(self.kn))
         for i, p in enumerate(self.qkv):
             self._fill_linear(d.qkv.part[i], p, grads)
         for i, p in enumerate(self.gate_up):

@@ -109,6 +109,11 @@ class EncoderPlan(Plan):
         d.qkv.n, d.qkv.width = len(qkv), 3 * H
         self.desc = d
         self.linears = [*enumerate(qkv), (3, o), (4, fin), (5, fout)]
+        part = d.qkv.part
+        for i, m in self.linears:
+            dst = (part[0], part[1], part[2], d.o_proj, d.in_, d.out)[i]
+            dst.n_out, dst.k_in = m.weight.shape
+            dst.ldw = m.weight.stride(0)
         self.norms = [(ln1, "ln1"), (ln2, "ln2")]
         self.params = [p for ln, _ in self.norms for p in (ln.weight, ln.bias)]
         self.params += [p for _, m in self.linears for p in (m.weight, m.bias)]
@@ -139,20 +144,24 @@ class EncoderPlan(Plan):
 
     def fill(self, grads: dict) -> LbEncoderDesc:
         """A descriptor of its own for the call (another thread may be in a pass of the same block),
-        with the tensors' present addresses; ``grads`` as in ``BlockPlan.fill``."""
+        with the tensors' present addresses; ``grads`` as in ``BlockPlan.fill``. (Sizes are part of
+        the signature; of a pass without gradients the accumulators stay null.)"""
         d = LbEncoderDesc.from_buffer_copy(self.desc)
-        part = d.qkv.part
+        part, bias = d.qkv.part, d.bias
+        (l1, _), (l2, _) = self.norms
+        d.ln1_w, d.ln1_b = l1.weight.data_ptr(), l1.bias.data_ptr()
+        d.ln2_w, d.ln2_b = l2.weight.data_ptr(), l2.bias.data_ptr()
         slots = (part[0], part[1], part[2], d.o_proj, d.in_, d.out)
-        for ln, name in self.norms:
-            setattr(d, name + "_w", ln.weight.data_ptr())
-            setattr(d, name + "_b", ln.bias.data_ptr())
-            setattr(d, name + "_wgrad", grads.get(id(ln.weight)))
-            setattr(d, name + "_bgrad", grads.get(id(ln.bias)))
         for i, m in self.linears:
-            dst, w = slots[i], m.weight
-            dst.w, dst.wgrad, dst.ldw = w.data_ptr(), grads.get(id(w)), w.stride(0)
-            dst.n_out, dst.k_in = w.shape
-            d.bias[i], d.bias_grad[i] = m.bias.data_ptr(), grads.get(id(m.bias))
+            slots[i].w = m.weight.data_ptr()
+            bias[i] = m.bias.data_ptr()
+        if grads:
+            for ln, name in self.norms:
+                setattr(d, name + "_wgrad", grads.get(id(ln.weight)))
+                setattr(d, name + "_bgrad", grads.get(id(ln.bias)))
+            for i, m in self.linears:
+                slots[i].wgrad = grads.get(id(m.weight))
+                d.bias_grad[i] = grads.get(id(m.bias))
         return d
 
 
