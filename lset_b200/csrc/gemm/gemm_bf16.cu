@@ -1131,8 +1131,17 @@ extern "C" int lb_gemm_fp8(const void* A, const void* B, void* C, int M, int N, 
   if (!out_fp32 && (accumulate || splits > 1)) return -5;
   constexpr int BKE = 2 * BK;
   // CTA pairs from one 256 x 256 tile up, as for bf16: 21760 x 19456 x 2560 877 -> 791 us, 21760 x 2560 x
-  // 9728 376 -> 350, the weight gradient 2560 x 9728 x 21760 577 -> 457; even at 1000 x 2560 x 2560.
-  if (use_2cta() && bias == nullptr && bn == 0 && M >= 256 && N >= 256) {
+  // 9728 376 -> 350, the weight gradient 2560 x 9728 x 21760 577 -> 457; even at 1000 x 2560 x 2560. Not
+  // where rows to fill up their taller tiles cost waves: 300 x 12288 x 4096 (2 waves of pairs, 1 of the
+  // one-CTA kernel) 32.8 us on the one-CTA kernel, 40.8 on pairs, 800 x 9728 x 2560 (3, 2) 32.7 and 38.2,
+  // 800 x 24576 x 4096 (6, 5) 83.9 and 83.3. (Weight gradients, which split, are always faster on pairs.)
+  const long long pair_tiles = 1LL * ((M + 255) / 256) * ((N + 255) / 256);
+  const int one_bn = one_cta_bn(M, N), pairs = lb_gemm_2cta_pairs();
+  const long long one_tiles = 1LL * ((M + BM - 1) / BM) * ((N + one_bn - 1) / one_bn);
+  const long long pair_waves = (pair_tiles + pairs - 1) / pairs;
+  const double one_waves = double((one_tiles + num_sms() - 1) / num_sms()) * one_bn / 256;
+  const bool fill = accumulate || pair_waves <= 1.2 * one_waves;
+  if (use_2cta() && bias == nullptr && bn == 0 && M >= 256 && N >= 256 && fill) {
     int s2 = splits;
     if (s2 == 0)
       s2 = (out_fp32 && accumulate)
@@ -1143,14 +1152,7 @@ extern "C" int lb_gemm_fp8(const void* A, const void* B, void* C, int M, int N, 
   }
   const int tiles_m = (M + BM - 1) / BM;
   const int sms = num_sms();
-  if (bn != 128 && bn != 256) {
-    auto eff = [&](int b) {
-      const long long t = 1LL * tiles_m * ((N + b - 1) / b);
-      const long long waves = (t + sms - 1) / sms;
-      return double(t) * b / double(waves * sms);
-    };
-    bn = (N > 128 && eff(256) >= eff(128)) ? 256 : 128;
-  }
+  if (bn != 128 && bn != 256) bn = one_bn;
   const int tiles_n = (N + bn - 1) / bn;
   const int kb_total = (K + BKE - 1) / BKE;
   if (splits == 0)
