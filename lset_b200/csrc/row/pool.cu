@@ -100,7 +100,49 @@ __global__ void __launch_bounds__(kRowThreads)
   }
 }
 
-// Means over a segment's tokens: what bounds this is the latency of a long segment's loads (its sums are
+// Many or short segments: one CTA per segment, threads are (column-vector, token-subset) pairs with 16
+// bytes a load. Enough CTAs run side by side to hide the latency that bounds the kernel below, which
+// pays for 16 times as many (5000 segments of one token x 768: 32 us here, 128 there; 20000 of 3 x 1024 133
+// and 674; 600 of 30 x 1024 18 and 25, of 300 84 and 91; but 300 of 300 68 and 57). The same sums in the
+// same order from 64 columns up.
+__global__ void __launch_bounds__(kRowThreads)
+    segment_mean_rows_kernel(const bf16* __restrict__ x, const int* __restrict__ cu,
+                             bf16* __restrict__ out, int H, int weighted) {
+  extern __shared__ float sacc[];  // [S, H]
+  const int seg = blockIdx.x;
+  const int t0 = cu[seg], t1 = cu[seg + 1];
+  const int len = t1 - t0;
+  const int CV = min(H / 8, kRowThreads);
+  const int S = kRowThreads / CV;
+  const int cvi = threadIdx.x % CV;
+  const int sub = threadIdx.x / CV;
+  const bool active = sub < S;
+  const float wden = weighted ? 0.5f * float(len) * float(len + 1) : float(len);
+  for (int c = cvi * 8; c < H; c += CV * 8) {
+    float acc[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] = 0.f;
+    if (active) {
+      for (int tok = t0 + sub; tok < t1; tok += S) {
+        float v[8];
+        unpack8(ld16(x + 1LL * tok * H + c), v);
+        const float wt = weighted ? float(tok - t0 + 1) : 1.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[i] += wt * v[i];
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) sacc[sub * H + c + i] = acc[i];
+    }
+  }
+  __syncthreads();
+  for (int c = threadIdx.x; c < H; c += kRowThreads) {
+    float s = 0.f;
+    for (int k = 0; k < S; ++k) s += sacc[k * H + c];
+    out[1LL * seg * H + c] = __float2bfloat16_rn(len > 0 ? s / wden : 0.f);
+  }
+}
+
+// Means over the tokens of few segments: what bounds this is the latency of a long segment's loads (its sums are
 // serial in each token subset, and their order is kept). One CTA per segment with a lane per eight
 // columns and one load in flight took 611 us for 17 segments of 4096 x 1024 and 1208 for a longest one
 // of 8192; with 64 columns a CTA, a lane per two and 32 loads in flight 135 and 244 (24 of 30 x 768:
@@ -221,13 +263,21 @@ extern "C" int lb_l2norm_bwd(const void* gy, long long ldgy, const void* y, long
   return launch_rc();
 }
 
-extern "C" int lb_segment_mean_fwd(const void* x, const int* cu_seqlens, void* out, int M, int H,
+// T: tokens in x, of all segments.
+extern "C" int lb_segment_mean_fwd(const void* x, const int* cu_seqlens, void* out, int T, int M, int H,
                                    int weighted, void* stream) {
   if (M <= 0) return 0;
   if ((H & 7) || H > 12288) return -3;
   // token subsets as many as lanes of eight columns leave of a CTA of kRowThreads, at most 32
   const int CV = (H / 8) < kRowThreads ? (H / 8) : kRowThreads;
   int S = kRowThreads / CV;
+  const bool aligned = (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+  if (aligned && (M >= 3 * row_num_sms() || T <= 16LL * M)) {
+    segment_mean_rows_kernel<<<M, kRowThreads, size_t(S) * H * sizeof(float),
+                               reinterpret_cast<cudaStream_t>(stream)>>>(
+        (const bf16*)x, cu_seqlens, (bf16*)out, H, weighted);
+    return launch_rc();
+  }
   if (S > kSegMaxSubsets) S = kSegMaxSubsets;
   segment_mean_fwd_kernel<<<dim3(M, (H + kSegCols - 1) / kSegCols), 32 * S, 0,
                             reinterpret_cast<cudaStream_t>(stream)>>>(

@@ -85,7 +85,7 @@ class _SegmentMean(torch.autograd.Function):
         out = torch.empty(M, H, dtype=x.dtype, device=x.device)
         rc = nv.load().lb_segment_mean_fwd(
             nv.c_void_p(x.data_ptr()), nv.c_void_p(cu.data_ptr()), nv.c_void_p(out.data_ptr()),
-            nv.c_int(M), nv.c_int(H), nv.c_int(int(weighted)), nv.c_void_p(nv.stream_ptr()))
+            nv.c_int(x.shape[0]), nv.c_int(M), nv.c_int(H), nv.c_int(int(weighted)), nv.c_void_p(nv.stream_ptr()))
         nv.check_rc(rc, "lb_segment_mean_fwd")
         nv.count_launch()
         ctx.save_for_backward(cu)

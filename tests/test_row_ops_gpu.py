@@ -277,6 +277,32 @@ def test_segment_mean_chunk_edges(H, weighted):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("H", [8, 64, 136, 1024, 2560])
+def test_segment_mean_of_many_or_short_segments(H, weighted):
+    """These have a kernel of their own: the sums of the other one, in its order from 64 columns up."""
+    from lset_b200.ops.pooling import segment_mean
+
+    lens = [1, 0, 3, 40, 17, 33, 100]
+    one = torch.randn(sum(lens), H, generator=torch.Generator().manual_seed(H)).bfloat16().cuda()
+    few = segment_mean(one, torch.tensor([0] + lens).cumsum(0).int().cuda(), weighted)
+    cu = torch.tensor([0] + lens * 90).cumsum(0).int().cuda()
+    many = segment_mean(one.repeat(90, 1), cu, weighted).view(90, len(lens), H)
+    assert torch.equal(many, many[:1].expand_as(many))
+    if H >= 64:
+        assert torch.equal(many[0], few)
+    ref = torch.stack([(s.double() * (torch.arange(1, n + 1, device="cuda").double()[:, None]
+                                      if weighted else 1)).sum(0)
+                       / max(1.0, n * (n + 1) / 2 if weighted else n)
+                       for n, s in zip(lens, one.split(lens))])
+    # one rounding to bf16 and fp32 sums of at most 100 terms
+    assert ((many[0].double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-4).all()
+    short = segment_mean(one[:20], torch.tensor([0, 1, 1, 5, 20]).int().cuda(), weighted)
+    if H >= 64:
+        assert torch.equal(short[0], few[0])
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("offset", [1, 4])
 @pytest.mark.parametrize("H", [64, 136, 1024, 2560])
 def test_rms_norm_takes_a_weight_that_starts_anywhere(H, offset):
