@@ -3,9 +3,10 @@
 // What bounds it: per 128 x 128 block of scores the two products take 1024 tensor clocks at
 // head dim 128 and the 16384 exponentials 1024 clocks of the SM's 16-a-clock unit, so neither may
 // wait for the other. A kernel in which the same 128 threads wait for the score product, do the
-// softmax and then wait for P·V (attn_fwd_kernel below, two CTAs per SM) spends most of its time in
-// those waits. Here the roles are separate warps and one CTA (one per SM) works on two query
-// tiles of one sequence and KV head, which share every K and V tile:
+// softmax and then wait for P·V (attn_fwd_kernel in attn_fwd.cu, two CTAs per SM) spends most of its
+// time in those waits. Here the roles are separate warps and one CTA (one per SM) works on two query
+// tiles of one sequence and KV head, which share every K and V tile (the arrangement published for
+// FlashAttention-4, with its rescale only where the maximum rose by more than 2^8):
 //
 //   warps 0-3   softmax of tile 0 (thread = row)      warps 4-7   softmax of tile 1
 //   warp 8      work items, TMA loads                 warp 9      tcgen05.mma issuer
@@ -22,7 +23,8 @@
 //   10 x 4096 tokens, 16/8 heads of 128, causal     1584 -> 741 (930 TFLOP/s), bidirectional 1355
 //   128 sequences of 128..512, same heads           266  -> 207
 //   64 of 16..64 and 64 of 128..512, same heads     151  -> 127
-// The short ones pay per work item: its first products and its store overlap with nothing.
+// The short ones pay per work item: its first products and its store overlap with nothing. Where most
+// sequences fit in one tile the one-tile kernel is faster (AttnPlan._one_tile).
 //
 // Tensor memory: S0 | S1 | O0 | O1, 128 columns each.
 #pragma once

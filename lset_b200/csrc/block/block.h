@@ -73,11 +73,12 @@ struct LbStreamCtx {
   const int* plan_kv;    // tile list for 128 tokens per tile
   int cap_kv;
   int* status;           // device status word for bounded waits
+  // of a pass that records gradients, written by its backward only:
   float* norm_scratch;   // lb_norm_bwd_partial_rows() * H floats
   float* rope_scratch;   // lb_rope_bwd_partial_rows() * 2 * hd floats
   float* wg_tmp;         // 2 * hd floats (QK-norm weight gradient staging)
   void* stream;
-  int may_split;         // inference: contractions may be summed in pieces (LbSmallGemm::may_split)
+  int may_split;         // a pass declared inference: contractions may be summed in pieces (see LbSmallGemm)
 };
 
 // Tensor parallelism with a token-sharded residual stream (sequence parallelism): the block's

@@ -4,8 +4,9 @@ Op by op a block is eight launches forward and about thirty backward, each with 
 a foreign call of its own: at the batch sizes such encoders are used with, the host needs several
 times longer to issue them than the GPU to run them. ``run`` hands the sequence to
 ``lb_encoder_fwd`` / ``lb_encoder_bwd`` (``csrc/block/block.cu``), as ``ops/block.py`` does for the
-decoder block; autograd sees one node. Forward values have the bits of the op-by-op path; bias
-gradients are added to their fp32 accumulators without a rounding to bf16 in between.
+decoder block; autograd sees one node. Forward values have the bits of the op-by-op path, except in
+passes declared to be inference (``ops.block.inference_pass``), whose products may be summed in
+pieces; bias gradients are added to their fp32 accumulators without a rounding to bf16 in between.
 
 Taken for blocks of plain bf16 ``Linear`` layers with biases (fused or separate query / key / value)
 on the GPU; everything else (tensor parallelism, 8-bit layers, adapters, selective activation

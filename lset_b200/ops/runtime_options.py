@@ -23,7 +23,9 @@ class RuntimeOptions:
     fused_double_rmsnorm: bool = True
     block_runner: bool = True       # whole decoder / encoder blocks issued by the native block runner
     tp_block_runner: bool = True    # ... also tensor-parallel blocks on a token-sharded stream
-    fused_glu_gemm: bool = False    # gated-MLP activation in the epilogue of the gate/up GEMM (measured slower: off)
+    # gated-MLP activation in the epilogue of the one-CTA gate/up GEMM, op by op (measured slower: off).
+    # The block runner has kernels of its own for it and takes them by size, whatever this says.
+    fused_glu_gemm: bool = False
     attention_backend: str = "auto"  # auto | native | sdpa
 
 
