@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(kBwdThreads)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4);
 
   const int tid = threadIdx.x;
-  const int warp = tid >> 5;
+  const int warp = warp_index();
   const int half = warp >> 2;  // which 32 of the 64 KV columns this thread handles
   auto load_kv = [&](int j) {
     mbar_expect_tx(bar_kv, 2 * C::KV_BYTES);
@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(kBwdThreads)
   // products itself; whether a wait ran out anywhere is agreed on at the barrier.
   for (int j = 0; j < nblk && !failed; ++j) {
     bool ok = true;
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
       ok = mbar_wait(bar_kv, j & 1);
       if (ok) {
         tc_fence_after();
@@ -355,7 +355,7 @@ __global__ void __launch_bounds__(kBwdThreads)
       failed = true;
       break;
     }
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
       tc_fence_after();
       const uint32_t sa = smem_u32(sdS);
       const uint32_t ka = smem_u32(sK);
@@ -467,7 +467,7 @@ __global__ void __launch_bounds__(kDkvThreads, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_work + 2);
 
   const int tid = threadIdx.x;
-  const int warp = tid >> 5;
+  const int warp = warp_index();
   const int lane = tid & 31;
 
   if (tid == kDkvMath) {
@@ -526,7 +526,7 @@ __global__ void __launch_bounds__(kDkvThreads, 1)
       // K and V of the item as soon as the last one's scores are complete: under its last math,
       // its accumulation products and its store
       ok = __all_sync(0xffffffffu, mbar_wait(bar_kve, (it & 1) ^ 1u));
-      if (ok && lane == 0) {
+      if (ok && elect_one()) {
         mbar_expect_tx(bar_kv, 2 * C::KV_BYTES);
 #pragma unroll
         for (int p = 0; p < C::PANELS; ++p) {
@@ -578,7 +578,7 @@ __global__ void __launch_bounds__(kDkvThreads, 1)
     __syncwarp();
   } else if (warp == kDkvMath / 32 + 1) {
     // -------------------------------------------------------------------- products
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, 64, 0, 0);
       constexpr uint32_t idesc_acc = umma_idesc_bf16(128, HD, 0, 1);
       const uint64_t kd = umma_smem_desc(smem_u32(sK), 16, 1024);

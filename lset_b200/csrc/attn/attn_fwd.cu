@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(128)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 5);
 
   const int tid = threadIdx.x;
-  const int warp = tid >> 5;
+  const int warp = warp_index();
   __shared__ int s_next[2];  // next work item of this CTA, published by thread 0 one tile ahead
 
   // KV block n of this CTA's whole run (all tiles) lives in slot n & 1; its barrier phase is
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(128)
           break;
         }
       }
-      if (tid == 0) {
+      if (warp == 0 && elect_one()) {
         tc_fence_after();
         const uint32_t qa = smem_u32(sQ);
         const uint32_t ka = smem_u32(sK + buf * C::KV_BYTES);
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(128)
       }
       tc_fence_after();
       // the last score product of this tile has read Q: the next tile's Q may land now
-      if (tid == 0 && last && has_next) load_q(nxt);
+      if (warp == 0 && last && has_next && elect_one()) load_q(nxt);
       float s[kAttnKvBlock];
       {
         uint32_t t0[32], t1[32];
@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(128)
         }
         tc_fence_after();
       }
-      if (tid == 0) {
+      if (warp == 0 && elect_one()) {
         if (!last) load_kv(cur, j + 1, n + 1);
         else if (has_next) load_kv(nxt, 0, n + 1);  // first block of the next work item
       }
@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(128)
       tc_fence_before();
       __syncthreads();
       // 5. O += P V
-      if (tid == 0) {
+      if (warp == 0 && elect_one()) {
         tc_fence_after();
         const uint32_t pa = smem_u32(sP);
         const uint32_t va = smem_u32(sV + buf * C::KV_BYTES);

@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_work + 2);
   uint8_t* sOut = reinterpret_cast<uint8_t*>(bars) + 256;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const int G = a.Hq / a.Hk;
   const int QT = 128 / G;               // a power of two, as G
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
 
   if (warp == 8) {
     // -------------------------------------------------------------------- work items, loads
-    if (lane == 0) {
+    if (elect_one()) {
       // Heads vary fastest, tiles run from the last to the first: under a causal mask the longest
       // items of a sequence come first.
       AttnPlanView plan{a.plan};
@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     __syncwarp();
   } else if (warp == 9) {
     // -------------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_o = umma_idesc_bf16(128, HD, 0, 1);
       // One copy of each product's instructions for both tiles: the kernel's code is fetched through
       // an instruction cache (see pair_wait).

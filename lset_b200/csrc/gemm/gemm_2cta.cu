@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(kThreads + (GATHER ? 32 * kPullWarps : 0), 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
   float* epi_stage = reinterpret_cast<float*>(smem + kStages * STAGE_BYTES + 512);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();   // 0 = leader
   const bool leader = rank == 0;
@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(kThreads + (GATHER ? 32 * kPullWarps : 0), 1)
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -384,7 +384,7 @@ __global__ void __launch_bounds__(kThreads + (GATHER ? 32 * kPullWarps : 0), 1)
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0 && leader) {
+    if (leader && elect_one()) {
       // ---------------------------------------------------------------- MMA issuer (leader)
       const uint32_t idesc = F8 ? umma_idesc_f8(2 * BMc, BNp, g.f8_a_e5m2, g.f8_b_e5m2)
                                 : umma_idesc_bf16(2 * BMc, BNp, A_MN, B_MN);

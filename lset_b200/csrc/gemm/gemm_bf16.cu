@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(gemm_threads<EPI, GATHER, F8>(), 1)
   [[maybe_unused]] float* epi_stage =
       reinterpret_cast<float*>(smem + C::STAGES * C::STAGE_BYTES + 256);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(gemm_threads<EPI, GATHER, F8>(), 1)
 
   if (warp == 0 && cta >= 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(gemm_threads<EPI, GATHER, F8>(), 1)
     __syncwarp();
   } else if (warp == 1 && cta >= 0) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = F8 ? umma_idesc_f8(BM, BN, g.f8_a_e5m2, g.f8_b_e5m2)
                                 : umma_idesc_bf16(BM, BN, A_MN, B_MN);
       int stage = 0;

@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(kThreads)
   uint64_t* tfull = empty + C::STAGES;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tfull + 1);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = warp_index();
   const int lane = threadIdx.x & 31;
   const int S = g.splits;
   const int rank = S > 1 ? int(cta_rank()) : 0;
@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(kThreads)
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       auto load_a = [&](int i) {
         uint8_t* sa = smem + (i % C::STAGES) * C::STAGE_BYTES;
         uint64_t* bar = &full[i % C::STAGES];
@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(kThreads)
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = umma_idesc_bf16(BM, BN, A_MN, B_MN);
       bool ok = true;
       for (int i = 0; i < nkb; ++i) {
