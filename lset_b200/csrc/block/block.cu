@@ -303,12 +303,12 @@ int glu_proj_fwd(const LbBlockDesc* d, const __nv_bfloat16* x, __nv_bfloat16* gu
     g.N = 2 * I;
     g.K = d->H;
     g.b_ready = 1;
-    // On the CTA-pair kernel the activation costs the epilogue (3 us of the model) and saves a launch and
+    // On the CTA-pair kernel the activation costs the epilogue (6 us of the model) and saves a launch and
     // its passes over memory. With one fused weight and the products kept that is even up to some
     // thousand tokens (2048: 46.8 against 45.3 us, 4100: 71 against 68, 22627: 257 against 266).
     const bool pair = T >= 256 && I >= 256 && g.ldb[0] == g.ldb[1] && lb_gemm_use_2cta(-1) &&
                       (p.n == 2 || !keep_gu || T >= 8192);
-    double other = 3.0;
+    double other = 6.0;
     if (pair) {
       other += lb_gemm_tile_cost(T, 2 * I, d->H, 0);
     } else {

@@ -25,6 +25,7 @@
 #include "../common/ptx.cuh"
 #include "../common/tma_desc.h"
 #include "gemm_small.h"
+#include "../common/pdl.h"
 
 namespace lb {
 
@@ -969,9 +970,10 @@ static int one_cta_bn(int M, int N) {
   return (N > 128 && eff(256) >= eff(128)) ? 256 : 128;
 }
 
-// Fitted with lb_gemm_small_plan, against which it is compared: a launch, and per wave of tiles and 64 of
-// contraction depth 0.33 us on CTA pairs, on the one-CTA kernel (for products smaller than a pair's
-// tile) 0.37 with 256 columns a tile and 0.27 with 128; a split weight gradient adds its reductions.
+// Microseconds per launch, to compare with lb_gemm_small_plan; fitted to the same kind of measurements (140
+// products of those widths at 8 to 3000 tokens, 10 % rms): a launch, per wave of tiles its set-up and
+// store and for each 64 of contraction depth 0.35 us on CTA pairs, on the one-CTA kernel (for products
+// smaller than a pair's tile) 0.3 with 256 columns a tile and 0.22 with 128; the bytes bound both.
 extern "C" double lb_gemm_tile_cost(int M, int N, int K, int fp32) {
   const bool pair = M >= 256 && N >= 256;
   const int bm = pair ? 256 : lb::BM, bn = pair ? 256 : one_cta_bn(M, N);
@@ -980,8 +982,13 @@ extern "C" double lb_gemm_tile_cost(int M, int N, int K, int fp32) {
   const int kb = (K + lb::BK - 1) / lb::BK;
   const int s = fp32 ? lb::auto_splits(tiles, kb, slots) : 1;
   const long long waves = (tiles * s + slots - 1) / slots;
-  const double block = pair ? 0.33 : (bn == 256 ? 0.37 : 0.27);
-  return 11.0 + double(waves) * ((kb + s - 1) / s) * block + (s > 1 ? 4.0 : 0.0);
+  const double block = pair ? 0.35 : (bn == 256 ? 0.3 : 0.22);
+  const double cost = 3.2 + double(waves) * (((kb + s - 1) / s) * block + 2.2) + (s > 1 ? 0.6 : 0.0);
+  const double memory =
+      3.0 + (2.0 * K * (double(M) + N) + (fp32 ? 8.0 : 2.0) * double(M) * N) / 3.73e6;
+  // in a chain of dependent launches these kernels, which are ordinary ones, wait for the end of the one
+  // in front of them where the other's set-up and first loads run under it (1.3 to 2 us)
+  return (cost > memory ? cost : memory) + (lb::pdl_enabled() ? 1.5 : 0.0);
 }
 
 static int gemm_bf16_impl(const void* A, const void* B, void* C, int M, int N, int K,

@@ -2,13 +2,13 @@
 // tokens (a query, a small training batch) against weights of any size.
 //
 // Such a product is bound by how fast the weights reach the tensor cores, and one SM takes in
-// about 64 bytes a clock however few rows there are. So the work is cut until every SM has some:
-// 128 x BN tiles (BN 64 or 128), and the contraction of a tile split over a cluster of up to eight
+// about 100 bytes a clock however few rows there are. So the work is cut until every SM has some:
+// 128 x 128 down to 64 x 32 tiles, and the contraction of a tile split over a cluster of up to eight
 // CTAs. Each CTA of the cluster leaves its fp32 partial tile in its own shared memory; after a
 // cluster barrier every CTA sums a share of the tile over the cluster through distributed shared
 // memory, in rank order (no atomics: the result does not depend on timing), and stores it. One
-// tile per CTA, about 100 KB of shared memory, so that two CTAs share an SM and one's set-up and
-// epilogue run under the other's main loop.
+// tile per CTA; up to four CTAs share an SM, and one's set-up and epilogue run under the others' main
+// loops; a CTA with an SM of its own takes all of the shared memory for its operand ring.
 //
 //   warp 0      TMA producer          warp 1   tcgen05.mma issuer
 //   warps 2-5   accumulator -> shared memory -> (cluster sum) -> global memory
@@ -30,10 +30,11 @@ namespace lb {
 
 namespace {
 
-constexpr int BM = 128;
 constexpr int BK = 64;
 constexpr int kThreads = 192;
 constexpr int kMaxSplits = 8;
+constexpr int kMaxStages = 16;          // of the operand ring
+constexpr int kRingExtra = 1024 + 512;  // alignment, barriers
 
 struct SmallArgs {
   int M, N;
@@ -49,21 +50,21 @@ struct SmallArgs {
   long long ld_h;
   int b_ready;
   int by_part;      // kParallelK of several parts: CTA r of a cluster contracts part r
-  int stage_bytes;  // what the loads of one stage bring
+  int block_bytes;  // what the loads of one k-block bring
+  int stages, kps;  // of the operand ring: stages of kps k-blocks
   int* status;
 };
 
-template <int BN>
+template <int BM, int BN>
 struct SCfg {
   static constexpr int A_BYTES = BM * BK * 2;
   static constexpr int B_BYTES = BN * BK * 2;
-  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = BN == 64 ? 4 : 3;
+  static constexpr int BLOCK_BYTES = A_BYTES + B_BYTES;
   static constexpr int PITCH = BN + 4;  // floats per row of the partial tile: 16-byte row accesses
                                         // of eight lanes then fall into different banks
-  static constexpr int RING = STAGES * STAGE_BYTES;
-  static constexpr int SMEM_BYTES = RING + 1024 + 256;
-  static_assert(BM * PITCH * 4 <= RING, "the partial tile reuses the operand ring");
+  // the partial tile reuses the operand ring
+  static constexpr int MIN_BLOCKS = (BM * PITCH * 4 + BLOCK_BYTES - 1) / BLOCK_BYTES;
+  static constexpr int smem_bytes(int blocks) { return blocks * BLOCK_BYTES + kRingExtra; }
 };
 
 __device__ __forceinline__ uint32_t cta_rank() {
@@ -150,19 +151,20 @@ __device__ __forceinline__ float4 cluster_sum4(uint32_t base, uint32_t off, int 
   return acc;
 }
 
-template <int A_MN, int B_MN, int BN, typename OutT, int GLU>
+template <int A_MN, int B_MN, int BM, int BN, typename OutT, int GLU>
 __global__ void __launch_bounds__(kThreads)
     gemm_small_kernel(const __grid_constant__ CUtensorMap tmA,
                       const __grid_constant__ CUtensorMap tmB0,
                       const __grid_constant__ CUtensorMap tmB1,
                       const __grid_constant__ CUtensorMap tmB2, SmallArgs g) {
-  using C = SCfg<BN>;
+  using C = SCfg<BM, BN>;
+  const int stages = g.stages, kps = g.kps;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + C::RING);
-  uint64_t* empty = full + C::STAGES;
-  uint64_t* tfull = empty + C::STAGES;
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + stages * kps * C::BLOCK_BYTES);
+  uint64_t* empty = full + kMaxStages;
+  uint64_t* tfull = empty + kMaxStages;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tfull + 1);
 
   const int warp = warp_index();
@@ -197,7 +199,7 @@ __global__ void __launch_bounds__(kThreads)
   if (GLU) n_ext = g.ext[0];
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < C::STAGES; ++s) {
+    for (int s = 0; s < stages; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
@@ -218,9 +220,12 @@ __global__ void __launch_bounds__(kThreads)
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (elect_one()) {
-      auto load_a = [&](int i) {
-        uint8_t* sa = smem + (i % C::STAGES) * C::STAGE_BYTES;
-        uint64_t* bar = &full[i % C::STAGES];
+      const int bp = g.mode == kParallelN ? part : (g.by_part ? rank : 0);
+      const CUtensorMap* tb = bp == 0 ? &tmB0 : (bp == 1 ? &tmB1 : &tmB2);
+      const int kb_b = kb0 - (g.by_part ? g.first[rank] : 0);
+      auto load_a = [&](int i, int s) {   // i: k-block, s: ring position in blocks
+        uint8_t* sa = smem + s * C::BLOCK_BYTES;
+        uint64_t* bar = &full[kps == 1 ? s : s >> 1];
         const int kc = (kb0 + i) * BK;
         if (A_MN) {
 #pragma unroll
@@ -230,17 +235,10 @@ __global__ void __launch_bounds__(kThreads)
           tma_load_2d(sa, &tmA, bar, kc, am0);
         }
       };
-      auto load_b = [&](int i) {
-        uint8_t* sb = smem + (i % C::STAGES) * C::STAGE_BYTES + C::A_BYTES;
-        uint64_t* bar = &full[i % C::STAGES];
-        const int kb = kb0 + i;
-        int p = g.mode == kParallelN ? part : 0, kl = kb;
-        if (g.mode == kParallelK) {
-          while (p + 1 < g.nparts && kb >= g.first[p + 1]) ++p;
-          kl = kb - g.first[p];
-        }
-        const CUtensorMap* tb = p == 0 ? &tmB0 : (p == 1 ? &tmB1 : &tmB2);
-        const int kc = kl * BK;
+      auto load_b = [&](int i, int s) {
+        uint8_t* sb = smem + s * C::BLOCK_BYTES + C::A_BYTES;
+        uint64_t* bar = &full[kps == 1 ? s : s >> 1];
+        const int kc = (kb_b + i) * BK;
         if (GLU) {  // gate rows, then up rows of the same features
           tma_load_2d(sb, &tmB0, bar, kc, n0);
           tma_load_2d(sb + (BN / 2) * 128, &tmB1, bar, kc, n0);
@@ -252,30 +250,40 @@ __global__ void __launch_bounds__(kThreads)
           tma_load_2d(sb, tb, bar, kc, n0);
         }
       };
-      const int pre = nkb < C::STAGES ? nkb : C::STAGES;
-      for (int i = 0; i < pre; ++i) mbar_expect_tx(&full[i], g.stage_bytes);
+      const int pre = min(nkb, stages * kps);
+      for (int i = 0, s = 0; i < pre; i += kps, ++s)
+        mbar_expect_tx(&full[s], g.block_bytes * min(kps, nkb - i));
       if (g.b_ready) {
-        for (int i = 0; i < pre; ++i) load_b(i);
+        for (int i = 0; i < pre; ++i) load_b(i, i);
         pdl_wait();
-        for (int i = 0; i < pre; ++i) load_a(i);
+        for (int i = 0; i < pre; ++i) load_a(i, i);
       } else {
         pdl_wait();
         for (int i = 0; i < pre; ++i) {
-          load_a(i);
-          load_b(i);
+          load_a(i, i);
+          load_b(i, i);
         }
       }
       bool ok = true;
-      for (int i = pre; i < nkb; ++i) {
-        const int s = i % C::STAGES;
-        if (!mbar_wait(&empty[s], ((i / C::STAGES) & 1) ^ 1u)) {
+      int s = 0;
+      uint32_t phase = 0;
+      for (int i = pre; i < nkb; i += kps) {
+        if (!mbar_wait(&empty[s], phase)) {
           report_status(g.status, kStatusTimeoutProducer);
           ok = false;
           break;
         }
-        mbar_expect_tx(&full[s], g.stage_bytes);
-        load_a(i);
-        load_b(i);
+        const int here = min(kps, nkb - i);
+        mbar_expect_tx(&full[s], g.block_bytes * here);
+#pragma unroll 1
+        for (int j = 0; j < here; ++j) {
+          load_a(i + j, s * kps + j);
+          load_b(i + j, s * kps + j);
+        }
+        if (++s == stages) {
+          s = 0;
+          phase ^= 1u;
+        }
       }
       if (!ok) {
         // copies already requested land within microseconds: a bounded grace period before exit
@@ -290,25 +298,34 @@ __global__ void __launch_bounds__(kThreads)
     if (elect_one()) {
       constexpr uint32_t idesc = umma_idesc_bf16(BM, BN, A_MN, B_MN);
       bool ok = true;
-      for (int i = 0; i < nkb; ++i) {
-        const int s = i % C::STAGES;
-        if (!mbar_wait(&full[s], (i / C::STAGES) & 1)) {
+      int s = 0;
+      uint32_t phase = 0;
+      for (int i = 0; i < nkb; i += kps) {
+        if (!mbar_wait(&full[s], phase)) {
           report_status(g.status, kStatusTimeoutMma);
           ok = false;
           break;
         }
         tc_fence_after();
-        const uint32_t sa = smem_u32(smem + s * C::STAGE_BYTES);
-        const uint32_t sb = sa + C::A_BYTES;
+        const int here = min(kps, nkb - i);
+#pragma unroll 1
+        for (int j = 0; j < here; ++j) {
+          const uint32_t sa = smem_u32(smem + (s * kps + j) * C::BLOCK_BYTES);
+          const uint32_t sb = sa + C::A_BYTES;
 #pragma unroll
-        for (int k = 0; k < BK / 16; ++k) {
-          const uint64_t adesc = A_MN ? umma_smem_desc(sa + k * 2048, BK * 128, 1024)
-                                      : umma_smem_desc(sa + k * 32, 16, 1024);
-          const uint64_t bdesc = B_MN ? umma_smem_desc(sb + k * 2048, BK * 128, 1024)
-                                      : umma_smem_desc(sb + k * 32, 16, 1024);
-          umma_bf16(tmem_base, adesc, bdesc, idesc, (i > 0 || k > 0) ? 1u : 0u);
+          for (int k = 0; k < BK / 16; ++k) {
+            const uint64_t adesc = A_MN ? umma_smem_desc(sa + k * 2048, BK * 128, 1024)
+                                        : umma_smem_desc(sa + k * 32, 16, 1024);
+            const uint64_t bdesc = B_MN ? umma_smem_desc(sb + k * 2048, BK * 128, 1024)
+                                        : umma_smem_desc(sb + k * 32, 16, 1024);
+            umma_bf16(tmem_base, adesc, bdesc, idesc, (i + j > 0 || k > 0) ? 1u : 0u);
+          }
         }
         umma_commit(&empty[s]);
+        if (++s == stages) {
+          s = 0;
+          phase ^= 1u;
+        }
       }
       if (ok) umma_commit(tfull);
     }
@@ -321,13 +338,16 @@ __global__ void __launch_bounds__(kThreads)
     const bool ok = mbar_wait(tfull, 0);
     if (!ok && lane == 0) report_status(g.status, kStatusTimeoutEpilogue);
     tc_fence_after();
-    if (__all_sync(0xffffffffu, ok) && m0 + q * 32 < m_ext) {
-      float* prow = reinterpret_cast<float*>(smem) + (q * 32 + lane) * C::PITCH;
+    // 64-row tiles: 16 rows in the lower half of each warp's lanes
+    constexpr int kRows = BM / 4;
+    if (__all_sync(0xffffffffu, ok) && m0 + q * kRows < m_ext) {
+      float* prow = reinterpret_cast<float*>(smem) + (q * kRows + lane) * C::PITCH;
 #pragma unroll
       for (int c = 0; c < BN / 32; ++c) {
         uint32_t r[32];
         tmem_ld_32x32b_x32(tmem_base + (uint32_t(q * 32) << 16) + c * 32, r);
         tmem_ld_wait();
+        if (lane < kRows)
 #pragma unroll
         for (int j = 0; j < 8; ++j)
           *reinterpret_cast<float4*>(prow + c * 32 + 4 * j) =
@@ -449,10 +469,44 @@ int tiles_along(const LbSmallGemm* p, int mode, int whole, int tile) {
   return n;
 }
 
+constexpr int kSmemLimit = 227 * 1024;
+struct SmallTile {
+  int bm, bn, min_blocks;
+};
+// 64-row tiles cut a long contraction of few tokens finer (what a CTA takes in bounds it), 32 columns
+// more so; 128 x 128 has the least traffic per product, for many tiles.
+constexpr SmallTile kSmallTiles[] = {{128, 128, SCfg<128, 128>::MIN_BLOCKS},
+                                     {128, 64, SCfg<128, 64>::MIN_BLOCKS},
+                                     {64, 64, SCfg<64, 64>::MIN_BLOCKS},
+                                     {64, 32, SCfg<64, 32>::MIN_BLOCKS}};
+
+// The operand ring of each of `grid` CTAs: the k-blocks in it and per stage. The CTAs that find place
+// on an SM side by side share its memory: with few CTAs one has all of it, and its loads cover the
+// latency of the weights (4 blocks of 24 KB in flight: 17.3 us for 160 x 1024 x 3072, 8: 12.9).
+// Returns how many CTAs an SM holds.
+int ring_of(int bm, int bn, int grid, int cluster, int* blocks_out, int* kps_out) {
+  const int block_bytes = (bm + bn) * BK * 2;
+  int min_blocks = 0;
+  for (const SmallTile& t : kSmallTiles)
+    if (t.bm == bm && t.bn == bn) min_blocks = t.min_blocks;
+  // (clusters do not fill every SM: one CTA per SM each, 144 CTAs in clusters of three or four took two waves)
+  int per_sm = ceil_div(grid, cluster > 1 ? small_sms() * 3 / 4 : small_sms());
+  if (per_sm > 4) per_sm = 4;
+  int blocks = (224 * 1024 / per_sm - 1024 - kRingExtra) / block_bytes;
+  if (blocks > kMaxStages) blocks = kMaxStages;
+  if (blocks < min_blocks) blocks = min_blocks;
+  // two blocks a stage halve the hand-overs between the threads that load and issue; a short ring is
+  // handed over in single blocks
+  *kps_out = blocks >= 6 ? 2 : 1;
+  *blocks_out = blocks = blocks / *kps_out * *kps_out;
+  const int fit = kSmemLimit / (blocks * block_bytes + kRingExtra + 1024);
+  return fit < per_sm ? fit : per_sm;
+}
+
 bool by_part(const LbSmallGemm* p) { return p->mode == kParallelK && p->nparts > 1; }
 
-int count_tiles(const LbSmallGemm* p, int bn, int* tiles_n) {
-  const int tm = tiles_along(p, kParallelM, p->M, BM);
+int count_tiles(const LbSmallGemm* p, int bm, int bn, int* tiles_n) {
+  const int tm = tiles_along(p, kParallelM, p->M, bm);
   const int tn = p->glu_h != nullptr ? ceil_div(p->ext[0], bn / 2)
                                      : tiles_along(p, kParallelN, p->N, bn);
   *tiles_n = tn;
@@ -485,30 +539,37 @@ bool shape_ok(const LbSmallGemm* p) {
   return true;
 }
 
-template <int A_MN, int B_MN, int BN, typename OutT, int GLU>
+template <int A_MN, int B_MN, int BM, int BN, typename OutT, int GLU>
 int launch_small(const CUtensorMap& tA, const CUtensorMap* tB, const SmallArgs& g, int grid,
                  cudaStream_t st) {
-  auto kern = gemm_small_kernel<A_MN, B_MN, BN, OutT, GLU>;
+  using C = SCfg<BM, BN>;
+  auto kern = gemm_small_kernel<A_MN, B_MN, BM, BN, OutT, GLU>;
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             SCfg<BN>::SMEM_BYTES) != cudaSuccess)
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit) !=
+        cudaSuccess)
       return -10;
     configured = true;
   }
-  return launch_pdl(kern, dim3(grid), dim3(kThreads), SCfg<BN>::SMEM_BYTES, st, pdl_enabled(),
-                    g.splits, tA, tB[0], tB[1], tB[2], g);
+  SmallArgs a = g;
+  int blocks;
+  ring_of(BM, BN, grid, g.splits, &blocks, &a.kps);
+  a.stages = blocks / a.kps;
+  return launch_pdl(kern, dim3(grid), dim3(kThreads), C::smem_bytes(blocks), st, pdl_enabled(),
+                    g.splits, tA, tB[0], tB[1], tB[2], a);
 }
 
-template <int BN>
+template <int BM, int BN>
 int dispatch(const LbSmallGemm* p, const CUtensorMap& tA, const CUtensorMap* tB, const SmallArgs& g,
              int grid, cudaStream_t st) {
   if (p->glu_h != nullptr)
-    return p->glu_kind == 0 ? launch_small<0, 0, BN, __nv_bfloat16, 1>(tA, tB, g, grid, st)
-                            : launch_small<0, 0, BN, __nv_bfloat16, 2>(tA, tB, g, grid, st);
-  if (p->a_mn) return launch_small<1, 1, BN, float, 0>(tA, tB, g, grid, st);
-  if (p->b_mn) return launch_small<0, 1, BN, __nv_bfloat16, 0>(tA, tB, g, grid, st);
-  return launch_small<0, 0, BN, __nv_bfloat16, 0>(tA, tB, g, grid, st);
+    return p->glu_kind == 0 ? launch_small<0, 0, BM, BN, __nv_bfloat16, 1>(tA, tB, g, grid, st)
+                            : launch_small<0, 0, BM, BN, __nv_bfloat16, 2>(tA, tB, g, grid, st);
+  if constexpr (BN >= 64) {
+    if (p->a_mn) return launch_small<1, 1, BM, BN, float, 0>(tA, tB, g, grid, st);
+    if (p->b_mn) return launch_small<0, 1, BM, BN, __nv_bfloat16, 0>(tA, tB, g, grid, st);
+  }
+  return launch_small<0, 0, BM, BN, __nv_bfloat16, 0>(tA, tB, g, grid, st);
 }
 
 }  // namespace
@@ -516,24 +577,23 @@ int dispatch(const LbSmallGemm* p, const CUtensorMap& tA, const CUtensorMap* tB,
 
 using namespace lb;
 
-// Microseconds, fitted to measurements of 40 products of transformer blocks (widths 768 to 4096, their
-// FFNs up to 12288, rank-16 adapters) at 1 to 20000 tokens with both tile widths and all splits: no
-// choice between this kernel and the tile kernels that it leads to is more than 3 % behind the other. W waves of two CTAs per SM pay for launch, set-up, pipeline fill and
-// the store of the tile, a split for the cluster's barriers; a k-block costs what the SM needs to
-// take it in, but no less than its share of the latency of the loads in flight in every wave.
-//   tokens x N x K                     tile kernels      this kernel (us, L2 flushed)
-//   32 x (2048, 1024, 1024) x 1024     37.8 (3 launches) 12.7
-//   32 x 1024 x 3072                   26.2              12.7
-//   660 x (768, 768, 768) x 768        39.8 (3 launches) 12.7
-//   1024 x (3072, 3072) x 1024         31.7 (2 launches) 26.3
-//   1024 x 1024 x (2048, 1024, 1024)   48.0 (3 launches) 30.2
-//   (3072, 3072) x 1024 x 1024 (grad)  35.2 (2 launches) 28.9
-// (about 5 us of each are the measurement's own).
+// Microseconds, fitted (10 % rms) to 2300 measurements of products of transformer blocks (widths 768 to
+// 2560, FFNs up to 9728) at 1 to 1400 tokens with every tile and split, weights cold; what it chooses is
+// 1.7 % slower than the best of them in the geometric mean. A launch, and per wave of resident CTAs its
+// set-up, a split's cluster barriers, and for each k-block the largest of what the SM takes in (103
+// bytes a clock), the issue of its products and the latency of the loads in flight; the store of the
+// tiles; and no less than the bytes take from memory.
+//   tokens x N x K                     before    now (us per launch of a graph, weights cold)
+//   32 x 1024 x 3072                   19.3      10.1   64 x 32 tiles, sixteen k-blocks in flight
+//   160 x 1024 x 3072                  20.0      10.4
+//   660 x 1024 x 2048                  15.2      10.5
+//   160 x (2048, 1024, 1024) x 1024    10.6       8.2
+//   160 x 1024 x (3072, 3072) (dgrad)  22.5      16.2
+//   32 x 1024 x 3072, split            9.0        7.2
 extern "C" double lb_gemm_small_plan(const LbSmallGemm* p, int* bn_out, int* splits_out) {
   if (!shape_ok(p)) return -1.0;
   const int sms = small_sms();
   const int kb = kblocks(p);
-  const int a_rows = p->M < BM && !p->a_mn ? p->M : BM;
   // Split only where the caller takes sums in another order (in a training step a different
   // rounding of one layer shows in the loss after the next update): an unsplit product has the bits
   // that the tile kernels give. Nothing is lost for the weight gradients, which are never faster
@@ -543,25 +603,37 @@ extern "C" double lb_gemm_small_plan(const LbSmallGemm* p, int* bn_out, int* spl
   int kb_part = 0;
   for (int i = 0; parts && i < p->nparts; ++i)
     kb_part = ceil_div(p->ext[i], BK) > kb_part ? ceil_div(p->ext[i], BK) : kb_part;
+  const double out_cols = p->glu_h != nullptr ? p->ext[0] : p->N;
+  const double bytes = 2.0 * p->K * (double(p->M) + p->N) + (p->out_fp32 ? 8.0 : 2.0) * p->M * out_cols;
   double best = 1e30;
-  for (int bn = 64; bn <= 128; bn += 64) {
+  for (const SmallTile& t : kSmallTiles) {
+    if (t.bn < 64 && p->b_mn) continue;   // (rows of 64 columns are the unit of those loads)
+    const int a_rows = p->M < t.bm && !p->a_mn ? p->M : t.bm;
     int tn;
-    const int tiles = count_tiles(p, bn, &tn);
-    const double stages = bn == 64 ? SCfg<64>::STAGES : SCfg<128>::STAGES;
+    const int tiles = count_tiles(p, t.bm, t.bn, &tn);
     for (int s1 = 1; s1 <= max_splits && s1 <= kb; s1 *= 2) {
       const int s = parts ? p->nparts : s1;
       const int ctas = tiles * s;
-      const double waves = ceil_div(ctas, 2 * sms);
-      const double per_sm = ctas < sms ? 1.0 : (s == 1 ? ceil_div(ctas, sms) : double(ctas) / sms);
-      const double store = (p->out_fp32 ? 1.8 : 2.6) * a_rows * bn / 8192.0;
-      const double split = (s > 1 ? 2.3 : 0.0) + (s > 2 ? 0.7 : 0.0) + (s > 4 ? 1.8 : 0.0);
-      const double block = per_sm * (a_rows + bn) * 2.0, latency = waves * 2600.0 / stages;
-      const double cost = 2.0 + waves * (1.1 + split + store) +
-                          (parts ? kb_part : ceil_div(kb, s)) *
-                              (block > latency ? block : latency) / 1900.0;
+      int blocks, kps;
+      const int res = ring_of(t.bm, t.bn, ctas, s, &blocks, &kps);
+      const int capacity = res * (sms - (s == 8 ? 20 : (s == 4 ? 8 : (s == 3 ? 7 : 0))));
+      const int waves = ceil_div(ctas, capacity);
+      int rest = ceil_div(ctas - (waves - 1) * capacity, sms);
+      if (rest > res) rest = res;
+      const double in = (a_rows + t.bn) * 128.0 / 103.0;
+      const double least = kps == 2 ? 290.0 : 600.0, flight = 2500.0 / blocks;
+      const double floor_clk = least > flight ? least : flight;
+      const double full = in * res > floor_clk ? in * res : floor_clk;
+      const double last = in * rest > floor_clk ? in * rest : floor_clk;
+      const double split = s == 1 ? 0.0 : (s <= 3 ? 1.3 : (s == 4 ? 1.7 : 2.8));
+      double cost = 3.4 + waves * (0.8 + split) +
+                    (p->out_fp32 ? 1.28 : 1.43) * a_rows * t.bn / 8192.0 * ceil_div(ctas, sms) +
+                    (parts ? kb_part : ceil_div(kb, s)) * ((waves - 1) * full + last) / 1900.0;
+      const double memory = 3.0 + bytes / 3.96e6;
+      if (cost < memory) cost = memory + 1e-3 * cost;   // (of several at that bound the least busy)
       if (cost < best) {
         best = cost;
-        *bn_out = bn;
+        *bn_out = t.bn | t.bm << 16;
         *splits_out = s;
       }
     }
@@ -572,14 +644,19 @@ extern "C" double lb_gemm_small_plan(const LbSmallGemm* p, int* bn_out, int* spl
 extern "C" int lb_gemm_small(const LbSmallGemm* p) {
   if (p->M <= 0 || p->N <= 0) return 0;
   if (!shape_ok(p)) return -3;
-  int bn = p->bn, splits = p->splits;
-  if (bn != 64 && bn != 128) bn = 0;
-  if (bn == 0 || splits <= 0) {
-    int b2 = 64, s2 = 1;
-    lb_gemm_small_plan(p, &b2, &s2);
-    if (bn == 0) bn = b2;
+  // tile: columns, and rows in the upper half (0: 128)
+  int tile = p->bn, splits = p->splits;
+  if (tile == 64 || tile == 128) tile |= 128 << 16;
+  bool known = false;
+  for (const SmallTile& t : kSmallTiles)
+    known = known || (tile == (t.bn | t.bm << 16) && !(t.bn < 64 && p->b_mn));
+  if (!known || splits <= 0) {
+    int t2 = 64, s2 = 1;
+    lb_gemm_small_plan(p, &t2, &s2);
+    if (!known) tile = t2;
     if (splits <= 0) splits = s2;
   }
+  const int bn = tile & 0xffff, BM = tile >> 16;
   const int kb = kblocks(p);
   if (by_part(p)) {
     splits = p->nparts;
@@ -634,14 +711,18 @@ extern "C" int lb_gemm_small(const LbSmallGemm* p) {
       at += ceil_div(p->ext[i], unit);
     }
   }
-  const int tiles = count_tiles(p, bn, &g.tiles_n);
+  const int tiles = count_tiles(p, BM, bn, &g.tiles_n);
   g.glu_h = p->glu_h;
   g.ld_h = p->ld_h;
   g.b_ready = p->b_ready && pdl_enabled();
   g.by_part = by_part(p);
-  g.stage_bytes = (a_box + b_box) * BK * 2;
+  g.block_bytes = (a_box + b_box) * BK * 2;
   g.status = p->status;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(p->stream);
   const int grid = tiles * splits;
-  return bn == 64 ? dispatch<64>(p, tA, tB, g, grid, st) : dispatch<128>(p, tA, tB, g, grid, st);
+  if (BM == 64)
+    return bn == 32 ? dispatch<64, 32>(p, tA, tB, g, grid, st)
+                    : dispatch<64, 64>(p, tA, tB, g, grid, st);
+  return bn == 64 ? dispatch<128, 64>(p, tA, tB, g, grid, st)
+                  : dispatch<128, 128>(p, tA, tB, g, grid, st);
 }

@@ -152,6 +152,37 @@ def test_gated_pair(T, I, keep):
     nv.check_status()
 
 
+@pytest.mark.parametrize("T", [1, 63, 65, 200])
+@pytest.mark.parametrize("N,K", [(8, 64), (72, 1096), (1024, 200)])
+def test_tiles_of_64_rows(T, N, K):
+    """64 x 64 and 64 x 32 tiles: the bits of the 128 x 64 tiles, in every form that takes them; the
+    longest contraction goes round the operand ring more than once."""
+    torch.manual_seed(T)
+    a, b, w = _rand(T, K), _rand(N, K), [_rand(64, N), _rand(K - K % 64, N)]
+    wide, bias, x = _rand(T, 64 + K - K % 64), _rand(N), _rand(T, N)
+
+    def both(run, out):
+        want = out()
+        assert run(want, 64) == 0
+        for tile in (64 | 64 << 16, 32 | 64 << 16):
+            got = out()
+            assert run(got, tile) == 0
+            assert torch.equal(got, want), tile & 0xffff
+
+    bf = lambda *s: lambda: torch.full(s, 3.0, device="cuda", dtype=torch.bfloat16)
+    both(lambda c, t: _call(a, [b], [c], T, N, K, [N], N_PARTS, bias=[bias], bn=t, splits=1), bf(T, N))
+    both(lambda c, t: _call(a, [b, b], [], T, 2 * N, K, [N, N], N_PARTS, h=c, bn=t, splits=1), bf(T, N))
+    both(lambda c, t: _call(wide, w, [c], T, N, wide.shape[1], [64, K - K % 64], K_PARTS, b_mn=1, bn=t,
+                            splits=2), bf(T, N))
+    both(lambda c, t: _call(a, [x], [c], K, N, T, [K], M_PARTS, a_mn=1, b_mn=1, fp32=1, bn=t, splits=1),
+         lambda: torch.full((K, N), 3.0, device="cuda"))
+    # a split sum: fp32 pieces, one rounding
+    c = bf(T, N)()
+    assert _call(a, [b], [c], T, N, K, [N], N_PARTS, bn=32 | 64 << 16, splits=4) == 0
+    assert _rel(c, a.double() @ b.double().t()) < ROUND
+    nv.check_status()
+
+
 def test_shapes_it_does_not_take():
     a, b, c = _rand(8, 64), _rand(16, 64), _rand(8, 16)
     assert _call(a, [b], [c], 8, 12, 64, [12], N_PARTS) == -3          # columns not a multiple of 8
