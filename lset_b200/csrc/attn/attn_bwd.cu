@@ -20,6 +20,7 @@
 // Counterpart of the flash_attn / varlen_attn backward used by the reference through autograd
 // (lset/models/decoder/qwen3/attention.py:203-234).
 #include "../common/api.h"
+#include "../common/pdl.h"
 #include "../common/ptx.cuh"
 #include "../common/row.cuh"
 #include "../common/tma_desc.h"
@@ -29,35 +30,6 @@ namespace lb {
 namespace {
 
 using bf16 = __nv_bfloat16;
-
-// ------------------------------------------------------------------------------------ delta
-template <int HD>
-__global__ void __launch_bounds__(256)
-    attn_delta_kernel(const bf16* __restrict__ dO, long long lddo, const bf16* __restrict__ O,
-                      long long ldo, float* __restrict__ delta, int T, int Hq) {
-  constexpr int LPH = HD / 8;
-  constexpr int UPB = 256 / LPH;
-  const int l = threadIdx.x % LPH;
-  const long long units = 1LL * T * Hq;
-  for (long long u0 = 1LL * blockIdx.x * UPB; u0 < units; u0 += 1LL * gridDim.x * UPB) {
-    const long long u = u0 + threadIdx.x / LPH;
-    float s = 0.f;
-    long long tok = 0;
-    int h = 0;
-    if (u < units) {
-      tok = u / Hq;
-      h = int(u % Hq);
-      float a[8], b[8];
-      unpack8(ld16(dO + tok * lddo + h * HD + l * 8), a);
-      unpack8(ld16(O + tok * ldo + h * HD + l * 8), b);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) s += a[i] * b[i];
-    }
-#pragma unroll
-    for (int o = LPH / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (u < units && l == 0) delta[1LL * h * T + tok] = s;
-  }
-}
 
 struct AttnBwdArgs {
   const int* seq_start;  // first token of each sequence
@@ -79,6 +51,42 @@ struct AttnBwdArgs {
   int capacity;      // of the plan
   unsigned* counter; // its work counter (persistent kernel; see finish_grid)
 };
+
+// ------------------------------------------------------------------------------------ delta
+template <int HD>
+__global__ void __launch_bounds__(256)
+    attn_delta_kernel(const bf16* __restrict__ dO, long long lddo, const bf16* __restrict__ O,
+                      long long ldo, float* __restrict__ delta, AttnBwdArgs a) {
+  const int T = a.T, Hq = a.Hq;
+  pdl_wait();
+  pdl_trigger();
+  // the gradient rows of tokens outside every sequence are written by no other kernel
+  clear_outside(a.plan, a.capacity, a.seq_start, a.seq_end, a.dQ, a.lddq, T, Hq * HD / 8);
+  clear_outside(a.plan, a.capacity, a.seq_start, a.seq_end, a.dK, a.lddk, T, a.Hk * HD / 8);
+  clear_outside(a.plan, a.capacity, a.seq_start, a.seq_end, a.dV, a.lddv, T, a.Hk * HD / 8);
+  constexpr int LPH = HD / 8;
+  constexpr int UPB = 256 / LPH;
+  const int l = threadIdx.x % LPH;
+  const long long units = 1LL * T * Hq;
+  for (long long u0 = 1LL * blockIdx.x * UPB; u0 < units; u0 += 1LL * gridDim.x * UPB) {
+    const long long u = u0 + threadIdx.x / LPH;
+    float s = 0.f;
+    long long tok = 0;
+    int h = 0;
+    if (u < units) {
+      tok = u / Hq;
+      h = int(u % Hq);
+      float x[8], y[8];
+      unpack8(ld16(dO + tok * lddo + h * HD + l * 8), x);
+      unpack8(ld16(O + tok * ldo + h * HD + l * 8), y);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) s += x[i] * y[i];
+    }
+#pragma unroll
+    for (int o = LPH / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (u < units && l == 0) delta[1LL * h * T + tok] = s;
+  }
+}
 
 __device__ __forceinline__ void ld_row32(uint32_t taddr, float (&s)[32]) {
   uint32_t t0[32];
@@ -215,6 +223,8 @@ __global__ void __launch_bounds__(kBwdThreads)
                    const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                    AttnBwdArgs a) {
   using C = DqCfg<HD>;
+  pdl_wait();
+  pdl_trigger();
   AttnPlanView plan{a.plan};
   if (int(blockIdx.x) >= plan.count()) return;
   const int b = plan.seq(blockIdx.x);
@@ -496,6 +506,8 @@ __global__ void __launch_bounds__(kDkvThreads, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
+  pdl_trigger();
 
   if (warp == kDkvMath / 32) {
     // -------------------------------------------------------------------- work items, loads
@@ -738,8 +750,13 @@ int launch_bwd(const void* dO, long long lddo, const void* q, long long ldq, con
     long long grid = (1LL * a.T * a.Hq + UPB - 1) / UPB;
     const long long cap = 1LL * row_num_sms() * 16;
     if (grid > cap) grid = cap;
-    attn_delta_kernel<HD><<<int(grid), 256, 0, st>>>((const bf16*)dO, lddo, (const bf16*)o, ldo,
-                                                     delta, a.T, a.Hq);
+    a.plan = plan_q;
+    a.capacity = cap_q;
+    const int rc = [&] {
+      return launch_pdl(attn_delta_kernel<HD>, dim3(int(grid)), dim3(256), 0, st, pdl_enabled(), 1,
+                        (const bf16*)dO, lddo, (const bf16*)o, ldo, delta, a);
+    }();
+    if (rc) return rc;
   }
   CUtensorMap tmQ, tmdO, tmK, tmV;
   int rc;
@@ -759,7 +776,9 @@ int launch_bwd(const void* dO, long long lddo, const void* q, long long ldq, con
       configured = true;
     }
     a.plan = plan_q;
-    kern<<<dim3(cap_q, a.Hk), kBwdThreads, C::SMEM_BYTES, st>>>(tmQ, tmdO, tmK, tmV, a);
+    rc = launch_pdl(kern, dim3(cap_q, a.Hk), dim3(kBwdThreads), C::SMEM_BYTES, st, pdl_enabled(), 1,
+                    tmQ, tmdO, tmK, tmV, a);
+    if (rc) return rc;
   }
   // dK/dV kernel: resident K / V tiles of 128 rows, Q / dO blocks of 64 tokens.
   if ((rc = make_tmap_2d(&tmQ, q, 2, (uint64_t)a.Hq * HD, a.T, (uint64_t)ldq * 2, 64, 64, true))) return rc;
@@ -781,9 +800,9 @@ int launch_bwd(const void* dO, long long lddo, const void* q, long long ldq, con
     a.counter = reinterpret_cast<unsigned*>(const_cast<int*>(plan_kv)) + 1 + 2 * cap_kv;
     const long long upper = 1LL * cap_kv * a.Hk;
     const int grid = int(upper < row_num_sms() ? upper : row_num_sms());
-    kern<<<grid, kDkvThreads, C::SMEM_BYTES, st>>>(tmQ, tmdO, tmK, tmV, a);
+    return launch_pdl(kern, dim3(grid), dim3(kDkvThreads), C::SMEM_BYTES, st, pdl_enabled(), 1, tmQ,
+                      tmdO, tmK, tmV, a);
   }
-  return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
 }  // namespace
@@ -809,10 +828,6 @@ extern "C" int lb_attn_bwd(const void* dO, long long lddo, const void* q, long l
                 T, Hq, Hk, softmax_scale, softmax_scale * kLog2eF, causal, status, 0, nullptr};
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (hd != 128 && hd != 64) return -3;
-  // gradient rows of tokens behind the last sequence are written by no kernel below
-  if (int rc = lb_attn_zero_tail(plan_q, cap_q, T, dq, lddq, Hq * hd, dk, lddk, Hk * hd, dv, lddv,
-                                 Hk * hd, stream))
-    return rc;
   if (hd == 128)
     return launch_bwd<128>(dO, lddo, q, ldq, k, ldk, v, ldv, o, ldo, delta, plan_q, cap_q, plan_kv,
                            cap_kv, a, st);

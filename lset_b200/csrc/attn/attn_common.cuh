@@ -28,15 +28,35 @@ struct AttnPlanView {
   __device__ __forceinline__ int tile(int i) const { return data[2 + 2 * i]; }
 };
 
-// Rows of the stream behind the last sequence belong to no work item: every CTA clears a share of O's
-// (`vec` = 16-byte pieces of a row).
-__device__ __forceinline__ void clear_tail(const int* plan, int capacity, __nv_bfloat16* O,
-                                           long long ldo, int T, int vec) {
-  const int end = plan[1 + 2 * capacity + 1];
-  if (end < 0) return;
-  for (int row = end + int(blockIdx.x); row < T; row += gridDim.x)
+// The plan's word on the rows of the stream that belong to no sequence: one past the last token of the
+// last one, and whether there are others in front of it (padding).
+constexpr int kPlanGaps = 1 << 30;
+
+// Clears the rows of P (`vec` 16-byte pieces each) that belong to no sequence, and so to no work item;
+// every CTA takes a share. The sequences lie in ascending order; the padding in front of one is cleared
+// with its first tile.
+__device__ __forceinline__ void clear_outside(const int* plan, int capacity, const int* seq_start,
+                                              const int* seq_end, __nv_bfloat16* P, long long ld, int T,
+                                              int vec) {
+  const int word = plan[1 + 2 * capacity + 1];
+  if (word < 0) return;
+  auto clear = [&](int row) {
     for (int v = threadIdx.x; v < vec; v += blockDim.x)
-      *reinterpret_cast<uint4*>(O + 1LL * row * ldo + v * 8) = make_uint4(0u, 0u, 0u, 0u);
+      *reinterpret_cast<uint4*>(P + 1LL * row * ld + v * 8) = make_uint4(0u, 0u, 0u, 0u);
+  };
+  for (int row = (word & ~kPlanGaps) + int(blockIdx.x); row < T; row += gridDim.x) clear(row);
+  if ((word & kPlanGaps) == 0) return;
+  const AttnPlanView view{plan};
+  const int n = view.count();
+  const int per = int(gridDim.x) > n && n > 0 ? int(gridDim.x) / n : 1;   // CTAs per tile
+  for (int w = blockIdx.x; w < n * per; w += gridDim.x) {
+    const int i = w % n;
+    if (view.tile(i) != 0) continue;
+    int lo = view.seq(i);
+    const int end = seq_start[lo];
+    while (lo > 0 && seq_end[lo - 1] <= seq_start[lo - 1]) --lo;   // (sequences without tokens have no tile)
+    for (int row = (lo > 0 ? seq_end[lo - 1] : 0) + w / n; row < end; row += per) clear(row);
+  }
 }
 
 // Called by every CTA of a persistent kernel when it takes no more work: the last one puts the plan's

@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(128)
   const int tiles = plan.count();
   const int total = tiles * a.Hk;
   if (int(blockIdx.x) >= total) {
-    clear_tail(a.plan, a.capacity, a.O, a.ldo, a.T, a.Hq * HD / 8);
+    clear_outside(a.plan, a.capacity, a.seq_start, a.seq_end, a.O, a.ldo, a.T, a.Hq * HD / 8);
     finish_grid(a.plan, a.capacity);
     return;
   }
@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(128)
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem_base, C::TMEM_COLS);
-  clear_tail(a.plan, a.capacity, a.O, a.ldo, a.T, a.Hq * HD / 8);
+  clear_outside(a.plan, a.capacity, a.seq_start, a.seq_end, a.O, a.ldo, a.T, a.Hq * HD / 8);
   finish_grid(a.plan, a.capacity);
 }
 
@@ -365,13 +365,17 @@ __global__ void __launch_bounds__(128)
 __global__ void attn_plan_kernel(const int* __restrict__ seq_start,
                                  const int* __restrict__ seq_end, int B, int tile_tokens,
                                  int* __restrict__ plan, int capacity) {
-  __shared__ int s_base;
-  if (threadIdx.x == 0) s_base = 0;
+  __shared__ int s_base, s_tokens, s_end;
+  if (threadIdx.x == 0) s_base = s_tokens = s_end = 0;
   __syncthreads();
   for (int b0 = 0; b0 < B; b0 += blockDim.x) {
     const int b = b0 + threadIdx.x;
     int nt = 0;
-    if (b < B) nt = max(0, (seq_end[b] - seq_start[b] + tile_tokens - 1) / tile_tokens);
+    if (b < B && seq_end[b] > seq_start[b]) {
+      nt = (seq_end[b] - seq_start[b] + tile_tokens - 1) / tile_tokens;
+      atomicAdd(&s_tokens, seq_end[b] - seq_start[b]);
+      atomicMax(&s_end, seq_end[b]);
+    }
     // inclusive scan over the block (simple Hillis-Steele in shared memory)
     __shared__ int scan[256];
     scan[threadIdx.x] = nt;
@@ -395,33 +399,12 @@ __global__ void attn_plan_kernel(const int* __restrict__ seq_start,
   }
   if (threadIdx.x == 0) {
     plan[0] = s_base < capacity ? s_base : capacity;
-    // spare words: the forward kernel's work counter; one past the last token that belongs to a
-    // sequence (tokens behind it, of a stream padded to a fixed budget, are no work item's: the
-    // forward kernel and the backward's launcher clear those rows); CTAs that have finished.
+    // spare words: the forward kernel's work counter; the rows that belong to no sequence (of padded
+    // batches and of streams padded to a fixed budget: no work item's, see clear_outside); CTAs
+    // that have finished.
     plan[1 + 2 * capacity] = 0;
-    plan[1 + 2 * capacity + 1] = seq_end[B - 1];
+    plan[1 + 2 * capacity + 1] = s_end | (s_tokens != s_end ? kPlanGaps : 0);
     plan[1 + 2 * capacity + 2] = 0;
-  }
-}
-
-// Rows [*end, T) of up to three [T, w] bf16 matrices := 0 (nothing to do when *end >= T).
-__global__ void __launch_bounds__(256)
-    attn_zero_tail_kernel(const int* __restrict__ end_ptr, int T, bf16* p0, long long ld0, int w0,
-                          bf16* p1, long long ld1, int w1, bf16* p2, long long ld2, int w2) {
-  const int end = *end_ptr;
-  if (end >= T || end < 0) return;
-  bf16* ps[3] = {p0, p1, p2};
-  const long long lds[3] = {ld0, ld1, ld2};
-  const int ws[3] = {w0, w1, w2};
-  for (int m = 0; m < 3; ++m) {
-    if (ps[m] == nullptr) continue;
-    const int vec = ws[m] / 8;
-    const long long total = 1LL * (T - end) * vec;
-    for (long long i = 1LL * blockIdx.x * blockDim.x + threadIdx.x; i < total;
-         i += 1LL * gridDim.x * blockDim.x) {
-      const long long r = end + i / vec, c = (i % vec) * 8;
-      *reinterpret_cast<uint4*>(ps[m] + r * lds[m] + c) = make_uint4(0u, 0u, 0u, 0u);
-    }
   }
 }
 
@@ -483,18 +466,6 @@ using namespace lb;
 
 // plan: int32 [1 + 2 * capacity + 3] (the last words are the attention kernels' own, see
 // attn_plan_kernel); capacity >= ceil(T / tile_tokens) + B always suffices.
-// Clears the rows behind the last sequence of a stream (see attn_plan_kernel). plan / capacity as
-// passed to lb_attn_plan; widths in elements, multiples of 8; unused matrices null.
-extern "C" int lb_attn_zero_tail(const int* plan, int capacity, int T, void* p0, long long ld0,
-                                 int w0, void* p1, long long ld1, int w1, void* p2, long long ld2,
-                                 int w2, void* stream) {
-  if (T <= 0) return 0;
-  if ((w0 | w1 | w2) & 7) return -3;
-  attn_zero_tail_kernel<<<64, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      plan + 1 + 2 * capacity + 1, T, (bf16*)p0, ld0, w0, (bf16*)p1, ld1, w1, (bf16*)p2, ld2, w2);
-  return cudaGetLastError() == cudaSuccess ? 0 : -11;
-}
-
 extern "C" int lb_attn_plan(const int* seq_start, const int* seq_end, int B, int tile_tokens,
                             int* plan, int capacity, void* stream) {
   if (B <= 0) return -3;

@@ -524,7 +524,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
   __syncthreads();
   tc_fence_after();
   if (warp == 9) tmem_dealloc(tmem_base, C::TMEM_COLS);
-  clear_tail(a.plan, a.capacity, a.O, a.ldo, a.T, a.Hq * HD / 8);
+  clear_outside(a.plan, a.capacity, a.seq_start, a.seq_end, a.O, a.ldo, a.T, a.Hq * HD / 8);
   finish_grid(a.plan, a.capacity);   // thread 0 belongs to warp 0; the item counter is final: the
                                      // barrier above came after the last item was drawn
 }

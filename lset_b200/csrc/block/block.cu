@@ -33,6 +33,8 @@ struct Arena {
 };
 
 __global__ void scale_bf16_kernel(__nv_bfloat16* x, long long n, float s) {
+  lb::pdl_wait();
+  lb::pdl_trigger();
   long long i = blockIdx.x * 1LL * blockDim.x + threadIdx.x;
   const long long step = 1LL * gridDim.x * blockDim.x;
   for (; i < n; i += step) x[i] = __float2bfloat16_rn(__bfloat162float(x[i]) * s);
@@ -42,8 +44,8 @@ int scale_bf16(__nv_bfloat16* x, long long n, float s, cudaStream_t st) {
   if (n <= 0) return 0;
   long long g = (n + 255) / 256;
   if (g > 1184) g = 1184;
-  scale_bf16_kernel<<<int(g), 256, 0, st>>>(x, n, s);
-  return cudaGetLastError() == cudaSuccess ? 0 : -11;
+  return lb::launch_pdl(scale_bf16_kernel, dim3(unsigned(g)), dim3(256), 0, st, lb::pdl_enabled(), 1, x,
+                        n, s);
 }
 
 struct Saved {
@@ -602,16 +604,18 @@ extern "C" int lb_block_fwd_launches(const LbBlockDesc* d, const LbStreamCtx* c,
     const LbLinear* l = linear_at(d, i);
     if (l != nullptr) n += lin_fwd_launches(*l);
   }
-  return n + (c->packed ? 0 : 1);
+  (void)c;
+  return n;
 }
 
 extern "C" int lb_block_bwd_launches(const LbBlockDesc* d, const LbStreamCtx* c,
                                      const LbTpCtx* tp) {
-  int n = 1 + 4 + 1;  // glu, attention (tail clear, delta, dq, dkv), rope
-  n += d->ln1_wgrad != nullptr ? 2 : 1;
-  n += d->ln2_wgrad != nullptr ? 2 : 1;
-  if (d->qk_norm && d->qn_wgrad != nullptr) n += d->kn_wgrad == d->qn_wgrad + d->hd ? 1 : 3;
+  (void)c;
+  int n = 1 + 3 + 1 + 2;  // glu, attention (delta, dq, dkv), rope, norms
+  const bool qk_sums = d->qk_norm && d->qn_wgrad != nullptr && d->kn_wgrad != nullptr;
   if (tp != nullptr) {
+    n += (d->ln1_wgrad != nullptr) + (d->ln2_wgrad != nullptr);
+    if (qk_sums) n += d->kn_wgrad == d->qn_wgrad + d->hd ? 1 : 3;
     n += 2 * 3 + 1 + 2 * 3;  // as in the forward, plus the copy of d_out into the publication area
     for (int i = 0; i < 7; ++i) {
       const LbLinear* l = linear_at(d, i);
@@ -619,11 +623,12 @@ extern "C" int lb_block_bwd_launches(const LbBlockDesc* d, const LbStreamCtx* c,
     }
     return n;
   }
+  n += d->ln1_wgrad != nullptr || d->ln2_wgrad != nullptr || qk_sums;   // sums of the partial rows
   for (int i = 0; i < 7; ++i) {
     const LbLinear* l = linear_at(d, i);
     if (l != nullptr) n += lin_bwd_launches(*l, (i == 1 || i == 2 || i == 5));
   }
-  return n + (c->packed ? 0 : 3);
+  return n;
 }
 
 static int block_fwd(const LbBlockDesc* d, const LbStreamCtx* c, const LbBlockIO* io) {
@@ -632,7 +637,6 @@ static int block_fwd(const LbBlockDesc* d, const LbStreamCtx* c, const LbBlockIO
   if (io->tp != nullptr) return block_fwd_tp(d, c, io);
   if (d->qkv.n < 1 || d->qkv.n > 3 || d->gate_up.n < 1 || d->gate_up.n > 2) return -3;
   if (d->qkv.width != (d->Hq + 2 * d->Hk) * d->hd || d->gate_up.width != 2 * d->I) return -3;
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(c->stream);
   Arena arena(io->saved);
   const Saved s = carve_saved(d, T, T, io->residual != nullptr, arena);
   const int H = d->H, hd = d->hd, Nq = d->Hq * hd, Nk = d->Hk * hd, W = d->qkv.width;
@@ -651,9 +655,6 @@ static int block_fwd(const LbBlockDesc* d, const LbStreamCtx* c, const LbBlockIO
                              d->qk_norm ? d->kn_w : nullptr, c->cos, c->sin, c->pos, c->pos_i64, 1,
                              s.qr, Nq, s.kr, Nk, s.q_rstd, s.k_rstd, T, d->Hq, d->Hk, hd, d->eps,
                              d->w_off, d->qk_norm, c->stream));
-  if (!c->packed) {  // rows of padding are never written by the attention kernel
-    if (cudaMemsetAsync(s.o, 0, (size_t)T * Nq * 2, st) != cudaSuccess) return -11;
-  }
   LB_TRY(lb_attn_fwd(s.qr, Nq, s.kr, Nk, s.qkv + Nq + Nk, W, c->seq_start, c->seq_end, c->plan_f,
                      c->cap_f, c->tile_f, s.o, Nq, s.lse, T, d->Hq, d->Hk, hd, d->softmax_scale,
                      d->causal, c->status, c->stream));
@@ -670,7 +671,6 @@ static int block_bwd(const LbBlockDesc* d, const LbStreamCtx* c, const LbBlockIO
   const int T = c->T;
   if (T <= 0) return 0;
   if (io->tp != nullptr) return block_bwd_tp(d, c, io);
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(c->stream);
   const bool has_res = io->residual != nullptr;
   Arena sa(io->saved);
   const Saved s = carve_saved(d, T, T, has_res, sa);
@@ -683,45 +683,45 @@ static int block_bwd(const LbBlockDesc* d, const LbStreamCtx* c, const LbBlockIO
 
   // ---- MLP
   LB_TRY(lin_dgrad(d->down, d_out, H, w.dh, T, false, w.us, c));
-  const lb::PdlScope pdl(true);  // from the second launch on, as in the forward
+  // From the second launch on, as in the forward: 2 us less from launch to launch, which is what a step of
+  // few tokens consists of (8 padded pairs on 28 layers of width 1024: 21.5 -> 19.4 ms together with
+  // padding cleared by the attention kernels and the norms' sums at the end of the call, 1915 -> 1551
+  // launches).
+  const lb::PdlScope pdl(true);
   LB_TRY(lin_wgrad(d->down, d_out, H, s.h, I, T, s.ts[6], w.us, c));
   LB_TRY(lb_glu_bwd(d->act_kind, w.dh, I, s.gu, s.gu + I, 2 * I, w.dgu, w.dgu + I, 2 * I, T, I,
                     c->stream));
   LB_TRY(proj_bwd(d->gate_up, w.dgu, s.x2, w.dx2, T, s.ts + 4, w.us, c));
   // second norm: the gradient of its input is both the attention branch's and the stream's
+  float* sums1 = c->norm_scratch + (size_t)lb_norm_bwd_partial_rows() * H;
   LB_TRY(lb_rms_norm_bwd(w.dx2, io->d_res_out, io->res_out, d->ln2_w, s.rstd2, w.dres2,
-                         c->norm_scratch, d->ln2_wgrad, 1, 1, T, H, d->w_off, c->stream));
+                         c->norm_scratch, nullptr, 1, 1, T, H, d->w_off, c->stream));
   // ---- attention
   LB_TRY(lin_dgrad(d->o_proj, w.dres2, H, w.dO, T, false, w.us, c));
   LB_TRY(lin_wgrad(d->o_proj, w.dres2, H, s.o, Nq, T, s.ts[3], w.us, c));
-  if (!c->packed) {
-    if (cudaMemsetAsync(w.dqr, 0, (size_t)T * Nq * 2, st) != cudaSuccess ||
-        cudaMemsetAsync(w.dkr, 0, (size_t)T * Nk * 2, st) != cudaSuccess ||
-        cudaMemsetAsync(w.dqkv, 0, (size_t)T * W * 2, st) != cudaSuccess)
-      return -11;
-  }
   LB_TRY(lb_attn_bwd(w.dO, Nq, s.qr, Nq, s.kr, Nk, s.qkv + Nq + Nk, W, s.o, Nq, s.lse, w.delta,
                      c->seq_start, c->seq_end, c->plan_q, c->cap_q, c->plan_kv, c->cap_kv, w.dqr, Nq,
                      w.dkr, Nk, w.dqkv + Nq + Nk, W, T, d->Hq, d->Hk, hd, d->softmax_scale,
                      d->causal, c->status, c->stream));
-  {
-    const bool want_dw = d->qk_norm && d->qn_wgrad != nullptr && d->kn_wgrad != nullptr;
-    const bool direct = want_dw && d->kn_wgrad == d->qn_wgrad + hd;
-    void* dw_out = !want_dw ? nullptr : (direct ? (void*)d->qn_wgrad : (void*)c->wg_tmp);
-    LB_TRY(lb_qk_norm_rope_bwd(w.dqr, Nq, w.dkr, Nk, s.qkv, W, s.qkv + Nq, W,
-                               d->qk_norm ? d->qn_w : nullptr, d->qk_norm ? d->kn_w : nullptr,
-                               c->cos, c->sin, c->pos, c->pos_i64, 1, s.q_rstd, s.k_rstd, w.dqkv, W,
-                               w.dqkv + Nq, W, d->qk_norm ? c->rope_scratch : nullptr, dw_out, 1,
-                               direct ? 1 : 0, T, d->Hq, d->Hk, hd, d->w_off, d->qk_norm,
-                               c->stream));
-    if (want_dw && !direct) {
-      LB_TRY(lb_colsum(c->wg_tmp, 1, hd, d->qn_wgrad, 1, 1, c->stream));
-      LB_TRY(lb_colsum(c->wg_tmp + hd, 1, hd, d->kn_wgrad, 1, 1, c->stream));
-    }
-  }
+  const bool want_dw = d->qk_norm && d->qn_wgrad != nullptr && d->kn_wgrad != nullptr;
+  LB_TRY(lb_qk_norm_rope_bwd(w.dqr, Nq, w.dkr, Nk, s.qkv, W, s.qkv + Nq, W,
+                             d->qk_norm ? d->qn_w : nullptr, d->qk_norm ? d->kn_w : nullptr, c->cos,
+                             c->sin, c->pos, c->pos_i64, 1, s.q_rstd, s.k_rstd, w.dqkv, W,
+                             w.dqkv + Nq, W, d->qk_norm ? c->rope_scratch : nullptr, nullptr, 1, 0, T,
+                             d->Hq, d->Hk, hd, d->w_off, d->qk_norm, c->stream));
   LB_TRY(proj_bwd(d->qkv, w.dqkv, s.x1, w.dx1, T, s.ts, w.us, c));
-  return lb_rms_norm_bwd(w.dx1, w.dres2, stream_in, d->ln1_w, s.rstd1, io->dx, c->norm_scratch,
-                         d->ln1_wgrad, 1, 1, T, H, d->w_off, c->stream);
+  LB_TRY(lb_rms_norm_bwd(w.dx1, w.dres2, stream_in, d->ln1_w, s.rstd1, io->dx, sums1, nullptr, 1, 1, T,
+                         H, d->w_off, c->stream));
+  // the norms' weight gradients out of their kernels' partial sums: one launch for all of them
+  LbColsum sums[kMaxColsums];
+  int n = 0;
+  const int rows = lb_norm_bwd_rows(T, H);
+  if (d->ln2_wgrad != nullptr) sums[n++] = {c->norm_scratch, rows, H, d->ln2_wgrad, nullptr, 0};
+  if (d->ln1_wgrad != nullptr) sums[n++] = {sums1, rows, H, d->ln1_wgrad, nullptr, 0};
+  if (want_dw)
+    sums[n++] = {c->rope_scratch, lb_rope_bwd_rows(T, d->Hq, d->Hk, hd), 2 * hd, d->qn_wgrad,
+                 d->kn_wgrad, hd};
+  return lb_colsums(sums, n, c->stream);
 }
 
 extern "C" int lb_block_fwd(const LbBlockDesc* d, const LbStreamCtx* c, LbBlockIO* io) {
@@ -788,25 +788,6 @@ EncWork carve_enc_work(const LbEncoderDesc* d, int T, Arena& a) {
   return w;
 }
 
-// Gradient of LN's input; weight and bias gradients straight into the accumulators where these lie
-// one behind the other.
-int enc_norm_bwd(const __nv_bfloat16* dy, const __nv_bfloat16* nr, const void* w, const float* mean,
-                 const float* rstd, __nv_bfloat16* dx, float* wgrad, float* bgrad, int T, int H,
-                 const LbStreamCtx* c, int* n) {
-  const bool want = wgrad != nullptr || bgrad != nullptr;
-  const bool direct = wgrad != nullptr && bgrad == wgrad + H;
-  float* dst = !want ? nullptr : (direct ? wgrad : c->wg_tmp);
-  LB_TRY(lb_layer_norm_bwd(dy, nullptr, nr, w, mean, rstd, dx, c->norm_scratch, dst, 1,
-                           direct ? 1 : 0, T, H, c->stream));
-  *n += want ? 2 : 1;
-  if (want && !direct) {
-    if (wgrad != nullptr) LB_TRY(lb_colsum(c->wg_tmp, 1, H, wgrad, 1, 1, c->stream));
-    if (bgrad != nullptr) LB_TRY(lb_colsum(c->wg_tmp + H, 1, H, bgrad, 1, 1, c->stream));
-    *n += (wgrad != nullptr) + (bgrad != nullptr);
-  }
-  return 0;
-}
-
 int enc_linear_bwd(const LbLinear& l, float* bgrad, const __nv_bfloat16* dy, const __nv_bfloat16* x,
                    __nv_bfloat16* dx, int T, const LbStreamCtx* c, int* n) {
   LB_TRY(lin_dgrad(l, dy, l.n_out, dx, T, false, nullptr, c));
@@ -847,11 +828,6 @@ extern "C" int lb_encoder_fwd(const LbEncoderDesc* d, const LbStreamCtx* c, LbBl
   const EncSaved s = carve_enc_saved(d, T, arena);
   const __nv_bfloat16* x = static_cast<const __nv_bfloat16*>(io->branch);
   __nv_bfloat16* no_ts[3] = {nullptr, nullptr, nullptr};
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(c->stream);
-  if (!c->packed) {  // rows of padding are never written by the attention kernel
-    if (cudaMemsetAsync(s.o, 0, (size_t)T * H * 2, st) != cudaSuccess) return -11;
-    ++io->launches;
-  }
   // ordered behind everything before it on the stream; the others as in block_fwd
   LB_TRY(proj_fwd(d->qkv, x, H, s.qkv, T, no_ts, c, d->bias));
   const lb::PdlScope pdl(true);
@@ -884,21 +860,17 @@ extern "C" int lb_encoder_bwd(const LbEncoderDesc* d, const LbStreamCtx* c, LbBl
   const __nv_bfloat16* dy = static_cast<const __nv_bfloat16*>(io->d_out);
   __nv_bfloat16* dx = static_cast<__nv_bfloat16*>(io->dx);
   __nv_bfloat16* no_ts[3] = {nullptr, nullptr, nullptr};
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(c->stream);
-  LB_TRY(enc_norm_bwd(dy, s.nr2, d->ln2_w, s.mean2, s.rstd2, w.dnr2, d->ln2_wgrad, d->ln2_bgrad, T, H,
-                      c, &n));
+  float* sums1 = c->norm_scratch + (size_t)lb_norm_bwd_partial_rows() * 2 * H;
+  LB_TRY(lb_layer_norm_bwd(dy, nullptr, s.nr2, d->ln2_w, s.mean2, s.rstd2, w.dnr2, c->norm_scratch,
+                           nullptr, 1, 1, T, H, c->stream));
   const lb::PdlScope pdl(true);
   LB_TRY(enc_linear_bwd(d->out, d->bias_grad[5], w.dnr2, s.g, w.dg, T, c, &n));
   LB_TRY(lb_gelu_bwd(w.dg, s.u, w.du, 1LL * T * d->I, c->stream));
   LB_TRY(enc_linear_bwd(d->in, d->bias_grad[4], w.du, s.y1, w.dy1, T, c, &n));
   LB_TRY(lb_add_bf16(w.dy1, w.dnr2, 1LL * T * H, c->stream));
-  LB_TRY(enc_norm_bwd(w.dy1, s.nr1, d->ln1_w, s.mean1, s.rstd1, w.dnr1, d->ln1_wgrad, d->ln1_bgrad, T,
-                      H, c, &n));
+  LB_TRY(lb_layer_norm_bwd(w.dy1, nullptr, s.nr1, d->ln1_w, s.mean1, s.rstd1, w.dnr1, sums1, nullptr, 1,
+                           1, T, H, c->stream));
   LB_TRY(enc_linear_bwd(d->o_proj, d->bias_grad[3], w.dnr1, s.o, w.dO, T, c, &n));
-  if (!c->packed) {
-    if (cudaMemsetAsync(w.dqkv, 0, (size_t)T * W * 2, st) != cudaSuccess) return -11;
-    ++n;
-  }
   LB_TRY(lb_attn_bwd(w.dO, H, s.qkv, W, s.qkv + H, W, s.qkv + 2 * H, W, s.o, H, s.lse, w.delta,
                      c->seq_start, c->seq_end, c->plan_q, c->cap_q, c->plan_kv, c->cap_kv, w.dqkv, W,
                      w.dqkv + H, W, w.dqkv + 2 * H, W, T, d->heads, d->heads, d->hd,
@@ -912,7 +884,17 @@ extern "C" int lb_encoder_bwd(const LbEncoderDesc* d, const LbStreamCtx* c, LbBl
     ++n;
   }
   LB_TRY(lb_add_bf16(dx, w.dnr1, 1LL * T * H, c->stream));
-  n += 3 + 4 + d->qkv.n;  // gelu, two additions; attention; input gradients of the projections
+  // both norms' weight and bias gradients out of their kernels' partial sums
+  LbColsum sums[2];
+  int k = 0;
+  const int rows = lb_norm_bwd_rows(T, H);
+  if (d->ln2_wgrad != nullptr || d->ln2_bgrad != nullptr)
+    sums[k++] = {c->norm_scratch, rows, 2 * H, d->ln2_wgrad, d->ln2_bgrad, H};
+  if (d->ln1_wgrad != nullptr || d->ln1_bgrad != nullptr)
+    sums[k++] = {sums1, rows, 2 * H, d->ln1_wgrad, d->ln1_bgrad, H};
+  LB_TRY(lb_colsums(sums, k, c->stream));
+  // norms; gelu, two additions; attention; input gradients of the projections
+  n += 2 + (k > 0) + 3 + 3 + d->qkv.n;
   for (int i = 0; i < d->qkv.n; ++i) n += d->qkv.part[i].wgrad != nullptr;
   io->launches = n - t_fewer;
   return 0;

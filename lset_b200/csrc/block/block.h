@@ -74,9 +74,9 @@ struct LbStreamCtx {
   int cap_kv;
   int* status;           // device status word for bounded waits
   // of a pass that records gradients, written by its backward only:
-  float* norm_scratch;   // lb_norm_bwd_partial_rows() * H floats
+  float* norm_scratch;   // 2 * lb_norm_bwd_partial_rows() * H floats (two norms)
   float* rope_scratch;   // lb_rope_bwd_partial_rows() * 2 * hd floats
-  float* wg_tmp;         // 2 * hd floats (QK-norm weight gradient staging)
+  float* wg_tmp;         // 2 * hd floats (QK-norm weight gradient staging of a token-sharded block)
   void* stream;
   int may_split;         // a pass declared inference: contractions may be summed in pieces (see LbSmallGemm)
 };
@@ -139,7 +139,7 @@ struct LbEncoderDesc {
   float* bias_grad[6];
 };
 // io: branch = x, out = y; d_out, dx and the arenas as for the decoder block. The stream context's
-// norm_scratch has room for 2 * H columns here, wg_tmp for 2 * H floats.
+// norm_scratch has room for twice 2 * H columns here; wg_tmp is not used.
 size_t lb_encoder_saved_bytes(const LbEncoderDesc* d, int T);
 size_t lb_encoder_work_bytes(const LbEncoderDesc* d, int T);
 int lb_encoder_fwd(const LbEncoderDesc* d, const LbStreamCtx* c, LbBlockIO* io);

@@ -6,6 +6,19 @@ extern "C" {
 
 int lb_colsum(const float* partial, int P, int C, void* out, int out_fp32, int accumulate,
               void* stream);
+// Column sums of `partial` [rows, cols], added to out; columns from `split` on (> 0) to out2. Null: not
+// wanted.
+struct LbColsum {
+  const float* partial;
+  int rows, cols;
+  void* out;
+  void* out2;
+  int split;
+};
+enum { kMaxColsums = 3 };
+int lb_colsums(const LbColsum* jobs, int n, void* stream);
+int lb_norm_bwd_rows(int N, int H);
+int lb_rope_bwd_rows(int T, int Hq, int Hk, int hd);
 
 // row/norm.cu
 int lb_norm_bwd_partial_rows();
@@ -51,9 +64,6 @@ int lb_bias_grad(const void* dy, long long ld, int T, int n0, int n1, int n2, fl
                  float* g2, void* stream);
 
 // attn/
-int lb_attn_zero_tail(const int* plan, int capacity, int T, void* p0, long long ld0, int w0,
-                      void* p1, long long ld1, int w1, void* p2, long long ld2, int w2,
-                      void* stream);
 int lb_attn_fwd(const void* q, long long ldq, const void* k, long long ldk, const void* v,
                 long long ldv, const int* seq_start, const int* seq_end, const int* plan,
                 int max_tiles, int tile_tokens, void* o, long long ldo, float* lse, int T, int Hq, int Hk,

@@ -31,6 +31,7 @@
 #include <cuda_bf16.h>
 #include <stdlib.h>
 
+#include "../common/pdl.h"
 #include "../common/ptx.cuh"
 #include "../common/tma_desc.h"
 
@@ -258,6 +259,8 @@ __global__ void __launch_bounds__(kThreads + (GATHER ? 32 * kPullWarps : 0), 1)
   __syncthreads();
   cluster_sync_all();   // both CTAs' barriers exist before anything arrives on them from afar
   tc_fence_after();
+  pdl_wait();
+  pdl_trigger();
   const uint32_t tmem_base = *tmem_slot;
 
   // gather: tiles are laid out rank by rank (a tile never spans two ranks' rows) and visited own
@@ -697,8 +700,9 @@ int launch2(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& t
     g_max_pairs = n;
   }
   const int pairs = (int)(total < g_max_pairs ? total : g_max_pairs);
-  cfg.gridDim = dim3(2 * pairs, 1, 1);
-  return cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmA2, tmB2, g) == cudaSuccess ? 0 : -11;
+  // (a gathering kernel is part of an exchange with other GPUs, not of such a chain)
+  return launch_pdl(kern, dim3(2 * pairs), cfg.blockDim, SMEM_BYTES, stream, !GATHER && pdl_enabled(),
+                    2, tmA, tmB, tmA2, tmB2, g);
 }
 
 int sm_count() {

@@ -22,10 +22,10 @@
 #include <cuda_bf16.h>
 #include <stdlib.h>
 
+#include "../common/pdl.h"
 #include "../common/ptx.cuh"
 #include "../common/tma_desc.h"
 #include "gemm_small.h"
-#include "../common/pdl.h"
 
 namespace lb {
 
@@ -208,6 +208,8 @@ __global__ void __launch_bounds__(gemm_threads<EPI, GATHER, F8>(), 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
+  pdl_trigger();
 
   // CTAs that compute tiles are numbered 0 .. ncta-1 (a gather launch puts its copy CTAs first)
   [[maybe_unused]] const int n_copy = GATHER ? g.copy_ctas : 0;
@@ -867,9 +869,10 @@ int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmArgs& g, in
       return -10;
     configured = true;
   }
-  kern<<<grid, gemm_threads<EPI, GATHER, F8>(), C::SMEM_BYTES, stream>>>(
-      tmA, tmB, tmA2 != nullptr ? *tmA2 : tmA, tmB2 != nullptr ? *tmB2 : tmB, g);
-  return cudaGetLastError() == cudaSuccess ? 0 : -11;
+  // (a gathering kernel is part of an exchange with other GPUs, not of such a chain)
+  return launch_pdl(kern, dim3(grid), dim3(gemm_threads<EPI, GATHER, F8>()), C::SMEM_BYTES, stream,
+                    !GATHER && pdl_enabled(), 1, tmA, tmB, tmA2 != nullptr ? *tmA2 : tmA,
+                    tmB2 != nullptr ? *tmB2 : tmB, g);
 }
 
 // Split of the contraction for a product whose output tiles alone do not fill the SMs evenly
@@ -986,9 +989,7 @@ extern "C" double lb_gemm_tile_cost(int M, int N, int K, int fp32) {
   const double cost = 3.2 + double(waves) * (((kb + s - 1) / s) * block + 2.2) + (s > 1 ? 0.6 : 0.0);
   const double memory =
       3.0 + (2.0 * K * (double(M) + N) + (fp32 ? 8.0 : 2.0) * double(M) * N) / 3.73e6;
-  // in a chain of dependent launches these kernels, which are ordinary ones, wait for the end of the one
-  // in front of them where the other's set-up and first loads run under it (1.3 to 2 us)
-  return (cost > memory ? cost : memory) + (lb::pdl_enabled() ? 1.5 : 0.0);
+  return cost > memory ? cost : memory;
 }
 
 static int gemm_bf16_impl(const void* A, const void* B, void* C, int M, int N, int K,

@@ -56,6 +56,8 @@ __global__ void __launch_bounds__(256)
     glu_bwd_kernel(const bf16* __restrict__ dout, long long ld_dout, const bf16* __restrict__ gate,
                    const bf16* __restrict__ up, long long ld_in, bf16* __restrict__ dgate,
                    bf16* __restrict__ dup, long long ld_d, long long T, int I) {
+  pdl_wait();
+  pdl_trigger();
   const int vec_per_row = I / 8;
   const long long total = T * vec_per_row;
   for (long long i = 1LL * blockIdx.x * blockDim.x + threadIdx.x; i < total;
@@ -248,16 +250,10 @@ extern "C" int lb_glu_bwd(int kind, const void* dout, long long ld_dout, const v
   if (T <= 0 || I <= 0) return 0;
   if ((I & 7) || (ld_in & 7) || (ld_dout & 7) || (ld_d & 7)) return -3;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  const int grid = flat_grid(T * (I / 8));
-  if (kind == kSwiglu)
-    glu_bwd_kernel<kSwiglu><<<grid, 256, 0, st>>>((const bf16*)dout, ld_dout, (const bf16*)gate,
-                                                  (const bf16*)up, ld_in, (bf16*)dgate, (bf16*)dup,
-                                                  ld_d, T, I);
-  else
-    glu_bwd_kernel<kGeglu><<<grid, 256, 0, st>>>((const bf16*)dout, ld_dout, (const bf16*)gate,
-                                                 (const bf16*)up, ld_in, (bf16*)dgate, (bf16*)dup,
-                                                 ld_d, T, I);
-  return launch_rc();
+  return launch_pdl(kind == kSwiglu ? glu_bwd_kernel<kSwiglu> : glu_bwd_kernel<kGeglu>,
+                    dim3(flat_grid(T * (I / 8))), dim3(256), 0, st, pdl_enabled(), 1,
+                    (const bf16*)dout, ld_dout, (const bf16*)gate, (const bf16*)up, ld_in,
+                    (bf16*)dgate, (bf16*)dup, ld_d, T, I);
 }
 
 extern "C" int lb_gelu_fwd(const void* x, void* y, long long n, void* stream) {

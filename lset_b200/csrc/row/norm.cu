@@ -10,6 +10,7 @@
 //
 // Backward runs on a persistent grid; every CTA writes one fp32 partial row of dW (and dB) to a
 // caller-provided scratch buffer, and a second small kernel sums the partials.
+#include "../common/api.h"
 #include "../common/pdl.h"
 #include "../common/row.cuh"
 
@@ -189,6 +190,8 @@ __global__ void __launch_bounds__(kRowThreads, 3)
     sw[i] = __bfloat162float(w[i]) + w_off;
   }
   __syncthreads();
+  pdl_wait();
+  pdl_trigger();
 
   for (long long row0 = 1LL * blockIdx.x * ROWS; row0 < N; row0 += 1LL * gridDim.x * ROWS) {
     const long long row = row0 + r;
@@ -359,6 +362,8 @@ __global__ void __launch_bounds__(kRowThreads)
     if (idx < H) unpack8(ld16(w + idx), wv[v]);
   }
   for (int i = threadIdx.x; i < 2 * H; i += kRowThreads) sdw[i] = 0.f;
+  pdl_wait();
+  pdl_trigger();
 
   for (long long row0 = 1LL * blockIdx.x * ROWS; row0 < N; row0 += 1LL * gridDim.x * ROWS) {
     const long long row = row0 + r;
@@ -422,14 +427,25 @@ __global__ void __launch_bounds__(kRowThreads)
 }
 
 // out[c] (+)= sum_p partial[p, c]. A CTA owns 32 columns; its 32 warps each sum a slice of the
-// partial rows (coalesced 128-byte reads), then the slices are combined in shared memory.
-__global__ void __launch_bounds__(1024)
-    colsum_kernel(const float* __restrict__ partial, int P, int C, void* out, int out_fp32,
-                  int accumulate) {
+// partial rows (coalesced 128-byte reads), then the slices are combined in shared memory. Several sums of
+// one block's backward are one launch.
+struct ColsumJobs {
+  LbColsum job[kMaxColsums];
+  int first[kMaxColsums + 1];   // CTAs
+};
+
+__global__ void __launch_bounds__(1024) colsum_kernel(ColsumJobs jobs, int out_fp32, int accumulate) {
   __shared__ float sm[32][33];
+  int j = 0;
+  while (j + 1 < kMaxColsums && int(blockIdx.x) >= jobs.first[j + 1]) ++j;
+  const LbColsum& job = jobs.job[j];
   const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
-  const int c = blockIdx.x * 32 + lane;
+  const int c = (int(blockIdx.x) - jobs.first[j]) * 32 + lane;
+  const int P = job.rows, C = job.cols;
+  const float* partial = job.partial;
   float s = 0.f;
+  pdl_wait();
+  pdl_trigger();
   if (c < C)
     for (int p = grp; p < P; p += 32) s += partial[1LL * p * C + c];
   sm[grp][lane] = s;
@@ -438,14 +454,39 @@ __global__ void __launch_bounds__(1024)
     float tot = 0.f;
 #pragma unroll
     for (int g2 = 0; g2 < 32; ++g2) tot += sm[g2][lane];
+    const bool upper = job.split > 0 && c >= job.split;
+    void* out = upper ? job.out2 : job.out;
+    const int at = upper ? c - job.split : c;
+    if (out == nullptr) return;
     if (out_fp32) {
       float* o = reinterpret_cast<float*>(out);
-      o[c] = accumulate ? o[c] + tot : tot;
+      o[at] = accumulate ? o[at] + tot : tot;
     } else {
       bf16* o = reinterpret_cast<bf16*>(out);
-      o[c] = __float2bfloat16_rn(accumulate ? __bfloat162float(o[c]) + tot : tot);
+      o[at] = __float2bfloat16_rn(accumulate ? __bfloat162float(o[at]) + tot : tot);
     }
   }
+}
+
+int launch_colsums(const LbColsum* jobs, int n, int out_fp32, int accumulate, cudaStream_t st) {
+  ColsumJobs a = {};
+  int ctas = 0, k = 0;
+  for (int i = 0; i < n; ++i) {
+    if (jobs[i].cols <= 0) continue;
+    a.job[k] = jobs[i];
+    a.first[k++] = ctas;
+    ctas += (jobs[i].cols + 31) / 32;
+  }
+  for (; k <= kMaxColsums; ++k) a.first[k] = ctas;
+  if (ctas == 0) return 0;
+  return launch_pdl(colsum_kernel, dim3(ctas), dim3(1024), 0, st, pdl_enabled(), 1, a, out_fp32,
+                    accumulate);
+}
+
+int launch_colsum(const float* partial, int P, int C, void* out, int out_fp32, int accumulate,
+                  cudaStream_t st) {
+  const LbColsum job = {partial, P, C, out, nullptr, 0};
+  return launch_colsums(&job, 1, out_fp32, accumulate, st);
 }
 
 int bwd_grid(int N, int rows_per_cta) {
@@ -514,13 +555,24 @@ extern "C" int lb_rms_norm_bwd(const void* dy, const void* dres, const void* xin
     if (2 * H * sizeof(float) > 48 * 1024)  // wide rows: opt in above the 48 KB default
       cudaFuncSetAttribute(rms_bwd_kernel<TPR, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            2 * H * (int)sizeof(float));
-    rms_bwd_kernel<TPR, NV><<<grid, kRowThreads, 2 * H * sizeof(float), st>>>(
-        (const bf16*)dy, (const bf16*)dres, (const bf16*)xin, (const bf16*)w, rstd, (bf16*)dx,
-        scratch, N, H, w_off);
+    const int rc = [&] {
+      return launch_pdl(rms_bwd_kernel<TPR, NV>, dim3(grid), dim3(kRowThreads),
+                        2 * H * sizeof(float), st, pdl_enabled(), 1, (const bf16*)dy,
+                        (const bf16*)dres, (const bf16*)xin, (const bf16*)w, rstd, (bf16*)dx,
+                        scratch, N, H, w_off);
+    }();
+    if (rc) return rc;
   });
   if (dw_out != nullptr)
-    colsum_kernel<<<(H + 31) / 32, 1024, 0, st>>>(scratch, grid, H, dw_out, dw_fp32, dw_accumulate);
+    return launch_colsum(scratch, grid, H, dw_out, dw_fp32, dw_accumulate, st);
   return launch_rc();
+}
+
+// Partial rows that the backward kernels leave in their scratch for N rows of width H.
+extern "C" int lb_norm_bwd_rows(int N, int H) {
+  if (N <= 0 || H <= 0) return 0;
+  LB_ROW_DISPATCH_NARROW(H, { return bwd_grid(N, kRowThreads / TPR); });
+  return 0;
 }
 
 extern "C" int lb_layer_norm_fwd(const void* x, const void* res_in, const void* w, const void* b,
@@ -553,22 +605,29 @@ extern "C" int lb_layer_norm_bwd(const void* dy, const void* dres, const void* x
     if (2 * H * sizeof(float) > 48 * 1024)
       cudaFuncSetAttribute(ln_bwd_kernel<TPR, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            2 * H * (int)sizeof(float));
-    ln_bwd_kernel<TPR, NV><<<grid, kRowThreads, 2 * H * sizeof(float), st>>>(
-        (const bf16*)dy, (const bf16*)dres, (const bf16*)xin, (const bf16*)w, mean, rstd, (bf16*)dx,
-        scratch, N, H);
+    const int rc = [&] {
+      return launch_pdl(ln_bwd_kernel<TPR, NV>, dim3(grid), dim3(kRowThreads),
+                        2 * H * sizeof(float), st, pdl_enabled(), 1, (const bf16*)dy,
+                        (const bf16*)dres, (const bf16*)xin, (const bf16*)w, mean, rstd, (bf16*)dx,
+                        scratch, N, H);
+    }();
+    if (rc) return rc;
   });
   if (dwb_out != nullptr)
-    colsum_kernel<<<(2 * H + 31) / 32, 1024, 0, st>>>(scratch, grid, 2 * H, dwb_out, dw_fp32,
-                                                       dw_accumulate);
+    return launch_colsum(scratch, grid, 2 * H, dwb_out, dw_fp32, dw_accumulate, st);
   return launch_rc();
 }
 
 extern "C" int lb_colsum(const float* partial, int P, int C, void* out, int out_fp32,
                          int accumulate, void* stream) {
   if (C <= 0) return 0;
-  colsum_kernel<<<(C + 31) / 32, 1024, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      partial, P, C, out, out_fp32, accumulate);
-  return launch_rc();
+  return launch_colsum(partial, P, C, out, out_fp32, accumulate, reinterpret_cast<cudaStream_t>(stream));
+}
+
+// Up to kMaxColsums sums of fp32 partial rows in one launch, added to fp32 outputs.
+extern "C" int lb_colsums(const LbColsum* jobs, int n, void* stream) {
+  if (n < 0 || n > kMaxColsums) return -3;
+  return launch_colsums(jobs, n, 1, 1, reinterpret_cast<cudaStream_t>(stream));
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -647,6 +706,6 @@ extern "C" int lb_rms_norm_bwd_noalloc(const void* dy, const void* dres, const v
         scratch, N, H, w_off);
   });
   if (dw_out != nullptr)
-    colsum_kernel<<<(H + 31) / 32, 1024, 0, st>>>(scratch, grid, H, dw_out, dw_fp32, dw_accumulate);
+    return launch_colsum(scratch, grid, H, dw_out, dw_fp32, dw_accumulate, st);
   return launch_rc();
 }

@@ -349,6 +349,16 @@ extern "C" int lb_qk_norm_rope_fwd(const void* q_in, long long ldq_in, const voi
   return -3;
 }
 
+// CTAs of the backward, each of which leaves a partial row in its scratch.
+extern "C" int lb_rope_bwd_rows(int T, int Hq, int Hk, int hd) {
+  int parts, part_heads;
+  const int tpb = kRowThreads / (hd / 8);
+  rope_parts(T, Hq + Hk, tpb, &parts, &part_heads);
+  const long long g = (1LL * T * parts + tpb - 1) / tpb;
+  const long long cap = 1LL * row_num_sms() * 4;
+  return int(g < cap ? g : cap);
+}
+
 // dw_out: [2, hd] (q weight grad then k weight grad); scratch: lb_rope_bwd_partial_rows()*2*hd floats.
 extern "C" int lb_qk_norm_rope_bwd(const void* dq, long long lddq, const void* dk, long long lddk,
                                    const void* q_in, long long ldq_in, const void* k_in,
@@ -367,13 +377,9 @@ extern "C" int lb_qk_norm_rope_bwd(const void* dq, long long lddq, const void* d
                 pos_mod > 0 ? pos_mod : 1, q_rstd, k_rstd, (bf16*)dq_in, (bf16*)dk_in, lddq_in,
                 lddk_in, scratch, T, Hq, Hk, w_off, do_norm, 1, 0};
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  int grid = 1;
+  const int grid = lb_rope_bwd_rows(T, Hq, Hk, hd);
   auto run = [&](auto kern, int lph) {
-    const int tpb = kRowThreads / lph;
-    rope_parts(T, Hq + Hk, tpb, &a.parts, &a.part_heads);
-    const long long g = (1LL * T * a.parts + tpb - 1) / tpb;
-    const long long cap = 1LL * row_num_sms() * 4;
-    grid = int(g < cap ? g : cap);
+    rope_parts(T, Hq + Hk, kRowThreads / lph, &a.parts, &a.part_heads);
     return launch_pdl(kern, dim3(grid), dim3(kRowThreads), 0, st, pdl_enabled(), 1, a);
   };
   int rc = -3;

@@ -56,7 +56,7 @@ class AttnPlan:
             return hit
         cap = (self.T + tile_tokens - 1) // tile_tokens + self.B
         # three spare words behind the entries: the work counter of the persistent kernels (forward,
-        # dK/dV), the end of the last sequence (rows behind it are cleared) and the CTAs that have
+        # dK/dV), which rows belong to no sequence (they are cleared) and the CTAs that have
         # finished: launches with one plan follow each other on a stream
         plan = torch.empty(1 + 2 * cap + 3, dtype=torch.int32, device=self.seq_start.device)
         rc = nv.load().lb_attn_plan(nv.c_void_p(self.seq_start.data_ptr()),
@@ -163,7 +163,7 @@ def _native_bwd(do, q, k, v, o, lse, plan: AttnPlan, causal, scale, dq, dk, dv):
         nv.c_int(hd), nv.c_float(scale), nv.c_int(int(causal)),
         nv.c_void_p(nv.status_word(q.device).data_ptr()), nv.c_void_p(nv.stream_ptr()))
     nv.check_rc(rc, "lb_attn_bwd")
-    nv.count_launch(4)
+    nv.count_launch(3)
 
 
 def _unit_inner(t):

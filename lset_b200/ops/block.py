@@ -458,7 +458,7 @@ def _stream_struct(ctx, plan: BlockPlan, device, training: bool) -> LbStreamCtx:
     # callers' passes, which would grow or write a shared buffer
     sums = None
     if grad:
-        norm, rope = lib.lb_norm_bwd_partial_rows() * d.H, lib.lb_rope_bwd_partial_rows() * 2 * d.hd
+        norm, rope = 2 * lib.lb_norm_bwd_partial_rows() * d.H, lib.lb_rope_bwd_partial_rows() * 2 * d.hd
         sums = torch.empty(norm + rope + 2 * d.hd, dtype=torch.float32, device=device)
         s.norm_scratch = sums.data_ptr()
         s.rope_scratch = sums.data_ptr() + 4 * norm

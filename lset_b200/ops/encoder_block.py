@@ -229,7 +229,7 @@ def _stream_struct(ctx, plan: EncoderPlan, device, training: bool) -> LbStreamCt
     # callers' passes, which would grow or write a shared buffer
     sums = None
     if grad:
-        partial = _library().lb_norm_bwd_partial_rows() * 2 * d.H
+        partial = 2 * _library().lb_norm_bwd_partial_rows() * 2 * d.H
         sums = torch.empty(partial + 2 * d.H, dtype=torch.float32, device=device)
         s.norm_scratch, s.wg_tmp = sums.data_ptr(), sums.data_ptr() + 4 * partial
     s.may_split = int(split)

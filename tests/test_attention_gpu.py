@@ -181,3 +181,36 @@ def test_short_sequences_take_the_one_tile_kernel():
     assert tile(256, 128, 16, 16, 128) == 128
     assert tile(1, 30, 16, 8, 128) == 128          # fewer sequences than SMs
     assert tile(256, 300, 4, 4, 256) == 128
+
+
+@pytest.mark.parametrize("Hq,Hk,hd", [(4, 2, 128), (3, 3, 64)])
+@pytest.mark.parametrize("one_tile", [False, True])
+@pytest.mark.parametrize("spans", [[(0, 40), (50, 96), (0, 0), (90, 96)], [(0, 0), (0, 0), (3, 96)],
+                                   [(0, 96), (0, 96)], [(0, 96), (0, 7), (0, 0), (0, 0)], [(0, 0)]])
+def test_kernels_clear_the_rows_of_no_sequence(Hq, Hk, hd, one_tile, spans, monkeypatch):
+    """Padding left, right and between, rows without a token first, last and next to each other: the
+    kernels write every row of buffers that hold garbage, zeros where there is no sequence."""
+    from lset_b200.ops.attention import _native_bwd, _native_fwd
+
+    if one_tile:
+        monkeypatch.setattr(AttnPlan, "_one_tile", lambda *a: True)
+    torch.manual_seed(0)
+    S, scale = 96, hd ** -0.5
+    mask = torch.zeros(len(spans), S, dtype=torch.long, device="cuda")
+    for row, (a, b) in zip(mask, spans):
+        row[a:b] = 1
+    T, live = mask.numel(), mask.reshape(-1) > 0
+    plan = AttnPlan.from_mask(mask)
+    q, k, v, do = (torch.randn(T, h, hd, device="cuda").to(torch.bfloat16) for h in (Hq, Hk, Hk, Hq))
+    want, _ = _native_fwd(q, k, v, plan, True, scale)      # into zeros
+    nan = lambda t, *a, **kw: torch.full_like(t, float("nan"))  # noqa: E731
+    monkeypatch.setattr(torch, "zeros", lambda *s, **kw: torch.full(s, float("nan"), **kw))
+    o, lse = _native_fwd(q, k, v, plan, True, scale)
+    monkeypatch.undo()
+    assert torch.equal(o, want) and not o[~live].any()
+    grads = [[f(t) for t in (q, k, v)] for f in (torch.zeros_like, nan)]
+    for g in grads:
+        _native_bwd(do, q, k, v, o, lse, plan, True, scale, *g)
+    nv.check_status()
+    for a, b in zip(*grads):
+        assert torch.equal(a, b) and not b[~live].any() and not b[live].isnan().any()
