@@ -241,8 +241,8 @@ class BlockPlan(Plan):
 
     @staticmethod
     def _signature(block):
-        """Changes when a projection is wrapped, replaced, moved or cast after the plan was made.
-        (Modules and parameters are looked up in their dicts: attribute access on a module costs
+        """Changes when a projection, a norm or a weight is wrapped, replaced, moved or cast after the
+        plan was made (which keeps them alive: an id stands for one object). (Modules and parameters are looked up in their dicts: attribute access on a module costs
         more than the rest of this, which runs for every block of every pass.)"""
         att, mlp = block._modules["self_attn"], block._modules["mlp"]
         am, mm = att._modules, mlp._modules
@@ -255,8 +255,12 @@ class BlockPlan(Plan):
             w = d["_parameters"].get("weight")
             if w is None:
                 w = m.weight
-            sig.append((id(m), type(m), "forward" in d, id(d.get("_sp_state")), w.dtype, w.device,
+            sig.append((id(m), type(m), id(w), "forward" in d, id(d.get("_sp_state")), w.dtype, w.device,
                         d["training"]))
+        bm = block._modules
+        for m in (bm["input_layernorm"], bm["post_attention_layernorm"], am.get("q_norm"), am.get("k_norm")):
+            if m is not None:
+                sig.append((id(m), id(m.__dict__["_parameters"].get("weight"))))
         return sig
 
     def still_valid(self, block) -> bool:

@@ -207,3 +207,23 @@ def test_models_of_different_width_with_interleaved_passes():
     for m, grads in zip(models, want):
         for n, p in m.named_parameters():
             assert (p.grad.float() - grads[n]).norm().item() <= 2e-2 * grads[n].norm().item(), n
+
+
+@pytest.mark.parametrize("name", ["mlp.down_proj", "self_attn.q_proj", "input_layernorm", "self_attn.k_norm"])
+def test_replaced_parameters_and_modules_are_seen(name):
+    """A weight or a norm put in place of another after the runner has looked at the block."""
+    import copy
+
+    model, inputs = _build("qwen3", False), _packed_inputs(lens=(9, 20, 3))
+    _run(model, inputs, True)
+    for replace in ("parameter", "module"):
+        parent, _, leaf = name.rpartition(".")
+        owner = model.layers[1].get_submodule(parent)
+        m = copy.deepcopy(getattr(owner, leaf)) if replace == "module" else getattr(owner, leaf)
+        m.weight = torch.nn.Parameter(m.weight.detach() * -1.5)
+        setattr(owner, leaf, m)
+        got = _run(model, inputs, True)
+        grad = m.weight.grad.clone()
+        assert torch.equal(got, _run(model, inputs, False)), replace
+        assert torch.allclose(grad.float(), m.weight.grad.float(), rtol=2e-2,
+                              atol=2e-2 * grad.abs().max().item()), replace
