@@ -644,11 +644,14 @@ static int block_fwd(const LbBlockDesc* d, const LbStreamCtx* c, const LbBlockIO
   const __nv_bfloat16* stream_in = io->residual != nullptr ? s.res1 : branch;
   __nv_bfloat16* out = static_cast<__nv_bfloat16*>(io->out);
 
-  // The first launch of a call is ordered behind everything before it on the stream, weight updates
+  // The first launch of a pass is ordered behind everything before it on the stream, weight updates
   // and events of other streams included; the others may start while the one in front of them runs
   // and read weights meanwhile.
-  LB_TRY(lb_rms_norm_fwd(branch, io->residual, d->ln1_w, s.x1, s.res1, s.rstd1, T, H, d->eps,
-                         d->w_off, c->stream));
+  {
+    const lb::PdlScope first(io->chained != 0);
+    LB_TRY(lb_rms_norm_fwd(branch, io->residual, d->ln1_w, s.x1, s.res1, s.rstd1, T, H, d->eps,
+                           d->w_off, c->stream));
+  }
   const lb::PdlScope pdl(true);
   LB_TRY(proj_fwd(d->qkv, s.x1, H, s.qkv, T, s.ts, c));
   LB_TRY(lb_qk_norm_rope_fwd(s.qkv, W, s.qkv + Nq, W, d->qk_norm ? d->qn_w : nullptr,
@@ -828,8 +831,10 @@ extern "C" int lb_encoder_fwd(const LbEncoderDesc* d, const LbStreamCtx* c, LbBl
   const EncSaved s = carve_enc_saved(d, T, arena);
   const __nv_bfloat16* x = static_cast<const __nv_bfloat16*>(io->branch);
   __nv_bfloat16* no_ts[3] = {nullptr, nullptr, nullptr};
-  // ordered behind everything before it on the stream; the others as in block_fwd
-  LB_TRY(proj_fwd(d->qkv, x, H, s.qkv, T, no_ts, c, d->bias));
+  {  // as in block_fwd
+    const lb::PdlScope first(io->chained != 0);
+    LB_TRY(proj_fwd(d->qkv, x, H, s.qkv, T, no_ts, c, d->bias));
+  }
   const lb::PdlScope pdl(true);
   LB_TRY(lb_attn_fwd(s.qkv, W, s.qkv + H, W, s.qkv + 2 * H, W, c->seq_start, c->seq_end, c->plan_f,
                      c->cap_f, c->tile_f, s.o, H, s.lse, T, d->heads, d->heads, d->hd,

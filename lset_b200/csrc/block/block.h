@@ -123,6 +123,8 @@ struct LbBlockIO {
   const LbTpCtx* tp;     // null: the stream is not token-sharded
   int fewer_launches;    // out: launches saved against lb_block_*_launches (several linears in one)
   int launches;          // out: launches of an encoder block's call
+  int chained;           // forward: the launch in front on the stream is the last one of another
+                         // block's call of the same pass (no weight update, no event in between)
 };
 
 // A post-LayerNorm encoder block (BERT): projections with biases, bidirectional attention, two

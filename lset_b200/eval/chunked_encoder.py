@@ -25,7 +25,7 @@ import numpy as np
 import torch
 
 from ..ops.block import inference_pass
-from ..ops.pooling import packed_pool
+from ..ops.pooling import gather_normalize, segment_mean
 from ..train.data.packing import pack_sequences
 
 DEFAULT_CHUNK_LEN = 4096
@@ -108,12 +108,25 @@ def encode_chunked(model, tokenize_fn, pool_fn, texts: Sequence[str], *, device,
 
     def run(idx: List[int]) -> torch.Tensor:
         packed = pack_sequences([chunks[i] for i in idx])
-        ids = packed["input_ids"].to(device)
-        cu = packed["cu_seqlens"].to(device)
+        ids, pos, cu = packed["input_ids"], packed["position_ids"], packed["cu_seqlens"]
+        T, n = ids.numel(), len(idx)
+        if pooling == "mean":
+            rows = torch.zeros(0, dtype=torch.int64)
+        else:
+            rows = (cu[1:] - 1 if pooling == "last_token" else cu[:-1]).long()
+        # one copy to the device: ids, positions, the pooled rows, the bounds in 32 bits
+        words = torch.empty(2 * T + rows.numel() + n // 2 + 1, dtype=torch.int64)
+        words[:T], words[T:2 * T], words[2 * T:2 * T + rows.numel()] = ids, pos, rows
+        words[2 * T + rows.numel():].view(torch.int32)[:n + 1] = cu
+        words = words.to(device)
+        ids, pos, rows, cu = (words[:T], words[T:2 * T], words[2 * T:2 * T + rows.numel()],
+                              words[2 * T + rows.numel():].view(torch.int32)[:n + 1])
         with torch.no_grad(), inference_pass():
-            hid = model(ids, position_ids=packed["position_ids"].to(device), cu_seqlens=cu,
+            hid = model(ids, position_ids=pos, cu_seqlens=cu,
                         max_seqlen=packed["max_seqlen"])["hidden_states"]
-            return packed_pool(hid, cu, pooling, False).float()
+            if pooling == "mean":
+                return segment_mean(hid, cu).float()
+            return gather_normalize(hid, rows, False).float()
 
     def run_with_retry(idx: List[int]) -> torch.Tensor:
         try:
@@ -125,19 +138,26 @@ def encode_chunked(model, tokenize_fn, pool_fn, texts: Sequence[str], *, device,
             half = len(idx) // 2
             return torch.cat([run_with_retry(idx[:half]), run_with_retry(idx[half:])])
 
-    acc = None
-    weight = torch.zeros(N, dtype=torch.float32, device=device)
-    owners_t = torch.tensor(owners, device=device)
-    lens_t = torch.tensor(lens, dtype=torch.float32, device=device)
-    for stream in plan_streams(lens, token_budget):
-        emb = run_with_retry(stream)
-        if acc is None:
-            acc = torch.zeros(N, emb.shape[1], dtype=torch.float32, device=device)
-        sel = torch.tensor(stream, device=device)
-        w = lens_t[sel]
-        acc.index_add_(0, owners_t[sel], emb * w[:, None])
-        weight.index_add_(0, owners_t[sel], w)
-    out = acc / weight.clamp(min=1.0)[:, None]
+    streams = plan_streams(lens, token_budget)
+    order = None
+    if len(chunks) == N:     # no document was split: the rows only have to be put in order, on the host
+        embs = [run_with_retry(stream) for stream in streams]
+        out = embs[0] if len(embs) == 1 else torch.cat(embs)
+        order = [i for stream in streams for i in stream]
+    else:
+        acc = None
+        weight = torch.zeros(N, dtype=torch.float32, device=device)
+        owners_t = torch.tensor(owners, device=device)
+        lens_t = torch.tensor(lens, dtype=torch.float32, device=device)
+        for stream in streams:
+            emb = run_with_retry(stream)
+            if acc is None:
+                acc = torch.zeros(N, emb.shape[1], dtype=torch.float32, device=device)
+            sel = torch.tensor(stream, device=device)
+            w = lens_t[sel]
+            acc.index_add_(0, owners_t[sel], emb * w[:, None])
+            weight.index_add_(0, owners_t[sel], w)
+        out = acc / weight.clamp(min=1.0)[:, None]
     if post_pooling is not None:   # dense projection between pooling and normalisation
         with torch.no_grad():
             w_dtype = next(iter(post_pooling.buffers())).dtype
@@ -145,6 +165,9 @@ def encode_chunked(model, tokenize_fn, pool_fn, texts: Sequence[str], *, device,
     if normalize:
         out = torch.nn.functional.normalize(out, dim=-1, eps=1e-12)
     result = out.cpu().numpy().astype(np.float32)
+    if order is not None:
+        rows, result = result, np.empty_like(result)
+        result[order] = rows
     if out_path and N >= CPU_STREAM_THRESHOLD:
         mm = np.lib.format.open_memmap(out_path, mode="w+", dtype=np.float32, shape=result.shape)
         mm[:] = result

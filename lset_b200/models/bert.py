@@ -117,7 +117,8 @@ class BertEncoder(nn.Module):
         ctx = make_stream_ctx(input_ids, attention_mask, position_ids, cu_seqlens, max_seqlen)
         types = token_type_ids.reshape(-1) if token_type_ids is not None else None
         x = self.embeddings(input_ids.reshape(-1), ctx.pos, types)
-        for layer in self.layers:
+        done, x = block_ops.run_inference(BertBlock, self.layers, x, ctx)
+        for layer in list(self.layers)[done:]:
             x = layer(x, ctx)
         if ctx.padded_shape is not None:
             x = x.view(*ctx.padded_shape, x.shape[-1])

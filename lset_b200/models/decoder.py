@@ -137,8 +137,10 @@ class DecoderModel(nn.Module):
 
             T = branch.shape[0]
             branch = tp_fused.shard_tokens(branch, sp)  # blocks see this rank's tokens only
-        prev_post = None
-        for layer in self.layers:
+        prev_post, done = None, 0
+        if sp is None and not self.traits.sandwich_norms:
+            done, branch, residual = block_ops.run_inference(DecoderBlock, self.layers, branch, ctx)
+        for layer in list(self.layers)[done:]:
             branch, residual = layer(branch, residual, ctx, prev_post)
             prev_post = layer.post_feedforward_layernorm if self.traits.sandwich_norms else None
         n = self.norm

@@ -27,6 +27,8 @@ import threading
 
 import torch
 
+from torch.nn.modules.module import _has_any_global_hook
+
 from . import _ac
 from . import _native as nv
 from ._grads import main_grad_of
@@ -79,7 +81,8 @@ class LbTpCtx(ctypes.Structure):
 class LbBlockIO(ctypes.Structure):
     _fields_ = [("branch", _vp), ("residual", _vp), ("out", _vp), ("res_out", _vp),
                 ("saved", _vp), ("d_out", _vp), ("d_res_out", _vp), ("dx", _vp), ("work", _vp),
-                ("tp", _vp), ("fewer_launches", ctypes.c_int), ("launches", ctypes.c_int)]
+                ("tp", _vp), ("fewer_launches", ctypes.c_int), ("launches", ctypes.c_int),
+                ("chained", ctypes.c_int)]
 
 
 _lib = None
@@ -576,3 +579,145 @@ def run(block, branch, residual, ctx):
     plan = block.__dict__["_lb_plan"]
     sctx = _stream_struct(ctx, plan, branch.device, block.training)
     return _BlockFn.apply(branch, residual, plan, sctx, ctx, *node_inputs(plan.params))
+
+
+# --------------------------------------------------------------------------- passes without derivatives
+def records_nothing() -> bool:
+    """Whether this pass is for its results alone, as torch sees it: no derivatives of any kind, no
+    transform, no trace to which a call behind torch's back would be missing."""
+    return (not torch.is_grad_enabled() and torch.autograd.forward_ad._current_level < 0
+            and torch._C._functorch.peek_interpreter_stack() is None
+            and not torch.jit.is_tracing() and not torch.compiler.is_compiling())
+
+
+def unhooked(d: dict) -> bool:
+    """``d``: the ``__dict__`` of a module. Whether calling it runs its class's forward alone."""
+    return not ("forward" in d or d["_forward_hooks"] or d["_forward_pre_hooks"]
+                or d["_backward_hooks"] or d["_backward_pre_hooks"])
+
+
+class Watch:
+    """Tensors (parameters by module and name) as a descriptor was filled from them; ``same`` looks at
+    each of them: at a parameter that was replaced, and at data exchanged under one."""
+
+    def __init__(self, params):
+        self.items = []
+        for owner, name in params:
+            t = owner._parameters[name]
+            self.items.append((owner._parameters, name, t, t.data_ptr(), t.dtype, t.shape, t.stride()))
+
+    def same(self) -> bool:
+        for where, name, t, ptr, dtype, shape, stride in self.items:
+            if (where.get(name) is not t or t.data_ptr() != ptr or t.dtype != dtype
+                    or t.shape != shape or t.stride() != stride):
+                return False
+        return True
+
+
+class _Inference(Plan):
+    """What a pass without derivatives keeps of one block: the descriptor, filled in, and what to look
+    at before it is used again. Never changed once made: another thread may be in a pass with it."""
+
+    def __init__(self, block, plan):
+        att, mlp = block.self_attn, block.mlp
+        qkv = [(att, n) for n in (("qkv_proj",) if att.fused_qkv else ("q_proj", "k_proj", "v_proj"))]
+        gu = [(mlp, n) for n in (("gate_up_proj",) if mlp.fused_gate_up else ("gate_proj", "up_proj"))]
+        names = qkv + [(att, "o_proj")] + gu + [(mlp, "down_proj")]
+        self.modules = [(owner._modules, n, owner._modules[n], owner._modules[n].__dict__)
+                        for owner, n in names]
+        self.ok = plan.sp is None and all(_plain_linear(m) for _, _, m, _ in self.modules)
+        if not self.ok:
+            return
+        norms = [block.input_layernorm, block.post_attention_layernorm]
+        if plan.qn is not None:
+            norms += [att.q_norm, att.k_norm]
+        self.halves = (att, mlp, *norms[:2], att._modules.get("q_norm"), att._modules.get("k_norm"))
+        self.plan = plan
+        self.watch = Watch([(m, "weight") for m in norms] + [(m, "weight") for _, _, m, _ in self.modules])
+        self.desc = plan.fill({})
+        self.addr = ctypes.addressof(self.desc)
+
+    def same(self, block) -> bool:
+        mods = block._modules
+        att, mlp = mods["self_attn"], mods["mlp"]
+        am = att._modules
+        if (att, mlp, mods["input_layernorm"], mods["post_attention_layernorm"]) != self.halves[:4]:
+            return False
+        if (am.get("q_norm"), am.get("k_norm")) != self.halves[4:]:
+            return False
+        for where, name, m, d in self.modules:
+            if where[name] is not m or "forward" in d or "_tp_kind" in d or d["_parameters"]["bias"] is not None:
+                return False
+        return self.watch.same()
+
+
+def _inference_of(block):
+    kept = block.__dict__.get("_lb_inference")
+    if kept is not None and kept.ok and kept.same(block):
+        return kept
+    plan = plan_of(block)
+    if plan is None:
+        return None
+    kept = _Inference(block, plan)
+    block.__dict__["_lb_inference"] = kept
+    return kept if kept.ok else None
+
+
+def run_inference(block_type, layers, branch, ctx):
+    """The blocks of a pass without derivatives, one after the other, with one activation arena and one
+    pair of stream buffers for all of them and no autograd node each. Takes the blocks from the first on
+    that are plain ones; returns ``(how many, branch, residual)``."""
+    if not (records_nothing() and branch.is_cuda and branch.dtype == torch.bfloat16
+            and branch.dim() == 2 and branch.is_contiguous() and branch.shape[0] > 0
+            and ctx.pos.shape[0] == branch.shape[0]):
+        return 0, branch, None
+    if _ac._active is not None or _rt.attention_backend == "sdpa" or _has_any_global_hook():
+        return 0, branch, None
+    for name in ("block_runner", "fused_rmsnorm", "fused_residual_rmsnorm", "fused_qk_norm_rope"):
+        if not enabled(name):
+            return 0, branch, None
+    lib = _library()
+    dev = branch.device
+    T, H = branch.shape
+    io, sctx, key, sizes, out, residual, n, launches = LbBlockIO(), None, None, None, None, None, 0, 0
+    io_at = ctypes.addressof(io)
+    x = branch
+    for block in layers:
+        d = block.__dict__
+        if type(block) is not block_type or not unhooked(d) or not _own_forwards(block):
+            break
+        kept = _inference_of(block)
+        if kept is None or kept.desc.H != H:
+            break
+        plan = kept.plan
+        k = (plan.desc.hd, plan.desc.Hq // plan.desc.Hk, plan.rope[1], id(plan.rope[2]), d["training"])
+        if k != key:
+            key = k
+            sctx = _stream_struct(ctx, plan, dev, d["training"])
+            sctx.stream = nv.stream_ptr()
+            sctx_at = ctypes.addressof(sctx)
+        size = (kept.desc.Hq, kept.desc.Hk, kept.desc.hd, kept.desc.I)
+        if size != sizes:
+            sizes = size
+            arena = torch.empty(_arena_size(lib.lb_block_saved_bytes(kept.addr, T, 1, None)),
+                                dtype=torch.uint8, device=dev)
+            io.saved = arena.data_ptr()
+            per_block = lib.lb_block_fwd_launches(kept.addr, sctx_at, 1, None)
+        if out is None:
+            out, res = torch.empty_like(branch), torch.empty_like(branch)
+            io.out, io.res_out = out.data_ptr(), res.data_ptr()
+        # (a block has read its inputs before it writes its outputs: from the second one on they are
+        # the same buffers)
+        io.branch = x.data_ptr()
+        io.residual = residual.data_ptr() if residual is not None else None
+        io.chained = int(n > 0)
+        rc = lib.lb_block_fwd(kept.addr, sctx_at, io_at)
+        if rc != 0:
+            nv.check_rc(rc, "lb_block_fwd")
+        launches += per_block - io.fewer_launches
+        x, residual = out, res
+        n += 1
+    if n:
+        nv.count_launch(launches)
+        calls["dp"] += n
+    return n, x, residual

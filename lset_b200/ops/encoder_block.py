@@ -25,8 +25,8 @@ from torch.nn.modules.module import _has_any_global_hook
 from . import _ac
 from . import _native as nv
 from ._grads import main_grad_of
-from .block import (LbBlockIO, LbLinear, LbProjection, LbStreamCtx, Plan, _arena_size, _fp, _vp,
-                    _work_arena, may_split, node_inputs)
+from .block import (LbBlockIO, LbLinear, LbProjection, LbStreamCtx, Plan, Watch, _arena_size, _fp, _vp,
+                    _work_arena, may_split, node_inputs, records_nothing, unhooked)
 from .runtime_options import enabled, options as _rt
 
 
@@ -299,3 +299,91 @@ def run(block, x, ctx):
     plan = block.__dict__["_lb_plan"]     # ``usable`` has just accepted it
     sctx = _stream_struct(ctx, plan, x.device, block.training)
     return _EncoderBlockFn.apply(x, plan, sctx, ctx, *node_inputs(plan.params))
+
+
+class _Inference(Plan):
+    """What a pass without derivatives keeps of one block (see ``ops.block._Inference``)."""
+
+    def __init__(self, block, plan):
+        qkv, o, fin, fout, ln1, ln2 = _modules(block)
+        att, mlp = block.attention, block.mlp
+        names = ("qkv_proj",) if att.fused_qkv else ("query", "key", "value")
+        names = [(att, n) for n in names + ("dense", "LayerNorm")] + [
+            (mlp, n) for n in ("dense_in", "dense_out", "LayerNorm")]
+        self.modules = [(owner._modules, n, owner._modules[n], owner._modules[n].__dict__)
+                        for owner, n in names]
+        self.halves, self.eps, self.norms = (att, mlp), ln1.eps, (ln1.__dict__, ln2.__dict__)
+        self.plan = plan
+        self.watch = Watch([(m, p) for _, _, m, _ in self.modules for p in ("weight", "bias")])
+        self.desc = plan.fill({})
+        self.addr = ctypes.addressof(self.desc)
+
+    def same(self, block) -> bool:
+        mods = block._modules
+        if mods["attention"] is not self.halves[0] or mods["mlp"] is not self.halves[1]:
+            return False
+        for where, name, m, d in self.modules:
+            if where[name] is not m or not unhooked(d) or "_tp_kind" in d:
+                return False
+        return (self.norms[0]["eps"] == self.eps and self.norms[1]["eps"] == self.eps
+                and self.watch.same())
+
+
+def _inference_of(block):
+    kept = block.__dict__.get("_lb_inference")
+    if kept is not None and kept.same(block):
+        return kept
+    plan = plan_of(block)
+    if plan is None:
+        return None
+    kept = block.__dict__["_lb_inference"] = _Inference(block, plan)
+    return kept
+
+
+def run_inference(block_type, layers, x, ctx):
+    """The blocks of a pass without derivatives (see ``ops.block.run_inference``); returns ``(how many,
+    x)``."""
+    if not (records_nothing() and x.is_cuda and x.dtype == torch.bfloat16 and x.dim() == 2
+            and x.is_contiguous() and x.shape[0] > 0 and ctx.pos.shape[0] == x.shape[0]):
+        return 0, x
+    if (_ac._active is not None or _rt.attention_backend == "sdpa" or _has_any_global_hook()
+            or not enabled("block_runner") or not enabled("fused_layernorm")):
+        return 0, x
+    global calls
+    lib = _library()
+    T, H = x.shape
+    io, key, size, outs, n, launches = LbBlockIO(), None, None, None, 0, 0
+    io_at = ctypes.addressof(io)
+    for block in layers:
+        d = block.__dict__
+        if type(block) is not block_type or not unhooked(d) or not _own_forwards(block):
+            break
+        kept = _inference_of(block)
+        if kept is None or kept.desc.H != H:
+            break
+        k = (kept.desc.hd, d["training"])
+        if k != key:
+            key = k
+            sctx = _stream_struct(ctx, kept.plan, x.device, d["training"])
+            sctx.stream = nv.stream_ptr()
+            sctx_at = ctypes.addressof(sctx)
+        if kept.desc.I != size:
+            size = kept.desc.I
+            arena = torch.empty(_arena_size(lib.lb_encoder_saved_bytes(kept.addr, T)),
+                                dtype=torch.uint8, device=x.device)
+            io.saved = arena.data_ptr()
+        if outs is None:
+            outs = torch.empty_like(x), torch.empty_like(x)
+        out = outs[n & 1]
+        io.branch, io.out = x.data_ptr(), out.data_ptr()
+        io.chained = int(n > 0)
+        rc = lib.lb_encoder_fwd(kept.addr, sctx_at, io_at)
+        if rc != 0:
+            nv.check_rc(rc, "lb_encoder_fwd")
+        launches += io.launches
+        x = out
+        n += 1
+    if n:
+        nv.count_launch(launches)
+        calls += n
+    return n, x

@@ -227,3 +227,58 @@ def test_replaced_parameters_and_modules_are_seen(name):
         assert torch.equal(got, _run(model, inputs, False)), replace
         assert torch.allclose(grad.float(), m.weight.grad.float(), rtol=2e-2,
                               atol=2e-2 * grad.abs().max().item()), replace
+
+
+@pytest.mark.parametrize("family", ["decoder", "encoder"])
+def test_passes_without_gradients_see_what_changed_since_the_last(family):
+    """They keep the blocks' descriptors from pass to pass: a parameter replaced, data exchanged under
+    one, another layout of the same storage, a block replaced, a hook set, all show in the next pass."""
+    import copy
+
+    if family == "decoder":
+        model = _build("qwen3", False).eval()
+        name, square = "mlp.down_proj", "mlp.up_proj"
+    else:
+        from lset_b200.models import BertConfig
+        from lset_b200.models.bert import BertEncoder
+
+        torch.manual_seed(2)
+        model = BertEncoder(BertConfig(vocab_size=1024, hidden_size=256, intermediate_size=256,
+                                       num_hidden_layers=2, num_attention_heads=4)).eval()
+        for p in model.parameters():
+            if p.dim() > 1:
+                torch.nn.init.normal_(p, std=0.05)
+        model, name, square = model.cuda().to(torch.bfloat16), "mlp.dense_out", "mlp.dense_in"
+    inputs = _packed_inputs(lens=(9, 20, 3))
+    seen = []
+
+    def passes():
+        with torch.no_grad():
+            got = model(**inputs)["hidden_states"].clone()
+        want = model(**inputs)["hidden_states"].detach()
+        nv.check_status()
+        assert torch.equal(got, want)
+        return got
+
+    m, sq = model.layers[1].get_submodule(name), model.layers[0].get_submodule(square)
+    m.weight.requires_grad_(False)
+    sq.weight.requires_grad_(False)
+
+    def mirrored():
+        w = sq.weight.data
+        sq.weight.data = w[:256, :256].t().contiguous().t() if w.shape[0] == w.shape[1] else w * 1.5
+
+    changes = [lambda: m.weight.mul_(2),
+               lambda: setattr(m, "weight", torch.nn.Parameter(m.weight.data * -1)),
+               lambda: setattr(m.weight, "data", m.weight.data * 0.5), mirrored,
+               lambda: setattr(model.layers[0], "mlp", copy.deepcopy(model.layers[1].mlp)),
+               lambda: model.layers.__setitem__(0, copy.deepcopy(model.layers[1])),
+               lambda: model.layers[1].register_forward_hook(lambda *a: seen.append(1))]
+    last = [passes()]
+    for i, change in enumerate(changes):
+        change()
+        now = passes()
+        if i not in (3, len(changes) - 1):
+            assert not torch.equal(now, last[0]), i
+        last[0] = now
+    assert len(seen) == 2
