@@ -45,22 +45,25 @@ __device__ __forceinline__ int token_pos(const RopeArgs& a, long long tok) {
                    : reinterpret_cast<const int*>(a.pos)[tok];
 }
 
-// A group of HD/8 lanes owns one token at a time (or, with few tokens, a part of its heads, see
+// A group of HD/16 lanes owns one token at a time (or, with few tokens, a part of its heads, see
 // rope_parts) and walks over its heads UB at a time: the cos/sin
 // row and the position are fetched once per token, and the 16-byte loads of the next UB heads are
-// already in flight while the current UB heads are normalised, rotated and stored (the kernel is
-// bound by memory latency otherwise).
+// already in flight while the current UB heads are normalised, rotated and stored. A lane holds eight
+// elements of either half of a head, the two partners of eight rotations, so that nothing but the sum of
+// squares crosses lanes. (With a lane per eight neighbouring elements, every element came over once by
+// shuffle, and the shuffles bound the kernel; the sum of squares is added up in the same order.)
+// Measured (us, tokens x heads of 128, L2 flushed): 22627 x 24 72 -> 64, 40280 x 24 117 -> 94, 33280 x 40
+// 156 -> 132 (65 % -> 81 % of copy bandwidth at 40280); 22627 x 40 heads of 64 59 -> 51.
 template <int HD>
 __global__ void __launch_bounds__(kRowThreads, 3) qk_rope_fwd_kernel(RopeArgs a) {
-  constexpr int LPH = HD / 8;  // lanes per head
+  constexpr int LPH = HD / 16;  // lanes per head
   constexpr int TPB = kRowThreads / LPH;
-  constexpr int UB = 4;
+  constexpr int UB = 2;
+  constexpr int HALF = HD / 2;
   __shared__ float swt[2 * HD];  // q then k norm weights (+ offset)
   const int l = threadIdx.x % LPH;
   const int g = threadIdx.x / LPH;
   const int e0 = l * 8;
-  const int c0 = e0 % (HD / 2);
-  const bool first_half = l < LPH / 2;
   for (int i = threadIdx.x; i < 2 * HD; i += kRowThreads)
     swt[i] = a.do_norm ? __bfloat162float(i < HD ? a.qw[i] : a.kw[i - HD]) + a.w_off : 1.f;
   __syncthreads();
@@ -77,31 +80,31 @@ __global__ void __launch_bounds__(kRowThreads, 3) qk_rope_fwd_kernel(RopeArgs a)
     const bf16* krow = a.k_in + tok * a.ldk_in + e0;
     bf16* qdst = a.q_out + tok * a.ldq_out + e0;
     bf16* kdst = a.k_out + tok * a.ldk_out + e0;
-    auto load_batch = [&](int h0, uint4 (&raw)[UB]) {
+    auto load_batch = [&](int h0, uint4 (&raw)[UB][2]) {
 #pragma unroll
       for (int j = 0; j < UB; ++j) {
         const int h = h0 + j;
-        raw[j] = make_uint4(0u, 0u, 0u, 0u);
-        if (valid && h < heads) raw[j] = ld16(h < a.Hq ? qrow + h * HD : krow + (h - a.Hq) * HD);
+        raw[j][0] = raw[j][1] = make_uint4(0u, 0u, 0u, 0u);
+        if (valid && h < heads) {
+          const bf16* p = h < a.Hq ? qrow + h * HD : krow + (h - a.Hq) * HD;
+          raw[j][0] = ld16(p);
+          raw[j][1] = ld16(p + HALF);
+        }
       }
     };
-    uint4 cur[UB], nxt[UB];
+    uint4 cur[UB][2], nxt[UB][2];
     load_batch(h_first, cur);
     float c[8], s[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) c[i] = s[i] = 0.f;
     if (valid) {
       const int pos = token_pos(a, tok);
-      const float4* cp = reinterpret_cast<const float4*>(a.cos + 1LL * pos * (HD / 2) + c0);
-      const float4* sp = reinterpret_cast<const float4*>(a.sin + 1LL * pos * (HD / 2) + c0);
+      const float4* cp = reinterpret_cast<const float4*>(a.cos + 1LL * pos * HALF + e0);
+      const float4* sp = reinterpret_cast<const float4*>(a.sin + 1LL * pos * HALF + e0);
       *reinterpret_cast<float4*>(c) = cp[0];
       *reinterpret_cast<float4*>(c + 4) = cp[1];
       *reinterpret_cast<float4*>(s) = sp[0];
       *reinterpret_cast<float4*>(s + 4) = sp[1];
-    }
-    if (!first_half) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) s[i] = -s[i];  // y = x*c - partner*s (first half), + (second)
     }
     for (int b0 = 0; b0 < a.part_heads; b0 += UB) {   // uniform over the CTA
       const int h0 = h_first + b0;
@@ -111,36 +114,50 @@ __global__ void __launch_bounds__(kRowThreads, 3) qk_rope_fwd_kernel(RopeArgs a)
         const int h = h0 + j;
         const bool live = valid && h < heads;
         const bool is_q = h < a.Hq;
-        float x[8];
-        unpack8(cur[j], x);
+        float x[2][8];
+        unpack8(cur[j][0], x[0]);
+        unpack8(cur[j][1], x[1]);
         if (a.do_norm) {
-          float ss = 0.f;
+          float ss[2] = {0.f, 0.f};
 #pragma unroll
-          for (int i = 0; i < 8; ++i) ss += x[i] * x[i];
+          for (int k = 0; k < 2; ++k)
 #pragma unroll
-          for (int o = LPH / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-          const float rstd = rsqrtf(ss / float(HD) + a.eps);
+            for (int i = 0; i < 8; ++i) ss[k] += x[k][i] * x[k][i];
+          float sum = ss[0] + ss[1];
+#pragma unroll
+          for (int o = LPH / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+          const float rstd = rsqrtf(sum / float(HD) + a.eps);
           if (live && l == 0) {
             if (is_q) a.q_rstd[tok * a.Hq + h] = rstd;
             else a.k_rstd[tok * a.Hk + (h - a.Hq)] = rstd;
           }
-          const float* wt = swt + (is_q ? 0 : HD) + e0;
-          const float4 w0 = *reinterpret_cast<const float4*>(wt);
-          const float4 w1 = *reinterpret_cast<const float4*>(wt + 4);
-          const float wl[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
 #pragma unroll
-          for (int i = 0; i < 8; ++i) x[i] = bf16_round(x[i] * rstd) * wl[i];
+          for (int k = 0; k < 2; ++k) {
+            const float* wt = swt + (is_q ? 0 : HD) + k * HALF + e0;
+            const float4 w0 = *reinterpret_cast<const float4*>(wt);
+            const float4 w1 = *reinterpret_cast<const float4*>(wt + 4);
+            const float wl[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+            for (int i = 0; i < 8; ++i) x[k][i] = bf16_round(x[k][i] * rstd) * wl[i];
+          }
         }
-        float y[8];
+        float y[2][8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          const float p = __shfl_xor_sync(0xffffffffu, x[i], LPH / 2);
-          y[i] = x[i] * c[i] - p * s[i];
+          y[0][i] = x[0][i] * c[i] - x[1][i] * s[i];
+          y[1][i] = x[1][i] * c[i] - x[0][i] * -s[i];
         }
-        if (live) st16(is_q ? qdst + h * HD : kdst + (h - a.Hq) * HD, pack8(y));
+        if (live) {
+          bf16* p = is_q ? qdst + h * HD : kdst + (h - a.Hq) * HD;
+          st16(p, pack8(y[0]));
+          st16(p + HALF, pack8(y[1]));
+        }
       }
 #pragma unroll
-      for (int j = 0; j < UB; ++j) cur[j] = nxt[j];
+      for (int j = 0; j < UB; ++j) {
+        cur[j][0] = nxt[j][0];
+        cur[j][1] = nxt[j][1];
+      }
     }
   }
 }
@@ -171,23 +188,30 @@ struct RopeBwdArgs {
   int parts, part_heads;
 };
 
-// Same token-per-lane-group walk as the forward kernel, UB heads at a time: the gradient rows, the
-// forward inputs and the saved rstd of UB heads are requested before any of them is used.
-template <int HD>
+// Same token-per-lane-group walk as the forward kernel, UB heads at a time: the gradient rows, the forward
+// inputs and the saved rstd of UB heads are requested before any of them is used. With few tokens a lane
+// holds eight elements of either half of a head, as in the forward (HALVES 2): half the lanes a head, so
+// half the CTAs, one wave of them. With many tokens registers bound the loads in flight, and eight
+// neighbouring elements a lane, the partner's by shuffle (HALVES 1), are as fast or faster.
+// Measured (us, tokens x 24 heads of 128, HALVES 1 / 2): 920 18.4 / 10.7, 2500 23 / 15, 6000 49 / 35,
+// 22627 106 / 108, 40280 174 / 172; 22627 x 40 heads of 64 106 / 119.
+template <int HD, int HALVES>
 __global__ void __launch_bounds__(kRowThreads, 2) qk_rope_bwd_kernel(RopeBwdArgs a) {
-  constexpr int LPH = HD / 8;
+  constexpr int LPH = HD / 8 / HALVES;
   constexpr int TPB = kRowThreads / LPH;
-  constexpr int UB = 4;
+  constexpr int UB = 4 / HALVES;
+  constexpr int HALF = HD / 2;
   __shared__ float sdw[2 * HD];
   __shared__ float swt[2 * HD];  // q then k norm weights (+ offset)
   const int l = threadIdx.x % LPH;
   const int g = threadIdx.x / LPH;
   const int e0 = l * 8;
-  const int c0 = e0 % (HD / 2);
-  const bool first_half = l < LPH / 2;
-  float dwq[8], dwk[8];
+  const int c0 = e0 % HALF;
+  float dwq[HALVES][8], dwk[HALVES][8];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) dwq[i] = dwk[i] = 0.f;
+  for (int k = 0; k < HALVES; ++k)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) dwq[k][i] = dwk[k][i] = 0.f;
   for (int i = threadIdx.x; i < 2 * HD; i += kRowThreads) {
     sdw[i] = 0.f;
     swt[i] = a.do_norm ? __bfloat162float(i < HD ? a.qw[i] : a.kw[i - HD]) + a.w_off : 1.f;
@@ -212,16 +236,16 @@ __global__ void __launch_bounds__(kRowThreads, 2) qk_rope_bwd_kernel(RopeBwdArgs
     for (int i = 0; i < 8; ++i) c[i] = s[i] = 0.f;
     if (valid) {
       const int pos = token_pos(pa, tok);
-      const float4* cp = reinterpret_cast<const float4*>(a.cos + 1LL * pos * (HD / 2) + c0);
-      const float4* sp = reinterpret_cast<const float4*>(a.sin + 1LL * pos * (HD / 2) + c0);
+      const float4* cp = reinterpret_cast<const float4*>(a.cos + 1LL * pos * HALF + c0);
+      const float4* sp = reinterpret_cast<const float4*>(a.sin + 1LL * pos * HALF + c0);
       *reinterpret_cast<float4*>(c) = cp[0];
       *reinterpret_cast<float4*>(c + 4) = cp[1];
       *reinterpret_cast<float4*>(s) = sp[0];
       *reinterpret_cast<float4*>(s + 4) = sp[1];
     }
-    if (!first_half) {
+    if (e0 >= HALF) {   // (of a single half a lane: gn = g*c + partner*s in the first, - in the second)
 #pragma unroll
-      for (int i = 0; i < 8; ++i) s[i] = -s[i];  // gn = g*c + partner*s (first half), - (second)
+      for (int i = 0; i < 8; ++i) s[i] = -s[i];
     }
     const bf16* gq = a.dq + tok * a.lddq + e0;
     const bf16* gk = a.dk + tok * a.lddk + e0;
@@ -231,18 +255,23 @@ __global__ void __launch_bounds__(kRowThreads, 2) qk_rope_bwd_kernel(RopeBwdArgs
     bf16* ok = a.dk_in + tok * a.lddk_in + e0;
     for (int b0 = 0; b0 < a.part_heads; b0 += UB) {
       const int h0 = h_first + b0;
-      uint4 graw[UB], xraw[UB];
+      uint4 graw[UB][HALVES], xraw[UB][HALVES];
       float rs[UB];
 #pragma unroll
       for (int j = 0; j < UB; ++j) {
         const int h = h0 + j;
-        graw[j] = xraw[j] = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int k = 0; k < HALVES; ++k) graw[j][k] = xraw[j][k] = make_uint4(0u, 0u, 0u, 0u);
         rs[j] = 0.f;
         if (valid && h < heads) {
           const bool is_q = h < a.Hq;
-          graw[j] = ld16(is_q ? gq + h * HD : gk + (h - a.Hq) * HD);
+          const bf16* gp = is_q ? gq + h * HD : gk + (h - a.Hq) * HD;
+#pragma unroll
+          for (int k = 0; k < HALVES; ++k) graw[j][k] = ld16(gp + k * HALF);
           if (a.do_norm) {
-            xraw[j] = ld16(is_q ? xq + h * HD : xk + (h - a.Hq) * HD);
+            const bf16* xp = is_q ? xq + h * HD : xk + (h - a.Hq) * HD;
+#pragma unroll
+            for (int k = 0; k < HALVES; ++k) xraw[j][k] = ld16(xp + k * HALF);
             rs[j] = is_q ? a.q_rstd[tok * a.Hq + h] : a.k_rstd[tok * a.Hk + (h - a.Hq)];
           }
         }
@@ -252,50 +281,77 @@ __global__ void __launch_bounds__(kRowThreads, 2) qk_rope_bwd_kernel(RopeBwdArgs
         const int h = h0 + j;
         const bool live = valid && h < heads;   // (loads of the others are zero, and add nothing)
         const bool is_q = h < a.Hq;
-        float gv[8], gn[8], o[8];
-        unpack8(graw[j], gv);
+        float gv[HALVES][8], gn[HALVES][8], o[HALVES][8];
+#pragma unroll
+        for (int k = 0; k < HALVES; ++k) unpack8(graw[j][k], gv[k]);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          const float p = __shfl_xor_sync(0xffffffffu, gv[i], LPH / 2);
-          gn[i] = gv[i] * c[i] + p * s[i];
+          if constexpr (HALVES == 2) {
+            gn[0][i] = gv[0][i] * c[i] + gv[1][i] * s[i];
+            gn[1][i] = gv[1][i] * c[i] + gv[0][i] * -s[i];
+          } else {
+            const float p = __shfl_xor_sync(0xffffffffu, gv[0][i], LPH / 2);
+            gn[0][i] = gv[0][i] * c[i] + p * s[i];
+          }
         }
         if (a.do_norm) {
-          float x[8], m[8];
-          unpack8(xraw[j], x);
+          float x[HALVES][8], m[HALVES][8], dots[HALVES] = {};
           const float rstd = rs[j];
-          const float* wt = swt + (is_q ? 0 : HD) + e0;
-          const float4 w0 = *reinterpret_cast<const float4*>(wt);
-          const float4 w1 = *reinterpret_cast<const float4*>(wt + 4);
-          const float wl[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-          float dot = 0.f;
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            x[i] *= rstd;  // xhat
-            m[i] = gn[i] * wl[i];
-            dot += m[i] * x[i];
-            const float dwv = gn[i] * bf16_round(x[i]);
-            if (is_q) dwq[i] += dwv;
-            else dwk[i] += dwv;
+          for (int k = 0; k < HALVES; ++k) {
+            unpack8(xraw[j][k], x[k]);
+            const float* wt = swt + (is_q ? 0 : HD) + k * HALF + e0;
+            const float4 w0 = *reinterpret_cast<const float4*>(wt);
+            const float4 w1 = *reinterpret_cast<const float4*>(wt + 4);
+            const float wl[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              x[k][i] *= rstd;  // xhat
+              m[k][i] = gn[k][i] * wl[i];
+              dots[k] += m[k][i] * x[k][i];
+              const float dwv = gn[k][i] * bf16_round(x[k][i]);
+              if (is_q) dwq[k][i] += dwv;
+              else dwk[k][i] += dwv;
+            }
           }
+          float dot = HALVES == 2 ? dots[0] + dots[HALVES - 1] : dots[0];
 #pragma unroll
           for (int sh = LPH / 2; sh > 0; sh >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, sh);
           dot /= float(HD);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) o[i] = rstd * (m[i] - x[i] * dot);
+          for (int k = 0; k < HALVES; ++k)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o[k][i] = rstd * (m[k][i] - x[k][i] * dot);
         } else {
 #pragma unroll
-          for (int i = 0; i < 8; ++i) o[i] = gn[i];
+          for (int k = 0; k < HALVES; ++k)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o[k][i] = gn[k][i];
         }
-        if (live) st16(is_q ? oq + h * HD : ok + (h - a.Hq) * HD, pack8(o));
+        if (live) {
+          bf16* p = is_q ? oq + h * HD : ok + (h - a.Hq) * HD;
+#pragma unroll
+          for (int k = 0; k < HALVES; ++k) st16(p + k * HALF, pack8(o[k]));
+        }
       }
     }
   }
   if (a.do_norm && a.dw_partial != nullptr) {
+    // the groups of a warp first: as many fewer additions to the same words of shared memory
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      atomicAdd(&sdw[e0 + i], dwq[i]);
-      atomicAdd(&sdw[HD + e0 + i], dwk[i]);
-    }
+    for (int k = 0; k < HALVES; ++k)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+#pragma unroll
+        for (int sh = 16; sh >= LPH; sh >>= 1) {
+          dwq[k][i] += __shfl_xor_sync(0xffffffffu, dwq[k][i], sh);
+          dwk[k][i] += __shfl_xor_sync(0xffffffffu, dwk[k][i], sh);
+        }
+        if ((threadIdx.x & 31) < LPH) {
+          atomicAdd(&sdw[k * HALF + e0 + i], dwq[k][i]);
+          atomicAdd(&sdw[HD + k * HALF + e0 + i], dwk[k][i]);
+        }
+      }
     __syncthreads();
     for (int i = threadIdx.x; i < 2 * HD; i += kRowThreads)
       a.dw_partial[1LL * blockIdx.x * 2 * HD + i] = sdw[i];
@@ -310,13 +366,15 @@ using namespace lb;
 // Lane groups per token. One walks over all heads, the next loads in flight under the current heads'
 // arithmetic, which is what the kernels are bound by with many tokens (a group for every four heads:
 // 142 against 127 us at 40280 tokens of 16 + 8 heads of 128). With so few tokens that the groups
-// are fewer than the SMs hold, the walk is a chain of latencies, and four heads a group are faster
-// (32 tokens: 21 against 29 us, 1024: 20 against 27; about 10 us of each are the measurement's own).
-static void rope_parts(int T, int heads, int tokens_per_cta, int* parts, int* part_heads) {
-  const int all = (heads + 3) / 4;
-  const bool few = 1LL * T < 3LL * row_num_sms() * tokens_per_cta / 2;
+// are fewer than the SMs hold, the walk is a chain of latencies, and a group for every few heads is
+// faster (32 tokens: 21 against 29 us, 1024: 20 against 27; about 10 us of each are the measurement's own).
+static bool few_tokens(int T, int hd) {
+  return 1LL * T < 3LL * row_num_sms() * (kRowThreads / (hd / 16)) / 2;
+}
+static void rope_parts(bool few, int heads, int unit, int* parts, int* part_heads) {
+  const int all = (heads + unit - 1) / unit;
   *parts = few ? all : 1;
-  *part_heads = few ? 4 : all * 4;
+  *part_heads = few ? unit : all * unit;
 }
 
 extern "C" int lb_rope_bwd_partial_rows() { return row_num_sms() * 8; }
@@ -337,25 +395,27 @@ extern "C" int lb_qk_norm_rope_fwd(const void* q_in, long long ldq_in, const voi
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   auto run = [&](auto kern, int lph) {
     const int tpb = kRowThreads / lph;
-    rope_parts(T, Hq + Hk, tpb, &a.parts, &a.part_heads);
+    rope_parts(few_tokens(T, hd), Hq + Hk, 2, &a.parts, &a.part_heads);
     const long long g = (1LL * T * a.parts + tpb - 1) / tpb;
-    const long long cap = 1LL * row_num_sms() * 6;  // two waves at three CTAs per SM
+    const long long cap = 1LL * row_num_sms() * 3;  // one wave at three CTAs per SM
     return launch_pdl(kern, dim3(unsigned(g < cap ? g : cap)), dim3(kRowThreads), 0, st,
                       pdl_enabled(), 1, a);
   };
-  if (hd == 128) return run(qk_rope_fwd_kernel<128>, 16);
-  if (hd == 64) return run(qk_rope_fwd_kernel<64>, 8);
-  if (hd == 256) return run(qk_rope_fwd_kernel<256>, 32);
+  if (hd == 128) return run(qk_rope_fwd_kernel<128>, 8);
+  if (hd == 64) return run(qk_rope_fwd_kernel<64>, 4);
+  if (hd == 256) return run(qk_rope_fwd_kernel<256>, 16);
   return -3;
 }
 
 // CTAs of the backward, each of which leaves a partial row in its scratch.
 extern "C" int lb_rope_bwd_rows(int T, int Hq, int Hk, int hd) {
+  if (T <= 0 || hd < 64) return 0;
+  const bool few = few_tokens(T, hd);
   int parts, part_heads;
-  const int tpb = kRowThreads / (hd / 8);
-  rope_parts(T, Hq + Hk, tpb, &parts, &part_heads);
+  rope_parts(few, Hq + Hk, few ? 2 : 4, &parts, &part_heads);
+  const int tpb = kRowThreads / (hd / (few ? 16 : 8));
   const long long g = (1LL * T * parts + tpb - 1) / tpb;
-  const long long cap = 1LL * row_num_sms() * 4;
+  const long long cap = 1LL * row_num_sms() * (few ? 2 : 4);
   return int(g < cap ? g : cap);
 }
 
@@ -378,14 +438,15 @@ extern "C" int lb_qk_norm_rope_bwd(const void* dq, long long lddq, const void* d
                 lddk_in, scratch, T, Hq, Hk, w_off, do_norm, 1, 0};
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int grid = lb_rope_bwd_rows(T, Hq, Hk, hd);
-  auto run = [&](auto kern, int lph) {
-    rope_parts(T, Hq + Hk, kRowThreads / lph, &a.parts, &a.part_heads);
+  const bool few = few_tokens(T, hd);
+  rope_parts(few, Hq + Hk, few ? 2 : 4, &a.parts, &a.part_heads);
+  auto run = [&](auto kern) {
     return launch_pdl(kern, dim3(grid), dim3(kRowThreads), 0, st, pdl_enabled(), 1, a);
   };
   int rc = -3;
-  if (hd == 128) rc = run(qk_rope_bwd_kernel<128>, 16);
-  else if (hd == 64) rc = run(qk_rope_bwd_kernel<64>, 8);
-  else if (hd == 256) rc = run(qk_rope_bwd_kernel<256>, 32);
+  if (hd == 128) rc = few ? run(qk_rope_bwd_kernel<128, 2>) : run(qk_rope_bwd_kernel<128, 1>);
+  else if (hd == 64) rc = few ? run(qk_rope_bwd_kernel<64, 2>) : run(qk_rope_bwd_kernel<64, 1>);
+  else if (hd == 256) rc = few ? run(qk_rope_bwd_kernel<256, 2>) : run(qk_rope_bwd_kernel<256, 1>);
   if (rc) return rc;
   if (do_norm && dw_out != nullptr && scratch != nullptr) {
     return lb_colsum(scratch, grid, 2 * hd, dw_out, dw_fp32, dw_accumulate, stream);

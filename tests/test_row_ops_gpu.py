@@ -317,3 +317,39 @@ def test_rms_norm_takes_a_weight_that_starts_anywhere(H, offset):
     assert torch.equal(rms_norm(x, w), rms_norm(x, w.clone()))
     for a, b in zip(residual_rms_norm(r, x, w), residual_rms_norm(r, x, w.clone())):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("Hq,Hk,hd", [(16, 8, 128), (5, 1, 64), (3, 1, 256)])
+@pytest.mark.parametrize("norm", [True, False])
+def test_rope_of_few_and_of_many_tokens_has_the_same_bits(Hq, Hk, hd, norm):
+    """Few tokens are cut into groups of heads, and their backward has lanes of its own; values and input
+    gradients of a token do not depend on how many there are. Weight gradients: fp32 sums."""
+    from lset_b200.ops.rope import qk_norm_rope
+
+    torch.manual_seed(hd)
+    T, parts = 16000, [1, 33, 4000, 11966]      # more than 3 * 148 * 4096 / hd / 2 of them: many
+    q, k = (torch.randn(T, h, hd, device="cuda").to(torch.bfloat16) for h in (Hq, Hk))
+    gq, gk = torch.randn_like(q), torch.randn_like(k)
+    ws = [(torch.rand(hd, device="cuda") + 0.5).to(torch.bfloat16).requires_grad_() for _ in range(2)]
+    cos, sin = torch.randn(512, hd // 2, device="cuda"), torch.randn(512, hd // 2, device="cuda")
+    pos = torch.randint(0, 512, (T,), device="cuda")
+
+    def run(rows):
+        a, b = q[rows].clone().requires_grad_(), k[rows].clone().requires_grad_()
+        out = qk_norm_rope(a, b, *(ws if norm else (None, None)), cos, sin, pos[rows])
+        for w in ws:
+            w.grad = None
+        torch.autograd.backward(out, (gq[rows], gk[rows]))
+        return [*(o.detach() for o in out), a.grad, b.grad], [w.grad.double() for w in ws if norm]
+
+    whole, wsum = run(slice(0, T))
+    total, at = [0.0, 0.0], 0
+    for n in parts:
+        part, wg = run(slice(at, at + n))
+        for x, y in zip(part, whole):
+            assert torch.equal(x, y[at:at + n]), n
+        total = [a + b for a, b in zip(total, wg)]
+        at += n
+    assert at == T
+    for a, b in zip(total, wsum):      # four bf16 roundings of the parts' sums
+        assert ((a - b).norm() / b.norm()).item() < 4 * 2 ** -8
