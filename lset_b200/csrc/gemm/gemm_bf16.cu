@@ -25,7 +25,9 @@
 #include "../common/pdl.h"
 #include "../common/ptx.cuh"
 #include "../common/tma_desc.h"
+#include "../common/api.h"
 #include "gemm_small.h"
+#include "loss.h"
 
 namespace lb {
 
@@ -35,14 +37,15 @@ constexpr int BM = 128;
 constexpr int BK = 64;
 constexpr int kGatherThreads = 256;  // + 2 pull warps
 
-// Number of epilogue warps. The plain store / reduce epilogue of the bf16 kernel runs on eight
-// (two per tensor-memory lane quarter, each taking half of the tile's columns): at K = 1024 the
-// main loop of a 128 x 256 tile lasts about as long as four warps need to drain it, and the drain
-// then bounds the kernel. The loss / GLU epilogues, the 8-bit kernel and the peer-gather variants
-// (which already carry two pull warps) keep four.
+// Number of epilogue warps. The plain store / reduce epilogue of the bf16 kernel and the loss epilogues
+// of more than one column tile run on eight (two per tensor-memory lane quarter, each taking half of
+// the tile's columns): at K = 1024 the main loop of a 128 x 256 tile lasts about as long as four warps
+// need to drain it, and the drain then bounds the kernel; where every CTA has one tile, nothing hides
+// it at all. The GLU epilogue, the 8-bit kernel, the peer-gather variants (which already carry two pull
+// warps) and losses of one column tile (EPI_LSE_ROW, EPI_PGRAD_ROW: one sum per row) keep four.
 template <int EPI, int GATHER, int F8>
 constexpr int epi_warps() {
-  return (EPI == 0 /*EPI_STORE*/ && GATHER == 0 && F8 == 0) ? 8 : 4;
+  return (EPI <= 2 /*EPI_STORE, EPI_LSE, EPI_PGRAD*/ && GATHER == 0 && F8 == 0) ? 8 : 4;
 }
 template <int EPI, int GATHER, int F8>
 constexpr int gemm_threads() {
@@ -65,7 +68,9 @@ struct GemmArgs {
   const float* lse;           // [M] natural-log LSE (EPI_PGRAD input)
   float* part;                // [tiles_n, M, 2] running (max, sum) in log2 domain (EPI_LSE output)
   float* pos;                 // [M] score of the target column (EPI_LSE output)
-  const float* coef;          // device scalar multiplied into the probabilities' gradient
+  const float* coef;          // device scalar multiplied into the probabilities' gradient,
+  float coef_scale;           // times this
+  float* zero;                // cleared by a forward launch (the loss that the next one adds to), or null
   long long target_offset;    // target column of row r is r + target_offset
   // label-matrix losses (labels != nullptr): int8 labels [M, ld_labels] (1 positive, 0 negative,
   // < 0 ignored; ld_labels a multiple of 32 and >= N, padding = ignored), optional target weights
@@ -120,7 +125,7 @@ struct GemmArgs {
   int* status;
 };
 
-enum { EPI_STORE = 0, EPI_LSE = 1, EPI_PGRAD = 2, EPI_GLU = 3 };
+enum { EPI_STORE = 0, EPI_LSE = 1, EPI_PGRAD = 2, EPI_GLU = 3, EPI_LSE_ROW = 4, EPI_PGRAD_ROW = 5 };
 constexpr float kLog2e = 1.4426950408889634f;
 
 template <int BN, int EW = 4, int F8 = 0>
@@ -158,12 +163,13 @@ __device__ __forceinline__ void red_add8_bf16(void* dst, const uint4& v) {
                : "memory");
 }
 
-template <int A_MN, int B_MN, int BN, typename OutT, int EPI, int GATHER = 0, int F8 = 0>
-__global__ void __launch_bounds__(gemm_threads<EPI, GATHER, F8>(), 1)
+template <int A_MN, int B_MN, int BN, typename OutT, int EPI_, int GATHER = 0, int F8 = 0>
+__global__ void __launch_bounds__(gemm_threads<EPI_, GATHER, F8>(), 1)
     gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                      const __grid_constant__ CUtensorMap tmA2,
                      const __grid_constant__ CUtensorMap tmB2, GemmArgs g) {
-  constexpr int EW = epi_warps<EPI, GATHER, F8>();
+  constexpr int EW = epi_warps<EPI_, GATHER, F8>();
+  constexpr int EPI = EPI_ == EPI_LSE_ROW ? EPI_LSE : (EPI_ == EPI_PGRAD_ROW ? EPI_PGRAD : EPI_);
   using C = Cfg<BN, EW, F8>;
   // 8-bit operands: K-major only; a k-block is still 128 bytes of every row, i.e. 128 elements,
   // and the shared-memory tiles, swizzle and descriptors are byte-for-byte those of the bf16 form.
@@ -210,6 +216,9 @@ __global__ void __launch_bounds__(gemm_threads<EPI, GATHER, F8>(), 1)
   const uint32_t tmem_base = *tmem_slot;
   pdl_wait();
   pdl_trigger();
+  if constexpr (EPI == EPI_LSE) {
+    if (blockIdx.x == 0 && threadIdx.x == 0 && g.zero != nullptr) *g.zero = 0.f;
+  }
 
   // CTAs that compute tiles are numbered 0 .. ncta-1 (a gather launch puts its copy CTAs first)
   [[maybe_unused]] const int n_copy = GATHER ? g.copy_ctas : 0;
@@ -571,7 +580,7 @@ __global__ void __launch_bounds__(gemm_threads<EPI, GATHER, F8>(), 1)
       }
       if constexpr (EPI == EPI_PGRAD) {
         lse2 = (row < m_limit) ? g.lse[row] * kLog2e : 0.f;
-        cf = g.coef != nullptr ? g.coef[0] : 1.f;
+        cf = g.coef[0] * g.coef_scale;
         if (lbl && row < m_limit) {
           cf *= g.row_w[row];
           rscale = g.row_scale[row];
@@ -822,7 +831,7 @@ __global__ void __launch_bounds__(gemm_threads<EPI, GATHER, F8>(), 1)
       }
       if constexpr (EPI == EPI_LSE) {
         if (row < m_limit) {
-          const int part_idx = GATHER == 1 ? chunk : n0 / BN;
+          const int part_idx = GATHER == 1 ? chunk : (EW == 8 ? 2 * (n0 / BN) + half : n0 / BN);
           float* pp = g.part + (static_cast<long long>(part_idx) * g.M + row) * 2;
           pp[0] = m_run;
           pp[1] = l_run;
@@ -1230,85 +1239,113 @@ extern "C" int lb_gemm_bf16_scatter(const void* A, const void* B, const void* co
 namespace lb {
 namespace {
 
-// lse[r] = ln(sum_j exp(s_rj)); loss_sum += sum_r (lse[r] − pos[r]) (one atomicAdd per block).
+// lse[r] = ln(sum_j exp(s_rj)) out of the (max, sum) pairs of `parts` column ranges; loss += loss_scale *
+// sum_r (lse[r] − pos[r]) (one atomicAdd per block). LABELS: loss += loss_scale * sum_r row_w[r] *
+// (lse[r] − row_scale[r] · pos[r]), and rows without a valid column get lse = 0 (their row_w is 0).
+// A block has 32 rows, and of each every eighth range per warp (8192 rows of 32 ranges: 9 us with a thread
+// per row, which is a chain of loads on a fifth of the SMs, 4 here).
+template <bool LABELS>
 __global__ void __launch_bounds__(256)
-    lse_merge_kernel(const float* __restrict__ part, int tiles_n, int M, const float* __restrict__ pos,
-                     float* __restrict__ lse, float* __restrict__ loss_sum) {
-  __shared__ float sred[8];
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    lse_merge_kernel(const float* __restrict__ part, int parts, int M, const float* __restrict__ pos,
+                     const float* __restrict__ row_scale, const float* __restrict__ row_w,
+                     float* __restrict__ lse, float* __restrict__ loss, float loss_scale) {
+  __shared__ float sm[8][32], sl[8][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int r = blockIdx.x * 32 + lane;
+  pdl_wait();
+  pdl_trigger();
+  float m = -INFINITY, l = 0.f;
+  auto add = [&](float mt, float lt) {
+    const float mn = fmaxf(m, mt);
+    if (mn > -INFINITY) l = l * exp2f(m - mn) + lt * exp2f(mt - mn);
+    m = mn;
+  };
+  if (r < M) {
+    const float2* p = reinterpret_cast<const float2*>(part);
+    int t = w;
+    for (; t + 24 < parts; t += 32) {   // four loads in flight
+      float2 v[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[i] = p[1LL * (t + 8 * i) * M + r];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) add(v[i].x, v[i].y);
+    }
+    for (; t < parts; t += 8) {
+      const float2 v = p[1LL * t * M + r];
+      add(v.x, v.y);
+    }
+  }
+  sm[w][lane] = m;
+  sl[w][lane] = l;
+  __syncthreads();
+  if (w != 0) return;
+#pragma unroll
+  for (int i = 1; i < 8; ++i) add(sm[i][lane], sl[i][lane]);
   float contrib = 0.f;
   if (r < M) {
-    float m = -INFINITY, l = 0.f;
-    for (int t = 0; t < tiles_n; ++t) {
-      const float mt = part[(1LL * t * M + r) * 2], lt = part[(1LL * t * M + r) * 2 + 1];
-      const float mn = fmaxf(m, mt);
-      if (mn > -INFINITY) l = l * exp2f(m - mn) + lt * exp2f(mt - mn);
-      m = mn;
-    }
-    const float v = (m + log2f(l)) * 0.6931471805599453f;
+    const float v = !LABELS || l > 0.f ? (m + log2f(l)) * 0.6931471805599453f : 0.f;
     lse[r] = v;
-    contrib = v - pos[r];
+    if constexpr (LABELS) {
+      const float rw = row_w[r];
+      if (rw != 0.f) contrib = rw * (v - row_scale[r] * pos[r]);
+    } else {
+      contrib = v - pos[r];
+    }
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) contrib += __shfl_xor_sync(0xffffffffu, contrib, o);
-  if ((threadIdx.x & 31) == 0) sred[threadIdx.x >> 5] = contrib;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float s = 0.f;
-    for (int i = 0; i < 8; ++i) s += sred[i];
-    atomicAdd(loss_sum, s);
-  }
+  if (lane == 0) atomicAdd(loss, contrib * loss_scale);
 }
 
-// Label-matrix variant: per_q = lse − row_scale · pos; loss_sum += sum_r row_w[r] · per_q. Rows
-// without a valid column get lse = 0 (their row_w is 0).
-__global__ void __launch_bounds__(256)
-    lse_merge_label_kernel(const float* __restrict__ part, int tiles_n, int M,
-                           const float* __restrict__ pos, const float* __restrict__ row_scale,
-                           const float* __restrict__ row_w, float* __restrict__ lse,
-                           float* __restrict__ loss_sum) {
-  __shared__ float sred[8];
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  float contrib = 0.f;
-  if (r < M) {
-    float m = -INFINITY, l = 0.f;
-    for (int t = 0; t < tiles_n; ++t) {
-      const float mt = part[(1LL * t * M + r) * 2], lt = part[(1LL * t * M + r) * 2 + 1];
-      const float mn = fmaxf(m, mt);
-      if (mn > -INFINITY) l = l * exp2f(m - mn) + lt * exp2f(mt - mn);
-      m = mn;
-    }
-    const float v = l > 0.f ? (m + log2f(l)) * 0.6931471805599453f : 0.f;
-    lse[r] = v;
-    const float w = row_w[r];
-    if (w != 0.f) contrib = w * (v - row_scale[r] * pos[r]);
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) contrib += __shfl_xor_sync(0xffffffffu, contrib, o);
-  if ((threadIdx.x & 31) == 0) sred[threadIdx.x >> 5] = contrib;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float s = 0.f;
-    for (int i = 0; i < 8; ++i) s += sred[i];
-    atomicAdd(loss_sum, s);
-  }
-}
+int num_sms();
 
+// Columns of a tile: 128 where tiles of 256 would leave more than half of the SMs without one (1024 x
+// 1024 x 768: scores 11.4 -> 7.2 us, with their gradient 13.4 -> 7.8, eight
+// epilogue warps included; those alone: 1009 x 4036 x 1024 with labels 33 -> 22 and 45 -> 26, 8192 x 8192 x
+// 1024 with gradient 117 -> 111).
 int loss_tile_bn(int M, int N) {
-  (void)M;
-  return N > 128 ? 256 : 128;
+  if (N <= 128) return 128;
+  return 2LL * ((M + BM - 1) / BM) * ((N + 255) / 256) <= num_sms() && N > 256 ? 128 : 256;
+}
+// Column ranges that a row's (max, sum) pairs come from: two per tile, one where a single tile has all
+// columns (the sums of small batches, whose bits a training run repeats).
+bool loss_one_tile(int M, int N) { return N <= loss_tile_bn(M, N); }
+int loss_parts(int M, int N) {
+  const int bn = loss_tile_bn(M, N);
+  return loss_one_tile(M, N) ? 1 : 2 * ((N + bn - 1) / bn);
 }
 
-int prep_loss(const void* Q, const void* Kd, int M, int N, int D, long long ldq, long long ldk,
+template <int EPI, int EPI_ROW>
+int launch_loss(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmArgs& g, int grid,
+                cudaStream_t stream) {
+  const bool wide = loss_tile_bn(g.M, g.N) == 256;
+  if (loss_one_tile(g.M, g.N))
+    return wide ? launch<0, 0, 256, __nv_bfloat16, EPI_ROW>(tmA, tmB, g, grid, stream)
+                : launch<0, 0, 128, __nv_bfloat16, EPI_ROW>(tmA, tmB, g, grid, stream);
+  return wide ? launch<0, 0, 256, __nv_bfloat16, EPI>(tmA, tmB, g, grid, stream)
+              : launch<0, 0, 128, __nv_bfloat16, EPI>(tmA, tmB, g, grid, stream);
+}
+
+template <bool LABELS>
+int merge_lse(const GemmArgs& g, int parts, float* lse, float* loss, float loss_scale,
+              cudaStream_t stream) {
+  return launch_pdl(lse_merge_kernel<LABELS>, dim3((g.M + 31) / 32), dim3(256), 0, stream,
+                    pdl_enabled(), 1, (const float*)g.part, parts, g.M, (const float*)g.pos,
+                    g.row_scale, g.row_w, lse, loss, loss_scale);
+}
+
+// (k_rows: passages in memory; columns from there to N have no product and are zero)
+int prep_loss(const void* Q, const void* Kd, int M, int N, int k_rows, int D, long long ldq, long long ldk,
               int bn, CUtensorMap* tmA, CUtensorMap* tmB, GemmArgs* g, int* grid) {
   if (M <= 0 || N <= 0 || D <= 0) return -4;
   if ((ldq & 7) || (ldk & 7)) return -3;
   int rc = make_tmap_2d(tmA, Q, 2, (uint64_t)D, (uint64_t)M, (uint64_t)ldq * 2, BK, BM, true);
   if (rc) return rc;
-  rc = make_tmap_2d(tmB, Kd, 2, (uint64_t)D, (uint64_t)N, (uint64_t)ldk * 2, BK, bn, true);
+  rc = make_tmap_2d(tmB, Kd, 2, (uint64_t)D, (uint64_t)k_rows, (uint64_t)ldk * 2, BK, bn, true);
   if (rc) return rc;
   const int tiles_m = (M + BM - 1) / BM, tiles_n = (N + bn - 1) / bn;
   *g = GemmArgs{};
+  g->coef_scale = 1.f;
   g->M = M;
   g->N = N;
   g->K = D;
@@ -1447,35 +1484,103 @@ extern "C" int lb_gemm_bf16_ext(const void* A, const void* B, const void* A2, co
 }
 
 extern "C" long long lb_infonce_scratch_floats(int M, int N) {
-  const int bn = lb::loss_tile_bn(M, N);
-  return 2LL * ((N + bn - 1) / bn) * M + M;
+  return 2LL * lb::loss_parts(M, N) * M + M;
 }
 
-// q: [M, D] bf16 (row stride ldq), k: [N, D] bf16 (row stride ldk). The positive of query r is
-// passage r + target_offset. Outputs: lse [M] fp32, loss_sum (device scalar, += sum_r (lse − pos)).
-// scratch: lb_infonce_scratch_floats(M, N) floats.
-extern "C" int lb_infonce_fwd(const void* q, long long ldq, const void* k, long long ldk, int M,
-                              int N, int D, float inv_temperature, long long target_offset,
-                              float* scratch, float* lse, float* loss_sum, int* status,
-                              void* stream_) {
-  using namespace lb;
-  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
-  const int bn = loss_tile_bn(M, N);
+namespace lb {
+namespace {
+
+// The arguments of one product of scores: columns [c0, c0 + n) of the loss.
+int loss_product(const LbLoss& p, int c0, int n, CUtensorMap* tmA, CUtensorMap* tmB, GemmArgs* g,
+                 int* grid) {
+  const bool lbl = p.labels != nullptr;
+  if (lbl && ((p.ld_labels & 31) || p.ld_labels < p.N)) return -3;
+  if (p.tw != nullptr && (!lbl || (p.ld_tw & 31) || p.ld_tw < p.N)) return -3;
+  if (!lbl && (n & 7)) return -3;
+  const int np = (n + 7) / 8 * 8;   // (columns beyond n are ignored: their labels are padding)
+  const char* k = static_cast<const char*>(p.k) + 2LL * c0 * p.ldk;
+  if (int rc = prep_loss(p.q, k, p.M, np, n, p.D, p.ldq, p.ldk, loss_tile_bn(p.M, np), tmA, tmB, g, grid))
+    return rc;
+  g->scale = p.inv_temperature;
+  g->target_offset = p.target_offset - c0;
+  if (lbl) {
+    g->labels = static_cast<const signed char*>(p.labels) + c0;
+    g->tw = p.tw != nullptr ? p.tw + c0 : nullptr;
+    g->ld_labels = p.ld_labels;
+    g->ld_tw = p.ld_tw;
+    g->row_scale = p.row_scale;
+    g->row_w = p.row_w;
+    g->loss_mode = p.loss_mode;
+  }
+  g->status = p.status;
+  return 0;
+}
+
+// W[:, c] of columns [c0, c0 + n), see LbLoss.
+int loss_pgrad(const LbLoss& p, int c0, int n, cudaStream_t stream) {
+  if (p.ldw & 7) return -3;
   CUtensorMap tmA, tmB;
   GemmArgs g;
   int grid;
-  if (int rc = prep_loss(q, k, M, N, D, ldq, ldk, bn, &tmA, &tmB, &g, &grid)) return rc;
-  const int tiles_n = (N + bn - 1) / bn;
-  g.scale = inv_temperature;
-  g.part = scratch;
-  g.pos = scratch + 2LL * tiles_n * M;
-  g.target_offset = target_offset;
-  g.status = status;
-  int rc = bn == 256 ? launch<0, 0, 256, __nv_bfloat16, EPI_LSE>(tmA, tmB, g, grid, stream)
-                     : launch<0, 0, 128, __nv_bfloat16, EPI_LSE>(tmA, tmB, g, grid, stream);
-  if (rc) return rc;
-  lse_merge_kernel<<<(M + 255) / 256, 256, 0, stream>>>(g.part, tiles_n, M, g.pos, lse, loss_sum);
-  return cudaGetLastError() == cudaSuccess ? 0 : -11;
+  if (int rc = loss_product(p, c0, n, &tmA, &tmB, &g, &grid)) return rc;
+  g.lse = p.lse;
+  g.coef = p.grad;
+  g.coef_scale = p.grad_scale;
+  g.C = p.W;
+  g.ldc = p.ldw;
+  return launch_loss<EPI_PGRAD, EPI_PGRAD_ROW>(tmA, tmB, g, grid, stream);
+}
+
+}  // namespace
+}  // namespace lb
+
+// Forward: p->lse and p->loss (see LbLoss). Scratch: lb_infonce_scratch_floats(M, N rounded up to 8).
+extern "C" int lb_loss_fwd(const LbLoss* p) {
+  using namespace lb;
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(p->stream);
+  CUtensorMap tmA, tmB;
+  GemmArgs g;
+  int grid;
+  if (int rc = loss_product(*p, 0, p->N, &tmA, &tmB, &g, &grid)) return rc;
+  const int parts = loss_parts(g.M, g.N);
+  g.part = p->scratch;
+  g.pos = p->scratch + 2LL * parts * g.M;
+  g.zero = p->loss;
+  if (p->labels != nullptr &&
+      cudaMemsetAsync(g.pos, 0, sizeof(float) * g.M, stream) != cudaSuccess)
+    return -12;
+  if (int rc = launch_loss<EPI_LSE, EPI_LSE_ROW>(tmA, tmB, g, grid, stream)) return rc;
+  const PdlScope pdl(true);
+  return p->labels != nullptr ? merge_lse<true>(g, parts, p->lse, p->loss, p->loss_scale, stream)
+                              : merge_lse<false>(g, parts, p->lse, p->loss, p->loss_scale, stream);
+}
+
+// Backward in panels of p->panel columns (the last one may have fewer): W of the panel, then dK of its
+// passages complete, and dQ: at once where there is one panel, else summed over the panels in dq32.
+extern "C" int lb_loss_bwd(const LbLoss* p) {
+  using namespace lb;
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(p->stream);
+  if (p->panel <= 0 || (p->panel < p->N && (p->panel & 255))) return -3;   // (label rows: 16-byte aligned)
+  const bool single = p->panel >= p->N;
+  if (!single && p->dq != nullptr && p->dq32 == nullptr) return -3;
+  for (int c0 = 0; c0 < p->N; c0 += p->panel) {
+    const int n = p->N - c0 < p->panel ? p->N - c0 : p->panel;
+    if (int rc = loss_pgrad(*p, c0, n, stream)) return rc;
+    const PdlScope chain(true);   // the first launch is ordered behind everything before it
+    const char* k = static_cast<const char*>(p->k) + 2LL * c0 * p->ldk;
+    if (p->dq != nullptr) {
+      const int rc = lb_gemm_bf16(p->W, k, single ? p->dq : (void*)p->dq32, p->M, p->D, n, p->ldw, p->ldk,
+                                  p->D, 0, 1, !single, !single && c0 > 0, nullptr, 1, 0, p->status,
+                                  p->stream);
+      if (rc) return rc;
+    }
+    if (p->dk != nullptr) {
+      const int rc = lb_gemm_bf16(p->W, p->q, static_cast<char*>(p->dk) + 2LL * c0 * p->D, n, p->D, p->M,
+                                  p->ldw, p->ldq, p->D, 1, 1, 0, 0, nullptr, 1, 0, p->status, p->stream);
+      if (rc) return rc;
+    }
+  }
+  return 0;
 }
 
 // W[r, c] = (exp(s_rc − lse[r]) − [c == r + target_offset]) * coef[0], bf16, row stride ldw
@@ -1484,102 +1589,23 @@ extern "C" int lb_infonce_pgrad(const void* q, long long ldq, const void* k, lon
                                 int N, int D, float inv_temperature, long long target_offset,
                                 const float* lse, const float* coef, void* W, long long ldw,
                                 int* status, void* stream_) {
-  using namespace lb;
-  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
-  if ((N & 7) || (ldw & 7)) return -3;
-  const int bn = loss_tile_bn(M, N);
-  CUtensorMap tmA, tmB;
-  GemmArgs g;
-  int grid;
-  if (int rc = prep_loss(q, k, M, N, D, ldq, ldk, bn, &tmA, &tmB, &g, &grid)) return rc;
-  g.scale = inv_temperature;
-  g.lse = lse;
-  g.coef = coef;
-  g.C = W;
-  g.ldc = ldw;
-  g.target_offset = target_offset;
-  g.status = status;
-  return bn == 256 ? launch<0, 0, 256, __nv_bfloat16, EPI_PGRAD>(tmA, tmB, g, grid, stream)
-                   : launch<0, 0, 128, __nv_bfloat16, EPI_PGRAD>(tmA, tmB, g, grid, stream);
-}
-
-// Label-matrix contrastive loss (multi-positive NCE and soft-label cross-entropy) on the same
-// streaming kernels: loss_sum += sum_r row_w[r] · (LSE_{valid c} s_rc − row_scale[r] · sum_c t_rc s_rc)
-// with t = max(label, 0) (tw == nullptr) or t = tw. labels: int8 [M, ld_labels], ld_labels % 32 == 0,
-// >= N, padded with a negative value; tw: fp32 [M, ld_tw] or nullptr, same padding rule (zeros).
-// loss_mode 1 (multi-positive NCE): lse[r] is the LSE over the negatives (label == 0) only and
-// loss_sum is not meaningful; the caller forms the loss from lse and the positives' scores.
-// scratch: lb_infonce_scratch_floats(M, N) floats.
-extern "C" int lb_label_loss_fwd(const void* q, long long ldq, const void* k, long long ldk, int M,
-                                 int N, int D, float inv_temperature, const void* labels,
-                                 long long ld_labels, const float* tw, long long ld_tw,
-                                 const float* row_scale, const float* row_w, int loss_mode,
-                                 float* scratch, float* lse, float* loss_sum, int* status,
-                                 void* stream_) {
-  using namespace lb;
-  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
-  if (labels == nullptr || (ld_labels & 31) || ld_labels < N) return -3;
-  if (tw != nullptr && ((ld_tw & 31) || ld_tw < N)) return -3;
-  const int bn = loss_tile_bn(M, N);
-  CUtensorMap tmA, tmB;
-  GemmArgs g;
-  int grid;
-  if (int rc = prep_loss(q, k, M, N, D, ldq, ldk, bn, &tmA, &tmB, &g, &grid)) return rc;
-  const int tiles_n = (N + bn - 1) / bn;
-  g.scale = inv_temperature;
-  g.part = scratch;
-  g.pos = scratch + 2LL * tiles_n * M;
-  g.labels = static_cast<const signed char*>(labels);
-  g.ld_labels = ld_labels;
-  g.tw = tw;
-  g.ld_tw = ld_tw;
-  g.row_scale = row_scale;
-  g.row_w = row_w;
-  g.loss_mode = loss_mode;
-  g.status = status;
-  if (cudaMemsetAsync(g.pos, 0, sizeof(float) * M, stream) != cudaSuccess) return -12;
-  int rc = bn == 256 ? launch<0, 0, 256, __nv_bfloat16, EPI_LSE>(tmA, tmB, g, grid, stream)
-                     : launch<0, 0, 128, __nv_bfloat16, EPI_LSE>(tmA, tmB, g, grid, stream);
-  if (rc) return rc;
-  lse_merge_label_kernel<<<(M + 255) / 256, 256, 0, stream>>>(g.part, tiles_n, M, g.pos, row_scale,
-                                                             row_w, lse, loss_sum);
-  return cudaGetLastError() == cudaSuccess ? 0 : -11;
-}
-
-// W[r, c] = ([label_rc >= 0] · exp(s_rc − lse[r]) − row_scale[r] · t_rc) · row_w[r] · coef[0], bf16
-// (loss_mode 0); loss_mode 1: positives (sigmoid(s − lse) − 1) · row_w · coef, negatives
-// exp(s − lse) · row_scale · row_w · coef.
-extern "C" int lb_label_loss_pgrad(const void* q, long long ldq, const void* k, long long ldk, int M,
-                                   int N, int D, float inv_temperature, const void* labels,
-                                   long long ld_labels, const float* tw, long long ld_tw,
-                                   const float* row_scale, const float* row_w, int loss_mode,
-                                   const float* lse, const float* coef, void* W, long long ldw,
-                                   int* status, void* stream_) {
-  using namespace lb;
-  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
-  if ((N & 7) || (ldw & 7)) return -3;
-  if (labels == nullptr || (ld_labels & 31) || ld_labels < N) return -3;
-  if (tw != nullptr && ((ld_tw & 31) || ld_tw < N)) return -3;
-  const int bn = loss_tile_bn(M, N);
-  CUtensorMap tmA, tmB;
-  GemmArgs g;
-  int grid;
-  if (int rc = prep_loss(q, k, M, N, D, ldq, ldk, bn, &tmA, &tmB, &g, &grid)) return rc;
-  g.scale = inv_temperature;
-  g.lse = lse;
-  g.coef = coef;
-  g.C = W;
-  g.ldc = ldw;
-  g.labels = static_cast<const signed char*>(labels);
-  g.ld_labels = ld_labels;
-  g.tw = tw;
-  g.ld_tw = ld_tw;
-  g.row_scale = row_scale;
-  g.row_w = row_w;
-  g.loss_mode = loss_mode;
-  g.status = status;
-  return bn == 256 ? launch<0, 0, 256, __nv_bfloat16, EPI_PGRAD>(tmA, tmB, g, grid, stream)
-                   : launch<0, 0, 128, __nv_bfloat16, EPI_PGRAD>(tmA, tmB, g, grid, stream);
+  LbLoss p = {};
+  p.q = q;
+  p.k = k;
+  p.ldq = ldq;
+  p.ldk = ldk;
+  p.M = M;
+  p.N = N;
+  p.D = D;
+  p.inv_temperature = inv_temperature;
+  p.target_offset = target_offset;
+  p.lse = const_cast<float*>(lse);
+  p.grad = coef;
+  p.grad_scale = 1.f;
+  p.W = W;
+  p.ldw = ldw;
+  p.status = status;
+  return lb::loss_pgrad(p, 0, N, reinterpret_cast<cudaStream_t>(stream_));
 }
 
 // Cross-rank InfoNCE forward: the passages of all `world` ranks (n_local rows each, in symmetric
@@ -1628,7 +1654,7 @@ extern "C" int lb_infonce_fwd_xrank(const void* q, long long ldq, const void* co
   CUtensorMap tmA, tmB;
   GemmArgs g;
   int grid;
-  if (int rc = prep_loss(q, k_all, M, N, D, ldq, ldk, 256, &tmA, &tmB, &g, &grid)) return rc;
+  if (int rc = prep_loss(q, k_all, M, N, N, D, ldq, ldk, 256, &tmA, &tmB, &g, &grid)) return rc;
   const int tiles_per_peer = (n_local + 255) / 256;
   const int chunks = world * tiles_per_peer;
   const long long total = 1LL * ((M + BM - 1) / BM) * chunks;
@@ -1652,8 +1678,7 @@ extern "C" int lb_infonce_fwd_xrank(const void* q, long long ldq, const void* co
   if (cudaMemsetAsync(counter, 0, sizeof(unsigned), stream) != cudaSuccess) return -12;
   int rc = launch<0, 0, 256, __nv_bfloat16, EPI_LSE, 1>(tmA, tmB, g, grid, stream);
   if (rc) return rc;
-  lse_merge_kernel<<<(M + 255) / 256, 256, 0, stream>>>(g.part, chunks, M, g.pos, lse, loss_sum);
-  return cudaGetLastError() == cudaSuccess ? 0 : -11;
+  return merge_lse<false>(g, chunks, lse, loss_sum, 1.f, stream);
 }
 
 // All-gather fused into a GEMM (tensor-parallel column layers and the input-gradient of row

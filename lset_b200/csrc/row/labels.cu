@@ -18,7 +18,7 @@ template <typename T>
 __global__ void __launch_bounds__(kLabelThreads)
     label_prep_kernel(const T* __restrict__ labels, long long ld, int Q, int K, int Kp,
                       signed char* __restrict__ lab8, float* __restrict__ row_scale,
-                      float* row_w, int* counters /* kept rows, CTAs done; zero on entry and exit */) {
+                      float* row_w, int* counters /* kept rows, CTAs done; zero on entry */) {
   __shared__ int s_sum[kLabelThreads / 32], s_max[kLabelThreads / 32];
   __shared__ bool s_last;
   int kept = 0;
@@ -75,8 +75,6 @@ __global__ void __launch_bounds__(kLabelThreads)
   const float w = 1.f / float(n > 1 ? n : 1);
   for (int r = threadIdx.x; r < Q; r += kLabelThreads)
     row_w[r] = *reinterpret_cast<volatile float*>(row_w + r) != 0.f ? w : 0.f;
-  __syncthreads();
-  if (threadIdx.x == 0) counters[0] = counters[1] = 0;
 }
 
 }  // namespace
@@ -85,13 +83,14 @@ __global__ void __launch_bounds__(kLabelThreads)
 using namespace lb;
 
 // labels [Q, K], rows ld elements apart; kind: 0 = fp32, 1 = int64, 2 = int32, 3 = int8 / bool. Kp: K
-// rounded up to a multiple of 32. counters: two ints, zero.
+// rounded up to a multiple of 32. counters: two ints.
 extern "C" int lb_label_prep(const void* labels, int kind, long long ld, int Q, int K, int Kp,
                              void* lab8, float* row_scale, float* row_w, int* counters,
                              void* stream) {
   if (Q <= 0) return 0;
   if (K <= 0 || (Kp & 31) || Kp < K) return -3;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (cudaMemsetAsync(counters, 0, 2 * sizeof(int), st) != cudaSuccess) return -12;
   const int cap = row_num_sms() * 8;
   const int grid = Q < cap ? Q : cap;
   signed char* out = static_cast<signed char*>(lab8);

@@ -7,6 +7,8 @@ Replaces the cuBLAS matmul of lset/losses/infonce.py:20 and lset/losses/contrast
 """
 from __future__ import annotations
 
+import ctypes
+
 import torch
 
 from . import _native as nv
@@ -71,7 +73,8 @@ def panel_cols(M: int, N: int) -> int:
 
 def streamed_loss_backward(launch_pgrad, q, k, need_dq: bool, need_dk: bool):
     """``launch_pgrad(c0, c1, W)`` fills ``W [M, c1 - c0]`` (bf16) for the passage columns
-    ``[c0, c1)``. Returns ``(dq, dk)`` in the inputs' dtype."""
+    ``[c0, c1)``. Returns ``(dq, dk)`` in the inputs' dtype. (The losses of one rank do the same in
+    one native call, ``lb_loss_bwd``.)"""
     M, D = q.shape
     N = k.shape[0]
     step = panel_cols(M, N)
@@ -99,55 +102,102 @@ def streamed_loss_backward(launch_pgrad, q, k, need_dq: bool, need_dk: bool):
 
 
 # ------------------------------------------------------------------------------------------------
-# Streaming InfoNCE: scores never materialise in fp32; see lb_infonce_fwd / lb_infonce_pgrad.
+# Streaming losses: scores never materialise in fp32; see csrc/gemm/loss.h. One native call each way.
 # ------------------------------------------------------------------------------------------------
+class LbLoss(ctypes.Structure):      # csrc/gemm/loss.h
+    _fields_ = [("q", ctypes.c_void_p), ("k", ctypes.c_void_p), ("ldq", ctypes.c_longlong),
+                ("ldk", ctypes.c_longlong), ("M", ctypes.c_int), ("N", ctypes.c_int), ("D", ctypes.c_int),
+                ("inv_temperature", ctypes.c_float), ("target_offset", ctypes.c_longlong),
+                ("labels", ctypes.c_void_p), ("ld_labels", ctypes.c_longlong), ("tw", ctypes.c_void_p),
+                ("ld_tw", ctypes.c_longlong), ("row_scale", ctypes.c_void_p), ("row_w", ctypes.c_void_p),
+                ("loss_mode", ctypes.c_int), ("loss_scale", ctypes.c_float),
+                ("scratch", ctypes.c_void_p), ("lse", ctypes.c_void_p), ("loss", ctypes.c_void_p),
+                ("grad", ctypes.c_void_p), ("grad_scale", ctypes.c_float), ("panel", ctypes.c_int),
+                ("W", ctypes.c_void_p), ("ldw", ctypes.c_longlong), ("dq", ctypes.c_void_p),
+                ("dq32", ctypes.c_void_p), ("dk", ctypes.c_void_p), ("status", ctypes.c_void_p),
+                ("stream", ctypes.c_void_p)]
+
+
+_lib = None
+
+
+def _library():
+    global _lib
+    if _lib is None:
+        lib = nv.load()
+        lib.lb_infonce_scratch_floats.restype = ctypes.c_longlong
+        lib.lb_infonce_scratch_floats.argtypes = [ctypes.c_int, ctypes.c_int]
+        lib.lb_loss_fwd.argtypes = lib.lb_loss_bwd.argtypes = [ctypes.c_void_p]
+        _lib = lib
+    return _lib
+
+
+def _loss_struct(q, k, inv_t, target_offset=0, labels8=None, tw=None, row_scale=None, row_w=None,
+                 mode=0) -> LbLoss:
+    p = LbLoss()
+    p.q, p.k, p.ldq, p.ldk = q.data_ptr(), k.data_ptr(), q.stride(0), k.stride(0)
+    p.M, p.D = q.shape
+    p.N = k.shape[0]
+    p.inv_temperature, p.target_offset = inv_t, target_offset
+    if labels8 is not None:
+        p.labels, p.ld_labels = labels8.data_ptr(), labels8.stride(0)
+        p.row_scale, p.row_w, p.loss_mode = row_scale.data_ptr(), row_w.data_ptr(), mode
+        if tw is not None:
+            p.tw, p.ld_tw = tw.data_ptr(), tw.stride(0)
+    p.status, p.stream = nv.status_word(q.device).data_ptr(), nv.stream_ptr()
+    return p
+
+
+def _loss_fwd(p: LbLoss, q, loss_scale: float):
+    """``(loss [], lse [M])``."""
+    lib = _library()
+    scr = torch.empty(lib.lb_infonce_scratch_floats(p.M, (p.N + 7) // 8 * 8), dtype=torch.float32,
+                      device=q.device)
+    lse = torch.empty(p.M, dtype=torch.float32, device=q.device)
+    loss = torch.empty((), dtype=torch.float32, device=q.device)
+    p.scratch, p.lse, p.loss, p.loss_scale = scr.data_ptr(), lse.data_ptr(), loss.data_ptr(), loss_scale
+    nv.check_rc(lib.lb_loss_fwd(ctypes.addressof(p)), "lb_loss_fwd")
+    nv.count_launch(2)
+    return loss, lse
+
+
+def _loss_bwd(p: LbLoss, q, k, lse, grad, grad_scale: float, need_dq: bool, need_dk: bool):
+    """``(dq, dk)``, in panels of columns of at most ``PANEL_BYTES`` of probability gradient."""
+    step = panel_cols(p.M, p.N)
+    grad = grad if grad.dtype == torch.float32 else grad.float()
+    ldw = (step + 7) // 8 * 8
+    W = torch.empty(p.M, ldw, dtype=torch.bfloat16, device=q.device)
+    dq = torch.empty(p.M, p.D, dtype=torch.bfloat16 if step >= p.N else torch.float32,
+                     device=q.device) if need_dq else None
+    dk = torch.empty(p.N, p.D, dtype=torch.bfloat16, device=q.device) if need_dk else None
+    p.lse, p.grad, p.grad_scale = lse.data_ptr(), grad.data_ptr(), grad_scale
+    p.panel, p.W, p.ldw = step, W.data_ptr(), ldw
+    if need_dq:
+        p.dq = dq.data_ptr()
+        if step < p.N:
+            p.dq32 = dq.data_ptr()
+    p.dk = dk.data_ptr() if need_dk else None
+    nv.check_rc(_library().lb_loss_bwd(ctypes.addressof(p)), "lb_loss_bwd")
+    nv.count_launch((1 + need_dq + need_dk) * ((p.N + step - 1) // step))
+    if need_dq and step < p.N:
+        dq = dq.to(q.dtype)
+    return dq, dk
+
+
 class _FusedInfoNCE(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, inv_t, target_offset, denom):
-        M, D = q.shape
-        N = k.shape[0]
-        lib = nv.load()
-        lib.lb_infonce_scratch_floats.restype = nv.c_ll
-        scr = torch.empty(int(lib.lb_infonce_scratch_floats(nv.c_int(M), nv.c_int(N))),
-                          dtype=torch.float32, device=q.device)
-        lse = torch.empty(M, dtype=torch.float32, device=q.device)
-        loss_sum = torch.zeros(1, dtype=torch.float32, device=q.device)
-        rc = lib.lb_infonce_fwd(
-            nv.c_void_p(q.data_ptr()), nv.c_ll(q.stride(0)), nv.c_void_p(k.data_ptr()),
-            nv.c_ll(k.stride(0)), nv.c_int(M), nv.c_int(N), nv.c_int(D), nv.c_float(inv_t),
-            nv.c_ll(target_offset), nv.c_void_p(scr.data_ptr()), nv.c_void_p(lse.data_ptr()),
-            nv.c_void_p(loss_sum.data_ptr()), nv.c_void_p(nv.status_word(q.device).data_ptr()),
-            nv.c_void_p(nv.stream_ptr()))
-        nv.check_rc(rc, "lb_infonce_fwd")
-        nv.count_launch(2)
+        loss, lse = _loss_fwd(_loss_struct(q, k, inv_t, target_offset), q, 1.0 / denom)
         ctx.save_for_backward(q, k, lse)
         ctx.meta = (inv_t, target_offset, denom)
-        return loss_sum[0] / denom
+        return loss
 
     @staticmethod
     def backward(ctx, g):
         q, k, lse = ctx.saved_tensors
         inv_t, target_offset, denom = ctx.meta
-        M, D = q.shape
-        N = k.shape[0]
-        coef = (g.float() * (inv_t / denom)).reshape(1).contiguous()
-        lib = nv.load()
-        status = nv.status_word(q.device).data_ptr()
-
-        def pgrad(c0, c1, W):
-            # columns [c0, c1): the passages start at row c0, the target column moves by -c0
-            rc = lib.lb_infonce_pgrad(
-                nv.c_void_p(q.data_ptr()), nv.c_ll(q.stride(0)),
-                nv.c_void_p(k.data_ptr() + c0 * k.stride(0) * k.element_size()),
-                nv.c_ll(k.stride(0)), nv.c_int(M), nv.c_int(c1 - c0), nv.c_int(D), nv.c_float(inv_t),
-                nv.c_ll(target_offset - c0), nv.c_void_p(lse.data_ptr()),
-                nv.c_void_p(coef.data_ptr()), nv.c_void_p(W.data_ptr()), nv.c_ll(W.stride(0)),
-                nv.c_void_p(status), nv.c_void_p(nv.stream_ptr()))
-            nv.check_rc(rc, "lb_infonce_pgrad")
-            nv.count_launch()
-
-        dq, dk = streamed_loss_backward(pgrad, q, k, ctx.needs_input_grad[0],
-                                        ctx.needs_input_grad[1])
+        dq, dk = _loss_bwd(_loss_struct(q, k, inv_t, target_offset), q, k, lse, g, inv_t / denom,
+                           ctx.needs_input_grad[0], ctx.needs_input_grad[1])
         return dq, dk, None, None, None
 
 
@@ -166,76 +216,27 @@ def fused_infonce(q, k, temperature: float, target_offset: int = 0, denom: float
 
 # ------------------------------------------------------------------------------------------------
 # Streaming label-matrix loss (multi-positive NCE / soft-label cross-entropy): the [Q, K] scores
-# exist only as tensor-core accumulators; see lb_label_loss_fwd / lb_label_loss_pgrad.
+# exist only as tensor-core accumulators.
 # ------------------------------------------------------------------------------------------------
 class _FusedLabelLoss(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, labels8, tw, row_scale, row_w, inv_t):
-        M, D = q.shape
-        N = k.shape[0]
-        lib = nv.load()
-        lib.lb_infonce_scratch_floats.restype = nv.c_ll
-        scr = torch.empty(int(lib.lb_infonce_scratch_floats(nv.c_int(M), nv.c_int(N))),
-                          dtype=torch.float32, device=q.device)
-        lse = torch.empty(M, dtype=torch.float32, device=q.device)
-        loss_sum = torch.zeros(1, dtype=torch.float32, device=q.device)
-        rc = lib.lb_label_loss_fwd(
-            nv.c_void_p(q.data_ptr()), nv.c_ll(q.stride(0)), nv.c_void_p(k.data_ptr()),
-            nv.c_ll(k.stride(0)), nv.c_int(M), nv.c_int(N), nv.c_int(D), nv.c_float(inv_t),
-            nv.c_void_p(labels8.data_ptr()), nv.c_ll(labels8.stride(0)),
-            nv.c_void_p(tw.data_ptr() if tw is not None else None),
-            nv.c_ll(tw.stride(0) if tw is not None else 0), nv.c_void_p(row_scale.data_ptr()),
-            nv.c_void_p(row_w.data_ptr()), nv.c_int(0), nv.c_void_p(scr.data_ptr()),
-            nv.c_void_p(lse.data_ptr()),
-            nv.c_void_p(loss_sum.data_ptr()), nv.c_void_p(nv.status_word(q.device).data_ptr()),
-            nv.c_void_p(nv.stream_ptr()))
-        nv.check_rc(rc, "lb_label_loss_fwd")
-        nv.count_launch(2)
+        loss, lse = _loss_fwd(_loss_struct(q, k, inv_t, 0, labels8, tw, row_scale, row_w), q, 1.0)
         ctx.save_for_backward(q, k, lse, labels8, row_scale, row_w, *([tw] if tw is not None else []))
         ctx.inv_t = inv_t
-        return loss_sum[0]
+        return loss
 
     @staticmethod
     def backward(ctx, g):
         q, k, lse, labels8, row_scale, row_w, *rest = ctx.saved_tensors
-        tw = rest[0] if rest else None
-        inv_t = ctx.inv_t
-        M, D = q.shape
-        N = k.shape[0]
-        coef = (g.float() * inv_t).reshape(1).contiguous()
-        lib = nv.load()
-        status = nv.status_word(q.device).data_ptr()
-
-        def pgrad(c0, c1, W):
-            # panel starts are multiples of 256 columns: the int8 label rows stay 16-byte aligned
-            rc = lib.lb_label_loss_pgrad(
-                nv.c_void_p(q.data_ptr()), nv.c_ll(q.stride(0)),
-                nv.c_void_p(k.data_ptr() + c0 * k.stride(0) * k.element_size()),
-                nv.c_ll(k.stride(0)), nv.c_int(M), nv.c_int(c1 - c0), nv.c_int(D), nv.c_float(inv_t),
-                nv.c_void_p(labels8.data_ptr() + c0), nv.c_ll(labels8.stride(0)),
-                nv.c_void_p(tw.data_ptr() + 4 * c0 if tw is not None else None),
-                nv.c_ll(tw.stride(0) if tw is not None else 0), nv.c_void_p(row_scale.data_ptr()),
-                nv.c_void_p(row_w.data_ptr()), nv.c_int(0), nv.c_void_p(lse.data_ptr()),
-                nv.c_void_p(coef.data_ptr()), nv.c_void_p(W.data_ptr()), nv.c_ll(W.stride(0)),
-                nv.c_void_p(status), nv.c_void_p(nv.stream_ptr()))
-            nv.check_rc(rc, "lb_label_loss_pgrad")
-            nv.count_launch()
-
-        dq, dk = streamed_loss_backward(pgrad, q, k, ctx.needs_input_grad[0],
-                                        ctx.needs_input_grad[1])
+        p = _loss_struct(q, k, ctx.inv_t, 0, labels8, rest[0] if rest else None, row_scale, row_w)
+        dq, dk = _loss_bwd(p, q, k, lse, g, ctx.inv_t, ctx.needs_input_grad[0], ctx.needs_input_grad[1])
         return dq, dk, None, None, None, None, None
 
 
 def fused_label_loss_supported(q, k) -> bool:
     return (nv.use_native(q, k) and q.dtype == torch.bfloat16 and k.dtype == torch.bfloat16
             and q.shape[1] % 8 == 0 and q.shape[1] == k.shape[1])
-
-
-def _pad_rows8(k):
-    """Passages padded with zero rows to a multiple of 8 (the kernels' granularity); the label
-    padding marks those columns as ignored, and autograd drops their gradient rows."""
-    extra = (-k.shape[0]) % 8
-    return k if extra == 0 else torch.cat([k, k.new_zeros(extra, k.shape[1])], dim=0)
 
 
 _LABEL_KINDS = {torch.float32: 0, torch.int64: 1, torch.int32: 2, torch.int8: 3, torch.bool: 3}
@@ -246,16 +247,15 @@ def _label_prep(labels, kind: int, Kp: int):
     Q, K = labels.shape
     dev = labels.device
     lab8 = torch.empty(Q, Kp, dtype=torch.int8, device=dev)
-    stats = torch.empty(2, Q, dtype=torch.float32, device=dev)
-    counters = torch.zeros(2, dtype=torch.int32, device=dev)
+    stats = torch.empty(2 * Q + 2, dtype=torch.float32, device=dev)     # two words of counters behind
+    at = stats.data_ptr()
     rc = nv.load().lb_label_prep(
         nv.c_void_p(labels.data_ptr()), nv.c_int(kind), nv.c_ll(labels.stride(0)), nv.c_int(Q),
-        nv.c_int(K), nv.c_int(Kp), nv.c_void_p(lab8.data_ptr()), nv.c_void_p(stats.data_ptr()),
-        nv.c_void_p(stats.data_ptr() + 4 * Q), nv.c_void_p(counters.data_ptr()),
-        nv.c_void_p(nv.stream_ptr()))
+        nv.c_int(K), nv.c_int(Kp), nv.c_void_p(lab8.data_ptr()), nv.c_void_p(at),
+        nv.c_void_p(at + 4 * Q), nv.c_void_p(at + 8 * Q), nv.c_void_p(nv.stream_ptr()))
     nv.check_rc(rc, "lb_label_prep")
     nv.count_launch()
-    return lab8, stats[0], stats[1]
+    return lab8, stats[:Q], stats[Q:2 * Q]
 
 
 def fused_label_loss(q, k, labels, temperature: float, scores=None):
@@ -271,7 +271,7 @@ def fused_label_loss(q, k, labels, temperature: float, scores=None):
     if (scores is None and kind is not None and labels.device == dev and Q > 0 and K > 0
             and (K == 1 or labels.stride(1) == 1)):
         lab8, row_scale, row_w = _label_prep(labels, kind, Kp)
-        return _FusedLabelLoss.apply(q.contiguous(), _pad_rows8(k).contiguous(), lab8, None,
+        return _FusedLabelLoss.apply(q.contiguous(), k.contiguous(), lab8, None,
                                      row_scale, row_w, 1.0 / float(temperature))
     lab8 = torch.full((Q, Kp), -1, dtype=torch.int8, device=dev)
     lab8[:, :K].copy_(labels)           # converts in the copy: no fp32 [Q, K] temporary
@@ -292,7 +292,7 @@ def fused_label_loss(q, k, labels, temperature: float, scores=None):
         row_scale = 1.0 / n_pos.clamp(min=1).float()
     keepf = keep.float()
     row_w = keepf / keepf.sum().clamp(min=1.0)
-    return _FusedLabelLoss.apply(q.contiguous(), _pad_rows8(k).contiguous(), lab8, tw,
+    return _FusedLabelLoss.apply(q.contiguous(), k.contiguous(), lab8, tw,
                                  row_scale.contiguous(), row_w.contiguous(),
                                  1.0 / float(temperature))
 
@@ -323,27 +323,10 @@ class _FusedMpNce(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, q, k, labels8, pos_qi, pos_di, inv_t):
-        M, D = q.shape
-        N = k.shape[0]
-        dev = q.device
-        lib = nv.load()
-        lib.lb_infonce_scratch_floats.restype = nv.c_ll
-        scr = torch.empty(int(lib.lb_infonce_scratch_floats(nv.c_int(M), nv.c_int(N))),
-                          dtype=torch.float32, device=dev)
-        neg_lse = torch.empty(M, dtype=torch.float32, device=dev)
-        unused = torch.zeros(1, dtype=torch.float32, device=dev)
+        M, N, dev = q.shape[0], k.shape[0], q.device
         ones = torch.ones(M, dtype=torch.float32, device=dev)
         zeros = torch.zeros(M, dtype=torch.float32, device=dev)
-        rc = lib.lb_label_loss_fwd(
-            nv.c_void_p(q.data_ptr()), nv.c_ll(q.stride(0)), nv.c_void_p(k.data_ptr()),
-            nv.c_ll(k.stride(0)), nv.c_int(M), nv.c_int(N), nv.c_int(D), nv.c_float(inv_t),
-            nv.c_void_p(labels8.data_ptr()), nv.c_ll(labels8.stride(0)), nv.c_void_p(None),
-            nv.c_ll(0), nv.c_void_p(ones.data_ptr()), nv.c_void_p(zeros.data_ptr()), nv.c_int(1),
-            nv.c_void_p(scr.data_ptr()), nv.c_void_p(neg_lse.data_ptr()),
-            nv.c_void_p(unused.data_ptr()), nv.c_void_p(nv.status_word(dev).data_ptr()),
-            nv.c_void_p(nv.stream_ptr()))
-        nv.check_rc(rc, "lb_label_loss_fwd")
-        nv.count_launch(2)
+        _, neg_lse = _loss_fwd(_loss_struct(q, k, inv_t, 0, labels8, None, ones, zeros, mode=1), q, 1.0)
         lab = labels8[:, :N]
         num_pos = (lab > 0).sum(dim=1)
         has_neg = (lab == 0).any(dim=1)
@@ -366,28 +349,9 @@ class _FusedMpNce(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         q, k, labels8, neg_lse, aux, row_w = ctx.saved_tensors
-        inv_t = ctx.inv_t
-        M, D = q.shape
-        N = k.shape[0]
-        coef = (g.float() * inv_t).reshape(1).contiguous()
-        lib = nv.load()
-        status = nv.status_word(q.device).data_ptr()
-
-        def pgrad(c0, c1, W):
-            rc = lib.lb_label_loss_pgrad(
-                nv.c_void_p(q.data_ptr()), nv.c_ll(q.stride(0)),
-                nv.c_void_p(k.data_ptr() + c0 * k.stride(0) * k.element_size()),
-                nv.c_ll(k.stride(0)), nv.c_int(M), nv.c_int(c1 - c0), nv.c_int(D), nv.c_float(inv_t),
-                nv.c_void_p(labels8.data_ptr() + c0), nv.c_ll(labels8.stride(0)), nv.c_void_p(None),
-                nv.c_ll(0), nv.c_void_p(aux.data_ptr()), nv.c_void_p(row_w.data_ptr()), nv.c_int(1),
-                nv.c_void_p(neg_lse.data_ptr()), nv.c_void_p(coef.data_ptr()),
-                nv.c_void_p(W.data_ptr()), nv.c_ll(W.stride(0)), nv.c_void_p(status),
-                nv.c_void_p(nv.stream_ptr()))
-            nv.check_rc(rc, "lb_label_loss_pgrad")
-            nv.count_launch()
-
-        dq, dk = streamed_loss_backward(pgrad, q, k, ctx.needs_input_grad[0],
-                                        ctx.needs_input_grad[1])
+        p = _loss_struct(q, k, ctx.inv_t, 0, labels8, None, aux, row_w, mode=1)
+        dq, dk = _loss_bwd(p, q, k, neg_lse, g, ctx.inv_t, ctx.needs_input_grad[0],
+                           ctx.needs_input_grad[1])
         return dq, dk, None, None, None, None
 
 
@@ -408,7 +372,7 @@ def fused_dense_loss(q, k, labels, scale: float, loss_type: str = "multi", pos_q
         raise ValueError(f"unknown loss_type {loss_type!r}")
     lab8 = _pad_labels_int8(labels.to(q.device))
     K = labels.shape[1]
-    q, k = q.contiguous(), _pad_rows8(k).contiguous()
+    q, k = q.contiguous(), k.contiguous()
     if loss_type == "multi":
         if pos_qi is None or pos_di is None:
             pos_qi, pos_di = (lab8[:, :K] > 0).nonzero(as_tuple=True)

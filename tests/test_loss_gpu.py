@@ -270,3 +270,38 @@ def test_label_prep_is_the_elementwise_computation(dtype, Q, K):
         assert torch.equal(lab8, want)
         assert torch.equal(row_scale, 1.0 / n_pos.clamp(min=1).float())
         assert torch.equal(row_w, keep / keep.sum().clamp(min=1.0))
+
+
+@pytest.mark.parametrize("M,N", [(1, 8), (64, 256), (64, 264), (130, 1000), (1024, 1024), (1200, 2560)])
+@pytest.mark.parametrize("labels", [False, True])
+def test_losses_at_the_edges_of_their_tiles(M, N, labels):
+    """One column tile and several, of 128 and of 256 columns, against fp64; with labels also column
+    counts that are no multiple of anything. Probabilities (their gradient W) are rounded to bf16 once,
+    the gradients once more: 2^-8 of them in the 2-norm."""
+    from lset_b200.ops.loss import fused_label_loss
+
+    N += 3 if labels else 0
+    q, k = _emb(M, 256, 0).requires_grad_(), _emb(N, 256, 1).requires_grad_()
+    rows, pos = torch.arange(M, device="cuda"), torch.arange(M, device="cuda") * 7 % N
+    if labels:
+        lab = torch.zeros(M, N, device="cuda")
+        lab[rows, pos] = 1.0
+        lab[:, (pos[0] + 1) % N] = torch.where(lab[:, (pos[0] + 1) % N] > 0, 1.0, -1.0)   # ignored
+        loss = fused_label_loss(q, k, lab, 0.05)
+    else:
+        pos = rows + (N - M if N > M else 0)
+        if N < M:
+            pytest.skip("every query has a passage")
+        loss = fused_infonce(q, k, 0.05, int(pos[0]))
+    (loss * 3).backward()
+    nv.check_status()
+    s = q.detach().double() @ k.detach().double().t() / 0.05
+    if labels:
+        s = s.masked_fill(lab < 0, float("-inf"))
+    p = s.softmax(1)
+    want = (s.logsumexp(1) - s[rows, pos]).mean()
+    p[rows, pos] -= 1
+    p *= 3 / 0.05 / M
+    assert abs(loss.item() - want.item()) < 1e-4 * max(1.0, abs(want.item()))
+    for got, ref in ((q.grad, p @ k.detach().double()), (k.grad, p.t() @ q.detach().double())):
+        assert ((got.double() - ref).norm() / ref.norm()).item() < 2 ** -8
