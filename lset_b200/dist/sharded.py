@@ -11,7 +11,7 @@ compute parameters, fp32 gradient reduction and fp32 optimizer state) built for 
 * backward: as soon as a layer's backward has run, its gradient buffer is reduce-scattered (fp32,
   averaged) on a side stream, overlapping the rest of backward; with gradient accumulation the
   reduction only happens on the boundary micro-step;
-* step: global-norm clipping with the coefficient kept on the device, one fused AdamW kernel per
+* step: global-norm clipping with the coefficient kept on the device, one fused AdamW kernel over every
   group that also writes the new bf16 shard, then an all-gather of the shards that the next
   forward waits for per layer. With 180 GB per GPU the bf16 replica stays resident by default (no
   re-gather in backward).
@@ -30,6 +30,7 @@ reduce-scatter, the optimizer step and the parameter all-gather into two launche
 """
 from __future__ import annotations
 
+import ctypes
 import math
 from typing import Iterable, List, Optional, Sequence
 
@@ -42,6 +43,12 @@ from ..ops._grads import register_main_grad
 from ..ops.norm import scratch
 
 _ALIGN = 8  # elements; keeps every parameter 16-byte aligned in the bf16 buffer
+
+
+class LbOptGroup(ctypes.Structure):      # csrc/row/optim.h
+    _fields_ = [("p", ctypes.c_void_p), ("g", ctypes.c_void_p), ("m", ctypes.c_void_p),
+                ("v", ctypes.c_void_p), ("p_bf16", ctypes.c_void_p), ("n", ctypes.c_longlong),
+                ("slot", ctypes.c_int)]
 
 
 def _round_up(x: int, m: int) -> int:
@@ -589,13 +596,14 @@ class ParamStore:
 
     # ------------------------------------------------------------------ utilities
     def zero_grad(self) -> None:
+        bufs = [self.sumsq]
         for g in self.groups:
             if g.sharded:
                 g.has_grad = False          # the next reduction overwrites the shard
             else:
-                g.flat_grad.zero_()
+                bufs.append(g.flat_grad)
             g.reduced = False
-        self.sumsq.zero_()
+        torch._foreach_zero_(bufs)          # one launch for many buffers
 
     def memory_report(self) -> dict:
         """Bytes this rank holds for trainable parameters, gradients and optimizer state."""
@@ -699,6 +707,7 @@ class ShardedAdamW:
         # [clip coefficient, norm, skip flag]
         self._coef = torch.tensor([1.0, 0.0, 0.0], dtype=torch.float32, device=dev)
         self.state = {}  # torch.optim.Optimizer API expected by LR schedulers
+        self._list = self._listed = None
 
     # -- torch.optim-like surface ------------------------------------------------------------
     def zero_grad(self, set_to_none: bool = True) -> None:
@@ -712,32 +721,53 @@ class ShardedAdamW:
         """Global gradient norm of the last ``step`` (device scalar)."""
         return self._coef[1]
 
-    def _global_sumsq(self) -> None:
+    def _native_groups(self, groups):
+        """The buffers of ``groups`` as the kernels' list."""
+        tensors = [(g.master, g.grad_shard, g.exp_avg, g.exp_avg_sq,
+                    g.param_shard if g.sharded else g.flat_param) for g in groups]
+        at = [(g.lo, g.shard_numel, *(t.data_ptr() for t in ts)) for g, ts in zip(groups, tensors)]
+        if at != self._listed:
+            arr = (LbOptGroup * len(groups))()
+            for e, g, (lo, n, p, grad, m, v, low) in zip(arr, groups, at):
+                e.p, e.g, e.m, e.v, e.n = p, grad, m, v, n
+                if g.compute_dtype == torch.bfloat16:
+                    e.p_bf16 = low + (0 if g.sharded else 2 * lo)
+                e.slot = int(getattr(g, "tp_sharded", False))
+            self._list, self._listed = arr, at
+        return self._list
+
+    def _global_sumsq(self) -> bool:
         """Squared global gradient norm into ``self._sumsq``: shards of tensor-parallel parameters
         are summed over the tensor-parallel group, replicated ones counted once, then everything is
-        summed over the data-parallel shards."""
+        summed over the data-parallel shards. True if the clip coefficient was formed with it (a
+        single rank on the GPU)."""
         st = self.store
         native = st.device.type == "cuda"
         parts = self._parts
-        parts.zero_()
         if st.use_symm and not st.zero3:
             parts.copy_(st.sumsq)  # accumulated by the reduce kernels
+        elif native:
+            lib = nv.load()
+            groups = self._native_groups(st.groups)
+            scr = scratch("sumsq", lib.lb_sumsq_scratch_floats(nv.c_int(len(groups))), st.device)
+            rc = lib.lb_sumsq_groups(groups, nv.c_int(len(groups)), nv.c_void_p(scr.data_ptr()),
+                                     nv.c_void_p(parts.data_ptr()), nv.c_void_p(nv.stream_ptr()))
+            nv.check_rc(rc, "lb_sumsq_groups")
+            nv.count_launch(2)
         else:
+            parts.zero_()
             for g in st.groups:
-                slot = 1 if getattr(g, "tp_sharded", False) else 0
-                if native:
-                    lib = nv.load()
-                    scr = scratch("sumsq", lib.lb_sumsq_partial_rows(), st.device)
-                    rc = lib.lb_sumsq_f32(nv.c_void_p(g.grad_shard.data_ptr()),
-                                          nv.c_ll(g.grad_shard.numel()), nv.c_void_p(scr.data_ptr()),
-                                          nv.c_void_p(parts.data_ptr() + 4 * slot), nv.c_int(1),
-                                          nv.c_void_p(nv.stream_ptr()))
-                    nv.check_rc(rc, "lb_sumsq_f32")
-                    nv.count_launch(2)
-                else:
-                    gs = g.grad_shard.reshape(-1).float()
-                    parts[slot] += torch.dot(gs, gs)       # one pass, no temporary
+                gs = g.grad_shard.reshape(-1).float()
+                parts[int(getattr(g, "tp_sharded", False))] += torch.dot(gs, gs)   # no temporary
         tp_on = st.tp_group is not None and dist.get_world_size(st.tp_group) > 1
+        if native and not tp_on and st.world == 1:
+            rc = nv.load().lb_clip_coef_local(
+                nv.c_void_p(parts.data_ptr()), nv.c_void_p(nv.status_word(st.device).data_ptr()),
+                nv.c_float(self.grad_clip), nv.c_void_p(self._sumsq.data_ptr()),
+                nv.c_void_p(self._coef.data_ptr()), nv.c_void_p(nv.stream_ptr()))
+            nv.check_rc(rc, "lb_clip_coef_local")
+            nv.count_launch()
+            return True
         if tp_on:
             dist.all_reduce(parts[1:2], op=dist.ReduceOp.SUM, group=st.tp_group)
         torch.sum(parts, dim=0, keepdim=True, out=self._sumsq[0:1])
@@ -749,6 +779,7 @@ class ShardedAdamW:
                 dist.all_reduce(self._sumsq[1:2], op=dist.ReduceOp.SUM, group=st.tp_group)
         if st.world > 1:
             dist.all_reduce(self._sumsq, op=dist.ReduceOp.SUM, group=st.dp_group)
+        return False
 
     @torch.no_grad()
     def step(self) -> None:
@@ -759,9 +790,11 @@ class ShardedAdamW:
         lr, (b1, b2), eps, wd = pg["lr"], pg["betas"], pg["eps"], pg["weight_decay"]
         bc1 = 1.0 - b1 ** self.step_count
         bc2s = math.sqrt(1.0 - b2 ** self.step_count)
-        self._global_sumsq()
+        have_coef = self._global_sumsq()
         native = st.device.type == "cuda"
-        if native:
+        if have_coef:
+            pass
+        elif native:
             rc = nv.load().lb_clip_coef(nv.c_void_p(self._sumsq.data_ptr()), nv.c_float(self.grad_clip),
                                         nv.c_void_p(self._coef.data_ptr()),
                                         nv.c_void_p(self._sumsq.data_ptr() + 4),
@@ -773,6 +806,15 @@ class ShardedAdamW:
             self._coef[1] = norm[0]
             self._coef[0] = torch.clamp(self.grad_clip / (norm[0] + 1e-6), max=1.0) \
                 if self.grad_clip > 0 else 1.0
+        plain = [g for g in st.groups if not (st.use_symm and not g.sharded)] if native else []
+        if plain:
+            groups = self._native_groups(plain)
+            rc = nv.load().lb_adamw_groups(
+                groups, nv.c_int(len(groups)), nv.c_float(lr), nv.c_float(b1), nv.c_float(b2),
+                nv.c_float(eps), nv.c_float(wd), nv.c_float(bc1), nv.c_float(bc2s), nv.c_float(1.0),
+                nv.c_void_p(self._coef.data_ptr()), nv.c_int(0), nv.c_void_p(nv.stream_ptr()))
+            nv.check_rc(rc, "lb_adamw_groups")
+            nv.count_launch()
         for g in st.groups:
             pshard = g.param_shard if g.sharded else g.flat_param[g.lo:g.hi]
             if st.use_symm and not g.sharded:
@@ -786,16 +828,6 @@ class ShardedAdamW:
                 nv.check_rc(rc, "lb_adamw_push")
                 nv.count_launch()
             elif native:
-                rc = nv.load().lb_adamw_f32(
-                    nv.c_void_p(g.master.data_ptr()), nv.c_void_p(g.grad_shard.data_ptr()),
-                    nv.c_void_p(g.exp_avg.data_ptr()), nv.c_void_p(g.exp_avg_sq.data_ptr()),
-                    nv.c_void_p(pshard.data_ptr() if g.compute_dtype == torch.bfloat16 else 0),
-                    nv.c_ll(g.shard_numel), nv.c_float(lr), nv.c_float(b1), nv.c_float(b2),
-                    nv.c_float(eps), nv.c_float(wd), nv.c_float(bc1), nv.c_float(bc2s),
-                    nv.c_float(1.0), nv.c_void_p(self._coef.data_ptr()), nv.c_int(0),
-                    nv.c_void_p(nv.stream_ptr()))
-                nv.check_rc(rc, "lb_adamw_f32")
-                nv.count_launch()
                 if g.compute_dtype != torch.bfloat16:
                     pshard.copy_(g.master)
             elif _HAS_FUSED_CPU_ADAMW and g.master.dtype == torch.float32:
