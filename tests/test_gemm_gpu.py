@@ -53,6 +53,15 @@ def test_nt(M, N, K, bn):
     _check(c, a.float() @ b.float().t())
 
 
+@pytest.mark.parametrize("M", [40, 4096, 4361])
+@pytest.mark.parametrize("b_mn", [False, True])
+def test_wide_products_visit_every_tile(M, b_mn):
+    """More than 16 columns of tiles and a B of more than 32 MB: bands of 16 rows of tiles, less than one
+    of them, one, and one with two rows left."""
+    a, b = _rand(M, 4096), _rand(4096, 4360) if b_mn else _rand(4360, 4096)
+    _check(matmul_abt(a, b, b_mn=b_mn), a.float() @ (b.float() if b_mn else b.float().t()))
+
+
 @pytest.mark.parametrize("M,N,K", SHAPES)
 def test_nn_b_mn_major(M, N, K):
     a, b = _rand(M, K), _rand(K, N)
