@@ -74,8 +74,12 @@ __global__ void __launch_bounds__(256)
     long long tok = 0;
     int h = 0;
     if (u < units) {
-      tok = u / Hq;
-      h = int(u % Hq);
+      if (units <= 0xffffffffll) {   // (a 64-bit division is a third of the loop's instructions)
+        tok = unsigned(u) / unsigned(Hq);
+      } else {
+        tok = u / Hq;
+      }
+      h = int(u - tok * Hq);
       float x[8], y[8];
       unpack8(ld16(dO + tok * lddo + h * HD + l * 8), x);
       unpack8(ld16(O + tok * ldo + h * HD + l * 8), y);
@@ -753,7 +757,8 @@ int launch_bwd(const void* dO, long long lddo, const void* q, long long ldq, con
     a.plan = plan_q;
     a.capacity = cap_q;
     const int rc = [&] {
-      return launch_pdl(attn_delta_kernel<HD>, dim3(int(grid)), dim3(256), 0, st, pdl_enabled(), 1,
+      return launch_pdl(attn_delta_kernel<HD>, dim3(int(grid)), dim3(256), 0, st,
+                        pdl_enabled(4LL * a.T * a.Hq * HD), 1,
                         (const bf16*)dO, lddo, (const bf16*)o, ldo, delta, a);
     }();
     if (rc) return rc;

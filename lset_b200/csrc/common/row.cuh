@@ -37,6 +37,53 @@ __device__ __forceinline__ float bf16_round(float x) {
 __device__ __forceinline__ uint4 ld16(const void* p) { return *reinterpret_cast<const uint4*>(p); }
 __device__ __forceinline__ void st16(void* p, const uint4& v) { *reinterpret_cast<uint4*>(p) = v; }
 
+// Two fp32 values in a 64-bit register pair: one instruction for both, with the roundings of two.
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 f2_of(float lo, float hi) {
+  f2 v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+  return v;
+}
+__device__ __forceinline__ float2 f2_get(f2 v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
+}
+__device__ __forceinline__ f2 f2_add(f2 a, f2 b) {
+  f2 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f2 f2_mul(f2 a, f2 b) {
+  f2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
+  f2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+// the two bf16 of a word
+__device__ __forceinline__ f2 f2_bf16(uint32_t w) {
+  return f2_of(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+}
+__device__ __forceinline__ uint32_t bf16_of_f2(f2 v) {
+  const float2 f = f2_get(v);
+  const __nv_bfloat162 h = __floats2bfloat162_rn(f.x, f.y);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+__device__ __forceinline__ f2 f2_bf16_round(f2 v) { return f2_bf16(bf16_of_f2(v)); }
+__device__ __forceinline__ void unpack8(const uint4& q, f2 (&f)[4]) {
+  f[0] = f2_bf16(q.x);
+  f[1] = f2_bf16(q.y);
+  f[2] = f2_bf16(q.z);
+  f[3] = f2_bf16(q.w);
+}
+__device__ __forceinline__ uint4 pack8(const f2 (&f)[4]) {
+  return make_uint4(bf16_of_f2(f[0]), bf16_of_f2(f[1]), bf16_of_f2(f[2]), bf16_of_f2(f[3]));
+}
+
 // Streaming variants: data touched once should not displace what later kernels reuse from L2.
 __device__ __forceinline__ uint4 ld16_stream(const void* p) {
   uint4 v;

@@ -166,37 +166,76 @@ __global__ void __launch_bounds__(kRowThreads)
   }
 }
 
-// Backward keeps x and dy as packed bf16 in registers (unpacked twice) and the weights in shared
-// memory, so that only the fp32 dW accumulators are long-lived: two CTAs fit per SM.
+// Sum over the TPR threads of a row, one barrier a call among those threads only: `sred` alternates between
+// two slots from call to call. The values and the order of row_sum.
+template <int TPR>
+__device__ __forceinline__ float row_sum_alt(float v, float (&sred)[2][8], int slot) {
+#pragma unroll
+  for (int o = (TPR < 32 ? TPR : 32) / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if constexpr (TPR > 32) {
+    const int warp = threadIdx.x >> 5;
+    if ((threadIdx.x & 31) == 0) sred[slot][warp] = v;
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + int(threadIdx.x) / TPR), "n"(TPR) : "memory");
+    constexpr int W = TPR / 32;
+    const int w0 = (warp / W) * W;
+    float t = 0.f;
+#pragma unroll
+    for (int i = 0; i < W; ++i) t += sred[slot][w0 + i];
+    v = t;
+  }
+  return v;
+}
+
+// Bound by memory where enough rows are in flight. x and dy stay packed in registers (unpacked twice) and
+// the weights in shared memory, so that only the dW accumulators live as long as the CTA: 64 registers, four
+// CTAs a SM, one wave of them. Four columns of a thread are next to its neighbour's in shared memory (eight in
+// a row cost every access twice its banks); two columns an instruction; one barrier a row.
+// Measured before (three CTAs, two waves) / now (us, L2 flushed): 22627 x 1024 53 / 45, 33280 x 4096 201 / 180,
+// 21000 x 2560 107 / 92, 5000 x 8192 104 / 84. (A warp a row, with no barrier, needs twice the
+// registers: 59 at 22627 x 1024.)
 template <int TPR, int NV>
-__global__ void __launch_bounds__(kRowThreads, 3)
+constexpr int rms_bwd_smem(int H) { return (H + 8 * TPR * NV) * int(sizeof(float)); }
+
+template <int TPR, int NV>
+__global__ void __launch_bounds__(kRowThreads, NV > 2 ? 2 : 4)
     rms_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ dres,
                    const bf16* __restrict__ xin, const bf16* __restrict__ w,
                    const float* __restrict__ rstd_in, bf16* __restrict__ dx,
                    float* __restrict__ dw_partial, int N, int H, float w_off) {
-  __shared__ float sred[8];
-  extern __shared__ float sdw[];  // [H] dW accumulator of the CTA, then [H] weights
+  __shared__ float sred[2][8];
+  extern __shared__ float sdw[];  // [H] dW accumulator of the CTA, then [2 NV][TPR][4] weights
   float* sw = sdw + H;
   constexpr int ROWS = kRowThreads / TPR;
   const int t = threadIdx.x % TPR;
   const int r = threadIdx.x / TPR;
-  float dwacc[NV][8];
+  f2 dwacc[NV][4];
 #pragma unroll
   for (int v = 0; v < NV; ++v)
 #pragma unroll
-    for (int i = 0; i < 8; ++i) dwacc[v][i] = 0.f;
+    for (int i = 0; i < 4; ++i) dwacc[v][i] = 0ull;
   for (int i = threadIdx.x; i < H; i += kRowThreads) {
+    const int col = i % 8, at = i / 8;   // column `col` of thread at % TPR in vector at / TPR
     sdw[i] = 0.f;
-    sw[i] = __bfloat162float(w[i]) + w_off;
+    sw[((at / TPR * 2 + col / 4) * TPR + at % TPR) * 4 + col % 4] = __bfloat162float(w[i]) + w_off;
   }
   __syncthreads();
   pdl_wait();
   pdl_trigger();
 
+  auto load_w = [&](int v, f2 (&wl)[4]) {
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const float4 q = *reinterpret_cast<const float4*>(sw + ((v * 2 + k) * TPR + t) * 4);
+      wl[2 * k] = f2_of(q.x, q.y);
+      wl[2 * k + 1] = f2_of(q.z, q.w);
+    }
+  };
+  int slot = 0;
   for (long long row0 = 1LL * blockIdx.x * ROWS; row0 < N; row0 += 1LL * gridDim.x * ROWS) {
     const long long row = row0 + r;
     const bool valid = row < N;
     const float rstd = valid ? rstd_in[row] : 0.f;
+    const f2 rstd2 = f2_of(rstd, rstd);
     uint4 xq[NV], gq[NV], rq[NV];
     float dot = 0.f;
     // every load of the row is requested before the first use
@@ -213,38 +252,40 @@ __global__ void __launch_bounds__(kRowThreads, 3)
     for (int v = 0; v < NV; ++v) {
       const int idx = (v * TPR + t) * 8;
       if (valid && idx < H) {
-        float xh[8], g[8];
+        f2 g[4], xh[4];
         unpack8(xq[v], xh);
         unpack8(gq[v], g);
-        const float4 w0 = *reinterpret_cast<const float4*>(sw + idx);
-        const float4 w1 = *reinterpret_cast<const float4*>(sw + idx + 4);
-        const float wl[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+        f2 wl[4];
+        load_w(v, wl);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          xh[i] *= rstd;
-          dot += g[i] * wl[i] * xh[i];
-          dwacc[v][i] += g[i] * bf16_round(xh[i]);
+        for (int i = 0; i < 4; ++i) {
+          xh[i] = f2_mul(xh[i], rstd2);
+          const float2 a = f2_get(f2_mul(g[i], wl[i])), b = f2_get(xh[i]);
+          dot = fmaf(a.x, b.x, dot);
+          dot = fmaf(a.y, b.y, dot);
+          dwacc[v][i] = f2_fma(g[i], f2_bf16_round(xh[i]), dwacc[v][i]);
         }
       }
     }
-    dot = row_sum<TPR>(dot, sred) / float(H);
+    dot = row_sum_alt<TPR>(dot, sred, slot) / float(H);
+    slot ^= 1;
+    const f2 minus_dot = f2_of(-dot, -dot);
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
       const int idx = (v * TPR + t) * 8;
       if (valid && idx < H) {
-        float xh[8], g[8], o[8];
-        unpack8(xq[v], xh);
+        f2 g[4], o[4], wl[4];
+        load_w(v, wl);
         unpack8(gq[v], g);
-        const float4 w0 = *reinterpret_cast<const float4*>(sw + idx);
-        const float4 w1 = *reinterpret_cast<const float4*>(sw + idx + 4);
-        const float wl[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+        unpack8(xq[v], o);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) o[i] = rstd * (g[i] * wl[i] - xh[i] * rstd * dot);
+        for (int i = 0; i < 4; ++i)
+          o[i] = f2_mul(rstd2, f2_fma(g[i], wl[i], f2_mul(f2_mul(o[i], rstd2), minus_dot)));
         if (dres != nullptr) {
-          float dr[8];
+          f2 dr[4];
           unpack8(rq[v], dr);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) o[i] += dr[i];
+          for (int i = 0; i < 4; ++i) o[i] = f2_add(o[i], dr[i]);
         }
         st16(dx + row * H + idx, pack8(o));
       }
@@ -256,7 +297,11 @@ __global__ void __launch_bounds__(kRowThreads, 3)
     const int idx = (v * TPR + t) * 8;
     if (idx < H) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) atomicAdd(&sdw[idx + i], dwacc[v][i]);
+      for (int i = 0; i < 4; ++i) {
+        const float2 a = f2_get(dwacc[v][i]);
+        atomicAdd(&sdw[idx + 2 * i], a.x);
+        atomicAdd(&sdw[idx + 2 * i + 1], a.y);
+      }
     }
   }
   __syncthreads();
@@ -489,9 +534,12 @@ int launch_colsum(const float* partial, int P, int C, void* out, int out_fp32, i
   return launch_colsums(&job, 1, out_fp32, accumulate, st);
 }
 
-int bwd_grid(int N, int rows_per_cta) {
+// CTAs of the backward kernels for each SM: one wave of rms_bwd_kernel, two of ln_bwd_kernel.
+constexpr int kRmsBwdPerSm = 4, kLayerNormBwdPerSm = 6;
+
+int bwd_grid(int N, int rows_per_cta, int per_sm) {
   const int need = (N + rows_per_cta - 1) / rows_per_cta;
-  const int cap = row_num_sms() * 6;  // two waves at three CTAs per SM
+  const int cap = row_num_sms() * per_sm;
   return need < cap ? (need > 0 ? need : 1) : cap;
 }
 
@@ -515,7 +563,7 @@ extern "C" int lb_rms_norm_fwd(const void* x, const void* res_in, const void* w,
     const int grid = (N + ROWS - 1) / ROWS;
     const bool aligned = (reinterpret_cast<uintptr_t>(w) & 15u) == 0;
     return launch_pdl(aligned ? rms_fwd_kernel<TPR, NV, true> : rms_fwd_kernel<TPR, NV, false>,
-                      dim3(grid), dim3(kRowThreads), 0, st, pdl_enabled(), 1, (const bf16*)x,
+                      dim3(grid), dim3(kRowThreads), 0, st, pdl_enabled((res_in != nullptr ? 8LL : 4LL) * N * H), 1, (const bf16*)x,
                       (const bf16*)res_in, (const bf16*)w, (bf16*)y, (bf16*)res_out, rstd, N, H, eps,
                       w_off);
   });
@@ -551,13 +599,14 @@ extern "C" int lb_rms_norm_bwd(const void* dy, const void* dres, const void* xin
   int grid = 1;
   LB_ROW_DISPATCH_NARROW(H, {
     constexpr int ROWS = kRowThreads / TPR;
-    grid = bwd_grid(N, ROWS);
-    if (2 * H * sizeof(float) > 48 * 1024)  // wide rows: opt in above the 48 KB default
+    grid = bwd_grid(N, ROWS, kRmsBwdPerSm);
+    constexpr auto smem = rms_bwd_smem<TPR, NV>;
+    if (smem(H) > 48 * 1024)  // wide rows: opt in above the 48 KB default
       cudaFuncSetAttribute(rms_bwd_kernel<TPR, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           2 * H * (int)sizeof(float));
+                           smem(8 * TPR * NV));
     const int rc = [&] {
       return launch_pdl(rms_bwd_kernel<TPR, NV>, dim3(grid), dim3(kRowThreads),
-                        2 * H * sizeof(float), st, pdl_enabled(), 1, (const bf16*)dy,
+                        smem(H), st, pdl_enabled((dres != nullptr ? 8LL : 6LL) * N * H), 1, (const bf16*)dy,
                         (const bf16*)dres, (const bf16*)xin, (const bf16*)w, rstd, (bf16*)dx,
                         scratch, N, H, w_off);
     }();
@@ -569,9 +618,14 @@ extern "C" int lb_rms_norm_bwd(const void* dy, const void* dres, const void* xin
 }
 
 // Partial rows that the backward kernels leave in their scratch for N rows of width H.
-extern "C" int lb_norm_bwd_rows(int N, int H) {
+extern "C" int lb_rms_bwd_rows(int N, int H) {
   if (N <= 0 || H <= 0) return 0;
-  LB_ROW_DISPATCH_NARROW(H, { return bwd_grid(N, kRowThreads / TPR); });
+  LB_ROW_DISPATCH_NARROW(H, { return bwd_grid(N, kRowThreads / TPR, kRmsBwdPerSm); });
+  return 0;
+}
+extern "C" int lb_layer_norm_bwd_rows(int N, int H) {
+  if (N <= 0 || H <= 0) return 0;
+  LB_ROW_DISPATCH_NARROW(H, { return bwd_grid(N, kRowThreads / TPR, kLayerNormBwdPerSm); });
   return 0;
 }
 
@@ -584,7 +638,7 @@ extern "C" int lb_layer_norm_fwd(const void* x, const void* res_in, const void* 
   LB_ROW_DISPATCH(H, {
     constexpr int ROWS = kRowThreads / TPR;
     const int grid = (N + ROWS - 1) / ROWS;
-    return launch_pdl(ln_fwd_kernel<TPR, NV>, dim3(grid), dim3(kRowThreads), 0, st, pdl_enabled(),
+    return launch_pdl(ln_fwd_kernel<TPR, NV>, dim3(grid), dim3(kRowThreads), 0, st, pdl_enabled((res_in != nullptr ? 8LL : 4LL) * N * H),
                       1, (const bf16*)x, (const bf16*)res_in, (const bf16*)w, (const bf16*)b,
                       (bf16*)y, (bf16*)res_out, mean, rstd, N, H, eps);
   });
@@ -601,13 +655,13 @@ extern "C" int lb_layer_norm_bwd(const void* dy, const void* dres, const void* x
   int grid = 1;
   LB_ROW_DISPATCH_NARROW(H, {
     constexpr int ROWS = kRowThreads / TPR;
-    grid = bwd_grid(N, ROWS);
+    grid = bwd_grid(N, ROWS, kLayerNormBwdPerSm);
     if (2 * H * sizeof(float) > 48 * 1024)
       cudaFuncSetAttribute(ln_bwd_kernel<TPR, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            2 * H * (int)sizeof(float));
     const int rc = [&] {
       return launch_pdl(ln_bwd_kernel<TPR, NV>, dim3(grid), dim3(kRowThreads),
-                        2 * H * sizeof(float), st, pdl_enabled(), 1, (const bf16*)dy,
+                        2 * H * sizeof(float), st, pdl_enabled((dres != nullptr ? 8LL : 6LL) * N * H), 1, (const bf16*)dy,
                         (const bf16*)dres, (const bf16*)xin, (const bf16*)w, mean, rstd, (bf16*)dx,
                         scratch, N, H);
     }();
@@ -696,12 +750,13 @@ extern "C" int lb_rms_norm_bwd_noalloc(const void* dy, const void* dres, const v
   int grid = 1;
   LB_ROW_DISPATCH_NARROW(H, {
     constexpr int ROWS = kRowThreads / TPR;
-    grid = bwd_grid(N, ROWS);
+    grid = bwd_grid(N, ROWS, kRmsBwdPerSm);
     if (grid > LB_NOALLOC_MAX_PARTIAL_ROWS) grid = LB_NOALLOC_MAX_PARTIAL_ROWS;
-    if (2 * H * sizeof(float) > 48 * 1024)  // wide rows: opt in above the 48 KB default
+    constexpr auto smem = rms_bwd_smem<TPR, NV>;
+    if (smem(H) > 48 * 1024)  // wide rows: opt in above the 48 KB default
       cudaFuncSetAttribute(rms_bwd_kernel<TPR, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           2 * H * (int)sizeof(float));
-    rms_bwd_kernel<TPR, NV><<<grid, kRowThreads, 2 * H * sizeof(float), st>>>(
+                           smem(8 * TPR * NV));
+    rms_bwd_kernel<TPR, NV><<<grid, kRowThreads, smem(H), st>>>(
         (const bf16*)dy, (const bf16*)dres, (const bf16*)xin, (const bf16*)w, rstd, (bf16*)dx,
         scratch, N, H, w_off);
   });

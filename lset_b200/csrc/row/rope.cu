@@ -45,6 +45,38 @@ __device__ __forceinline__ int token_pos(const RopeArgs& a, long long tok) {
                    : reinterpret_cast<const int*>(a.pos)[tok];
 }
 
+// Where weight i of q's and k's 2 * HD is in shared memory: [q or k][half][4 of 8][lane][4], so that the
+// lanes of a head read neighbouring 16 bytes (eight floats in a row a lane cost twice the banks).
+template <int HD>
+__device__ __forceinline__ int weight_at(int i) {
+  constexpr int HALF = HD / 2, LPH = HD / 16;
+  const int e = i % HD, c = e % HALF;
+  return i - e + ((e / HALF * 2 + c % 8 / 4) * LPH + c / 8) * 4 + c % 4;
+}
+
+// The angles of a position (or zeros) for the eight elements from e0.
+template <int HALF>
+__device__ __forceinline__ void load_angles(const float* cos, const float* sin, int pos, int e0, f2 (&c)[4],
+                                            f2 (&s)[4]) {
+  float4 v[4] = {};
+  if (pos >= 0) {
+    const float4* cp = reinterpret_cast<const float4*>(cos + 1LL * pos * HALF + e0);
+    const float4* sp = reinterpret_cast<const float4*>(sin + 1LL * pos * HALF + e0);
+    v[0] = cp[0];
+    v[1] = cp[1];
+    v[2] = sp[0];
+    v[3] = sp[1];
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    c[2 * i] = f2_of(v[i].x, v[i].y);
+    c[2 * i + 1] = f2_of(v[i].z, v[i].w);
+    s[2 * i] = f2_of(v[2 + i].x, v[2 + i].y);
+    s[2 * i + 1] = f2_of(v[2 + i].z, v[2 + i].w);
+  }
+}
+__device__ __forceinline__ f2 f2_neg(f2 v) { return v ^ 0x8000000080000000ull; }
+
 // A group of HD/16 lanes owns one token at a time (or, with few tokens, a part of its heads, see
 // rope_parts) and walks over its heads UB at a time: the cos/sin
 // row and the position are fetched once per token, and the 16-byte loads of the next UB heads are
@@ -52,20 +84,23 @@ __device__ __forceinline__ int token_pos(const RopeArgs& a, long long tok) {
 // elements of either half of a head, the two partners of eight rotations, so that nothing but the sum of
 // squares crosses lanes. (With a lane per eight neighbouring elements, every element came over once by
 // shuffle, and the shuffles bound the kernel; the sum of squares is added up in the same order.)
-// Measured (us, tokens x heads of 128, L2 flushed): 22627 x 24 72 -> 64, 40280 x 24 117 -> 94, 33280 x 40
-// 156 -> 132 (65 % -> 81 % of copy bandwidth at 40280); 22627 x 40 heads of 64 59 -> 51.
+// Measured (us, tokens x heads of 128, L2 flushed): 22627 x 24 72 -> 62, 40280 x 24 117 -> 94, 33280 x 40
+// 156 -> 132 (65 % -> 81 % of copy bandwidth at 40280); 22627 x 40 heads of 64 59 -> 55. Two elements an
+// instruction, and weights without bank conflicts, change nothing there, but among GEMMs, which take the clock
+// down: 40280 x 24 116 -> 108, 22627 x 24 77 -> 73.
 template <int HD>
 __global__ void __launch_bounds__(kRowThreads, 3) qk_rope_fwd_kernel(RopeArgs a) {
   constexpr int LPH = HD / 16;  // lanes per head
   constexpr int TPB = kRowThreads / LPH;
   constexpr int UB = 2;
   constexpr int HALF = HD / 2;
-  __shared__ float swt[2 * HD];  // q then k norm weights (+ offset)
+  __shared__ __align__(16) float swt[2 * HD];  // q then k norm weights (+ offset): [half][4 of 8][lane][4]
   const int l = threadIdx.x % LPH;
   const int g = threadIdx.x / LPH;
   const int e0 = l * 8;
   for (int i = threadIdx.x; i < 2 * HD; i += kRowThreads)
-    swt[i] = a.do_norm ? __bfloat162float(i < HD ? a.qw[i] : a.kw[i - HD]) + a.w_off : 1.f;
+    swt[weight_at<HD>(i)] =
+        a.do_norm ? __bfloat162float(i < HD ? a.qw[i] : a.kw[i - HD]) + a.w_off : 1.f;
   __syncthreads();
   pdl_wait();
   pdl_trigger();
@@ -94,18 +129,8 @@ __global__ void __launch_bounds__(kRowThreads, 3) qk_rope_fwd_kernel(RopeArgs a)
     };
     uint4 cur[UB][2], nxt[UB][2];
     load_batch(h_first, cur);
-    float c[8], s[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) c[i] = s[i] = 0.f;
-    if (valid) {
-      const int pos = token_pos(a, tok);
-      const float4* cp = reinterpret_cast<const float4*>(a.cos + 1LL * pos * HALF + e0);
-      const float4* sp = reinterpret_cast<const float4*>(a.sin + 1LL * pos * HALF + e0);
-      *reinterpret_cast<float4*>(c) = cp[0];
-      *reinterpret_cast<float4*>(c + 4) = cp[1];
-      *reinterpret_cast<float4*>(s) = sp[0];
-      *reinterpret_cast<float4*>(s + 4) = sp[1];
-    }
+    f2 c[4], s[4];
+    load_angles<HALF>(a.cos, a.sin, valid ? token_pos(a, tok) : -1, e0, c, s);
     for (int b0 = 0; b0 < a.part_heads; b0 += UB) {   // uniform over the CTA
       const int h0 = h_first + b0;
       if (b0 + UB < a.part_heads) load_batch(h0 + UB, nxt);
@@ -114,16 +139,22 @@ __global__ void __launch_bounds__(kRowThreads, 3) qk_rope_fwd_kernel(RopeArgs a)
         const int h = h0 + j;
         const bool live = valid && h < heads;
         const bool is_q = h < a.Hq;
-        float x[2][8];
-        unpack8(cur[j][0], x[0]);
-        unpack8(cur[j][1], x[1]);
+        f2 x[2][4];
         if (a.do_norm) {
-          float ss[2] = {0.f, 0.f};
+          // element i of either half in one pair: two sums of squares, each in the order of its half
+          const uint32_t lo[4] = {cur[j][0].x, cur[j][0].y, cur[j][0].z, cur[j][0].w};
+          const uint32_t hi[4] = {cur[j][1].x, cur[j][1].y, cur[j][1].z, cur[j][1].w};
+          f2 p[8], ss = 0ull;
 #pragma unroll
-          for (int k = 0; k < 2; ++k)
+          for (int i = 0; i < 4; ++i) {
+            p[2 * i] = f2_of(__uint_as_float(lo[i] << 16), __uint_as_float(hi[i] << 16));
+            p[2 * i + 1] =
+                f2_of(__uint_as_float(lo[i] & 0xffff0000u), __uint_as_float(hi[i] & 0xffff0000u));
+          }
 #pragma unroll
-            for (int i = 0; i < 8; ++i) ss[k] += x[k][i] * x[k][i];
-          float sum = ss[0] + ss[1];
+          for (int i = 0; i < 8; ++i) ss = f2_fma(p[i], p[i], ss);
+          const float2 halves = f2_get(ss);
+          float sum = halves.x + halves.y;
 #pragma unroll
           for (int o = LPH / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
           const float rstd = rsqrtf(sum / float(HD) + a.eps);
@@ -131,21 +162,29 @@ __global__ void __launch_bounds__(kRowThreads, 3) qk_rope_fwd_kernel(RopeArgs a)
             if (is_q) a.q_rstd[tok * a.Hq + h] = rstd;
             else a.k_rstd[tok * a.Hk + (h - a.Hq)] = rstd;
           }
+          const f2 r2 = f2_of(rstd, rstd);
+          const float* wt = swt + (is_q ? 0 : HD) + l * 4;
 #pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            const float* wt = swt + (is_q ? 0 : HD) + k * HALF + e0;
-            const float4 w0 = *reinterpret_cast<const float4*>(wt);
-            const float4 w1 = *reinterpret_cast<const float4*>(wt + 4);
-            const float wl[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+          for (int q = 0; q < 2; ++q) {   // columns 4q .. 4q + 3 of either half
+            float2 y[4];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) x[k][i] = bf16_round(x[k][i] * rstd) * wl[i];
+            for (int i = 0; i < 4; ++i) y[i] = f2_get(f2_mul(p[4 * q + i], r2));
+            const float4 w0 = *reinterpret_cast<const float4*>(wt + q * LPH * 4);
+            const float4 w1 = *reinterpret_cast<const float4*>(wt + (2 + q) * LPH * 4);
+            x[0][2 * q] = f2_mul(f2_bf16_round(f2_of(y[0].x, y[1].x)), f2_of(w0.x, w0.y));
+            x[0][2 * q + 1] = f2_mul(f2_bf16_round(f2_of(y[2].x, y[3].x)), f2_of(w0.z, w0.w));
+            x[1][2 * q] = f2_mul(f2_bf16_round(f2_of(y[0].y, y[1].y)), f2_of(w1.x, w1.y));
+            x[1][2 * q + 1] = f2_mul(f2_bf16_round(f2_of(y[2].y, y[3].y)), f2_of(w1.z, w1.w));
           }
+        } else {
+          unpack8(cur[j][0], x[0]);
+          unpack8(cur[j][1], x[1]);
         }
-        float y[2][8];
+        f2 y[2][4];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          y[0][i] = x[0][i] * c[i] - x[1][i] * s[i];
-          y[1][i] = x[1][i] * c[i] - x[0][i] * -s[i];
+        for (int i = 0; i < 4; ++i) {
+          y[0][i] = f2_fma(x[0][i], c[i], f2_neg(f2_mul(x[1][i], s[i])));
+          y[1][i] = f2_fma(x[1][i], c[i], f2_mul(x[0][i], s[i]));
         }
         if (live) {
           bf16* p = is_q ? qdst + h * HD : kdst + (h - a.Hq) * HD;
@@ -185,94 +224,90 @@ struct RopeBwdArgs {
   int T, Hq, Hk;
   float w_off;
   int do_norm;
-  int parts, part_heads;
+  int grid_q;  // CTAs of q's heads; the others walk over k's
+  int parts_q, part_heads_q, parts_k, part_heads_k;
 };
 
 // Same token-per-lane-group walk as the forward kernel, UB heads at a time: the gradient rows, the forward
-// inputs and the saved rstd of UB heads are requested before any of them is used. With few tokens a lane
-// holds eight elements of either half of a head, as in the forward (HALVES 2): half the lanes a head, so
-// half the CTAs, one wave of them. With many tokens registers bound the loads in flight, and eight
-// neighbouring elements a lane, the partner's by shuffle (HALVES 1), are as fast or faster.
-// Measured (us, tokens x 24 heads of 128, HALVES 1 / 2): 920 18.4 / 10.7, 2500 23 / 15, 6000 49 / 35,
-// 22627 106 / 108, 40280 174 / 172; 22627 x 40 heads of 64 106 / 119.
-template <int HD, int HALVES>
+// inputs and the saved rstd of UB heads are requested before any of them is used, and registers bound how
+// many those are. So a CTA walks over q's heads or over k's, with the weights of the one in registers and one
+// set of dW accumulators, and a lane holds eight elements of either half of a head, as in the forward.
+// Measured before (both kinds a CTA, weights in shared memory, an element an instruction) / now (us, tokens x
+// 24 heads of 128, L2 flushed): 22627 103 / 88, 40280 171 / 139, 6000 35 / 32, 3000 23 / 21; 33280 x 40
+// 227 / 187; 22627 x 40 heads of 64 94 / 84. (Three CTAs a SM with a head at a time: 119 at 22627.)
+template <int HD>
 __global__ void __launch_bounds__(kRowThreads, 2) qk_rope_bwd_kernel(RopeBwdArgs a) {
-  constexpr int LPH = HD / 8 / HALVES;
+  constexpr int LPH = HD / 16;
   constexpr int TPB = kRowThreads / LPH;
-  constexpr int UB = 4 / HALVES;
+  constexpr int UB = 2;
   constexpr int HALF = HD / 2;
-  __shared__ float sdw[2 * HD];
-  __shared__ float swt[2 * HD];  // q then k norm weights (+ offset)
+  __shared__ float sdw[HD];
   const int l = threadIdx.x % LPH;
   const int g = threadIdx.x / LPH;
   const int e0 = l * 8;
-  const int c0 = e0 % HALF;
-  float dwq[HALVES][8], dwk[HALVES][8];
+  const bool is_q = int(blockIdx.x) < a.grid_q;
+  const unsigned cta = is_q ? blockIdx.x : blockIdx.x - a.grid_q;
+  const unsigned ctas = is_q ? a.grid_q : gridDim.x - a.grid_q;
+  const int H = is_q ? a.Hq : a.Hk;
+  const unsigned parts = is_q ? a.parts_q : a.parts_k;
+  const int part_heads = is_q ? a.part_heads_q : a.part_heads_k;
+  f2 dw[2][4], wt[2][4];
 #pragma unroll
-  for (int k = 0; k < HALVES; ++k)
+  for (int k = 0; k < 2; ++k) {
+    uint4 q = make_uint4(0u, 0u, 0u, 0u);
+    if (a.do_norm) {
+      float f[8];   // (a weight may start at any element)
 #pragma unroll
-    for (int i = 0; i < 8; ++i) dwq[k][i] = dwk[k][i] = 0.f;
-  for (int i = threadIdx.x; i < 2 * HD; i += kRowThreads) {
-    sdw[i] = 0.f;
-    swt[i] = a.do_norm ? __bfloat162float(i < HD ? a.qw[i] : a.kw[i - HD]) + a.w_off : 1.f;
+      for (int i = 0; i < 8; ++i) f[i] = __bfloat162float((is_q ? a.qw : a.kw)[k * HALF + e0 + i]) + a.w_off;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) wt[k][i] = f2_of(f[2 * i], f[2 * i + 1]);
+    } else {
+      unpack8(q, wt[k]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) dw[k][i] = 0ull;
   }
+  for (int i = threadIdx.x; i < HD; i += kRowThreads) sdw[i] = 0.f;
   __syncthreads();
   RopeArgs pa;  // only the position fields are used by token_pos
   pa.pos = a.pos;
   pa.pos_i64 = a.pos_i64;
   pa.pos_mod = a.pos_mod;
+  const bf16* gp = (is_q ? a.dq : a.dk) + e0;
+  const bf16* xp = (is_q ? a.q_in : a.k_in) + e0;
+  bf16* op = (is_q ? a.dq_in : a.dk_in) + e0;
+  const float* rp = is_q ? a.q_rstd : a.k_rstd;
+  const long long ldg = is_q ? a.lddq : a.lddk, ldx = is_q ? a.ldq_in : a.ldk_in;
+  const long long ldo = is_q ? a.lddq_in : a.lddk_in;
   pdl_wait();
   pdl_trigger();
 
-  const unsigned total = unsigned(a.T) * a.parts;
-  for (unsigned u0 = blockIdx.x * TPB; u0 < total; u0 += gridDim.x * TPB) {
-    const unsigned tok_u = (u0 + g) / a.parts;
+  const unsigned total = unsigned(a.T) * parts;
+  for (unsigned u0 = cta * TPB; u0 < total; u0 += ctas * TPB) {
+    const unsigned tok_u = (u0 + g) / parts;
     const long long tok = tok_u;
     const bool valid = tok < a.T;
-    const int h_first = int(u0 + g - tok_u * a.parts) * a.part_heads;
-    const int heads = min(h_first + a.part_heads, a.Hq + a.Hk);
-    float c[8], s[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) c[i] = s[i] = 0.f;
-    if (valid) {
-      const int pos = token_pos(pa, tok);
-      const float4* cp = reinterpret_cast<const float4*>(a.cos + 1LL * pos * HALF + c0);
-      const float4* sp = reinterpret_cast<const float4*>(a.sin + 1LL * pos * HALF + c0);
-      *reinterpret_cast<float4*>(c) = cp[0];
-      *reinterpret_cast<float4*>(c + 4) = cp[1];
-      *reinterpret_cast<float4*>(s) = sp[0];
-      *reinterpret_cast<float4*>(s + 4) = sp[1];
-    }
-    if (e0 >= HALF) {   // (of a single half a lane: gn = g*c + partner*s in the first, - in the second)
-#pragma unroll
-      for (int i = 0; i < 8; ++i) s[i] = -s[i];
-    }
-    const bf16* gq = a.dq + tok * a.lddq + e0;
-    const bf16* gk = a.dk + tok * a.lddk + e0;
-    const bf16* xq = a.q_in + tok * a.ldq_in + e0;
-    const bf16* xk = a.k_in + tok * a.ldk_in + e0;
-    bf16* oq = a.dq_in + tok * a.lddq_in + e0;
-    bf16* ok = a.dk_in + tok * a.lddk_in + e0;
-    for (int b0 = 0; b0 < a.part_heads; b0 += UB) {
+    const int h_first = int(u0 + g - tok_u * parts) * part_heads;
+    const int heads = min(h_first + part_heads, H);
+    f2 c[4], s[4];
+    load_angles<HALF>(a.cos, a.sin, valid ? token_pos(pa, tok) : -1, e0, c, s);
+    for (int b0 = 0; b0 < part_heads; b0 += UB) {
       const int h0 = h_first + b0;
-      uint4 graw[UB][HALVES], xraw[UB][HALVES];
+      uint4 graw[UB][2], xraw[UB][2];
       float rs[UB];
 #pragma unroll
       for (int j = 0; j < UB; ++j) {
         const int h = h0 + j;
 #pragma unroll
-        for (int k = 0; k < HALVES; ++k) graw[j][k] = xraw[j][k] = make_uint4(0u, 0u, 0u, 0u);
+        for (int k = 0; k < 2; ++k) graw[j][k] = xraw[j][k] = make_uint4(0u, 0u, 0u, 0u);
         rs[j] = 0.f;
         if (valid && h < heads) {
-          const bool is_q = h < a.Hq;
-          const bf16* gp = is_q ? gq + h * HD : gk + (h - a.Hq) * HD;
 #pragma unroll
-          for (int k = 0; k < HALVES; ++k) graw[j][k] = ld16(gp + k * HALF);
+          for (int k = 0; k < 2; ++k) graw[j][k] = ld16(gp + tok * ldg + h * HD + k * HALF);
           if (a.do_norm) {
-            const bf16* xp = is_q ? xq + h * HD : xk + (h - a.Hq) * HD;
 #pragma unroll
-            for (int k = 0; k < HALVES; ++k) xraw[j][k] = ld16(xp + k * HALF);
-            rs[j] = is_q ? a.q_rstd[tok * a.Hq + h] : a.k_rstd[tok * a.Hk + (h - a.Hq)];
+            for (int k = 0; k < 2; ++k) xraw[j][k] = ld16(xp + tok * ldx + h * HD + k * HALF);
+            rs[j] = rp[tok * H + h];
           }
         }
       }
@@ -280,58 +315,45 @@ __global__ void __launch_bounds__(kRowThreads, 2) qk_rope_bwd_kernel(RopeBwdArgs
       for (int j = 0; j < UB; ++j) {
         const int h = h0 + j;
         const bool live = valid && h < heads;   // (loads of the others are zero, and add nothing)
-        const bool is_q = h < a.Hq;
-        float gv[HALVES][8], gn[HALVES][8], o[HALVES][8];
+        f2 gv[2][4], gn[2][4];
+        unpack8(graw[j][0], gv[0]);
+        unpack8(graw[j][1], gv[1]);
 #pragma unroll
-        for (int k = 0; k < HALVES; ++k) unpack8(graw[j][k], gv[k]);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          if constexpr (HALVES == 2) {
-            gn[0][i] = gv[0][i] * c[i] + gv[1][i] * s[i];
-            gn[1][i] = gv[1][i] * c[i] + gv[0][i] * -s[i];
-          } else {
-            const float p = __shfl_xor_sync(0xffffffffu, gv[0][i], LPH / 2);
-            gn[0][i] = gv[0][i] * c[i] + p * s[i];
-          }
+        for (int i = 0; i < 4; ++i) {
+          gn[0][i] = f2_fma(gv[0][i], c[i], f2_mul(gv[1][i], s[i]));
+          gn[1][i] = f2_fma(gv[1][i], c[i], f2_neg(f2_mul(gv[0][i], s[i])));
         }
         if (a.do_norm) {
-          float x[HALVES][8], m[HALVES][8], dots[HALVES] = {};
-          const float rstd = rs[j];
+          f2 x[2][4];
+          float dots[2] = {0.f, 0.f};
+          const f2 r2 = f2_of(rs[j], rs[j]);
 #pragma unroll
-          for (int k = 0; k < HALVES; ++k) {
+          for (int k = 0; k < 2; ++k) {
             unpack8(xraw[j][k], x[k]);
-            const float* wt = swt + (is_q ? 0 : HD) + k * HALF + e0;
-            const float4 w0 = *reinterpret_cast<const float4*>(wt);
-            const float4 w1 = *reinterpret_cast<const float4*>(wt + 4);
-            const float wl[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              x[k][i] *= rstd;  // xhat
-              m[k][i] = gn[k][i] * wl[i];
-              dots[k] += m[k][i] * x[k][i];
-              const float dwv = gn[k][i] * bf16_round(x[k][i]);
-              if (is_q) dwq[k][i] += dwv;
-              else dwk[k][i] += dwv;
+            for (int i = 0; i < 4; ++i) {
+              x[k][i] = f2_mul(x[k][i], r2);  // xhat
+              dw[k][i] = f2_fma(gn[k][i], f2_bf16_round(x[k][i]), dw[k][i]);
+              gn[k][i] = f2_mul(gn[k][i], wt[k][i]);
+              const float2 m = f2_get(gn[k][i]), xh = f2_get(x[k][i]);
+              dots[k] = fmaf(m.x, xh.x, dots[k]);
+              dots[k] = fmaf(m.y, xh.y, dots[k]);
             }
           }
-          float dot = HALVES == 2 ? dots[0] + dots[HALVES - 1] : dots[0];
+          float dot = dots[0] + dots[1];
 #pragma unroll
           for (int sh = LPH / 2; sh > 0; sh >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, sh);
           dot /= float(HD);
+          const f2 minus_dot = f2_of(-dot, -dot);
 #pragma unroll
-          for (int k = 0; k < HALVES; ++k)
+          for (int k = 0; k < 2; ++k)
 #pragma unroll
-            for (int i = 0; i < 8; ++i) o[k][i] = rstd * (m[k][i] - x[k][i] * dot);
-        } else {
-#pragma unroll
-          for (int k = 0; k < HALVES; ++k)
-#pragma unroll
-            for (int i = 0; i < 8; ++i) o[k][i] = gn[k][i];
+            for (int i = 0; i < 4; ++i)
+              gn[k][i] = f2_mul(r2, f2_fma(x[k][i], minus_dot, gn[k][i]));
         }
         if (live) {
-          bf16* p = is_q ? oq + h * HD : ok + (h - a.Hq) * HD;
 #pragma unroll
-          for (int k = 0; k < HALVES; ++k) st16(p + k * HALF, pack8(o[k]));
+          for (int k = 0; k < 2; ++k) st16(op + tok * ldo + h * HD + k * HALF, pack8(gn[k]));
         }
       }
     }
@@ -339,22 +361,23 @@ __global__ void __launch_bounds__(kRowThreads, 2) qk_rope_bwd_kernel(RopeBwdArgs
   if (a.do_norm && a.dw_partial != nullptr) {
     // the groups of a warp first: as many fewer additions to the same words of shared memory
 #pragma unroll
-    for (int k = 0; k < HALVES; ++k)
+    for (int k = 0; k < 2; ++k)
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
+      for (int i = 0; i < 4; ++i) {
+        float2 v = f2_get(dw[k][i]);
 #pragma unroll
         for (int sh = 16; sh >= LPH; sh >>= 1) {
-          dwq[k][i] += __shfl_xor_sync(0xffffffffu, dwq[k][i], sh);
-          dwk[k][i] += __shfl_xor_sync(0xffffffffu, dwk[k][i], sh);
+          v.x += __shfl_xor_sync(0xffffffffu, v.x, sh);
+          v.y += __shfl_xor_sync(0xffffffffu, v.y, sh);
         }
         if ((threadIdx.x & 31) < LPH) {
-          atomicAdd(&sdw[k * HALF + e0 + i], dwq[k][i]);
-          atomicAdd(&sdw[HD + k * HALF + e0 + i], dwk[k][i]);
+          atomicAdd(&sdw[k * HALF + e0 + 2 * i], v.x);
+          atomicAdd(&sdw[k * HALF + e0 + 2 * i + 1], v.y);
         }
       }
     __syncthreads();
     for (int i = threadIdx.x; i < 2 * HD; i += kRowThreads)
-      a.dw_partial[1LL * blockIdx.x * 2 * HD + i] = sdw[i];
+      a.dw_partial[1LL * blockIdx.x * 2 * HD + i] = (i < HD) == is_q ? sdw[i % HD] : 0.f;
   }
 }
 
@@ -399,7 +422,7 @@ extern "C" int lb_qk_norm_rope_fwd(const void* q_in, long long ldq_in, const voi
     const long long g = (1LL * T * a.parts + tpb - 1) / tpb;
     const long long cap = 1LL * row_num_sms() * 3;  // one wave at three CTAs per SM
     return launch_pdl(kern, dim3(unsigned(g < cap ? g : cap)), dim3(kRowThreads), 0, st,
-                      pdl_enabled(), 1, a);
+                      pdl_enabled(4LL * T * (Hq + Hk) * hd), 1, a);
   };
   if (hd == 128) return run(qk_rope_fwd_kernel<128>, 8);
   if (hd == 64) return run(qk_rope_fwd_kernel<64>, 4);
@@ -407,16 +430,31 @@ extern "C" int lb_qk_norm_rope_fwd(const void* q_in, long long ldq_in, const voi
   return -3;
 }
 
-// CTAs of the backward, each of which leaves a partial row in its scratch.
+// CTAs of the backward, each of which leaves a partial row in its scratch, and how many of them walk over
+// q's heads: of two a SM, q's share of the heads.
+static int rope_bwd_grid(int T, int Hq, int Hk, int hd, int* grid_q) {
+  const bool few = few_tokens(T, hd);
+  const int tpb = kRowThreads / (hd / 16);
+  auto need = [&](int heads) {
+    int parts, part_heads;
+    rope_parts(few, heads, 2, &parts, &part_heads);
+    return (1LL * T * parts + tpb - 1) / tpb;
+  };
+  const long long cap = 2LL * row_num_sms();
+  long long q = need(Hq), k = need(Hk);
+  if (q + k > cap) {
+    const long long share = cap * Hq / (Hq + Hk);
+    q = share < q ? (share > 0 ? share : 1) : q;
+    k = cap - q < k ? cap - q : k;
+    if (k < 1) k = 1;
+  }
+  *grid_q = int(q);
+  return int(q + k);
+}
 extern "C" int lb_rope_bwd_rows(int T, int Hq, int Hk, int hd) {
   if (T <= 0 || hd < 64) return 0;
-  const bool few = few_tokens(T, hd);
-  int parts, part_heads;
-  rope_parts(few, Hq + Hk, few ? 2 : 4, &parts, &part_heads);
-  const int tpb = kRowThreads / (hd / (few ? 16 : 8));
-  const long long g = (1LL * T * parts + tpb - 1) / tpb;
-  const long long cap = 1LL * row_num_sms() * (few ? 2 : 4);
-  return int(g < cap ? g : cap);
+  int grid_q;
+  return rope_bwd_grid(T, Hq, Hk, hd, &grid_q);
 }
 
 // dw_out: [2, hd] (q weight grad then k weight grad); scratch: lb_rope_bwd_partial_rows()*2*hd floats.
@@ -435,18 +473,20 @@ extern "C" int lb_qk_norm_rope_bwd(const void* dq, long long lddq, const void* d
   RopeBwdArgs a{(const bf16*)dq, (const bf16*)dk, lddq, lddk, (const bf16*)q_in, (const bf16*)k_in,
                 ldq_in, ldk_in, (const bf16*)qw, (const bf16*)kw, cos, sin, pos, pos_i64,
                 pos_mod > 0 ? pos_mod : 1, q_rstd, k_rstd, (bf16*)dq_in, (bf16*)dk_in, lddq_in,
-                lddk_in, scratch, T, Hq, Hk, w_off, do_norm, 1, 0};
+                lddk_in, scratch, T, Hq, Hk, w_off, do_norm};
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  const int grid = lb_rope_bwd_rows(T, Hq, Hk, hd);
+  const int grid = rope_bwd_grid(T, Hq, Hk, hd, &a.grid_q);
   const bool few = few_tokens(T, hd);
-  rope_parts(few, Hq + Hk, few ? 2 : 4, &a.parts, &a.part_heads);
+  rope_parts(few, Hq, 2, &a.parts_q, &a.part_heads_q);
+  rope_parts(few, Hk, 2, &a.parts_k, &a.part_heads_k);
   auto run = [&](auto kern) {
-    return launch_pdl(kern, dim3(grid), dim3(kRowThreads), 0, st, pdl_enabled(), 1, a);
+    return launch_pdl(kern, dim3(grid), dim3(kRowThreads), 0, st,
+                      pdl_enabled(6LL * T * (Hq + Hk) * hd), 1, a);
   };
   int rc = -3;
-  if (hd == 128) rc = few ? run(qk_rope_bwd_kernel<128, 2>) : run(qk_rope_bwd_kernel<128, 1>);
-  else if (hd == 64) rc = few ? run(qk_rope_bwd_kernel<64, 2>) : run(qk_rope_bwd_kernel<64, 1>);
-  else if (hd == 256) rc = few ? run(qk_rope_bwd_kernel<256, 2>) : run(qk_rope_bwd_kernel<256, 1>);
+  if (hd == 128) rc = run(qk_rope_bwd_kernel<128>);
+  else if (hd == 64) rc = run(qk_rope_bwd_kernel<64>);
+  else if (hd == 256) rc = run(qk_rope_bwd_kernel<256>);
   if (rc) return rc;
   if (do_norm && dw_out != nullptr && scratch != nullptr) {
     return lb_colsum(scratch, grid, 2 * hd, dw_out, dw_fp32, dw_accumulate, stream);

@@ -353,3 +353,27 @@ def test_rope_of_few_and_of_many_tokens_has_the_same_bits(Hq, Hk, hd, norm):
     assert at == T
     for a, b in zip(total, wsum):      # four bf16 roundings of the parts' sums
         assert ((a - b).norm() / b.norm()).item() < 4 * 2 ** -8
+
+
+@pytest.mark.parametrize("op", ["swiglu", "geglu", "rms"])
+def test_rows_of_many_have_the_bits_of_few(op):
+    """Walks that go round the grid several times, and end within a round; widths that fill no wave of
+    vectors. A row's values and input gradients do not depend on how many rows there are."""
+    torch.manual_seed(0)
+    T, H = (6401, 3080) if op != "rms" else (4801, 1000)    # above 64 * 256 * 148 vectors; 4 * 148 * 4 rows
+    x, g, g2 = _r(T, H if op == "rms" else 2 * H), _r(T, H), _r(T, H)
+    w, r = _r(H, scale=0.5), _r(T, H)
+
+    def run(rows):
+        if op == "rms":
+            outs, gr = _grads(lambda a, b, c: N.residual_rms_norm(a, b, c, 1e-6), [r[rows], x[rows], w],
+                              (g[rows], g2[rows]))
+            return [*outs, *gr[:2]]
+        outs, gr = _grads(lambda a: A.glu(a, op), [x[rows]], g[rows])
+        return [*outs, *gr]
+
+    whole, at = run(slice(0, T)), 0
+    for n in (1, 3, 700, T - 704):
+        for a, b in zip(run(slice(at, at + n)), whole):
+            assert torch.equal(a, b[at:at + n]), n
+        at += n
