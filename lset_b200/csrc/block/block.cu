@@ -230,6 +230,12 @@ bool plain(const LbProjection& p) {
 
 thread_local int t_fewer = 0;  // launches saved by the current call
 
+// Only where nothing is computed a second time: the tile kernels' results differ in their roundings.
+bool short_attn(const LbStreamCtx* c, int Hq, int Hk, int hd, int rotation) {
+  return c->may_split && c->plan_q == nullptr &&
+         lb_attn_short_ok(c->n_seq, c->max_len, Hq, Hk, hd, rotation);
+}
+
 LbSmallGemm small_gemm(const LbProjection& p, int mode, const LbStreamCtx* c) {
   LbSmallGemm g = {};
   g.nparts = p.n;
@@ -654,13 +660,21 @@ static int block_fwd(const LbBlockDesc* d, const LbStreamCtx* c, const LbBlockIO
   }
   const lb::PdlScope pdl(true);
   LB_TRY(proj_fwd(d->qkv, s.x1, H, s.qkv, T, s.ts, c));
-  LB_TRY(lb_qk_norm_rope_fwd(s.qkv, W, s.qkv + Nq, W, d->qk_norm ? d->qn_w : nullptr,
-                             d->qk_norm ? d->kn_w : nullptr, c->cos, c->sin, c->pos, c->pos_i64, 1,
-                             s.qr, Nq, s.kr, Nk, s.q_rstd, s.k_rstd, T, d->Hq, d->Hk, hd, d->eps,
-                             d->w_off, d->qk_norm, c->stream));
-  LB_TRY(lb_attn_fwd(s.qr, Nq, s.kr, Nk, s.qkv + Nq + Nk, W, c->seq_start, c->seq_end, c->plan_f,
-                     c->cap_f, c->tile_f, s.o, Nq, s.lse, T, d->Hq, d->Hk, hd, d->softmax_scale,
-                     d->causal, c->status, c->stream));
+  if (short_attn(c, d->Hq, d->Hk, hd, 1)) {
+    ++t_fewer;
+    LB_TRY(lb_attn_short(s.qkv, s.qkv + Nq, s.qkv + Nq + Nk, W, d->qk_norm ? d->qn_w : nullptr,
+                         d->qk_norm ? d->kn_w : nullptr, c->cos, c->sin, c->pos, c->pos_i64, c->seq_start,
+                         c->seq_end, c->plan_f, c->cap_f, s.o, Nq, T, c->n_seq, c->max_len, d->Hq, d->Hk, hd,
+                         d->eps, d->w_off, d->softmax_scale, d->causal, c->stream));
+  } else {
+    LB_TRY(lb_qk_norm_rope_fwd(s.qkv, W, s.qkv + Nq, W, d->qk_norm ? d->qn_w : nullptr,
+                               d->qk_norm ? d->kn_w : nullptr, c->cos, c->sin, c->pos, c->pos_i64, 1,
+                               s.qr, Nq, s.kr, Nk, s.q_rstd, s.k_rstd, T, d->Hq, d->Hk, hd, d->eps,
+                               d->w_off, d->qk_norm, c->stream));
+    LB_TRY(lb_attn_fwd(s.qr, Nq, s.kr, Nk, s.qkv + Nq + Nk, W, c->seq_start, c->seq_end, c->plan_f,
+                       c->cap_f, c->tile_f, s.o, Nq, s.lse, T, d->Hq, d->Hk, hd, d->softmax_scale,
+                       d->causal, c->status, c->stream));
+  }
   // attention branch output: staged in `out`, consumed by the second norm before the MLP writes there
   LB_TRY(lin_fwd(d->o_proj, s.o, Nq, out, H, T, s.ts[3], c));
   LB_TRY(lb_rms_norm_fwd(out, stream_in, d->ln2_w, s.x2, io->res_out, s.rstd2, T, H, d->eps,
@@ -836,9 +850,15 @@ extern "C" int lb_encoder_fwd(const LbEncoderDesc* d, const LbStreamCtx* c, LbBl
     LB_TRY(proj_fwd(d->qkv, x, H, s.qkv, T, no_ts, c, d->bias));
   }
   const lb::PdlScope pdl(true);
-  LB_TRY(lb_attn_fwd(s.qkv, W, s.qkv + H, W, s.qkv + 2 * H, W, c->seq_start, c->seq_end, c->plan_f,
-                     c->cap_f, c->tile_f, s.o, H, s.lse, T, d->heads, d->heads, d->hd,
-                     d->softmax_scale, 0, c->status, c->stream));
+  if (short_attn(c, d->heads, d->heads, d->hd, 0)) {
+    LB_TRY(lb_attn_short(s.qkv, s.qkv + H, s.qkv + 2 * H, W, nullptr, nullptr, nullptr, nullptr, nullptr, 0,
+                         c->seq_start, c->seq_end, c->plan_f, c->cap_f, s.o, H, T, c->n_seq, c->max_len,
+                         d->heads, d->heads, d->hd, 0.f, 0.f, d->softmax_scale, 0, c->stream));
+  } else {
+    LB_TRY(lb_attn_fwd(s.qkv, W, s.qkv + H, W, s.qkv + 2 * H, W, c->seq_start, c->seq_end, c->plan_f,
+                       c->cap_f, c->tile_f, s.o, H, s.lse, T, d->heads, d->heads, d->hd,
+                       d->softmax_scale, 0, c->status, c->stream));
+  }
   LB_TRY(lin_fwd(d->o_proj, s.o, H, s.tmp, H, T, nullptr, c, d->bias[3]));
   LB_TRY(lb_layer_norm_fwd(s.tmp, x, d->ln1_w, d->ln1_b, s.y1, s.nr1, s.mean1, s.rstd1, T, H, d->eps,
                            c->stream));

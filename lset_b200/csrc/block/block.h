@@ -79,6 +79,7 @@ struct LbStreamCtx {
   float* wg_tmp;         // 2 * hd floats (QK-norm weight gradient staging of a token-sharded block)
   void* stream;
   int may_split;         // a pass declared inference: contractions may be summed in pieces (see LbSmallGemm)
+  int n_seq, max_len;    // sequences, and what the caller takes for the longest one's tokens
 };
 
 // Tensor parallelism with a token-sharded residual stream (sequence parallelism): the block's

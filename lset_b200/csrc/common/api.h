@@ -51,6 +51,14 @@ int lb_qk_norm_rope_bwd(const void* dq, long long lddq, const void* dk, long lon
                         int dw_accumulate, int T, int Hq, int Hk, int hd, float w_off, int do_norm,
                         void* stream);
 
+// attn/attn_short.cu
+int lb_attn_short_ok(int B, int max_len, int Hq, int Hk, int hd, int rotation);
+int lb_attn_short(const void* q, const void* k, const void* v, long long ld, const void* qw,
+                  const void* kw, const float* cos, const float* sin, const void* pos, int pos_i64,
+                  const int* seq_start, const int* seq_end, const int* plan, int capacity, void* o,
+                  long long ldo, int T, int B, int max_len, int Hq, int Hk, int hd, float eps, float w_off,
+                  float softmax_scale, int causal, void* stream);
+
 // row/act.cu
 int lb_glu_fwd(int kind, const void* gate, const void* up, long long ld_in, void* out,
                long long ld_out, long long T, int I, void* stream);

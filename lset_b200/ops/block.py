@@ -66,7 +66,7 @@ class LbStreamCtx(ctypes.Structure):
                 ("plan_q", _ip), ("cap_q", ctypes.c_int), ("plan_kv", _ip),
                 ("cap_kv", ctypes.c_int), ("status", _ip), ("norm_scratch", _fp),
                 ("rope_scratch", _fp), ("wg_tmp", _fp), ("stream", _vp),
-                ("may_split", ctypes.c_int)]
+                ("may_split", ctypes.c_int), ("n_seq", ctypes.c_int), ("max_len", ctypes.c_int)]
 
 
 class LbTpCtx(ctypes.Structure):
@@ -472,6 +472,8 @@ def _stream_struct(ctx, plan: BlockPlan, device, training: bool) -> LbStreamCtx:
         s.wg_tmp = sums.data_ptr() + 4 * (norm + rope)
     s.stream = 0
     s.may_split = int(split)
+    # what the attention of short sequences is chosen by (0: not known)
+    s.n_seq, s.max_len = ap.seq_start.numel(), getattr(ap, "max_seqlen", 0)
     # keep the tensors the struct points to alive as long as the struct
     s._keep = (cos, sin, ctx.pos, ap, ptf, ptq, ptk, sums)
     ctx.tables[key] = s

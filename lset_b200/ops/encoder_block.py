@@ -233,6 +233,8 @@ def _stream_struct(ctx, plan: EncoderPlan, device, training: bool) -> LbStreamCt
         sums = torch.empty(partial + 2 * d.H, dtype=torch.float32, device=device)
         s.norm_scratch, s.wg_tmp = sums.data_ptr(), sums.data_ptr() + 4 * partial
     s.may_split = int(split)
+    # what the attention of short sequences is chosen by (0: not known)
+    s.n_seq, s.max_len = ap.seq_start.numel(), getattr(ap, "max_seqlen", 0)
     s._keep = (ctx.pos, ap, ptf, ptq, sums)
     ctx.tables[key] = s
     return s
