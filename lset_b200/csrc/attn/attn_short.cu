@@ -162,12 +162,13 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 3) attn_short_ker
 #pragma unroll
           for (int j = 0; j < UB; ++j) {
             const int u = u0 + j * GROUPS + g;
-            uint4 y[2];
-            rope_head<HD>(raw[j], a.do_norm, swt + (u < new_q ? 0 : HD) + lg * 4, a.eps, cs[j], sn[j], y);
+            f2 y[2][4];
+            rope_head<HD>(raw[j], a.do_norm, swt + (u < new_q ? 0 : HD) + lg * 4, a.eps, cs[j], sn[j], y,
+                          [](float) {});
             if (u < new_q + nk) {
               bf16* dst = u < new_q ? sQ + u * C::PITCH : sK + (u - new_q) * C::PITCH;
-              st16(dst + lg * 8, y[0]);
-              st16(dst + HD / 2 + lg * 8, y[1]);
+              st16(dst + lg * 8, pack8(y[0]));
+              st16(dst + HD / 2 + lg * 8, pack8(y[1]));
             }
           }
         }

@@ -106,16 +106,17 @@ __global__ void __launch_bounds__(kRowThreads, 3) qk_rope_fwd_kernel(RopeArgs a)
         const int h = h0 + j;
         const bool live = valid && h < heads;
         const bool is_q = h < a.Hq;
-        uint4 y[2];
-        const float rstd = rope_head<HD>(cur[j], a.do_norm, swt + (is_q ? 0 : HD) + l * 4, a.eps, c, s, y);
-        if (a.do_norm && live && l == 0) {
-          if (is_q) a.q_rstd[tok * a.Hq + h] = rstd;
-          else a.k_rstd[tok * a.Hk + (h - a.Hq)] = rstd;
-        }
+        f2 y[2][4];
+        rope_head<HD>(cur[j], a.do_norm, swt + (is_q ? 0 : HD) + l * 4, a.eps, c, s, y, [&](float rstd) {
+          if (live && l == 0) {
+            if (is_q) a.q_rstd[tok * a.Hq + h] = rstd;
+            else a.k_rstd[tok * a.Hk + (h - a.Hq)] = rstd;
+          }
+        });
         if (live) {
           bf16* p = is_q ? qdst + h * HD : kdst + (h - a.Hq) * HD;
-          st16(p, y[0]);
-          st16(p + HALF, y[1]);
+          st16(p, pack8(y[0]));
+          st16(p + HALF, pack8(y[1]));
         }
       }
 #pragma unroll

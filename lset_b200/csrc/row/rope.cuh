@@ -44,13 +44,13 @@ __device__ __forceinline__ void load_angles(const float* cos, const float* sin, 
 __device__ __forceinline__ f2 f2_neg(f2 v) { return v ^ 0x8000000080000000ull; }
 
 // A lane's eight elements of either half of a head (`raw`) to their rotated values; `wt`: its first weight
-// (see weight_at; only read with do_norm). All lanes of the warp call it. Returns the head's rstd.
-template <int HD>
-__device__ __forceinline__ float rope_head(const uint4 (&raw)[2], bool do_norm, const float* wt, float eps,
-                                           const f2 (&c)[4], const f2 (&s)[4], uint4 (&out)[2]) {
+// (see weight_at; only read with do_norm). All lanes of the warp call it. The head's rstd goes to `rstd_is`.
+template <int HD, typename Rstd>
+__device__ __forceinline__ void rope_head(const uint4 (&raw)[2], bool do_norm, const float* wt, float eps,
+                                           const f2 (&c)[4], const f2 (&s)[4], f2 (&y)[2][4],
+                                          Rstd rstd_is) {
   constexpr int LPH = HD / 16;
   f2 x[2][4];
-  float rstd = 0.f;
   if (do_norm) {
     // element i of either half in one pair: two sums of squares, each in the order of its half
     const uint32_t lo[4] = {raw[0].x, raw[0].y, raw[0].z, raw[0].w};
@@ -67,33 +67,30 @@ __device__ __forceinline__ float rope_head(const uint4 (&raw)[2], bool do_norm, 
     float sum = halves.x + halves.y;
 #pragma unroll
     for (int o = LPH / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    rstd = rsqrtf(sum / float(HD) + eps);
+    const float rstd = rsqrtf(sum / float(HD) + eps);
+    rstd_is(rstd);
     const f2 r2 = f2_of(rstd, rstd);
 #pragma unroll
     for (int q = 0; q < 2; ++q) {   // columns 4q .. 4q + 3 of either half
-      float2 y[4];
+      float2 n[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) y[i] = f2_get(f2_mul(p[4 * q + i], r2));
+      for (int i = 0; i < 4; ++i) n[i] = f2_get(f2_mul(p[4 * q + i], r2));
       const float4 w0 = *reinterpret_cast<const float4*>(wt + q * LPH * 4);
       const float4 w1 = *reinterpret_cast<const float4*>(wt + (2 + q) * LPH * 4);
-      x[0][2 * q] = f2_mul(f2_bf16_round(f2_of(y[0].x, y[1].x)), f2_of(w0.x, w0.y));
-      x[0][2 * q + 1] = f2_mul(f2_bf16_round(f2_of(y[2].x, y[3].x)), f2_of(w0.z, w0.w));
-      x[1][2 * q] = f2_mul(f2_bf16_round(f2_of(y[0].y, y[1].y)), f2_of(w1.x, w1.y));
-      x[1][2 * q + 1] = f2_mul(f2_bf16_round(f2_of(y[2].y, y[3].y)), f2_of(w1.z, w1.w));
+      x[0][2 * q] = f2_mul(f2_bf16_round(f2_of(n[0].x, n[1].x)), f2_of(w0.x, w0.y));
+      x[0][2 * q + 1] = f2_mul(f2_bf16_round(f2_of(n[2].x, n[3].x)), f2_of(w0.z, w0.w));
+      x[1][2 * q] = f2_mul(f2_bf16_round(f2_of(n[0].y, n[1].y)), f2_of(w1.x, w1.y));
+      x[1][2 * q + 1] = f2_mul(f2_bf16_round(f2_of(n[2].y, n[3].y)), f2_of(w1.z, w1.w));
     }
   } else {
     unpack8(raw[0], x[0]);
     unpack8(raw[1], x[1]);
   }
-  f2 y[2][4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     y[0][i] = f2_fma(x[0][i], c[i], f2_neg(f2_mul(x[1][i], s[i])));
     y[1][i] = f2_fma(x[1][i], c[i], f2_mul(x[0][i], s[i]));
   }
-  out[0] = pack8(y[0]);
-  out[1] = pack8(y[1]);
-  return rstd;
 }
 
 }  // namespace lb
