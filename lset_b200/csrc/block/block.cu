@@ -132,11 +132,35 @@ Work carve_work(const LbBlockDesc* d, int T, int R, bool sharded, Arena& a) {
     if (rc_ != 0) return rc_; \
   } while (0)
 
+thread_local int t_fewer = 0;  // launches saved by the current call
+
 // Fills in the tile width and split of `g`: whether it is modelled to take less than `alternative`.
 bool small_wins(LbSmallGemm* g, double alternative) {
   if (!lb_gemm_use_2cta(-1)) return false;
   const double cost = lb_gemm_small_plan(g, &g->bn, &g->splits);
   return cost >= 0.0 && cost < alternative;
+}
+
+LbSmallGemm small_linear(const LbLinear& l, const __nv_bfloat16* x, long long ldx, __nv_bfloat16* y,
+                         long long ldy, int T, const LbStreamCtx* c, const void* bias) {
+  LbSmallGemm g = {};
+  g.A = x;
+  g.B[0] = l.w;
+  g.C[0] = y;
+  g.lda = ldx;
+  g.ldb[0] = l.ldw;
+  g.ldc[0] = ldy;
+  g.M = T;
+  g.N = g.ext[0] = l.n_out;
+  g.K = l.k_in;
+  g.nparts = 1;
+  g.mode = kParallelN;
+  g.b_ready = 1;
+  g.may_split = c->may_split;
+  g.bias[0] = bias;
+  g.status = c->status;
+  g.stream = c->stream;
+  return g;
 }
 
 // y[:, :n_out] (row stride ldy) = x · Wᵀ (+ LoRA). `ts` receives s · x · Aᵀ when the linear has adapters.
@@ -152,27 +176,31 @@ int lin_fwd(const LbLinear& l, const __nv_bfloat16* x, long long ldx, __nv_bfloa
                             l.lora_r, l.lora_r, ldy, 0, nullptr, c->status, c->stream);
   }
   if (c->may_split) {
-    LbSmallGemm g = {};
-    g.A = x;
-    g.B[0] = l.w;
-    g.C[0] = y;
-    g.lda = ldx;
-    g.ldb[0] = l.ldw;
-    g.ldc[0] = ldy;
-    g.M = T;
-    g.N = g.ext[0] = l.n_out;
-    g.K = l.k_in;
-    g.nparts = 1;
-    g.mode = kParallelN;
-    g.b_ready = g.may_split = 1;
-    g.bias[0] = bias;
-    g.status = c->status;
-    g.stream = c->stream;
-    if (small_wins(&g, lb_gemm_tile_cost(T, l.n_out, l.k_in, 0)))
+    LbSmallGemm g = small_linear(l, x, ldx, y, ldy, T, c, bias);
+    if (small_wins(&g, lb_gemm_tile_cost(T, l.n_out, l.k_in, 0, bias != nullptr)))
       return lb_gemm_small(&g);
   }
   return lb_gemm_bf16(x, l.w, y, T, l.n_out, l.k_in, ldx, l.ldw, ldy, 0, 0, 0, 0, bias, 1, 0,
                       c->status, c->stream);
+}
+
+// g = GELU(u), u = x · Wᵀ + bias, both [T, n_out] contiguous; u is left unwritten where one launch does both
+// and it is not to be kept.
+int lin_gelu_fwd(const LbLinear& l, const __nv_bfloat16* x, long long ldx, __nv_bfloat16* u, bool keep_u,
+                 __nv_bfloat16* gelu, int I, int T, const LbStreamCtx* c, const void* bias) {
+  if (l.lora_r == 0) {
+    LbSmallGemm g = small_linear(l, x, ldx, keep_u ? u : nullptr, I, T, c, bias);
+    g.glu_h = gelu;
+    g.ld_h = I;
+    g.glu_kind = 2;
+    // (beside it the activation: a launch, two passes at 5 TB/s)
+    if (small_wins(&g, lb_gemm_tile_cost(T, l.n_out, l.k_in, 0, bias != nullptr) + 2.5 + 4.0 * T * I / 5e6)) {
+      ++t_fewer;
+      return lb_gemm_small(&g);
+    }
+  }
+  LB_TRY(lin_fwd(l, x, ldx, u, I, T, nullptr, c, bias));
+  return lb_gelu_fwd(u, gelu, 1LL * T * I, c->stream);
 }
 
 // dx[T, k_in] (contiguous) = or += dy · W (+ s · (dy · B) · A). `us` is scratch for s · dy · B and is
@@ -228,8 +256,6 @@ bool plain(const LbProjection& p) {
   return true;
 }
 
-thread_local int t_fewer = 0;  // launches saved by the current call
-
 // Only where nothing is computed a second time: the tile kernels' results differ in their roundings.
 bool short_attn(const LbStreamCtx* c, int Hq, int Hk, int hd, int rotation) {
   return c->may_split && c->plan_q == nullptr &&
@@ -263,7 +289,7 @@ int proj_fwd(const LbProjection& p, const __nv_bfloat16* x, long long ldx, __nv_
       g.bias[i] = bias != nullptr ? bias[i] : nullptr;
       g.ldc[i] = p.width;
       col += p.part[i].n_out;
-      apart += lb_gemm_tile_cost(T, p.part[i].n_out, p.part[i].k_in, 0);
+      apart += lb_gemm_tile_cost(T, p.part[i].n_out, p.part[i].k_in, 0, bias != nullptr);
     }
     g.A = x;
     g.lda = ldx;
@@ -318,10 +344,10 @@ int glu_proj_fwd(const LbBlockDesc* d, const __nv_bfloat16* x, __nv_bfloat16* gu
                       (p.n == 2 || !keep_gu || T >= 8192);
     double other = 6.0;
     if (pair) {
-      other += lb_gemm_tile_cost(T, 2 * I, d->H, 0);
+      other += lb_gemm_tile_cost(T, 2 * I, d->H, 0, 0);
     } else {
       other += 6.0 * T * I / 5e6;   // the activation: a launch, three passes at 5 TB/s
-      for (int i = 0; i < p.n; ++i) other += lb_gemm_tile_cost(T, p.part[i].n_out, d->H, 0);
+      for (int i = 0; i < p.n; ++i) other += lb_gemm_tile_cost(T, p.part[i].n_out, d->H, 0, 0);
     }
     // (measured, small / pair: 520 x 3072 x 1024 25 / 29 us, 800 x 9728 x 2560 175 / 121, 1500 x 1152 x 768
     // 21 / 25, 6000 x 1152 x 768 48 / 39)
@@ -349,8 +375,8 @@ int proj_bwd(const LbProjection& p, const __nv_bfloat16* dy, const __nv_bfloat16
     double apart = 0.0, apart_w = 0.0;
     bool all_w = true;
     for (int i = 0; i < p.n; ++i) {
-      apart += lb_gemm_tile_cost(T, K, p.part[i].n_out, 0);
-      apart_w += lb_gemm_tile_cost(p.part[i].n_out, K, T, 1);
+      apart += lb_gemm_tile_cost(T, K, p.part[i].n_out, 0, 0);
+      apart_w += lb_gemm_tile_cost(p.part[i].n_out, K, T, 1, 0);
       all_w = all_w && p.part[i].wgrad != nullptr;
     }
     LbSmallGemm g = small_gemm(p, kParallelK, c);
@@ -862,8 +888,7 @@ extern "C" int lb_encoder_fwd(const LbEncoderDesc* d, const LbStreamCtx* c, LbBl
   LB_TRY(lin_fwd(d->o_proj, s.o, H, s.tmp, H, T, nullptr, c, d->bias[3]));
   LB_TRY(lb_layer_norm_fwd(s.tmp, x, d->ln1_w, d->ln1_b, s.y1, s.nr1, s.mean1, s.rstd1, T, H, d->eps,
                            c->stream));
-  LB_TRY(lin_fwd(d->in, s.y1, H, s.u, I, T, nullptr, c, d->bias[4]));
-  LB_TRY(lb_gelu_fwd(s.u, s.g, 1LL * T * I, c->stream));
+  LB_TRY(lin_gelu_fwd(d->in, s.y1, H, s.u, c->plan_q != nullptr, s.g, I, T, c, d->bias[4]));
   LB_TRY(lin_fwd(d->out, s.g, I, s.tmp, H, T, nullptr, c, d->bias[5]));
   LB_TRY(lb_layer_norm_fwd(s.tmp, s.y1, d->ln2_w, d->ln2_b, io->out, s.nr2, s.mean2, s.rstd2, T, H,
                            d->eps, c->stream));

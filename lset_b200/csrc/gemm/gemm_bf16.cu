@@ -890,7 +890,10 @@ int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmArgs& g, in
 // the fp32 reduction epilogue of an item, hidden behind the next item's main loop only when that
 // is at least as long. More splits mean more reduction traffic, so a candidate must win by 2 %.
 int auto_splits(long long tiles, int kb_total, int sms) {
-  constexpr int kEpi = 32, kMinKb = 32;
+  // In k-blocks: the last epilogue, and what every epilogue adds to its wave although the next tile runs under
+  // it. (Without the latter 4096 x 1024 x 22627 was cut in eight for its last wave's sake: 171 us, 162 whole;
+  // 6144 x 1024 x 40280 in ten, 428, in three 415; 1024 x 2048 x 22627 in nine, 88, in two 86.)
+  constexpr int kEpi = 32, kEach = 8, kMinKb = 32;
   if (kb_total < 2 * kMinKb) return 1;
   int best = 1;
   double best_cost = 1e30;
@@ -900,8 +903,8 @@ int auto_splits(long long tiles, int kb_total, int sms) {
     const int se = (kb_total + kb_per - 1) / kb_per;
     const long long items = tiles * se;
     const long long waves = (items + sms - 1) / sms;
-    const double cost = double(waves) * (kb_per > kEpi ? kb_per : kEpi) + kEpi;
-    if (cost < best_cost * 0.98) {
+    const double cost = double(waves) * ((kb_per > kEpi ? kb_per : kEpi) + kEach) + kEpi;
+    if (cost < best_cost * 0.995) {
       best = se;
       best_cost = cost;
     }
@@ -985,17 +988,20 @@ static int one_cta_bn(int M, int N) {
 // Microseconds per launch, to compare with lb_gemm_small_plan; fitted to the same kind of measurements (140
 // products of those widths at 8 to 3000 tokens, 10 % rms): a launch, per wave of tiles its set-up and
 // store and for each 64 of contraction depth 0.35 us on CTA pairs, on the one-CTA kernel (for products
-// smaller than a pair's tile) 0.3 with 256 columns a tile and 0.22 with 128; the bytes bound both.
-extern "C" double lb_gemm_tile_cost(int M, int N, int K, int fp32) {
-  const bool pair = M >= 256 && N >= 256;
+// smaller than a pair's tile) 0.3 with 256 columns a tile and 0.22 with 128; the bytes bound both. With a
+// bias (one-CTA kernel at any size) the store of a tile of 256 columns takes 5 us (650 x 3072 x 768 11.8 us,
+// here 11.6; the model without it said 8.2 and lost to the small kernel's 8.0 only on paper).
+extern "C" double lb_gemm_tile_cost(int M, int N, int K, int fp32, int bias) {
+  const bool pair = M >= 256 && N >= 256 && !bias;
   const int bm = pair ? 256 : lb::BM, bn = pair ? 256 : one_cta_bn(M, N);
   const int slots = pair ? lb_gemm_2cta_pairs() : lb::num_sms();
   const long long tiles = 1LL * ((M + bm - 1) / bm) * ((N + bn - 1) / bn);
   const int kb = (K + lb::BK - 1) / lb::BK;
   const int s = fp32 ? lb::auto_splits(tiles, kb, slots) : 1;
   const long long waves = (tiles * s + slots - 1) / slots;
-  const double block = pair ? 0.35 : (bn == 256 ? 0.3 : 0.22);
-  const double cost = 3.2 + double(waves) * (((kb + s - 1) / s) * block + 2.2) + (s > 1 ? 0.6 : 0.0);
+  const double block = pair ? 0.35 : (bn == 256 ? (bias ? 0.28 : 0.3) : (bias ? 0.15 : 0.22));
+  const double store = bias && bn == 256 ? 5.0 : (bias ? 2.5 : 2.2);
+  const double cost = 3.2 + double(waves) * (((kb + s - 1) / s) * block + store) + (s > 1 ? 0.6 : 0.0);
   const double memory =
       3.0 + (2.0 * K * (double(M) + N) + (fp32 ? 8.0 : 2.0) * double(M) * N) / 3.73e6;
   return cost > memory ? cost : memory;
@@ -1049,7 +1055,7 @@ static int gemm_bf16_impl(const void* A, const void* B, void* C, int M, int N, i
     p.status = status;
     p.stream = stream_;
     const double cost = lb_gemm_small_plan(&p, &p.bn, &p.splits);
-    if (cost >= 0.0 && cost < lb_gemm_tile_cost(M, N, K, out_fp32))
+    if (cost >= 0.0 && cost < lb_gemm_tile_cost(M, N, K, out_fp32, bias != nullptr))
       return lb_gemm_small(&p);
   }
   if (use_2cta() && bias == nullptr && !scatter && bn == 0 && M >= 256 && N >= 256) {

@@ -15,7 +15,8 @@
 //
 // Projections that share an input, an output or a token contraction (q, k, v; gate, up) are one
 // launch: see LbSmallGemm. The gated pair takes gate and up rows of the same features into one
-// tile and writes act(gate) * up from the epilogue.
+// tile and writes act(gate) * up from the epilogue; the GELU of a single product (BERT's) is written there too
+// (650 x 3072 x 768: 8 us, with a launch of its own 12).
 //
 // Measurements: see lb_gemm_small_plan.
 #include "gemm_small.h"
@@ -92,12 +93,15 @@ __device__ __forceinline__ float4 ld_cluster4(uint32_t addr) {
   return v;
 }
 
-// The values of the stand-alone activation kernel (row/act.cu): the same bits. GLU: 1 = SiLU, 2 =
+// The values of the stand-alone activation kernels (row/act.cu): the same bits. GLU: 3 = GELU (erf), of the
+// product itself; of the gate of a pair 1 = SiLU, 2 =
 // tanh-GELU.
 template <int GLU>
 __device__ __forceinline__ float act_of(float x) {
   if constexpr (GLU == 1) {
     return x * __frcp_rn(1.f + __expf(-x));
+  } else if constexpr (GLU == 3) {
+    return 0.5f * x * (1.f + erff(x * 0.7071067811865476f));
   } else {
     const float k0 = 0.7978845608028654f, k1 = 0.044715f;
     return 0.5f * x * (1.f + tanhf(k0 * (x + k1 * x * x * x)));
@@ -185,9 +189,10 @@ __global__ void __launch_bounds__(kThreads)
     const int t = g.mode == kParallelN ? tn : tm;
     while (part + 1 < g.nparts && t >= g.first[part + 1]) ++part;
   }
-  constexpr int kCols = GLU ? BN / 2 : BN;             // output columns of a tile
+  constexpr bool PAIR = GLU == 1 || GLU == 2;
+  constexpr int kCols = PAIR ? BN / 2 : BN;            // output columns of a tile
   int m0 = tm * BM, n0 = tn * kCols, am0 = m0, m_ext = g.M, n_ext = g.N;
-  if (g.mode == kParallelN && !GLU) {
+  if (g.mode == kParallelN && !PAIR) {
     n0 = (tn - g.first[part]) * BN;
     n_ext = g.ext[part];
   } else if (g.mode == kParallelM) {
@@ -196,7 +201,7 @@ __global__ void __launch_bounds__(kThreads)
     am0 = m0;
     for (int p = 0; p < part; ++p) am0 += g.ext[p];
   }
-  if (GLU) n_ext = g.ext[0];
+  if (PAIR) n_ext = g.ext[0];
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) {
@@ -239,7 +244,7 @@ __global__ void __launch_bounds__(kThreads)
         uint8_t* sb = smem + s * C::BLOCK_BYTES + C::A_BYTES;
         uint64_t* bar = &full[kps == 1 ? s : s >> 1];
         const int kc = (kb_b + i) * BK;
-        if (GLU) {  // gate rows, then up rows of the same features
+        if (PAIR) {  // gate rows, then up rows of the same features
           tma_load_2d(sb, &tmB0, bar, kc, n0);
           tma_load_2d(sb + (BN / 2) * 128, &tmB1, bar, kc, n0);
         } else if (B_MN) {
@@ -378,7 +383,7 @@ __global__ void __launch_bounds__(kThreads)
       const uint32_t off = uint32_t(row * C::PITCH + c) * 4u;
       float4 a0 = cluster_sum4(base, off, S, g.by_part);
       float4 a1 = cluster_sum4(base, off + 16u, S, g.by_part);
-      if (!GLU && g.bias[part] != nullptr) {
+      if (!PAIR && g.bias[part] != nullptr) {
         const uint4 bq = *reinterpret_cast<const uint4*>(g.bias[part] + n0 + c);
         const float2 b0 = unpack_bf16x2(bq.x), b1 = unpack_bf16x2(bq.y);
         const float2 b2 = unpack_bf16x2(bq.z), b3 = unpack_bf16x2(bq.w);
@@ -391,7 +396,7 @@ __global__ void __launch_bounds__(kThreads)
       pk.z = pack_bf16x2(a1.x, a1.y);
       pk.w = pack_bf16x2(a1.z, a1.w);
       const long long grow = m0 + row;
-      if constexpr (GLU) {
+      if constexpr (PAIR) {
         const float4 u0 = cluster_sum4(base, off + BN / 2 * 4u, S);
         const float4 u1 = cluster_sum4(base, off + BN / 2 * 4u + 16u, S);
         uint4 pu;
@@ -415,8 +420,20 @@ __global__ void __launch_bounds__(kThreads)
         *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(g.glu_h) + grow * g.ld_h + n0 +
                                   c) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
       } else {
-        *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(g.C[part]) +
-                                  grow * g.ldc[part] + n0 + c) = pk;
+        if (GLU != 3 || g.C[0] != nullptr)
+          *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(g.C[part]) +
+                                    grow * g.ldc[part] + n0 + c) = pk;
+        if constexpr (GLU == 3) {
+          const uint32_t w[4] = {pk.x, pk.y, pk.z, pk.w};
+          uint32_t hw[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float2 v = unpack_bf16x2(w[j]);
+            hw[j] = pack_bf16x2(act_of<3>(v.x), act_of<3>(v.y));
+          }
+          *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(g.glu_h) + grow * g.ld_h + n0 + c) =
+              make_uint4(hw[0], hw[1], hw[2], hw[3]);
+        }
       }
     }
   } else {
@@ -503,11 +520,12 @@ int ring_of(int bm, int bn, int grid, int cluster, int* blocks_out, int* kps_out
   return fit < per_sm ? fit : per_sm;
 }
 
+bool gated(const LbSmallGemm* p) { return p->glu_h != nullptr && p->glu_kind != 2; }
 bool by_part(const LbSmallGemm* p) { return p->mode == kParallelK && p->nparts > 1; }
 
 int count_tiles(const LbSmallGemm* p, int bm, int bn, int* tiles_n) {
   const int tm = tiles_along(p, kParallelM, p->M, bm);
-  const int tn = p->glu_h != nullptr ? ceil_div(p->ext[0], bn / 2)
+  const int tn = gated(p) ? ceil_div(p->ext[0], bn / 2)
                                      : tiles_along(p, kParallelN, p->N, bn);
   *tiles_n = tn;
   return tm * tn;
@@ -526,14 +544,14 @@ bool shape_ok(const LbSmallGemm* p) {
   for (int i = 0; i < (p->mode == kParallelK ? 1 : p->nparts); ++i)
     if (p->C[i] != nullptr && (p->ldc[i] & (p->out_fp32 ? 3 : 7))) return false;
   if (p->glu_h != nullptr &&
-      (p->mode != kParallelN || p->nparts != 2 || p->ext[0] != p->ext[1] || p->a_mn || p->b_mn ||
-       p->out_fp32 || (p->ld_h & 7)))
+      (p->mode != kParallelN || p->a_mn || p->b_mn || p->out_fp32 || (p->ld_h & 7) ||
+       (gated(p) ? p->nparts != 2 || p->ext[0] != p->ext[1] : p->nparts != 1)))
     return false;
   if (p->a_mn && !p->b_mn) return false;        // not a product of a linear layer
   if (p->out_fp32 != (p->a_mn ? 1 : 0)) return false;
   for (int i = 0; i < p->nparts; ++i)
     if (p->bias[i] != nullptr &&
-        (p->mode != kParallelN || p->glu_h != nullptr || p->out_fp32 ||
+        (p->mode != kParallelN || gated(p) || p->out_fp32 ||
          (reinterpret_cast<uintptr_t>(p->bias[i]) & 15u) != 0))
       return false;
   return true;
@@ -562,6 +580,8 @@ int launch_small(const CUtensorMap& tA, const CUtensorMap* tB, const SmallArgs& 
 template <int BM, int BN>
 int dispatch(const LbSmallGemm* p, const CUtensorMap& tA, const CUtensorMap* tB, const SmallArgs& g,
              int grid, cudaStream_t st) {
+  if (p->glu_h != nullptr && !gated(p))
+    return launch_small<0, 0, BM, BN, __nv_bfloat16, 3>(tA, tB, g, grid, st);
   if (p->glu_h != nullptr)
     return p->glu_kind == 0 ? launch_small<0, 0, BM, BN, __nv_bfloat16, 1>(tA, tB, g, grid, st)
                             : launch_small<0, 0, BM, BN, __nv_bfloat16, 2>(tA, tB, g, grid, st);
@@ -603,7 +623,7 @@ extern "C" double lb_gemm_small_plan(const LbSmallGemm* p, int* bn_out, int* spl
   int kb_part = 0;
   for (int i = 0; parts && i < p->nparts; ++i)
     kb_part = ceil_div(p->ext[i], BK) > kb_part ? ceil_div(p->ext[i], BK) : kb_part;
-  const double out_cols = p->glu_h != nullptr ? p->ext[0] : p->N;
+  const double out_cols = gated(p) ? p->ext[0] : p->N;
   const double bytes = 2.0 * p->K * (double(p->M) + p->N) + (p->out_fp32 ? 8.0 : 2.0) * p->M * out_cols;
   double best = 1e30;
   for (const SmallTile& t : kSmallTiles) {
@@ -672,7 +692,7 @@ extern "C" int lb_gemm_small(const LbSmallGemm* p) {
   // 37.2 us, 25.7 without; 1 x 6144 x 4096 61.5, 40.8). What is left in shared memory below them goes
   // to accumulator rows and columns that nobody reads.
   const int a_box = !p->a_mn && p->M < BM ? p->M : BM;
-  const int b_box = !p->b_mn && p->glu_h == nullptr && p->nparts == 1 && p->N < bn ? p->N : bn;
+  const int b_box = !p->b_mn && !gated(p) && p->nparts == 1 && p->N < bn ? p->N : bn;
   int a_inner = p->a_mn ? p->M : p->K;
   rc = p->a_mn ? make_tmap_2d(&tA, p->A, 2, (uint64_t)a_inner, (uint64_t)p->K,
                               (uint64_t)p->lda * 2, 64, BK, true)
@@ -686,7 +706,7 @@ extern "C" int lb_gemm_small(const LbSmallGemm* p) {
     rc = p->b_mn ? make_tmap_2d(&tB[i], p->B[i], 2, (uint64_t)n, (uint64_t)k,
                                 (uint64_t)p->ldb[i] * 2, 64, BK, true)
                  : make_tmap_2d(&tB[i], p->B[i], 2, (uint64_t)k, (uint64_t)n,
-                                (uint64_t)p->ldb[i] * 2, BK, p->glu_h != nullptr ? bn / 2 : b_box,
+                                (uint64_t)p->ldb[i] * 2, BK, gated(p) ? bn / 2 : b_box,
                                 true);
     if (rc) return rc;
   }

@@ -22,9 +22,11 @@ struct LbSmallGemm {
   const void* bias[3]; // bf16, added to the columns of a part (kParallelN without glu_h); null: none
   // Gated pair (kParallelN, two parts of the same ext): also h = act(C_0) * C_1 [M, ext[0]], with both
   // factors rounded to bf16 first; C[0] == null leaves the products themselves unwritten.
+  // glu_kind 2 (kParallelN, one part): h = GELU(C_0) [M, N], of the rounded product with its bias; C[0] == null
+  // leaves that unwritten.
   void* glu_h;
   long long ld_h;
-  int glu_kind;        // 0 = SiLU, 1 = tanh-GELU
+  int glu_kind;        // 0 = SiLU, 1 = tanh-GELU, 2 = GELU (erf) of one product
   // The B operands were complete before the kernel in front of this one on the stream began, so
   // their tiles may be requested while that kernel is still running.
   int b_ready;
@@ -36,9 +38,9 @@ struct LbSmallGemm {
 
 // Modelled time of the product on this kernel and the tile width and split it would take (a negative
 // value: not taken), and of one product on the CTA-pair kernel (fp32: a weight gradient, whose
-// contraction that kernel splits).
+// contraction that kernel splits; bias: the one-CTA kernel's, which adds it).
 double lb_gemm_small_plan(const LbSmallGemm* p, int* bn, int* splits);
-double lb_gemm_tile_cost(int M, int N, int K, int fp32);
+double lb_gemm_tile_cost(int M, int N, int K, int fp32, int bias);
 int lb_gemm_small(const LbSmallGemm* p);
 
 }  // extern "C"

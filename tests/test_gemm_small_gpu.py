@@ -20,7 +20,7 @@ class SmallGemm(ctypes.Structure):      # LbSmallGemm of csrc/gemm/gemm_small.h
                 ("b_ready", _ci), ("may_split", _ci), ("bn", _ci), ("splits", _ci), ("status", _vp), ("stream", _vp)]
 
 
-def _call(a, bs, cs, M, N, K, ext, mode, a_mn=0, b_mn=0, fp32=0, bias=(), h=None, bn=0, splits=0):
+def _call(a, bs, cs, M, N, K, ext, mode, a_mn=0, b_mn=0, fp32=0, bias=(), h=None, bn=0, splits=0, kind=0):
     g = SmallGemm()
     g.A, g.lda = a.data_ptr(), a.stride(0)
     for i, b in enumerate(bs):
@@ -34,7 +34,7 @@ def _call(a, bs, cs, M, N, K, ext, mode, a_mn=0, b_mn=0, fp32=0, bias=(), h=None
     g.M, g.N, g.K, g.nparts, g.mode = M, N, K, len(ext), mode
     g.a_mn, g.b_mn, g.out_fp32, g.bn, g.splits = a_mn, b_mn, fp32, bn, splits
     if h is not None:
-        g.glu_h, g.ld_h = h.data_ptr(), h.stride(0)
+        g.glu_h, g.ld_h, g.glu_kind = h.data_ptr(), h.stride(0), kind
     g.status, g.stream = nv.status_word(a.device).data_ptr(), nv.stream_ptr()
     return nv.load().lb_gemm_small(ctypes.byref(g))
 
@@ -152,6 +152,24 @@ def test_gated_pair(T, I, keep):
     nv.check_status()
 
 
+@pytest.mark.parametrize("T,N,K", [(1, 8, 64), (65, 72, 1096), (130, 3072, 768)])
+@pytest.mark.parametrize("keep,biased", [(True, True), (False, True), (False, False)])
+def test_gelu_of_a_product(T, N, K, keep, biased):
+    """The bits of the product and a GELU of its own."""
+    from lset_b200.ops.activation import gelu
+
+    torch.manual_seed(N)
+    a, b, bias = _rand(T, K), _rand(N, K) * 0.05, [_rand(N)] if biased else ()
+    for bn, s in [*FORMS, (64 | 64 << 16, 1), (32 | 64 << 16, 4)]:
+        u, c, h = (torch.full((T, N), 3.0, device="cuda", dtype=torch.bfloat16) for _ in range(3))
+        assert _call(a, [b], [u], T, N, K, [N], N_PARTS, bias=bias, bn=bn, splits=s) == 0
+        assert _call(a, [b], [c] if keep else [], T, N, K, [N], N_PARTS, bias=bias, h=h, kind=2, bn=bn,
+                     splits=s) == 0
+        assert torch.equal(h, gelu(u)), (bn, s)
+        assert torch.equal(c, u) if keep else (c == 3).all()
+    nv.check_status()
+
+
 @pytest.mark.parametrize("T", [1, 63, 65, 200])
 @pytest.mark.parametrize("N,K", [(8, 64), (72, 1096), (1024, 200)])
 def test_tiles_of_64_rows(T, N, K):
@@ -189,6 +207,7 @@ def test_shapes_it_does_not_take():
     assert _call(a, [_rand(40, 16), _rand(24, 16)], [c], 8, 16, 64, [40, 24], K_PARTS,
                  b_mn=1) == -3                                          # a k-block over two weights
     assert _call(a, [b], [c.float()], 8, 16, 64, [16], N_PARTS, fp32=1) == -3
+    assert _call(a, [b, b], [], 8, 32, 64, [16, 16], N_PARTS, h=c, kind=2) == -3    # GELU of one product
 
 
 @pytest.mark.parametrize("T,N,K", [(40, 1024, 2048), (304, 768, 3072), (1000, 2048, 1024)])
