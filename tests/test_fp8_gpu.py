@@ -48,6 +48,15 @@ def test_cast_matches_eager(R, C, mode, e5m2):
             assert int(got.data[:, got.cols:].max().item() if got.data.shape[1] > got.cols else 0) == 0
 
 
+@pytest.mark.parametrize("R,C", [(128, 128), (129, 136), (255, 120), (12, 1032), (113, 248)])
+def test_both_outputs_of_a_cast_hold_the_same_bytes(R, C):
+    """Edges of the 128 x 128 tiles and of the blocks of four rows that are transposed in registers."""
+    q, q_t = f8.quantize_fp8(_rand(R, C), f8.PER_TENSOR, e5m2=False, want=True, want_t=True)
+    assert torch.equal(q.data[:, :C].t(), q_t.data[:, :R])
+    assert not q_t.data[:, R:].any()
+    assert q.data[:, :C].view(torch.float8_e4m3fn).float().abs().amax() == 448
+
+
 GEMM_SHAPES = [(128, 256, 128), (256, 512, 256), (300, 264, 208), (1000, 1024, 1024),
                (4096, 3072, 1024), (77, 128, 80), (513, 1032, 528), (23040, 1024, 3072)]
 
