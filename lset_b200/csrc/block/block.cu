@@ -163,15 +163,52 @@ LbSmallGemm small_linear(const LbLinear& l, const __nv_bfloat16* x, long long ld
   return g;
 }
 
+// Adapters: ts_i = s · x · A_iᵀ [T, r] of linears that share their input. One launch reads x for all of them
+// (33280 x 4096, rank 16, for q, k and v: 3 x 66 us and a launch for each scale apart, 98 together; gate and up
+// 74).
+int lora_fwd_products(const LbLinear* l, int n, const __nv_bfloat16* x, long long ldx, int T,
+                      __nv_bfloat16* const* ts, const LbStreamCtx* c) {
+  bool any = false;
+  for (int i = 0; i < n; ++i) any = any || l[i].lora_r > 0;
+  if (!any) return 0;
+  LbSmallGemm g = small_linear(l[0], x, ldx, nullptr, 0, T, c, nullptr);
+  double apart = 0.0;
+  bool same = true;
+  g.N = 0;
+  for (int i = 0; i < n; ++i) {
+    g.B[i] = l[i].lora_a;
+    g.ldb[i] = l[i].k_in;
+    g.C[i] = ts[i];
+    g.ldc[i] = g.ext[i] = l[i].lora_r;
+    g.N += l[i].lora_r;
+    apart += lb_gemm_tile_cost(T, l[i].lora_r, l[i].k_in, 0, 0) + 3.5;
+    same = same && l[i].lora_r > 0 && l[i].k_in == l[0].k_in && l[i].lora_scale == l[0].lora_scale;
+  }
+  g.nparts = n;
+  if (same && l[0].lora_scale != 0.f && small_wins(&g, apart)) {
+    t_fewer += 2 * n - 1;
+    return lb_gemm_small_scaled(&g, l[0].lora_scale);
+  }
+  for (int i = 0; i < n; ++i) {
+    if (l[i].lora_r == 0) continue;
+    if (n > 1) {
+      LB_TRY(lora_fwd_products(l + i, 1, x, ldx, T, ts + i, c));
+      continue;
+    }
+    LB_TRY(lb_gemm_bf16(x, l[i].lora_a, ts[i], T, l[i].lora_r, l[i].k_in, ldx, l[i].k_in, l[i].lora_r, 0, 0, 0,
+                        0, nullptr, 1, 0, c->status, c->stream));
+    LB_TRY(scale_bf16(ts[i], 1LL * T * l[i].lora_r, l[i].lora_scale,
+                      reinterpret_cast<cudaStream_t>(c->stream)));
+  }
+  return 0;
+}
+
 // y[:, :n_out] (row stride ldy) = x · Wᵀ (+ LoRA). `ts` receives s · x · Aᵀ when the linear has adapters.
 int lin_fwd(const LbLinear& l, const __nv_bfloat16* x, long long ldx, __nv_bfloat16* y,
             long long ldy, int T, __nv_bfloat16* ts, const LbStreamCtx* c,
-            const void* bias = nullptr) {
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(c->stream);
+            const void* bias = nullptr, bool ts_ready = false) {
   if (l.lora_r > 0) {
-    LB_TRY(lb_gemm_bf16(x, l.lora_a, ts, T, l.lora_r, l.k_in, ldx, l.k_in, l.lora_r, 0, 0, 0, 0,
-                        nullptr, 1, 0, c->status, c->stream));
-    LB_TRY(scale_bf16(ts, 1LL * T * l.lora_r, l.lora_scale, st));
+    if (!ts_ready) LB_TRY(lora_fwd_products(&l, 1, x, ldx, T, &ts, c));
     return lb_gemm_bf16_ext(x, l.w, ts, l.lora_b, y, T, l.n_out, l.k_in, l.lora_r, ldx, l.ldw,
                             l.lora_r, l.lora_r, ldy, 0, nullptr, c->status, c->stream);
   }
@@ -210,9 +247,19 @@ int lin_dgrad(const LbLinear& l, const __nv_bfloat16* dy, long long lddy, __nv_b
   cudaStream_t st = reinterpret_cast<cudaStream_t>(c->stream);
   const void* peers[1] = {dx};
   if (l.lora_r > 0) {
-    LB_TRY(lb_gemm_bf16(dy, l.lora_b, us, T, l.lora_r, l.n_out, lddy, l.lora_r, l.lora_r, 0, 1, 0, 0,
-                        nullptr, 1, 0, c->status, c->stream));
-    LB_TRY(scale_bf16(us, 1LL * T * l.lora_r, l.lora_scale, st));
+    LbSmallGemm g = small_linear(l, dy, lddy, us, l.lora_r, T, c, nullptr);
+    g.B[0] = l.lora_b;
+    g.ldb[0] = g.N = g.ext[0] = l.lora_r;
+    g.K = l.n_out;
+    g.b_mn = 1;
+    if (l.lora_scale != 0.f && small_wins(&g, lb_gemm_tile_cost(T, l.lora_r, l.n_out, 0, 0) + 3.5)) {
+      ++t_fewer;
+      LB_TRY(lb_gemm_small_scaled(&g, l.lora_scale));
+    } else {
+      LB_TRY(lb_gemm_bf16(dy, l.lora_b, us, T, l.lora_r, l.n_out, lddy, l.lora_r, l.lora_r, 0, 1, 0, 0,
+                          nullptr, 1, 0, c->status, c->stream));
+      LB_TRY(scale_bf16(us, 1LL * T * l.lora_r, l.lora_scale, st));
+    }
     if (!accumulate)
       return lb_gemm_bf16_ext(dy, l.w, us, l.lora_a, dx, T, l.k_in, l.n_out, l.lora_r, lddy, l.ldw,
                               l.lora_r, l.k_in, l.k_in, 1, nullptr, c->status, c->stream);
@@ -302,8 +349,9 @@ int proj_fwd(const LbProjection& p, const __nv_bfloat16* x, long long ldx, __nv_
       return lb_gemm_small(&g);
     }
   }
+  LB_TRY(lora_fwd_products(p.part, p.n, x, ldx, T, ts, c));
   for (int i = 0; i < p.n; ++i) {
-    LB_TRY(lin_fwd(p.part[i], x, ldx, y, p.width, T, ts[i], c, bias != nullptr ? bias[i] : nullptr));
+    LB_TRY(lin_fwd(p.part[i], x, ldx, y, p.width, T, ts[i], c, bias != nullptr ? bias[i] : nullptr, true));
     y += p.part[i].n_out;
   }
   return 0;

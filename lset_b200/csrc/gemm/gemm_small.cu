@@ -49,6 +49,7 @@ struct SmallArgs {
   const __nv_bfloat16* bias[3];
   void* glu_h;
   long long ld_h;
+  float scale;      // of the rounded product (0: none)
   int b_ready;
   int by_part;      // kParallelK of several parts: CTA r of a cluster contracts part r
   int block_bytes;  // what the loads of one k-block bring
@@ -395,6 +396,15 @@ __global__ void __launch_bounds__(kThreads)
       pk.y = pack_bf16x2(a0.z, a0.w);
       pk.z = pack_bf16x2(a1.x, a1.y);
       pk.w = pack_bf16x2(a1.z, a1.w);
+      if (!GLU && g.scale != 0.f) {
+        uint32_t w[4] = {pk.x, pk.y, pk.z, pk.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 v = unpack_bf16x2(w[j]);
+          w[j] = pack_bf16x2(v.x * g.scale, v.y * g.scale);
+        }
+        pk = make_uint4(w[0], w[1], w[2], w[3]);
+      }
       const long long grow = m0 + row;
       if constexpr (PAIR) {
         const float4 u0 = cluster_sum4(base, off + BN / 2 * 4u, S);
@@ -661,9 +671,11 @@ extern "C" double lb_gemm_small_plan(const LbSmallGemm* p, int* bn_out, int* spl
   return best;
 }
 
-extern "C" int lb_gemm_small(const LbSmallGemm* p) {
+extern "C" int lb_gemm_small(const LbSmallGemm* p) { return lb_gemm_small_scaled(p, 0.f); }
+
+extern "C" int lb_gemm_small_scaled(const LbSmallGemm* p, float scale) {
   if (p->M <= 0 || p->N <= 0) return 0;
-  if (!shape_ok(p)) return -3;
+  if (!shape_ok(p) || (scale != 0.f && (p->out_fp32 || p->glu_h != nullptr))) return -3;
   // tile: columns, and rows in the upper half (0: 128)
   int tile = p->bn, splits = p->splits;
   if (tile == 64 || tile == 128) tile |= 128 << 16;
@@ -734,6 +746,7 @@ extern "C" int lb_gemm_small(const LbSmallGemm* p) {
   const int tiles = count_tiles(p, BM, bn, &g.tiles_n);
   g.glu_h = p->glu_h;
   g.ld_h = p->ld_h;
+  g.scale = scale;
   g.b_ready = p->b_ready && pdl_enabled();
   g.by_part = by_part(p);
   g.block_bytes = (a_box + b_box) * BK * 2;

@@ -42,6 +42,8 @@ struct LbSmallGemm {
 double lb_gemm_small_plan(const LbSmallGemm* p, int* bn, int* splits);
 double lb_gemm_tile_cost(int M, int N, int K, int fp32, int bias);
 int lb_gemm_small(const LbSmallGemm* p);
+// The same, a bf16 result (not an activation's) rounded, multiplied by `scale` and rounded again; 0: not.
+int lb_gemm_small_scaled(const LbSmallGemm* p, float scale);
 
 }  // extern "C"
 

@@ -20,7 +20,7 @@ class SmallGemm(ctypes.Structure):      # LbSmallGemm of csrc/gemm/gemm_small.h
                 ("b_ready", _ci), ("may_split", _ci), ("bn", _ci), ("splits", _ci), ("status", _vp), ("stream", _vp)]
 
 
-def _call(a, bs, cs, M, N, K, ext, mode, a_mn=0, b_mn=0, fp32=0, bias=(), h=None, bn=0, splits=0, kind=0):
+def _call(a, bs, cs, M, N, K, ext, mode, a_mn=0, b_mn=0, fp32=0, bias=(), h=None, bn=0, splits=0, kind=0, scale=None):
     g = SmallGemm()
     g.A, g.lda = a.data_ptr(), a.stride(0)
     for i, b in enumerate(bs):
@@ -36,6 +36,8 @@ def _call(a, bs, cs, M, N, K, ext, mode, a_mn=0, b_mn=0, fp32=0, bias=(), h=None
     if h is not None:
         g.glu_h, g.ld_h, g.glu_kind = h.data_ptr(), h.stride(0), kind
     g.status, g.stream = nv.status_word(a.device).data_ptr(), nv.stream_ptr()
+    if scale is not None:
+        return nv.load().lb_gemm_small_scaled(ctypes.byref(g), ctypes.c_float(scale))
     return nv.load().lb_gemm_small(ctypes.byref(g))
 
 
@@ -167,6 +169,20 @@ def test_gelu_of_a_product(T, N, K, keep, biased):
                      splits=s) == 0
         assert torch.equal(h, gelu(u)), (bn, s)
         assert torch.equal(c, u) if keep else (c == 3).all()
+    nv.check_status()
+
+
+@pytest.mark.parametrize("T", [1, 130, 5000])
+@pytest.mark.parametrize("ext,b_mn", [([16, 16, 16], 0), ([8, 64], 0), ([16], 1)])
+def test_scaled_products_are_rounded_before_and_after(T, ext, b_mn):
+    K = 512
+    a, bs = _rand(T, K), [_rand(K, e) if b_mn else _rand(e, K) for e in ext]
+    for bn, s in [*FORMS, (64 | 64 << 16, 1)]:
+        c, d = ([torch.full((T, e), 3.0, device="cuda", dtype=torch.bfloat16) for e in ext] for _ in range(2))
+        assert _call(a, bs, c, T, sum(ext), K, ext, N_PARTS, b_mn=b_mn, bn=bn, splits=s) == 0
+        assert _call(a, bs, d, T, sum(ext), K, ext, N_PARTS, b_mn=b_mn, bn=bn, splits=s, scale=0.3) == 0
+        for x, y in zip(c, d):
+            assert torch.equal(y, (x.float() * 0.3).to(torch.bfloat16)), (bn, s)
     nv.check_status()
 
 
