@@ -16,9 +16,10 @@ using bf16 = __nv_bfloat16;
 constexpr int kBatch = 40;       // buffers of one launch (its arguments hold the list)
 constexpr int kChunk = 4096;     // elements of one CTA at a time
 
+// Buffers of one launch, and the work items in front of each: chunks of the update, CTAs of the sums.
 struct Groups {
   LbOptGroup g[kBatch];
-  long long first[kBatch + 1];   // chunks in front of each buffer
+  long long first[kBatch + 1];
   int n;
 };
 
@@ -28,51 +29,67 @@ __device__ __forceinline__ long long find_chunk(const Groups& a, long long c, in
   return c - a.first[at];
 }
 
+// The sums of squares have one order, which depends on the sizes of the buffers alone and on no other
+// buffer in front: within a buffer a walk of its own, then its CTAs, then the buffers one after the other. The
+// clip coefficient multiplies every gradient, and a model of many layers turns one weight that is rounded to
+// another bf16 value for its sake into a loss of the next step that differs by up to some per cent in small
+// batches. (One walk over all buffers, in which a thread's sum runs from one to the next, has other last bits
+// with every other list.)
+//
+// Bound by memory: four loads of a thread are requested together.
 __global__ void __launch_bounds__(256)
     sumsq_partial_kernel(const __grid_constant__ Groups a, float* __restrict__ partial) {
   __shared__ float sred[8];
-  float s[2] = {0.f, 0.f};
   int at = 0;
-  for (long long c = blockIdx.x; c < a.first[a.n]; c += gridDim.x) {
-    const long long e0 = find_chunk(a, c, at) * kChunk;
-    const LbOptGroup& g = a.g[at];
-    const float* x = g.g + e0;
-    const int n = int(g.n - e0 < kChunk ? g.n - e0 : kChunk);
-    float t = 0.f;
-    if (n == kChunk) {
-      float4 v[4];
+  const long long cta = find_chunk(a, blockIdx.x, at);
+  const long long ctas = a.first[at + 1] - a.first[at];
+  const float* x = a.g[at].g;
+  const long long n = a.g[at].n, n4 = n / 4, step = ctas * 256;
+  const float4* x4 = reinterpret_cast<const float4*>(x);
+  float s = 0.f;
+  auto add = [&](const float4& v) { s += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w; };
+  long long i = cta * 256 + threadIdx.x;
+  for (; i + 3 * step < n4; i += 4 * step) {
+    float4 v[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) v[i] = reinterpret_cast<const float4*>(x)[i * 256 + threadIdx.x];
+    for (int j = 0; j < 4; ++j) v[j] = x4[i + j * step];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) t += v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
-    } else {
-      for (int i = threadIdx.x; i < n; i += 256) t += x[i] * x[i];
-    }
-    s[0] += g.slot == 0 ? t : 0.f;
-    s[1] += g.slot == 0 ? 0.f : t;
+    for (int j = 0; j < 4; ++j) add(v[j]);
   }
-#pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    const float t = row_sum<256>(s[k], sred);
-    if (threadIdx.x == 0) partial[2 * blockIdx.x + k] = t;
-    __syncthreads();
+  for (; i < n4; i += step) add(x4[i]);
+  if (cta == 0) {
+    for (long long j = n4 * 4 + threadIdx.x; j < n; j += 256) s += x[j] * x[j];
   }
+  s = row_sum<256>(s, sred);
+  if (threadIdx.x == 0) partial[blockIdx.x] = s;
 }
 
-// out[k] = sum of the partial sums of slot k.
+// sums[b], a CTA for each buffer: its sum in the component of its slot.
 __global__ void __launch_bounds__(256)
-    sumsq_final_kernel(const float* __restrict__ partial, int P, float* __restrict__ out) {
+    sumsq_buffer_kernel(const __grid_constant__ Groups a, const float* __restrict__ partial,
+                        float2* __restrict__ sums) {
   __shared__ float sred[8];
-  float s[2] = {0.f, 0.f};
-  for (int i = threadIdx.x; i < P; i += blockDim.x) {
-    s[0] += partial[2 * i];
-    s[1] += partial[2 * i + 1];
-  }
+  const int b = blockIdx.x;
+  float s = 0.f;
+  for (long long i = a.first[b] + threadIdx.x; i < a.first[b + 1]; i += 256) s += partial[i];
+  s = row_sum<256>(s, sred);
+  if (threadIdx.x == 0) sums[b] = a.g[b].slot == 0 ? make_float2(s, 0.f) : make_float2(0.f, s);
+}
+
+// out[k] = sum of the buffers' sums of slot k, one after the other.
+__global__ void sumsq_final_kernel(const float2* __restrict__ sums, int n, float* __restrict__ out) {
+  float2 t = make_float2(0.f, 0.f);
+  for (int b0 = 0; b0 < n; b0 += 32) {
+    const float2 v = b0 + int(threadIdx.x) < n ? sums[b0 + threadIdx.x] : make_float2(0.f, 0.f);
 #pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    const float t = row_sum<256>(s[k], sred);
-    if (threadIdx.x == 0) out[k] = t;
-    __syncthreads();
+    for (int l = 0; l < 32; ++l) {
+      t.x += __shfl_sync(0xffffffffu, v.x, l);
+      t.y += __shfl_sync(0xffffffffu, v.y, l);
+    }
+  }
+  if (threadIdx.x == 0) {
+    out[0] = t.x;
+    out[1] = t.y;
   }
 }
 
@@ -160,19 +177,26 @@ __global__ void __launch_bounds__(256) adamw_kernel(const __grid_constant__ Grou
   }
 }
 
-// The next buffers of a list that one launch takes.
-int take_groups(const LbOptGroup* groups, int count, int from, Groups* a) {
+// The next buffers of a list that one launch takes; `items`: work items of a buffer of n elements.
+template <typename Items>
+int take_groups(const LbOptGroup* groups, int count, int from, Groups* a, Items items) {
   *a = Groups{};
-  long long chunks = 0;
+  long long total = 0;
   int i = from;
   for (; i < count && a->n < kBatch; ++i) {
     if (groups[i].n <= 0) continue;
-    a->first[a->n] = chunks;
+    a->first[a->n] = total;
     a->g[a->n++] = groups[i];
-    chunks += (groups[i].n + kChunk - 1) / kChunk;
+    total += items(groups[i].n);
   }
-  a->first[a->n] = chunks;
+  a->first[a->n] = total;
   return i;
+}
+
+// CTAs that a buffer's sum of squares is cut into.
+int sumsq_ctas(long long n) {
+  const long long need = (n / 4 + 255) / 256, cap = 4LL * row_num_sms();
+  return int(need < 1 ? 1 : (need > cap ? cap : need));
 }
 
 bool aligned(const void* p, uintptr_t mask) { return (reinterpret_cast<uintptr_t>(p) & mask) == 0; }
@@ -182,29 +206,31 @@ bool aligned(const void* p, uintptr_t mask) { return (reinterpret_cast<uintptr_t
 
 using namespace lb;
 
-// Floats of scratch for the sum of squares over `count` buffers.
+// Floats of scratch for the sums of squares of `count` buffers: two of each, then its CTAs' partial sums.
 extern "C" int lb_sumsq_scratch_floats(int count) {
-  const int launches = (count + kBatch - 1) / kBatch;
-  return 2 * row_num_sms() * 4 * (launches > 0 ? launches : 1);
+  return (count > 0 ? count : 1) * (2 + 4 * row_num_sms());
 }
 
-// out[k] = sum(g^2) over the buffers of slot k (0, 1).
+// out[k] = sum(g^2) over the buffers of slot k (0, 1). scratch: 8-byte aligned.
 extern "C" int lb_sumsq_groups(const LbOptGroup* groups, int count, float* scratch, float* out,
                                void* stream) {
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  const int cap = row_num_sms() * 4;
-  int rows = 0;
+  if (!aligned(scratch, 7u)) return -3;
+  float2* sums = reinterpret_cast<float2*>(scratch);
+  float* partial = scratch + 2LL * (count > 0 ? count : 1);
+  int buffers = 0;
   for (int i = 0; i < count; ++i)
     if (!aligned(groups[i].g, 15u)) return -3;
   for (int from = 0; from < count;) {
     Groups a;
-    from = take_groups(groups, count, from, &a);
+    from = take_groups(groups, count, from, &a, sumsq_ctas);
     if (a.n == 0) break;
-    const int grid = int(a.first[a.n] < cap ? a.first[a.n] : cap);
-    sumsq_partial_kernel<<<grid, 256, 0, st>>>(a, scratch + 2 * rows);
-    rows += grid;
+    sumsq_partial_kernel<<<unsigned(a.first[a.n]), 256, 0, st>>>(a, partial);
+    sumsq_buffer_kernel<<<a.n, 256, 0, st>>>(a, partial, sums + buffers);
+    partial += a.first[a.n];
+    buffers += a.n;
   }
-  sumsq_final_kernel<<<1, 256, 0, st>>>(scratch, rows, out);
+  sumsq_final_kernel<<<1, 32, 0, st>>>(sums, buffers, out);
   return launch_rc();
 }
 
@@ -237,7 +263,7 @@ extern "C" int lb_adamw_groups(const LbOptGroup* groups, int count, float lr, fl
   const long long cap = 1LL * row_num_sms() * 16;
   for (int from = 0; from < count;) {
     Groups list;
-    from = take_groups(groups, count, from, &list);
+    from = take_groups(groups, count, from, &list, [](long long n) { return (n + kChunk - 1) / kChunk; });
     if (list.n == 0) break;
     const long long chunks = list.first[list.n];
     adamw_kernel<<<int(chunks < cap ? chunks : cap), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(

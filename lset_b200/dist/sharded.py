@@ -753,7 +753,7 @@ class ShardedAdamW:
             rc = lib.lb_sumsq_groups(groups, nv.c_int(len(groups)), nv.c_void_p(scr.data_ptr()),
                                      nv.c_void_p(parts.data_ptr()), nv.c_void_p(nv.stream_ptr()))
             nv.check_rc(rc, "lb_sumsq_groups")
-            nv.count_launch(2)
+            nv.count_launch(3)
         else:
             parts.zero_()
             for g in st.groups:

@@ -46,3 +46,29 @@ def test_lists_of_buffers(sizes):
             assert torch.allclose(got.double(), ref, rtol=2e-6, atol=2e-6)
         assert torch.equal(low[i], p[i].to(torch.bfloat16))
         assert not g[i].any()
+
+
+def _sums_of_squares(lib, tensors, slots):
+    groups = (LbOptGroup * len(tensors))()
+    for e, t, slot in zip(groups, tensors, slots):
+        e.g, e.n, e.slot = t.data_ptr(), t.numel(), slot
+    n = nv.c_int(len(tensors))
+    scratch = torch.empty(lib.lb_sumsq_scratch_floats(n), device="cuda")
+    out = torch.empty(2, device="cuda")
+    assert lib.lb_sumsq_groups(groups, n, nv.c_void_p(scratch.data_ptr()), nv.c_void_p(out.data_ptr()),
+                               nv.c_void_p(nv.stream_ptr())) == 0
+    return out.cpu()
+
+
+def test_sums_of_squares_are_added_buffer_by_buffer():
+    """Bits of the gradient norm, hence of every clipped step: the sum of each buffer by itself (whatever else
+    is in the list), one after the other."""
+    torch.manual_seed(0)
+    lib = nv.load()
+    tensors = [torch.randn(5 + 7919 * i, device="cuda") for i in range(60)]
+    tensors += [torch.randn(5_000_003, device="cuda"), torch.randn(8, device="cuda")]
+    slots = [int(i % 5 == 2) for i in range(len(tensors))]
+    want = torch.zeros(2)
+    for t, slot in zip(tensors, slots):
+        want[slot] += _sums_of_squares(lib, [t], [slot])[slot]
+    assert torch.equal(_sums_of_squares(lib, tensors, slots), want)
