@@ -890,21 +890,22 @@ int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmArgs& g, in
 // the fp32 reduction epilogue of an item, hidden behind the next item's main loop only when that
 // is at least as long. More splits mean more reduction traffic, so a candidate must win by 2 %.
 int auto_splits(long long tiles, int kb_total, int sms) {
-  // In k-blocks: the last epilogue, and what every epilogue adds to its wave although the next tile runs under
-  // it. (Without the latter 4096 x 1024 x 22627 was cut in eight for its last wave's sake: 171 us, 162 whole;
-  // 6144 x 1024 x 40280 in ten, 428, in three 415; 1024 x 2048 x 22627 in nine, 88, in two 86.)
-  constexpr int kEpi = 32, kEach = 8, kMinKb = 32;
-  if (kb_total < 2 * kMinKb) return 1;
+  // How a gradient is cut shows in its last bits, and through the clip coefficient in every weight of the step.
+  // (A model that also counts what an epilogue adds to its wave cuts some less: 4096 x 1024 x 22627 whole and not
+  // in eight, 162 for 171 us; 6144 x 1024 x 40280 415 for 428. It moved the loss of the third step of 12 pairs
+  // on two layers of width 2560 by 0.8 %, and was taken back.)
+  constexpr int kEpi = 32;
+  if (kb_total < kLongSum) return 1;
   int best = 1;
   double best_cost = 1e30;
   for (int s = 1; s <= 32; ++s) {
     const int kb_per = (kb_total + s - 1) / s;
-    if (s > 1 && kb_per < kMinKb) break;
+    if (s > 1 && kb_per < kLongSum / 2) break;
     const int se = (kb_total + kb_per - 1) / kb_per;
     const long long items = tiles * se;
     const long long waves = (items + sms - 1) / sms;
-    const double cost = double(waves) * ((kb_per > kEpi ? kb_per : kEpi) + kEach) + kEpi;
-    if (cost < best_cost * 0.995) {
+    const double cost = double(waves) * (kb_per > kEpi ? kb_per : kEpi) + kEpi;
+    if (cost < best_cost * 0.98) {
       best = se;
       best_cost = cost;
     }
@@ -991,6 +992,10 @@ static int one_cta_bn(int M, int N) {
 // smaller than a pair's tile) 0.3 with 256 columns a tile and 0.22 with 128; the bytes bound both. With a
 // bias (one-CTA kernel at any size) the store of a tile of 256 columns takes 5 us (650 x 3072 x 768 11.8 us,
 // here 11.6; the model without it said 8.2 and lost to the small kernel's 8.0 only on paper).
+//
+// Of a weight gradient over kLongSum k-blocks or more the choice decides whether it is summed whole or in
+// pieces, that is its bits. So there both models are the ones that training runs have been drawn by, see
+// long_sum_cost (gemm_small.cu).
 extern "C" double lb_gemm_tile_cost(int M, int N, int K, int fp32, int bias) {
   const bool pair = M >= 256 && N >= 256 && !bias;
   const int bm = pair ? 256 : lb::BM, bn = pair ? 256 : one_cta_bn(M, N);
@@ -999,9 +1004,12 @@ extern "C" double lb_gemm_tile_cost(int M, int N, int K, int fp32, int bias) {
   const int kb = (K + lb::BK - 1) / lb::BK;
   const int s = fp32 ? lb::auto_splits(tiles, kb, slots) : 1;
   const long long waves = (tiles * s + slots - 1) / slots;
+  const int depth = (kb + s - 1) / s;
+  if (fp32 && kb >= kLongSum)
+    return 11.0 + double(waves) * depth * (pair ? 0.33 : (bn == 256 ? 0.37 : 0.27)) + (s > 1 ? 4.0 : 0.0);
   const double block = pair ? 0.35 : (bn == 256 ? (bias ? 0.28 : 0.3) : (bias ? 0.15 : 0.22));
   const double store = bias && bn == 256 ? 5.0 : (bias ? 2.5 : 2.2);
-  const double cost = 3.2 + double(waves) * (((kb + s - 1) / s) * block + store) + (s > 1 ? 0.6 : 0.0);
+  const double cost = 3.2 + double(waves) * (depth * block + store);
   const double memory =
       3.0 + (2.0 * K * (double(M) + N) + (fp32 ? 8.0 : 2.0) * double(M) * N) / 3.73e6;
   return cost > memory ? cost : memory;

@@ -567,6 +567,25 @@ bool shape_ok(const LbSmallGemm* p) {
   return true;
 }
 
+// Modelled time of a weight gradient over kLongSum k-blocks or more, for the comparison with the tile kernels
+// alone: which of them takes it decides whether it is summed whole or in pieces, hence its bits and, through the
+// clip coefficient, those of every weight of the step. So this and its counterpart in lb_gemm_tile_cost stay
+// as they were fitted first (128-row tiles in rings of four and three stages), whatever the kernel has become
+// since.
+double long_sum_cost(const LbSmallGemm* p, int kb) {
+  double best = 1e30;
+  for (int bn = 64; bn <= 128; bn += 64) {
+    int tn;
+    const int tiles = count_tiles(p, 128, bn, &tn);
+    const double waves = ceil_div(tiles, 2 * small_sms()), per_sm = ceil_div(tiles, small_sms());
+    const double block = per_sm * (128 + bn) * 2.0, latency = waves * 2600.0 / (bn == 64 ? 4.0 : 3.0);
+    const double cost =
+        2.0 + waves * (1.1 + 1.8 * 128 * bn / 8192.0) + kb * (block > latency ? block : latency) / 1900.0;
+    if (cost < best) best = cost;
+  }
+  return best;
+}
+
 template <int A_MN, int B_MN, int BM, int BN, typename OutT, int GLU>
 int launch_small(const CUtensorMap& tA, const CUtensorMap* tB, const SmallArgs& g, int grid,
                  cudaStream_t st) {
@@ -668,7 +687,7 @@ extern "C" double lb_gemm_small_plan(const LbSmallGemm* p, int* bn_out, int* spl
       }
     }
   }
-  return best;
+  return p->out_fp32 && kb >= kLongSum ? long_sum_cost(p, kb) : best;
 }
 
 extern "C" int lb_gemm_small(const LbSmallGemm* p) { return lb_gemm_small_scaled(p, 0.f); }

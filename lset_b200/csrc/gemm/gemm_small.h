@@ -36,6 +36,9 @@ struct LbSmallGemm {
   void* stream;
 };
 
+// From this many k-blocks of 64 on the tile kernels may add up a weight gradient in pieces.
+enum { kLongSum = 64 };
+
 // Modelled time of the product on this kernel and the tile width and split it would take (a negative
 // value: not taken), and of one product on the CTA-pair kernel (fp32: a weight gradient, whose
 // contraction that kernel splits; bias: the one-CTA kernel's, which adds it).

@@ -274,3 +274,39 @@ def test_gated_pair_on_cta_pairs(T, I, K, kind, keep):
     nv.check_status()
     assert torch.equal(h, want)
     assert torch.equal(got, gu) if keep else torch.isnan(got).all()
+
+
+@pytest.mark.parametrize("M,N,T,half", [(2560, 9728, 5157, 2688), (768, 768, 5096, 2560), (16, 12288, 4096, 2048)])
+def test_weight_gradients_over_many_tokens_keep_their_two_pieces(M, N, T, half):
+    """Bits of a training step: the first ``half`` of the tokens (whole k-blocks of the kernel's) and the others,
+    each summed by itself. (Three pieces and more are added up as they come.)"""
+    from lset_b200.ops.gemm import matmul_abt
+
+    torch.manual_seed(T)
+    dy, x = _rand(T, M), _rand(T, N)
+
+    def grad(rows):
+        out = torch.zeros(M, N, device="cuda")
+        return matmul_abt(dy[rows], x[rows], a_mn=True, b_mn=True, out=out, accumulate=True, splits=0)
+
+    assert torch.equal(grad(slice(0, T)), grad(slice(0, half)).add_(grad(slice(half, T))))
+    nv.check_status()
+
+
+@pytest.mark.parametrize("ext,N,T,whole", [
+    ([2048, 1024, 1024], 1024, 9096, True), ([2048, 1024, 1024], 1024, 12096, False),
+    ([768, 256, 256], 768, 13096, True), ([768, 256, 256], 768, 14096, False),
+    ([2048, 512, 512], 2048, 5096, True), ([768, 768, 768], 768, 11096, True)])
+def test_which_joint_weight_gradients_are_summed_whole(ext, N, T, whole):
+    lib, g = nv.load(), SmallGemm()
+    g.A = g.B[0] = 4096
+    g.lda, g.ldb[0] = sum(ext), N
+    for i, e in enumerate(ext):
+        g.C[i], g.ldc[i], g.ext[i] = 4096, N, e
+    g.M, g.N, g.K, g.nparts, g.mode = sum(ext), N, T, len(ext), M_PARTS
+    g.a_mn = g.b_mn = g.out_fp32 = 1
+    plan, tile = lib.lb_gemm_small_plan, lib.lb_gemm_tile_cost
+    plan.restype = tile.restype = ctypes.c_double
+    cost = plan(ctypes.byref(g), ctypes.byref(_ci()), ctypes.byref(_ci()))
+    apart = sum(tile(_ci(e), _ci(N), _ci(T), _ci(1), _ci(0)) for e in ext)
+    assert (0 <= cost < apart) == whole
