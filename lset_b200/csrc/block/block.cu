@@ -806,7 +806,7 @@ static int block_bwd(const LbBlockDesc* d, const LbStreamCtx* c, const LbBlockIO
   // the norms' weight gradients out of their kernels' partial sums: one launch for all of them
   LbColsum sums[kMaxColsums];
   int n = 0;
-  const int rows = lb_rms_bwd_rows(T, H);
+  const int rows = lb_norm_bwd_rows(T, H);
   if (d->ln2_wgrad != nullptr) sums[n++] = {c->norm_scratch, rows, H, d->ln2_wgrad, nullptr, 0};
   if (d->ln1_wgrad != nullptr) sums[n++] = {sums1, rows, H, d->ln1_wgrad, nullptr, 0};
   if (want_dw)
@@ -985,7 +985,7 @@ extern "C" int lb_encoder_bwd(const LbEncoderDesc* d, const LbStreamCtx* c, LbBl
   // both norms' weight and bias gradients out of their kernels' partial sums
   LbColsum sums[2];
   int k = 0;
-  const int rows = lb_layer_norm_bwd_rows(T, H);
+  const int rows = lb_norm_bwd_rows(T, H);
   if (d->ln2_wgrad != nullptr || d->ln2_bgrad != nullptr)
     sums[k++] = {c->norm_scratch, rows, 2 * H, d->ln2_wgrad, d->ln2_bgrad, H};
   if (d->ln1_wgrad != nullptr || d->ln1_bgrad != nullptr)

@@ -17,8 +17,7 @@ struct LbColsum {
 };
 enum { kMaxColsums = 3 };
 int lb_colsums(const LbColsum* jobs, int n, void* stream);
-int lb_rms_bwd_rows(int N, int H);
-int lb_layer_norm_bwd_rows(int N, int H);
+int lb_norm_bwd_rows(int N, int H);
 int lb_rope_bwd_rows(int T, int Hq, int Hk, int hd);
 
 // row/norm.cu

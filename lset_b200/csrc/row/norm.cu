@@ -187,17 +187,19 @@ __device__ __forceinline__ float row_sum_alt(float v, float (&sred)[2][8], int s
 }
 
 // Bound by memory where enough rows are in flight. x and dy stay packed in registers (unpacked twice) and
-// the weights in shared memory, so that only the dW accumulators live as long as the CTA: 64 registers, four
-// CTAs a SM, one wave of them. Four columns of a thread are next to its neighbour's in shared memory (eight in
+// the weights in shared memory, so that only the dW accumulators live as long as the CTA: three CTAs a SM (two
+// above 4096 columns). Four columns of a thread are next to its neighbour's in shared memory (eight in
 // a row cost every access twice its banks); two columns an instruction; one barrier a row.
-// Measured before (three CTAs, two waves) / now (us, L2 flushed): 22627 x 1024 53 / 45, 33280 x 4096 201 / 180,
-// 21000 x 2560 107 / 92, 5000 x 8192 104 / 84. (A warp a row, with no barrier, needs twice the
-// registers: 59 at 22627 x 1024.)
+// Measured before / now (us, L2 flushed): 22627 x 1024 53 / 49, 40280 x 1024 76 / 72, 33280 x 4096 201 / 197,
+// 21000 x 2560 107 / 105, 5000 x 8192 104 / 92. (A warp a row, with no barrier, needs twice the
+// registers: 59 at 22627 x 1024.) One wave of four CTAs a SM, which 64 registers allow, takes 45, 68, 179, 92 and
+// 84, but cuts the sums of dW into other partial rows: the gradient norm then has other last bits, and every
+// weight of a clipped step.
 template <int TPR, int NV>
 constexpr int rms_bwd_smem(int H) { return (H + 8 * TPR * NV) * int(sizeof(float)); }
 
 template <int TPR, int NV>
-__global__ void __launch_bounds__(kRowThreads, NV > 2 ? 2 : 4)
+__global__ void __launch_bounds__(kRowThreads, NV > 2 ? 2 : 3)
     rms_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ dres,
                    const bf16* __restrict__ xin, const bf16* __restrict__ w,
                    const float* __restrict__ rstd_in, bf16* __restrict__ dx,
@@ -534,12 +536,13 @@ int launch_colsum(const float* partial, int P, int C, void* out, int out_fp32, i
   return launch_colsums(&job, 1, out_fp32, accumulate, st);
 }
 
-// CTAs of the backward kernels for each SM: one wave of rms_bwd_kernel, two of ln_bwd_kernel.
-constexpr int kRmsBwdPerSm = 4, kLayerNormBwdPerSm = 6;
+// CTAs of the backward kernels for each SM, and so the partial rows that their weight gradients are cut into: part of
+// the bits of a training step.
+constexpr int kBwdPerSm = 6;
 
-int bwd_grid(int N, int rows_per_cta, int per_sm) {
+int bwd_grid(int N, int rows_per_cta) {
   const int need = (N + rows_per_cta - 1) / rows_per_cta;
-  const int cap = row_num_sms() * per_sm;
+  const int cap = row_num_sms() * kBwdPerSm;
   return need < cap ? (need > 0 ? need : 1) : cap;
 }
 
@@ -599,7 +602,7 @@ extern "C" int lb_rms_norm_bwd(const void* dy, const void* dres, const void* xin
   int grid = 1;
   LB_ROW_DISPATCH_NARROW(H, {
     constexpr int ROWS = kRowThreads / TPR;
-    grid = bwd_grid(N, ROWS, kRmsBwdPerSm);
+    grid = bwd_grid(N, ROWS);
     constexpr auto smem = rms_bwd_smem<TPR, NV>;
     if (smem(H) > 48 * 1024)  // wide rows: opt in above the 48 KB default
       cudaFuncSetAttribute(rms_bwd_kernel<TPR, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -617,15 +620,10 @@ extern "C" int lb_rms_norm_bwd(const void* dy, const void* dres, const void* xin
   return launch_rc();
 }
 
-// Partial rows that the backward kernels leave in their scratch for N rows of width H.
-extern "C" int lb_rms_bwd_rows(int N, int H) {
+// Partial rows that either norm's backward leaves in its scratch for N rows of width H.
+extern "C" int lb_norm_bwd_rows(int N, int H) {
   if (N <= 0 || H <= 0) return 0;
-  LB_ROW_DISPATCH_NARROW(H, { return bwd_grid(N, kRowThreads / TPR, kRmsBwdPerSm); });
-  return 0;
-}
-extern "C" int lb_layer_norm_bwd_rows(int N, int H) {
-  if (N <= 0 || H <= 0) return 0;
-  LB_ROW_DISPATCH_NARROW(H, { return bwd_grid(N, kRowThreads / TPR, kLayerNormBwdPerSm); });
+  LB_ROW_DISPATCH_NARROW(H, { return bwd_grid(N, kRowThreads / TPR); });
   return 0;
 }
 
@@ -655,7 +653,7 @@ extern "C" int lb_layer_norm_bwd(const void* dy, const void* dres, const void* x
   int grid = 1;
   LB_ROW_DISPATCH_NARROW(H, {
     constexpr int ROWS = kRowThreads / TPR;
-    grid = bwd_grid(N, ROWS, kLayerNormBwdPerSm);
+    grid = bwd_grid(N, ROWS);
     if (2 * H * sizeof(float) > 48 * 1024)
       cudaFuncSetAttribute(ln_bwd_kernel<TPR, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            2 * H * (int)sizeof(float));
@@ -750,7 +748,7 @@ extern "C" int lb_rms_norm_bwd_noalloc(const void* dy, const void* dres, const v
   int grid = 1;
   LB_ROW_DISPATCH_NARROW(H, {
     constexpr int ROWS = kRowThreads / TPR;
-    grid = bwd_grid(N, ROWS, kRmsBwdPerSm);
+    grid = bwd_grid(N, ROWS);
     if (grid > LB_NOALLOC_MAX_PARTIAL_ROWS) grid = LB_NOALLOC_MAX_PARTIAL_ROWS;
     constexpr auto smem = rms_bwd_smem<TPR, NV>;
     if (smem(H) > 48 * 1024)  // wide rows: opt in above the 48 KB default

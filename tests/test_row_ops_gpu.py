@@ -377,3 +377,35 @@ def test_rows_of_many_have_the_bits_of_few(op):
         for a, b in zip(run(slice(at, at + n)), whole):
             assert torch.equal(a, b[at:at + n]), n
         at += n
+
+
+@pytest.mark.parametrize("N_,H", [(1, 1032), (700, 1032), (3000, 1032), (2, 2056), (2500, 2056)])
+def test_rms_norm_weight_gradient_is_summed_in_one_order(N_, H):
+    """Bits of a training step (the gradient norm, and through the clip coefficient every weight): six partial rows
+    an SM, each of them the sums of its rows (two at a time up to 2048 columns), then every 32nd partial row,
+    then those. bf16 products are exact in fp32."""
+    torch.manual_seed(H)
+    x, dy, w = _r(N_, H), _r(N_, H), _r(H, scale=0.5)
+    rstd, dx = torch.rand(N_, device="cuda") + 0.5, torch.empty_like(x)
+    lib = nv.load()
+    scratch = torch.empty(lib.lb_norm_bwd_partial_rows() * H, device="cuda")
+    dw = torch.empty(H, device="cuda")
+    p = lambda t: nv.c_void_p(t.data_ptr())  # noqa: E731
+    assert lib.lb_rms_norm_bwd(p(dy), nv.c_void_p(0), p(x), p(w), p(rstd), p(dx), p(scratch), p(dw), nv.c_int(1),
+                               nv.c_int(0), nv.c_int(N_), nv.c_int(H), nv.c_float(0.0),
+                               nv.c_void_p(nv.stream_ptr())) == 0
+    rows = 2 if H <= 2048 else 1
+    ctas = min((N_ + rows - 1) // rows, 6 * torch.cuda.get_device_properties(0).multi_processor_count)
+    terms = dy.float() * (x.float() * rstd[:, None]).to(torch.bfloat16).float()
+    terms = torch.nn.functional.pad(terms, (0, 0, 0, -N_ % (ctas * rows))).view(-1, ctas, rows, H)
+    part = torch.zeros(ctas, rows, H, device="cuda")
+    for t in terms:
+        part += t
+    part = torch.nn.functional.pad(part.sum(1), (0, 0, 0, -ctas % 32)).view(-1, 32, H)
+    groups = torch.zeros(32, H, device="cuda")
+    for t in part:
+        groups += t
+    want = torch.zeros(H, device="cuda")
+    for t in groups:
+        want += t
+    assert torch.equal(dw, want)
