@@ -151,33 +151,41 @@ struct RopeBwdArgs {
   int T, Hq, Hk;
   float w_off;
   int do_norm;
-  int grid_q;  // CTAs of q's heads; the others walk over k's
-  int parts_q, part_heads_q, parts_k, part_heads_k;
+  int grid;               // partial rows of dW; a CTA of each for q's heads, then one for k's
+  int parts, part_heads;  // as of the forward
 };
+
+// Threads of a CTA, and lane groups, each of which owns a token at a time.
+constexpr int kRopeBwdThreads = 128;
+constexpr int rope_bwd_groups(int hd) { return kRopeBwdThreads / (hd / 16); }
 
 // Same token-per-lane-group walk as the forward kernel, UB heads at a time: the gradient rows, the forward
 // inputs and the saved rstd of UB heads are requested before any of them is used, and registers bound how
 // many those are. So a CTA walks over q's heads or over k's, with the weights of the one in registers and one
 // set of dW accumulators, and a lane holds eight elements of either half of a head, as in the forward.
-// Measured before (both kinds a CTA, weights in shared memory, an element an instruction) / now (us, tokens x
-// 24 heads of 128, L2 flushed): 22627 103 / 88, 40280 171 / 139, 6000 35 / 32, 3000 23 / 21; 33280 x 40
-// 227 / 187; 22627 x 40 heads of 64 94 / 84. (Three CTAs a SM with a head at a time: 119 at 22627.)
+//
+// dW has one order of summation, part of the bits of a training step (the gradient norm, and through the clip
+// coefficient every weight): group g of row r of `grid` partial rows adds up its units' heads, in ascending order, of
+// units r * TPB + g + i * grid * TPB (a unit: part_heads of q's and k's heads of a token), then the
+// groups one after the other.
+// Measured with both kinds a CTA, weights in shared memory and an element an instruction / now (us, tokens x
+// 24 heads of 128, L2 flushed): 22627 105 / 84, 40280 174 / 135, 8000 52 / 37, 3000 31 / 25, 1200 24 / 16; 33280 x
+// 40 225 / 178; 22627 x 40 heads of 64 107 / 77. Groups of two heads of one kind for few tokens take 20 at 3000 and
+// 14 at 1200, in another order of summation. (Three CTAs a SM with a head at a time: 119 at 22627.)
 template <int HD>
-__global__ void __launch_bounds__(kRowThreads, 2) qk_rope_bwd_kernel(RopeBwdArgs a) {
+__global__ void __launch_bounds__(kRopeBwdThreads, 4) qk_rope_bwd_kernel(RopeBwdArgs a) {
   constexpr int LPH = HD / 16;
-  constexpr int TPB = kRowThreads / LPH;
+  constexpr int TPB = rope_bwd_groups(HD);
   constexpr int UB = 2;
   constexpr int HALF = HD / 2;
-  __shared__ float sdw[HD];
+  __shared__ float sdw[TPB][HD];
   const int l = threadIdx.x % LPH;
   const int g = threadIdx.x / LPH;
   const int e0 = l * 8;
-  const bool is_q = int(blockIdx.x) < a.grid_q;
-  const unsigned cta = is_q ? blockIdx.x : blockIdx.x - a.grid_q;
-  const unsigned ctas = is_q ? a.grid_q : gridDim.x - a.grid_q;
-  const int H = is_q ? a.Hq : a.Hk;
-  const unsigned parts = is_q ? a.parts_q : a.parts_k;
-  const int part_heads = is_q ? a.part_heads_q : a.part_heads_k;
+  const bool is_q = int(blockIdx.x) < a.grid;
+  const unsigned cta = is_q ? blockIdx.x : blockIdx.x - a.grid;
+  const int H = is_q ? a.Hq : a.Hk, h_from = is_q ? 0 : a.Hq;   // of the heads of both
+  const int span = min(H, a.part_heads);
   f2 dw[2][4], wt[2][4];
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
@@ -194,8 +202,6 @@ __global__ void __launch_bounds__(kRowThreads, 2) qk_rope_bwd_kernel(RopeBwdArgs
 #pragma unroll
     for (int i = 0; i < 4; ++i) dw[k][i] = 0ull;
   }
-  for (int i = threadIdx.x; i < HD; i += kRowThreads) sdw[i] = 0.f;
-  __syncthreads();
   RopeArgs pa;  // only the position fields are used by token_pos
   pa.pos = a.pos;
   pa.pos_i64 = a.pos_i64;
@@ -209,16 +215,17 @@ __global__ void __launch_bounds__(kRowThreads, 2) qk_rope_bwd_kernel(RopeBwdArgs
   pdl_wait();
   pdl_trigger();
 
-  const unsigned total = unsigned(a.T) * parts;
-  for (unsigned u0 = cta * TPB; u0 < total; u0 += ctas * TPB) {
-    const unsigned tok_u = (u0 + g) / parts;
+  const unsigned total = unsigned(a.T) * a.parts;
+  for (unsigned u0 = cta * TPB; u0 < total; u0 += a.grid * TPB) {
+    const unsigned tok_u = (u0 + g) / a.parts;
     const long long tok = tok_u;
-    const bool valid = tok < a.T;
-    const int h_first = int(u0 + g - tok_u * parts) * part_heads;
-    const int heads = min(h_first + part_heads, H);
+    const int first = int(u0 + g - tok_u * a.parts) * a.part_heads - h_from;
+    const int h_first = max(first, 0), heads = min(first + a.part_heads, H);
+    const bool valid = tok < a.T && h_first < heads;
+    if (__all_sync(0xffffffffu, !valid)) continue;   // (the warp's parts are heads of the other kind)
     f2 c[4], s[4];
     load_angles<HALF>(a.cos, a.sin, valid ? token_pos(pa, tok) : -1, e0, c, s);
-    for (int b0 = 0; b0 < part_heads; b0 += UB) {
+    for (int b0 = 0; b0 < span; b0 += UB) {
       const int h0 = h_first + b0;
       uint4 graw[UB][2], xraw[UB][2];
       float rs[UB];
@@ -286,25 +293,21 @@ __global__ void __launch_bounds__(kRowThreads, 2) qk_rope_bwd_kernel(RopeBwdArgs
     }
   }
   if (a.do_norm && a.dw_partial != nullptr) {
-    // the groups of a warp first: as many fewer additions to the same words of shared memory
 #pragma unroll
     for (int k = 0; k < 2; ++k)
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        float2 v = f2_get(dw[k][i]);
-#pragma unroll
-        for (int sh = 16; sh >= LPH; sh >>= 1) {
-          v.x += __shfl_xor_sync(0xffffffffu, v.x, sh);
-          v.y += __shfl_xor_sync(0xffffffffu, v.y, sh);
-        }
-        if ((threadIdx.x & 31) < LPH) {
-          atomicAdd(&sdw[k * HALF + e0 + 2 * i], v.x);
-          atomicAdd(&sdw[k * HALF + e0 + 2 * i + 1], v.y);
-        }
+        const float2 v = f2_get(dw[k][i]);
+        sdw[g][k * HALF + e0 + 2 * i] = v.x;
+        sdw[g][k * HALF + e0 + 2 * i + 1] = v.y;
       }
     __syncthreads();
-    for (int i = threadIdx.x; i < 2 * HD; i += kRowThreads)
-      a.dw_partial[1LL * blockIdx.x * 2 * HD + i] = (i < HD) == is_q ? sdw[i % HD] : 0.f;
+    for (int i = threadIdx.x; i < HD; i += kRopeBwdThreads) {
+      float t = 0.f;
+#pragma unroll
+      for (int j = 0; j < TPB; ++j) t += sdw[j][i];
+      a.dw_partial[(2LL * cta + (is_q ? 0 : 1)) * HD + i] = t;
+    }
   }
 }
 
@@ -318,10 +321,8 @@ using namespace lb;
 // 142 against 127 us at 40280 tokens of 16 + 8 heads of 128). With so few tokens that the groups
 // are fewer than the SMs hold, the walk is a chain of latencies, and a group for every few heads is
 // faster (32 tokens: 21 against 29 us, 1024: 20 against 27; about 10 us of each are the measurement's own).
-static bool few_tokens(int T, int hd) {
-  return 1LL * T < 3LL * row_num_sms() * (kRowThreads / (hd / 16)) / 2;
-}
-static void rope_parts(bool few, int heads, int unit, int* parts, int* part_heads) {
+static void rope_parts(int T, int tokens_per_cta, int heads, int unit, int* parts, int* part_heads) {
+  const bool few = 1LL * T < 3LL * row_num_sms() * tokens_per_cta / 2;
   const int all = (heads + unit - 1) / unit;
   *parts = few ? all : 1;
   *part_heads = few ? unit : all * unit;
@@ -345,7 +346,7 @@ extern "C" int lb_qk_norm_rope_fwd(const void* q_in, long long ldq_in, const voi
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   auto run = [&](auto kern, int lph) {
     const int tpb = kRowThreads / lph;
-    rope_parts(few_tokens(T, hd), Hq + Hk, 2, &a.parts, &a.part_heads);
+    rope_parts(T, tpb, Hq + Hk, 2, &a.parts, &a.part_heads);
     const long long g = (1LL * T * a.parts + tpb - 1) / tpb;
     const long long cap = 1LL * row_num_sms() * 3;  // one wave at three CTAs per SM
     return launch_pdl(kern, dim3(unsigned(g < cap ? g : cap)), dim3(kRowThreads), 0, st,
@@ -357,31 +358,17 @@ extern "C" int lb_qk_norm_rope_fwd(const void* q_in, long long ldq_in, const voi
   return -3;
 }
 
-// CTAs of the backward, each of which leaves a partial row in its scratch, and how many of them walk over
-// q's heads: of two a SM, q's share of the heads.
-static int rope_bwd_grid(int T, int Hq, int Hk, int hd, int* grid_q) {
-  const bool few = few_tokens(T, hd);
-  const int tpb = kRowThreads / (hd / 16);
-  auto need = [&](int heads) {
-    int parts, part_heads;
-    rope_parts(few, heads, 2, &parts, &part_heads);
-    return (1LL * T * parts + tpb - 1) / tpb;
-  };
-  const long long cap = 2LL * row_num_sms();
-  long long q = need(Hq), k = need(Hk);
-  if (q + k > cap) {
-    const long long share = cap * Hq / (Hq + Hk);
-    q = share < q ? (share > 0 ? share : 1) : q;
-    k = cap - q < k ? cap - q : k;
-    if (k < 1) k = 1;
-  }
-  *grid_q = int(q);
-  return int(q + k);
+// Partial rows of dW that the backward leaves in its scratch: with the parts, its order of summation.
+static int rope_bwd_plan(int T, int heads, int hd, int* parts, int* part_heads) {
+  const int groups = rope_bwd_groups(hd);
+  rope_parts(T, groups, heads, 4, parts, part_heads);
+  const long long need = (1LL * T * *parts + groups - 1) / groups, cap = 4LL * row_num_sms();
+  return int(need < cap ? need : cap);
 }
 extern "C" int lb_rope_bwd_rows(int T, int Hq, int Hk, int hd) {
   if (T <= 0 || hd < 64) return 0;
-  int grid_q;
-  return rope_bwd_grid(T, Hq, Hk, hd, &grid_q);
+  int parts, part_heads;
+  return rope_bwd_plan(T, Hq + Hk, hd, &parts, &part_heads);
 }
 
 // dw_out: [2, hd] (q weight grad then k weight grad); scratch: lb_rope_bwd_partial_rows()*2*hd floats.
@@ -402,12 +389,10 @@ extern "C" int lb_qk_norm_rope_bwd(const void* dq, long long lddq, const void* d
                 pos_mod > 0 ? pos_mod : 1, q_rstd, k_rstd, (bf16*)dq_in, (bf16*)dk_in, lddq_in,
                 lddk_in, scratch, T, Hq, Hk, w_off, do_norm};
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  const int grid = rope_bwd_grid(T, Hq, Hk, hd, &a.grid_q);
-  const bool few = few_tokens(T, hd);
-  rope_parts(few, Hq, 2, &a.parts_q, &a.part_heads_q);
-  rope_parts(few, Hk, 2, &a.parts_k, &a.part_heads_k);
+  if (hd != 64 && hd != 128 && hd != 256) return -3;
+  a.grid = rope_bwd_plan(T, Hq + Hk, hd, &a.parts, &a.part_heads);
   auto run = [&](auto kern) {
-    return launch_pdl(kern, dim3(grid), dim3(kRowThreads), 0, st,
+    return launch_pdl(kern, dim3(2 * a.grid), dim3(kRopeBwdThreads), 0, st,
                       pdl_enabled(6LL * T * (Hq + Hk) * hd), 1, a);
   };
   int rc = -3;
@@ -416,7 +401,7 @@ extern "C" int lb_qk_norm_rope_bwd(const void* dq, long long lddq, const void* d
   else if (hd == 256) rc = run(qk_rope_bwd_kernel<256>);
   if (rc) return rc;
   if (do_norm && dw_out != nullptr && scratch != nullptr) {
-    return lb_colsum(scratch, grid, 2 * hd, dw_out, dw_fp32, dw_accumulate, stream);
+    return lb_colsum(scratch, a.grid, 2 * hd, dw_out, dw_fp32, dw_accumulate, stream);
   }
   return launch_rc();
 }

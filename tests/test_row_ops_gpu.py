@@ -409,3 +409,53 @@ def test_rms_norm_weight_gradient_is_summed_in_one_order(N_, H):
     for t in groups:
         want += t
     assert torch.equal(dw, want)
+
+
+@pytest.mark.parametrize("T,Hq,Hk,hd", [(1, 2, 1, 128), (3000, 16, 8, 128), (2500, 5, 2, 64), (10000, 2, 1, 128),
+                                        (5000, 3, 1, 256)])
+def test_rope_weight_gradients_are_summed_in_one_order(T, Hq, Hk, hd):
+    """As for the norms: groups of lanes walk over units of heads (four of q's and k's in a row of few tokens, else
+    all of a token), a partial row has the groups of 16 tokens (of 128 columns), then every 32nd partial row, then
+    those. Without a rotation the terms are products of bf16 values, exact in fp32."""
+    torch.manual_seed(T)
+    H, dev = Hq + Hk, "cuda"
+    x, dy, dx = _r(T, H * hd), _r(T, H * hd), torch.empty(T, H * hd, device=dev, dtype=torch.bfloat16)
+    qw, kw, rstd = _r(hd), _r(hd), torch.rand(T, H, device=dev) + 0.5
+    rq, rk = rstd[:, :Hq].contiguous(), rstd[:, Hq:].contiguous()
+    cos, sin = torch.ones(1, hd // 2, device=dev), torch.zeros(1, hd // 2, device=dev)
+    pos = torch.zeros(T, dtype=torch.int32, device=dev)
+    lib = nv.load()
+    scratch = torch.empty(lib.lb_rope_bwd_partial_rows() * 2 * hd, device=dev)
+    dw = torch.empty(2, hd, device=dev)
+    p = lambda t, at=0: nv.c_void_p(t.data_ptr() + 2 * at)  # noqa: E731
+    ld, k_at = nv.c_ll(H * hd), Hq * hd
+    assert lib.lb_qk_norm_rope_bwd(
+        p(dy), ld, p(dy, k_at), ld, p(x), ld, p(x, k_at), ld, p(qw), p(kw), p(cos), p(sin), p(pos), nv.c_int(0),
+        nv.c_int(1), p(rq), p(rk), p(dx), ld, p(dx, k_at), ld, p(scratch), p(dw), nv.c_int(1), nv.c_int(0),
+        nv.c_int(T), nv.c_int(Hq), nv.c_int(Hk), nv.c_int(hd), nv.c_float(0.0), nv.c_int(1),
+        nv.c_void_p(nv.stream_ptr())) == 0
+    sms, groups = torch.cuda.get_device_properties(0).multi_processor_count, 2048 // hd
+    unit = 4 if T < 3 * sms * groups // 2 else H
+    parts = -(-H // unit)
+    rows = min(-(-T * parts // groups), 4 * sms)
+    terms = dy.view(T, H, hd).float() * (x.view(T, H, hd).float() * rstd[..., None]).to(torch.bfloat16).float()
+    terms = torch.nn.functional.pad(terms, (0, 0, 0, parts * unit - H)).view(T * parts, unit, hd)
+    is_k = (torch.arange(parts * unit, device=dev) >= Hq).view(parts, unit).repeat(T, 1)[..., None]
+    extra = -T * parts % (rows * groups)
+    for kind, got in ((False, dw[0]), (True, dw[1])):
+        t = torch.where(is_k == kind, terms, 0.0)
+        t = torch.nn.functional.pad(t, (0, 0, 0, 0, 0, extra)).view(-1, rows, groups, unit, hd)
+        acc = torch.zeros(rows, groups, hd, device=dev)
+        for step in t:
+            for j in range(unit):
+                acc += step[:, :, j]
+        part = torch.zeros(rows, hd, device=dev)
+        for j in range(groups):
+            part += acc[:, j]
+        part = torch.nn.functional.pad(part, (0, 0, 0, -rows % 32)).view(-1, 32, hd)
+        sums, want = torch.zeros(32, hd, device=dev), torch.zeros(hd, device=dev)
+        for q in part:
+            sums += q
+        for q in sums:
+            want += q
+        assert torch.equal(got, want), kind
