@@ -67,10 +67,11 @@ struct GemmArgs {
   float scale;                // 1 / temperature
   const float* lse;           // [M] natural-log LSE (EPI_PGRAD input)
   float* part;                // [tiles_n, M, 2] running (max, sum) in log2 domain (EPI_LSE output)
-  float* pos;                 // [M] score of the target column (EPI_LSE output)
+  float* pos;                 // EPI_LSE output: [M] score of the target column; of label losses
+                              // [parts, M] weighted score sums
   const float* coef;          // device scalar multiplied into the probabilities' gradient,
   float coef_scale;           // times this
-  float* zero;                // cleared by a forward launch (the loss that the next one adds to), or null
+  unsigned* zero;             // cleared by a forward launch (the counter of the next one), or null
   long long target_offset;    // target column of row r is r + target_offset
   // label-matrix losses (labels != nullptr): int8 labels [M, ld_labels] (1 positive, 0 negative,
   // < 0 ignored; ld_labels a multiple of 32 and >= N, padding = ignored), optional target weights
@@ -217,7 +218,7 @@ __global__ void __launch_bounds__(gemm_threads<EPI_, GATHER, F8>(), 1)
   pdl_wait();
   pdl_trigger();
   if constexpr (EPI == EPI_LSE) {
-    if (blockIdx.x == 0 && threadIdx.x == 0 && g.zero != nullptr) *g.zero = 0.f;
+    if (blockIdx.x == 0 && threadIdx.x == 0 && g.zero != nullptr) *g.zero = 0u;
   }
 
   // CTAs that compute tiles are numbered 0 .. ncta-1 (a gather launch puts its copy CTAs first)
@@ -836,7 +837,7 @@ __global__ void __launch_bounds__(gemm_threads<EPI_, GATHER, F8>(), 1)
           pp[0] = m_run;
           pp[1] = l_run;
           if (lbl) {
-            if (pos_val != 0.f) atomicAdd(&g.pos[row], pos_val);  // several column tiles add up
+            g.pos[static_cast<long long>(part_idx) * g.M + row] = pos_val;
           } else if (pos_here) {
             g.pos[row] = pos_val;
           }
@@ -1253,22 +1254,24 @@ extern "C" int lb_gemm_bf16_scatter(const void* A, const void* B, const void* co
 namespace lb {
 namespace {
 
-// lse[r] = ln(sum_j exp(s_rj)) out of the (max, sum) pairs of `parts` column ranges; loss += loss_scale *
-// sum_r (lse[r] − pos[r]) (one atomicAdd per block). LABELS: loss += loss_scale * sum_r row_w[r] *
-// (lse[r] − row_scale[r] · pos[r]), and rows without a valid column get lse = 0 (their row_w is 0).
+// lse[r] = ln(sum_j exp(s_rj)) out of the (max, sum) pairs of `parts` column ranges; loss = loss_scale *
+// sum_r (lse[r] − pos[r]). LABELS: loss = loss_scale * sum_r row_w[r] * (lse[r] − row_scale[r] · pos[r]), pos[r]
+// a sum over the ranges, and rows without a valid column get lse = 0 (their row_w is 0).
 // A block has 32 rows, and of each every eighth range per warp (8192 rows of 32 ranges: 9 us with a thread
-// per row, which is a chain of loads on a fifth of the SMs, 4 here).
+// per row, which is a chain of loads on a fifth of the SMs, 4 here). The last block to end adds up the blocks'
+// shares of the loss in their order, eight at a time: the same inputs have the same loss.
 template <bool LABELS>
 __global__ void __launch_bounds__(256)
     lse_merge_kernel(const float* __restrict__ part, int parts, int M, const float* __restrict__ pos,
                      const float* __restrict__ row_scale, const float* __restrict__ row_w,
-                     float* __restrict__ lse, float* __restrict__ loss, float loss_scale) {
-  __shared__ float sm[8][32], sl[8][32];
+                     float* __restrict__ lse, float* shares, unsigned* counter, float* __restrict__ loss,
+                     float loss_scale) {
+  __shared__ float sm[8][32], sl[8][32], sp[8][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int r = blockIdx.x * 32 + lane;
   pdl_wait();
   pdl_trigger();
-  float m = -INFINITY, l = 0.f;
+  float m = -INFINITY, l = 0.f, t_pos = 0.f;
   auto add = [&](float mt, float lt) {
     const float mn = fmaxf(m, mt);
     if (mn > -INFINITY) l = l * exp2f(m - mn) + lt * exp2f(mt - mn);
@@ -1279,36 +1282,69 @@ __global__ void __launch_bounds__(256)
     int t = w;
     for (; t + 24 < parts; t += 32) {   // four loads in flight
       float2 v[4];
+      float q[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) v[i] = p[1LL * (t + 8 * i) * M + r];
+      for (int i = 0; i < 4; ++i) {
+        v[i] = p[1LL * (t + 8 * i) * M + r];
+        q[i] = LABELS ? pos[1LL * (t + 8 * i) * M + r] : 0.f;
+      }
 #pragma unroll
-      for (int i = 0; i < 4; ++i) add(v[i].x, v[i].y);
+      for (int i = 0; i < 4; ++i) {
+        add(v[i].x, v[i].y);
+        t_pos += q[i];
+      }
     }
     for (; t < parts; t += 8) {
       const float2 v = p[1LL * t * M + r];
+      if (LABELS) t_pos += pos[1LL * t * M + r];
       add(v.x, v.y);
     }
   }
   sm[w][lane] = m;
   sl[w][lane] = l;
+  if (LABELS) sp[w][lane] = t_pos;
   __syncthreads();
   if (w != 0) return;
 #pragma unroll
-  for (int i = 1; i < 8; ++i) add(sm[i][lane], sl[i][lane]);
+  for (int i = 1; i < 8; ++i) {
+    add(sm[i][lane], sl[i][lane]);
+    if (LABELS) t_pos += sp[i][lane];
+  }
   float contrib = 0.f;
   if (r < M) {
     const float v = !LABELS || l > 0.f ? (m + log2f(l)) * 0.6931471805599453f : 0.f;
     lse[r] = v;
     if constexpr (LABELS) {
       const float rw = row_w[r];
-      if (rw != 0.f) contrib = rw * (v - row_scale[r] * pos[r]);
+      if (rw != 0.f) contrib = rw * (v - row_scale[r] * t_pos);
     } else {
       contrib = v - pos[r];
     }
   }
+  auto warp_sum = [](float x) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) contrib += __shfl_xor_sync(0xffffffffu, contrib, o);
-  if (lane == 0) atomicAdd(loss, contrib * loss_scale);
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+  };
+  contrib = warp_sum(contrib);
+  unsigned done = 0;
+  if (lane == 0) {
+    shares[blockIdx.x] = contrib;
+    __threadfence();
+    done = atomicAdd(counter, 1u) + 1u;
+  }
+  const int blocks = gridDim.x;
+  if (__shfl_sync(0xffffffffu, done, 0) != unsigned(blocks)) return;
+  __threadfence();
+  float total = 0.f;
+  for (int b0 = lane * 8; b0 < blocks; b0 += 32 * 8) {
+    float t = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) t += b0 + i < blocks ? __ldcg(shares + b0 + i) : 0.f;
+    total += t;
+  }
+  total = warp_sum(total);
+  if (lane == 0) *loss = total * loss_scale;
 }
 
 int num_sms();
@@ -1322,7 +1358,7 @@ int loss_tile_bn(int M, int N) {
   return 2LL * ((M + BM - 1) / BM) * ((N + 255) / 256) <= num_sms() && N > 256 ? 128 : 256;
 }
 // Column ranges that a row's (max, sum) pairs come from: two per tile, one where a single tile has all
-// columns (the sums of small batches, whose bits a training run repeats).
+// columns (the sums of small batches, whose bits a training run has had from the start).
 bool loss_one_tile(int M, int N) { return N <= loss_tile_bn(M, N); }
 int loss_parts(int M, int N) {
   const int bn = loss_tile_bn(M, N);
@@ -1340,12 +1376,23 @@ int launch_loss(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmArgs& 
               : launch<0, 0, 128, __nv_bfloat16, EPI>(tmA, tmB, g, grid, stream);
 }
 
+// Scratch of a forward, in floats: part [parts, M, 2], pos [pos_rows, M], the counter of merge_lse's blocks and
+// their shares of the loss.
+long long loss_scratch(int M, long long parts, long long pos_rows) {
+  return (2 * parts + pos_rows) * M + 1 + (M + 31) / 32;
+}
+void carve_loss(float* scratch, long long parts, long long pos_rows, GemmArgs* g) {
+  g->part = scratch;
+  g->pos = scratch + 2 * parts * g->M;
+  g->zero = reinterpret_cast<unsigned*>(g->pos + pos_rows * g->M);
+}
+
 template <bool LABELS>
 int merge_lse(const GemmArgs& g, int parts, float* lse, float* loss, float loss_scale,
               cudaStream_t stream) {
   return launch_pdl(lse_merge_kernel<LABELS>, dim3((g.M + 31) / 32), dim3(256), 0, stream,
                     pdl_enabled(), 1, (const float*)g.part, parts, g.M, (const float*)g.pos,
-                    g.row_scale, g.row_w, lse, loss, loss_scale);
+                    g.row_scale, g.row_w, lse, reinterpret_cast<float*>(g.zero + 1), g.zero, loss, loss_scale);
 }
 
 // (k_rows: passages in memory; columns from there to N have no product and are zero)
@@ -1375,7 +1422,6 @@ int prep_loss(const void* Q, const void* Kd, int M, int N, int k_rows, int D, lo
 }  // namespace
 }  // namespace lb
 
-// Number of floats of scratch that lb_infonce_fwd needs for M queries against N passages.
 // Same with bf16 accumulators in the owners' buffers (red.global.add on packed bf16x2): half the
 // NVLink bytes of the fp32 form, for activations whose reduce-scatter would be bf16 anyway.
 extern "C" int lb_gemm_bf16_scatter16(const void* A, const void* B, const void* const* c_peers,
@@ -1497,8 +1543,10 @@ extern "C" int lb_gemm_bf16_ext(const void* A, const void* B, const void* A2, co
                    : launch<0, 0, 128, __nv_bfloat16>(tmA, tmB, g, grid, stream, &tmA2, &tmB2);
 }
 
+// Number of floats of scratch that lb_loss_fwd needs for M queries against N passages (a multiple of 8).
 extern "C" long long lb_infonce_scratch_floats(int M, int N) {
-  return 2LL * lb::loss_parts(M, N) * M + M;
+  const int parts = lb::loss_parts(M, N);
+  return lb::loss_scratch(M, parts, parts);
 }
 
 namespace lb {
@@ -1557,12 +1605,7 @@ extern "C" int lb_loss_fwd(const LbLoss* p) {
   int grid;
   if (int rc = loss_product(*p, 0, p->N, &tmA, &tmB, &g, &grid)) return rc;
   const int parts = loss_parts(g.M, g.N);
-  g.part = p->scratch;
-  g.pos = p->scratch + 2LL * parts * g.M;
-  g.zero = p->loss;
-  if (p->labels != nullptr &&
-      cudaMemsetAsync(g.pos, 0, sizeof(float) * g.M, stream) != cudaSuccess)
-    return -12;
+  carve_loss(p->scratch, parts, p->labels != nullptr ? parts : 1, &g);
   if (int rc = launch_loss<EPI_LSE, EPI_LSE_ROW>(tmA, tmB, g, grid, stream)) return rc;
   const PdlScope pdl(true);
   return p->labels != nullptr ? merge_lse<true>(g, parts, p->lse, p->loss, p->loss_scale, stream)
@@ -1628,7 +1671,7 @@ extern "C" int lb_infonce_pgrad(const void* q, long long ldq, const void* k, lon
 // the launch after every rank has written its passages and keeps k_all for the backward.
 // flags: [world * ceil(n_local / 256)] zero-initialised once; counter: one u32; epoch: 1, 2, 3, …
 // on successive calls that use these flags (a flag counts the 16-row items pulled so far).
-// part/lse layout as in lb_infonce_fwd with tiles = world * ceil(n_local / 256).
+// A row's (max, sum) pairs are those of world * ceil(n_local / 256) tiles; *loss_sum is written.
 namespace lb {
 namespace {
 // Grid of a gather launch: the CTAs that compute tiles plus the copy CTAs in front of them (16 of
@@ -1653,7 +1696,7 @@ int gather_grid(long long total, int sms, int world, double pull_bytes, double f
 }  // namespace lb
 
 extern "C" long long lb_infonce_xrank_scratch_floats(int M, int n_local, int world) {
-  return 2LL * world * ((n_local + 255) / 256) * M + M;
+  return lb::loss_scratch(M, 1LL * world * ((n_local + 255) / 256), 1);
 }
 
 extern "C" int lb_infonce_fwd_xrank(const void* q, long long ldq, const void* const* k_peers,
@@ -1676,8 +1719,7 @@ extern "C" int lb_infonce_fwd_xrank(const void* q, long long ldq, const void* co
   grid = gather_grid(total, sms, world, 2.0 * (world - 1) * n_local * D, 2.0 * M * N * D,
                      &g.copy_ctas);
   g.scale = inv_temperature;
-  g.part = scratch;
-  g.pos = scratch + 2LL * chunks * M;
+  carve_loss(scratch, chunks, 1, &g);
   g.target_offset = target_offset;
   for (int i = 0; i < world; ++i) g.b_peers[i] = k_peers[i];
   g.b_local = k_all;

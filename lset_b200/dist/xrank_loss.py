@@ -88,7 +88,7 @@ class _CrossRankInfoNCE(torch.autograd.Function):
         scr = torch.empty(int(lib.lb_infonce_xrank_scratch_floats(
             nv.c_int(B), nv.c_int(n_local), nv.c_int(W))), dtype=torch.float32, device=q.device)
         lse = torch.empty(B, dtype=torch.float32, device=q.device)
-        loss_sum = torch.zeros(1, dtype=torch.float32, device=q.device)
+        loss_sum = torch.empty(1, dtype=torch.float32, device=q.device)
         rc = lib.lb_infonce_fwd_xrank(
             nv.c_void_p(q.data_ptr()), nv.c_ll(q.stride(0)), ksym.c_ptr_array(),
             nv.c_void_p(buf.k_all.data_ptr()), nv.c_ll(D), nv.c_int(B), nv.c_int(n_local),

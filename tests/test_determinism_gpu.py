@@ -123,3 +123,23 @@ def test_norms_rope_and_glu():
         return y, t.grad
 
     _same(glu)
+
+
+@pytest.mark.parametrize("M", [40, 96, 256, 1000])
+@pytest.mark.parametrize("labels", [False, True])
+def test_losses(M, labels):
+    """The loss is a sum over many blocks' rows (with labels, of several column tiles each); so are its
+    gradients."""
+    from lset_b200.ops.loss import fused_infonce, fused_label_loss
+
+    torch.manual_seed(4)
+    q, k = _r(M, 128), _r(1536, 128)
+    lab = (torch.rand(M, 1536, device="cuda") < 0.02).float()
+
+    def loss():
+        a, b = q.clone().requires_grad_(), k.clone().requires_grad_()
+        out = fused_label_loss(a, b, lab, 0.05) if labels else fused_infonce(a, b, 0.05)
+        return out, *torch.autograd.grad(out, (a, b))
+
+    for _ in range(10):
+        _same(loss)
