@@ -636,8 +636,10 @@ class _Inference(Plan):
         self.halves = (att, mlp, *norms[:2], att._modules.get("q_norm"), att._modules.get("k_norm"))
         self.plan = plan
         self.watch = Watch([(m, "weight") for m in norms] + [(m, "weight") for _, _, m, _ in self.modules])
-        self.desc = plan.fill({})
-        self.addr = ctypes.addressof(self.desc)
+        d = self.desc = plan.fill({})
+        self.addr = ctypes.addressof(d)
+        # all that the size of the block's activations and its number of launches follow from
+        self.sizes = (d.Hq, d.Hk, d.hd, d.I, d.qk_norm, d.qkv.n, d.gate_up.n)
 
     def same(self, block) -> bool:
         mods = block._modules
@@ -698,9 +700,8 @@ def run_inference(block_type, layers, branch, ctx):
             sctx = _stream_struct(ctx, plan, dev, d["training"])
             sctx.stream = nv.stream_ptr()
             sctx_at = ctypes.addressof(sctx)
-        size = (kept.desc.Hq, kept.desc.Hk, kept.desc.hd, kept.desc.I)
-        if size != sizes:
-            sizes = size
+        if kept.sizes != sizes:
+            sizes = kept.sizes
             arena = torch.empty(_arena_size(lib.lb_block_saved_bytes(kept.addr, T, 1, None)),
                                 dtype=torch.uint8, device=dev)
             io.saved = arena.data_ptr()

@@ -317,8 +317,9 @@ class _Inference(Plan):
         self.halves, self.eps, self.norms = (att, mlp), ln1.eps, (ln1.__dict__, ln2.__dict__)
         self.plan = plan
         self.watch = Watch([(m, p) for _, _, m, _ in self.modules for p in ("weight", "bias")])
-        self.desc = plan.fill({})
-        self.addr = ctypes.addressof(self.desc)
+        d = self.desc = plan.fill({})
+        self.addr = ctypes.addressof(d)
+        self.sizes = (d.heads, d.I)      # what the size of the block's activations follows from
 
     def same(self, block) -> bool:
         mods = block._modules
@@ -354,7 +355,7 @@ def run_inference(block_type, layers, x, ctx):
     global calls
     lib = _library()
     T, H = x.shape
-    io, key, size, outs, n, launches = LbBlockIO(), None, None, None, 0, 0
+    io, key, sizes, outs, n, launches = LbBlockIO(), None, None, None, 0, 0
     io_at = ctypes.addressof(io)
     for block in layers:
         d = block.__dict__
@@ -369,8 +370,8 @@ def run_inference(block_type, layers, x, ctx):
             sctx = _stream_struct(ctx, kept.plan, x.device, d["training"])
             sctx.stream = nv.stream_ptr()
             sctx_at = ctypes.addressof(sctx)
-        if kept.desc.I != size:
-            size = kept.desc.I
+        if kept.sizes != sizes:
+            sizes = kept.sizes
             arena = torch.empty(_arena_size(lib.lb_encoder_saved_bytes(kept.addr, T)),
                                 dtype=torch.uint8, device=x.device)
             io.saved = arena.data_ptr()

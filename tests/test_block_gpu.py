@@ -282,3 +282,14 @@ def test_passes_without_gradients_see_what_changed_since_the_last(family):
             assert not torch.equal(now, last[0]), i
         last[0] = now
     assert len(seen) == 2
+
+
+def test_inference_pass_over_blocks_with_and_without_head_norms():
+    model, inputs = _build("qwen3", False).eval(), _packed_inputs(lens=(9, 20, 3))
+    model.layers[0].self_attn.q_norm = model.layers[0].self_attn.k_norm = None
+    with torch.no_grad():
+        before = block_ops.calls["dp"]
+        got = model(**inputs)["hidden_states"].clone()
+        assert block_ops.calls["dp"] == before + 2
+    assert torch.equal(got, model(**inputs)["hidden_states"].detach())
+    nv.check_status()

@@ -211,3 +211,59 @@ def test_a_block_that_has_run_can_be_copied_and_pickled(make, plan, copied):
     assert other.__dict__["_lb_plan"] is None
     for a, b in zip(block.parameters(), other.parameters()):
         assert torch.equal(a, b)
+
+
+class _OnDevice(torch.Tensor):
+    is_cuda = True
+
+
+def _qwen(norms):
+    d = dec_ops.LbBlockDesc()
+    d.H, d.Hq, d.Hk, d.hd, d.I, d.qk_norm = 128, 2, 1, 64, 256, norms
+    return d
+
+
+def _bert(heads):
+    d = enc_ops.LbEncoderDesc()
+    d.H, d.heads, d.hd, d.I = 128, heads, 128 // heads, 256
+    return d
+
+
+@pytest.mark.parametrize("ops,descs", [(dec_ops, [_qwen(0), _qwen(1), _qwen(0)]), (enc_ops, [_bert(1), _bert(2)])])
+def test_every_block_of_an_inference_pass_has_room_for_its_activations(ops, descs, monkeypatch):
+    """Blocks of a stack need not be alike: q/k norms and heads have statistics of their own in the arena."""
+    desc_type, arenas, fits = type(descs[0]), [], []
+
+    def need(addr, T, *_):
+        d = desc_type.from_address(addr)
+        return T * (d.heads if ops is enc_ops else 8 + d.qk_norm * (d.Hq + d.Hk)) * 4
+
+    def forward(addr, sctx, io):
+        at = dec_ops.LbBlockIO.from_address(io).saved
+        fits.append(any(a.data_ptr() == at and need(addr, 5) <= a.numel() for a in arenas))
+        return 0
+
+    def arena(n, *a, **kw):
+        arenas.append(torch.zeros(n, dtype=torch.uint8))
+        return arenas[-1]
+
+    name = "lb_encoder" if ops is enc_ops else "lb_block"
+    lib = SimpleNamespace(lb_block_fwd_launches=lambda *a: 1,
+                          **{name + "_saved_bytes": need, name + "_fwd": forward})
+    kept = []
+    for d in descs:     # as a pass fills them in
+        monkeypatch.setattr(ops, "Watch", lambda params: None)
+        monkeypatch.setattr(ops, "_plain_linear", lambda m: True, raising=False)
+        plan = SimpleNamespace(fill=lambda grads, d=d: d, desc=d, rope=(64, 1e4, None), sp=None, qn=None)
+        kept.append(ops._Inference(_bert_block() if ops is enc_ops else _decoder_block(), plan))
+    blocks = torch.nn.ModuleList(torch.nn.Identity() for _ in descs)
+    monkeypatch.setattr(ops, "_library", lambda: lib)
+    monkeypatch.setattr(ops, "_own_forwards", lambda block: True)
+    monkeypatch.setattr(ops, "_inference_of", lambda block: kept[list(blocks).index(block)])
+    monkeypatch.setattr(ops, "_stream_struct", lambda *a: dec_ops.LbStreamCtx())
+    monkeypatch.setattr(ops.nv, "stream_ptr", lambda: 0)
+    monkeypatch.setattr(ops, "torch", SimpleNamespace(**{**vars(torch), "empty": arena}))
+    x = torch.zeros(5, 128, dtype=torch.bfloat16).as_subclass(_OnDevice)
+    with torch.no_grad():
+        done, *_ = ops.run_inference(torch.nn.Identity, blocks, x, SimpleNamespace(pos=torch.zeros(5)))
+    assert done == len(descs) and fits == [True] * len(descs)
