@@ -627,13 +627,16 @@ class _Inference(Plan):
         names = qkv + [(att, "o_proj")] + gu + [(mlp, "down_proj")]
         self.modules = [(owner._modules, n, owner._modules[n], owner._modules[n].__dict__)
                         for owner, n in names]
-        self.ok = plan.sp is None and all(_plain_linear(m) for _, _, m, _ in self.modules)
-        if not self.ok:
-            return
         norms = [block.input_layernorm, block.post_attention_layernorm]
         if plan.qn is not None:
             norms += [att.q_norm, att.k_norm]
+        # (a weight may be a buffer, or computed by its module: such a block is called by itself)
+        self.ok = (plan.sp is None and all(_plain_linear(m) for _, _, m, _ in self.modules)
+                   and all("weight" in m._parameters for m in norms + [m for _, _, m, _ in self.modules]))
+        if not self.ok:
+            return
         self.halves = (att, mlp, *norms[:2], att._modules.get("q_norm"), att._modules.get("k_norm"))
+        self.fused = att.fused_qkv, mlp.fused_gate_up
         self.plan = plan
         self.watch = Watch([(m, "weight") for m in norms] + [(m, "weight") for _, _, m, _ in self.modules])
         d = self.desc = plan.fill({})
@@ -649,8 +652,11 @@ class _Inference(Plan):
             return False
         if (am.get("q_norm"), am.get("k_norm")) != self.halves[4:]:
             return False
+        if (att.fused_qkv, mlp.fused_gate_up) != self.fused:
+            return False
         for where, name, m, d in self.modules:
-            if where[name] is not m or "forward" in d or "_tp_kind" in d or d["_parameters"]["bias"] is not None:
+            if (where.get(name) is not m or "forward" in d or "_tp_kind" in d
+                    or d["_parameters"].get("bias") is not None):
                 return False
         return self.watch.same()
 

@@ -315,6 +315,7 @@ class _Inference(Plan):
         self.modules = [(owner._modules, n, owner._modules[n], owner._modules[n].__dict__)
                         for owner, n in names]
         self.halves, self.eps, self.norms = (att, mlp), ln1.eps, (ln1.__dict__, ln2.__dict__)
+        self.fused = att.fused_qkv
         self.plan = plan
         self.watch = Watch([(m, p) for _, _, m, _ in self.modules for p in ("weight", "bias")])
         d = self.desc = plan.fill({})
@@ -323,10 +324,11 @@ class _Inference(Plan):
 
     def same(self, block) -> bool:
         mods = block._modules
-        if mods["attention"] is not self.halves[0] or mods["mlp"] is not self.halves[1]:
+        if (mods["attention"] is not self.halves[0] or mods["mlp"] is not self.halves[1]
+                or self.halves[0].fused_qkv != self.fused):
             return False
         for where, name, m, d in self.modules:
-            if where[name] is not m or not unhooked(d) or "_tp_kind" in d:
+            if where.get(name) is not m or not unhooked(d) or "_tp_kind" in d:
                 return False
         return (self.norms[0]["eps"] == self.eps and self.norms[1]["eps"] == self.eps
                 and self.watch.same())

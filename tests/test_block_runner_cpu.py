@@ -267,3 +267,31 @@ def test_every_block_of_an_inference_pass_has_room_for_its_activations(ops, desc
     with torch.no_grad():
         done, *_ = ops.run_inference(torch.nn.Identity, blocks, x, SimpleNamespace(pos=torch.zeros(5)))
     assert done == len(descs) and fits == [True] * len(descs)
+
+
+def _decoder_inference(block, monkeypatch):
+    monkeypatch.setattr(dec_ops, "_plain_linear", lambda m: True)
+    plan = SimpleNamespace(fill=lambda grads: _qwen(0), desc=_qwen(0), rope=(64, 1e4, None), sp=None, qn=None)
+    return dec_ops._Inference(block, plan)
+
+
+@pytest.mark.parametrize("name", ["mlp.down_proj", "input_layernorm"])
+def test_a_block_with_a_weight_that_is_no_parameter_is_called_by_itself(name, monkeypatch):
+    block = _decoder_block()
+    assert _decoder_inference(block, monkeypatch).ok
+    m = block.get_submodule(name)
+    w = m.weight.detach()
+    del m.weight
+    m.register_buffer("weight", w)
+    assert not _decoder_inference(block, monkeypatch).ok
+
+
+def test_what_is_kept_of_a_block_sees_a_projection_that_is_gone(monkeypatch):
+    block = _decoder_block()
+    kept = _decoder_inference(block, monkeypatch)
+    assert kept.same(block)
+    block.self_attn.fused_qkv = True
+    assert not kept.same(block)
+    block.self_attn.fused_qkv = False
+    del block.self_attn.q_proj
+    assert not kept.same(block)
