@@ -676,10 +676,36 @@ extern "C" int lb_colsum(const float* partial, int P, int C, void* out, int out_
   return launch_colsum(partial, P, C, out, out_fp32, accumulate, reinterpret_cast<cudaStream_t>(stream));
 }
 
-// Up to kMaxColsums sums of fp32 partial rows in one launch, added to fp32 outputs.
+// How many of the n sums from the first on may run side by side: none of them adds to another's output.
+static int colsum_batch(const LbColsum* jobs, int n) {
+  int k = 0;
+  for (; k < n && k < kMaxColsums; ++k)
+    for (int j = 0; j < k; ++j)
+      for (const void* a : {jobs[k].out, jobs[k].out2})
+        if (a != nullptr && (a == jobs[j].out || a == jobs[j].out2)) return k;
+  return k;
+}
+
+// Up to kMaxColsums sums of fp32 partial rows, added to fp32 outputs. They are one launch as long as each has
+// outputs of its own: a weight that two norms share is added to by one launch after the other.
 extern "C" int lb_colsums(const LbColsum* jobs, int n, void* stream) {
   if (n < 0 || n > kMaxColsums) return -3;
-  return launch_colsums(jobs, n, 1, 1, reinterpret_cast<cudaStream_t>(stream));
+  LbColsum each[2 * kMaxColsums];
+  int k = 0;
+  for (int i = 0; i < n; ++i) {
+    each[k++] = jobs[i];
+    if (jobs[i].split > 0 && jobs[i].out != nullptr && jobs[i].out == jobs[i].out2) {
+      each[k - 1].out2 = nullptr;
+      each[k] = jobs[i];
+      each[k++].out = nullptr;
+    }
+  }
+  for (int from = 0; from < k;) {
+    const int count = colsum_batch(each + from, k - from);
+    if (int rc = launch_colsums(each + from, count, 1, 1, reinterpret_cast<cudaStream_t>(stream))) return rc;
+    from += count;
+  }
+  return 0;
 }
 
 // ------------------------------------------------------------------------------------------------

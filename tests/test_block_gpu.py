@@ -293,3 +293,18 @@ def test_inference_pass_over_blocks_with_and_without_head_norms():
         assert block_ops.calls["dp"] == before + 2
     assert torch.equal(got, model(**inputs)["hidden_states"].detach())
     nv.check_status()
+
+
+@pytest.mark.parametrize("tied", [("input_layernorm", "post_attention_layernorm"),
+                                  ("self_attn.q_norm", "self_attn.k_norm")])
+def test_norms_that_share_a_weight_both_add_to_its_gradient(tied):
+    model, inputs = _build("qwen3", False), _packed_inputs(lens=(9, 20, 3))
+    for layer in model.layers:
+        first, second = (layer.get_submodule(n) for n in tied)
+        second.weight = first.weight
+    _run(model, inputs, False)
+    want = {n: p.grad.float() for n, p in model.named_parameters()}
+    for _ in range(3):
+        _run(model, inputs, True)
+        for n, p in model.named_parameters():       # (two bf16 gradients added up, or one fp32 sum rounded)
+            assert (p.grad.float() - want[n]).norm() <= 2 ** -7 * want[n].norm(), n

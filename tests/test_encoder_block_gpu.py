@@ -240,3 +240,18 @@ def test_bias_grad_sums_in_a_fixed_order(T):
         outs.append(out)
     assert all(torch.equal(o, outs[0]) for o in outs)
     assert (outs[0].double() - dy.double().sum(0)).abs().max().item() < T * 2 ** -23 * 8
+
+
+def test_norms_that_share_weights_both_add_to_their_gradients():
+    model, inputs = _model(128, 2, 256, False), _inputs([9, 20, 3], False)
+    for layer in model.layers:
+        first, second = layer.attention.LayerNorm, layer.mlp.LayerNorm
+        second.weight, second.bias = first.weight, first.bias
+    _run(model, inputs, False)
+    want = {n: p.grad.float() for n, p in model.named_parameters()}
+    before = enc_ops.calls
+    _run(model, inputs, True)
+    assert enc_ops.calls == before + len(model.layers)
+    for n, p in model.named_parameters():
+        size = want[n.replace("key.bias", "value.bias")].norm().item()
+        assert (p.grad.float() - want[n]).norm().item() < 2e-2 * size, n
