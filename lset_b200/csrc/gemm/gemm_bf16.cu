@@ -1558,8 +1558,7 @@ int loss_product(const LbLoss& p, int c0, int n, CUtensorMap* tmA, CUtensorMap* 
   const bool lbl = p.labels != nullptr;
   if (lbl && ((p.ld_labels & 31) || p.ld_labels < p.N)) return -3;
   if (p.tw != nullptr && (!lbl || (p.ld_tw & 31) || p.ld_tw < p.N)) return -3;
-  if (!lbl && (n & 7)) return -3;
-  const int np = (n + 7) / 8 * 8;   // (columns beyond n are ignored: their labels are padding)
+  const int np = lbl ? (n + 7) / 8 * 8 : n;   // (columns beyond n are ignored: their labels are padding)
   const char* k = static_cast<const char*>(p.k) + 2LL * c0 * p.ldk;
   if (int rc = prep_loss(p.q, k, p.M, np, n, p.D, p.ldq, p.ldk, loss_tile_bn(p.M, np), tmA, tmB, g, grid))
     return rc;
@@ -1580,7 +1579,7 @@ int loss_product(const LbLoss& p, int c0, int n, CUtensorMap* tmA, CUtensorMap* 
 
 // W[:, c] of columns [c0, c0 + n), see LbLoss.
 int loss_pgrad(const LbLoss& p, int c0, int n, cudaStream_t stream) {
-  if (p.ldw & 7) return -3;
+  if ((p.ldw & 7) || (p.labels == nullptr && (n & 7))) return -3;
   CUtensorMap tmA, tmB;
   GemmArgs g;
   int grid;

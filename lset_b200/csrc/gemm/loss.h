@@ -4,7 +4,8 @@
 extern "C" {
 
 // s = (q · kᵀ) * inv_temperature. Mirrored field by field in lset_b200/ops/loss.py.
-//   InfoNCE (labels null): the positive of query r is passage r + target_offset; N a multiple of 8.
+//   InfoNCE (labels null): the positive of query r is passage r + target_offset; N a multiple of 8 in the
+//     backward.
 //     loss = loss_scale * sum_r (LSE_c s_rc − s_r,positive)
 //     W[r, c] = (exp(s_rc − lse[r]) − [c is the positive]) * coef
 //   label matrix: int8 labels [M, ld_labels] (ld_labels a multiple of 32, >= N, padded with a negative

@@ -305,3 +305,16 @@ def test_losses_at_the_edges_of_their_tiles(M, N, labels):
     assert abs(loss.item() - want.item()) < 1e-4 * max(1.0, abs(want.item()))
     for got, ref in ((q.grad, p @ k.detach().double()), (k.grad, p.t() @ q.detach().double())):
         assert ((got.double() - ref).norm() / ref.norm()).item() < 2 ** -8
+
+
+@pytest.mark.parametrize("M,N", [(5, 13), (100, 250), (300, 1001)])
+def test_infonce_forward_takes_any_number_of_passages(M, N):
+    """The probability gradient has rows of a multiple of 8: the backward is refused."""
+    q, k = _emb(M, 256, 0).requires_grad_(), _emb(N, 256, 1)
+    loss = fused_infonce(q, k, 0.05)
+    s = q.detach().double() @ k.double().t() / 0.05
+    want = (s.logsumexp(1) - s.diagonal()).mean().item()
+    assert abs(loss.item() - want) < 1e-4 * max(1.0, abs(want))
+    with pytest.raises(RuntimeError):
+        loss.backward()
+    nv.check_status()
