@@ -756,11 +756,9 @@ int launch_bwd(const void* dO, long long lddo, const void* q, long long ldq, con
     if (grid > cap) grid = cap;
     a.plan = plan_q;
     a.capacity = cap_q;
-    const int rc = [&] {
-      return launch_pdl(attn_delta_kernel<HD>, dim3(int(grid)), dim3(256), 0, st,
-                        pdl_enabled(4LL * a.T * a.Hq * HD), 1,
-                        (const bf16*)dO, lddo, (const bf16*)o, ldo, delta, a);
-    }();
+    const int rc = launch_pdl(attn_delta_kernel<HD>, dim3(int(grid)), dim3(256), 0, st,
+                              pdl_enabled(4LL * a.T * a.Hq * HD), 1, (const bf16*)dO, lddo, (const bf16*)o,
+                              ldo, delta, a);
     if (rc) return rc;
   }
   CUtensorMap tmQ, tmdO, tmK, tmV;

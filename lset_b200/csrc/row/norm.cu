@@ -607,12 +607,10 @@ extern "C" int lb_rms_norm_bwd(const void* dy, const void* dres, const void* xin
     if (smem(H) > 48 * 1024)  // wide rows: opt in above the 48 KB default
       cudaFuncSetAttribute(rms_bwd_kernel<TPR, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            smem(8 * TPR * NV));
-    const int rc = [&] {
-      return launch_pdl(rms_bwd_kernel<TPR, NV>, dim3(grid), dim3(kRowThreads),
-                        smem(H), st, pdl_enabled((dres != nullptr ? 8LL : 6LL) * N * H), 1, (const bf16*)dy,
-                        (const bf16*)dres, (const bf16*)xin, (const bf16*)w, rstd, (bf16*)dx,
-                        scratch, N, H, w_off);
-    }();
+    const int rc = launch_pdl(rms_bwd_kernel<TPR, NV>, dim3(grid), dim3(kRowThreads), smem(H), st,
+                              pdl_enabled((dres != nullptr ? 8LL : 6LL) * N * H), 1, (const bf16*)dy,
+                              (const bf16*)dres, (const bf16*)xin, (const bf16*)w, rstd, (bf16*)dx,
+                              scratch, N, H, w_off);
     if (rc) return rc;
   });
   if (dw_out != nullptr)
@@ -657,12 +655,10 @@ extern "C" int lb_layer_norm_bwd(const void* dy, const void* dres, const void* x
     if (2 * H * sizeof(float) > 48 * 1024)
       cudaFuncSetAttribute(ln_bwd_kernel<TPR, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            2 * H * (int)sizeof(float));
-    const int rc = [&] {
-      return launch_pdl(ln_bwd_kernel<TPR, NV>, dim3(grid), dim3(kRowThreads),
-                        2 * H * sizeof(float), st, pdl_enabled((dres != nullptr ? 8LL : 6LL) * N * H), 1, (const bf16*)dy,
-                        (const bf16*)dres, (const bf16*)xin, (const bf16*)w, mean, rstd, (bf16*)dx,
-                        scratch, N, H);
-    }();
+    const int rc = launch_pdl(ln_bwd_kernel<TPR, NV>, dim3(grid), dim3(kRowThreads), 2 * H * sizeof(float),
+                              st, pdl_enabled((dres != nullptr ? 8LL : 6LL) * N * H), 1, (const bf16*)dy,
+                              (const bf16*)dres, (const bf16*)xin, (const bf16*)w, mean, rstd, (bf16*)dx,
+                              scratch, N, H);
     if (rc) return rc;
   });
   if (dwb_out != nullptr)

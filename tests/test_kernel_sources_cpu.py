@@ -28,7 +28,7 @@ def test_kernels_launched_as_programmatic_dependents_wait():
     names = set()
     for text in TEXTS.values():
         for fn in _functions(text):
-            if "return launch_pdl(" in fn:
+            if "launch_pdl(" in fn:
                 found = re.findall(r"\b\w+_kernel\b", fn)
                 assert found, fn[:200]
                 names.update(found)
