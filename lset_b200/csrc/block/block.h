@@ -142,7 +142,7 @@ struct LbEncoderDesc {
   float* bias_grad[6];
 };
 // io: branch = x, out = y; d_out, dx and the arenas as for the decoder block. The stream context's
-// norm_scratch has room for twice 2 * H columns here; wg_tmp is not used.
+// norm_scratch has room for twice 2 * H columns here; rope_scratch and wg_tmp are not used.
 size_t lb_encoder_saved_bytes(const LbEncoderDesc* d, int T);
 size_t lb_encoder_work_bytes(const LbEncoderDesc* d, int T);
 int lb_encoder_fwd(const LbEncoderDesc* d, const LbStreamCtx* c, LbBlockIO* io);

@@ -229,9 +229,9 @@ def _stream_struct(ctx, plan: EncoderPlan, device, training: bool) -> LbStreamCt
     # callers' passes, which would grow or write a shared buffer
     sums = None
     if grad:
-        partial = 2 * _library().lb_norm_bwd_partial_rows() * 2 * d.H
-        sums = torch.empty(partial + 2 * d.H, dtype=torch.float32, device=device)
-        s.norm_scratch, s.wg_tmp = sums.data_ptr(), sums.data_ptr() + 4 * partial
+        sums = torch.empty(2 * _library().lb_norm_bwd_partial_rows() * 2 * d.H, dtype=torch.float32,
+                           device=device)
+        s.norm_scratch = sums.data_ptr()
     s.may_split = int(split)
     # what the attention of short sequences is chosen by (0: not known)
     s.n_seq, s.max_len = ap.seq_start.numel(), getattr(ap, "max_seqlen", 0)
