@@ -84,15 +84,6 @@ __device__ __forceinline__ uint4 pack8(const f2 (&f)[4]) {
   return make_uint4(bf16_of_f2(f[0]), bf16_of_f2(f[1]), bf16_of_f2(f[2]), bf16_of_f2(f[3]));
 }
 
-// Streaming variants: data touched once should not displace what later kernels reuse from L2.
-__device__ __forceinline__ uint4 ld16_stream(const void* p) {
-  uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "l"(p));
-  return v;
-}
-
 // Sum over the TPR threads that own one row. `sred` is a shared float[8] (one slot per warp).
 // Must be called by every thread of the CTA when TPR > 32 (it contains __syncthreads).
 template <int TPR>

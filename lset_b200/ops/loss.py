@@ -57,7 +57,8 @@ def similarity(q: torch.Tensor, k: torch.Tensor) -> torch.Tensor:
 # walked in panels of columns, the panel's W is recomputed from the saved row LSE, dK of the panel
 # is complete after one product, and dQ accumulates over the panels in fp32. A panel's W is capped
 # at PANEL_BYTES (half of the 126 MB L2, so the two products that read it find it there); score
-# matrices below the cap take a single panel. Extra memory: the cap plus the fp32 accumulator of dQ.
+# matrices below the cap take a single panel. Extra memory: the cap plus the fp32 accumulator of dQ. (One
+# native call, lb_loss_bwd; across ranks dist/xrank_loss.py.)
 # ------------------------------------------------------------------------------------------------
 PANEL_BYTES = 64 << 20
 PANEL_MIN_COLS = 1024       # narrower panels leave the dK product too few tiles
@@ -69,36 +70,6 @@ def panel_cols(M: int, N: int) -> int:
     Mp = (M + 7) // 8 * 8
     cols = max(PANEL_MIN_COLS, (PANEL_BYTES // (2 * Mp)) // 256 * 256)
     return min(N, cols)
-
-
-def streamed_loss_backward(launch_pgrad, q, k, need_dq: bool, need_dk: bool):
-    """``launch_pgrad(c0, c1, W)`` fills ``W [M, c1 - c0]`` (bf16) for the passage columns
-    ``[c0, c1)``. Returns ``(dq, dk)`` in the inputs' dtype. (The losses of one rank do the same in
-    one native call, ``lb_loss_bwd``.)"""
-    M, D = q.shape
-    N = k.shape[0]
-    step = panel_cols(M, N)
-    single = step >= N
-    dq = dk = dq32 = None
-    if need_dk:
-        dk = torch.empty(N, D, dtype=k.dtype, device=k.device)
-    W = torch.empty(M, step, dtype=torch.bfloat16, device=q.device)
-    for c0 in range(0, N, step):
-        c1 = min(N, c0 + step)
-        Wp = W if c1 - c0 == step else W[:, :c1 - c0]
-        launch_pgrad(c0, c1, Wp)
-        if need_dq:
-            if single:
-                dq = matmul_abt(Wp, k, b_mn=True)                       # [M, D] = W · K
-            elif dq32 is None:
-                dq32 = matmul_abt(Wp, k[c0:c1], b_mn=True, out_dtype=torch.float32)
-            else:
-                matmul_abt(Wp, k[c0:c1], b_mn=True, out=dq32, accumulate=True)
-        if need_dk:
-            matmul_abt(Wp, q, a_mn=True, b_mn=True, out=dk[c0:c1])          # [n, D] = Wᵀ · Q
-    if need_dq and dq is None:
-        dq = dq32.to(q.dtype)
-    return dq, dk
 
 
 # ------------------------------------------------------------------------------------------------
