@@ -27,7 +27,8 @@ bool pdl_enabled();
 // their way need lines of what is left. So above 96 MB such a kernel waits for the end of the one in front.
 // Measured (us, early start / not, between its GEMMs): gated backward 22627 x 3072 144 / 111, 33280 x 12288
 // 904 / 709 (alone 642, and 814 with the division set to shared memory); RMSNorm backward 22627 x 1024
-// 49 / 42, 33280 x 4096 258 / 206; RMSNorm 40280 x 1024 60 / 50; rotation of 40280 x 24 heads 107 / 93. Steps
+// 49 / 42, 33280 x 4096 258 / 206 (with four CTAs an SM); RMSNorm 40280 x 1024 60 / 50; rotation of 40280 x 24
+// heads 107 / 93. Steps
 // with the line at 12 / 48 / 96 / 10^6 MB: 24 texts of 256 tokens encoded 5.68 / 5.62 / 5.55 / 5.55 ms,
 // 64 texts 13.72 / 13.74 / 13.71 / 13.78; 12 pairs trained on 22.2 / 22.05 / 21.9 / 22.1, 6 pairs 15.0 /
 // 14.8 / 14.8 / 14.8.
