@@ -245,8 +245,9 @@ class BlockPlan(Plan):
     @staticmethod
     def _signature(block):
         """Changes when a projection, a norm or a weight is wrapped, replaced, moved or cast after the
-        plan was made (which keeps them alive: an id stands for one object). (Modules and parameters are looked up in their dicts: attribute access on a module costs
-        more than the rest of this, which runs for every block of every pass.)"""
+        plan was made (which keeps them alive: an id stands for one object). (Modules and parameters
+        are looked up in their dicts: attribute access on a module costs more than the rest of this,
+        which runs for every block of every pass.)"""
         att, mlp = block._modules["self_attn"], block._modules["mlp"]
         am, mm = att._modules, mlp._modules
         mods = ((am["qkv_proj"],) if att.fused_qkv else (am["q_proj"], am["k_proj"], am["v_proj"]))

@@ -360,7 +360,7 @@ def test_rows_of_many_have_the_bits_of_few(op):
     """Walks that go round the grid several times, and end within a round; widths that fill no wave of
     vectors. A row's values and input gradients do not depend on how many rows there are."""
     torch.manual_seed(0)
-    T, H = (6401, 3080) if op != "rms" else (4801, 1000)    # above 64 * 256 * 148 vectors; 4 * 148 * 4 rows
+    T, H = (6401, 3080) if op != "rms" else (4801, 1000)    # above 64 * 256 * 148 vectors; 6 * 148 * 4 rows
     x, g, g2 = _r(T, H if op == "rms" else 2 * H), _r(T, H), _r(T, H)
     w, r = _r(H, scale=0.5), _r(T, H)
 
