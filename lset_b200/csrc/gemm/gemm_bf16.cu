@@ -995,8 +995,8 @@ static int one_cta_bn(int M, int N) {
 // here 11.6; the model without it said 8.2 and lost to the small kernel's 8.0 only on paper).
 //
 // Of a weight gradient over kLongSum k-blocks or more the choice decides whether it is summed whole or in
-// pieces, that is its bits. So there both models are the ones that training runs have been drawn by, see
-// long_sum_cost (gemm_small.cu).
+// pieces, that is its bits. So there both models stay as they were fitted first, see long_sum_cost
+// (gemm_small.cu).
 extern "C" double lb_gemm_tile_cost(int M, int N, int K, int fp32, int bias) {
   const bool pair = M >= 256 && N >= 256 && !bias;
   const int bm = pair ? 256 : lb::BM, bn = pair ? 256 : one_cta_bn(M, N);
